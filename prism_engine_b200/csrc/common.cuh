@@ -333,9 +333,6 @@ struct AttnArgs {
     uint64_t seq_stride;    // elements (fp16) or bytes (int8) between sequences in the cache
     uint32_t int8;          // cache holds [f32 scale][kvd x i8] per position
     uint32_t max_seq;
-    // fused kernel only: the `batch` rows are consecutive prompt tokens of cache sequence prefill_seq,
-    // row t at position pos + t (causal attention over the cache after their keys/values were appended)
-    uint32_t prefill = 0, prefill_seq = 0;
     // fused kernel only: paged cache (page table on the device, [sequence][tbl_stride] page numbers of 2^page_shift rows)
     const int32_t *page_tbl = nullptr;
     uint32_t page_shift = 0, tbl_stride = 0;
@@ -359,6 +356,22 @@ int launch_kv_append(prism_cuda_ctx *ctx, const KvAppendArgs &a);
 bool attn_fused_eligible(const AttnArgs &a);
 int launch_attn_fused(prism_cuda_ctx *ctx, const AttnArgs &a, const uint16_t *k_src, const uint16_t *v_src,
                       uint32_t rope_k, float rope_base);
+// The rotation frequencies base^(-2j/hd) on the device, kept until the context is destroyed.
+int rope_table(prism_cuda_ctx *ctx, uint32_t hd, float base, const float **out);
+
+// prefill_attn.cu: T consecutive tokens, at positions pos0 .., of each of n_seq sequences (row s*T + t of qkv: q | k | v
+// of a token, `stride` halfs apart): rotates q in place, rotates / copies k and v into the fp16 cache, causal attention.
+struct PrefillAttn {
+    uint16_t *qkv; uint32_t stride;
+    uint16_t *kc, *vc;        // cache of the layer: rows of nkv*hd
+    uint64_t cache_rows;      // rows of it, all sequences (or pages) together
+    uint16_t *out;            // [n_seq*T][nh*hd]
+    uint32_t nh, nkv, hd, T, n_seq, pos0;
+    uint32_t seq0, seq_rows, max_seq;  // cache sequence of the first, rows per sequence (contiguous cache), positions it can hold
+    uint32_t rope_k; float rope_base;
+    const int32_t *page_tbl; uint32_t page_shift, tbl_stride;
+};
+int launch_prefill_attn(prism_cuda_ctx *ctx, const PrefillAttn &a);
 
 }  // namespace prism
 

@@ -451,24 +451,23 @@ static int prefill_chunk(prism_cuda_engine *e, uint32_t b, uint32_t pos0, uint32
     const prism_model_config &c = e->cfg;
     const uint32_t H = e->H, I = e->I_l, wq = e->qd_l + 2 * e->kvd_l;
     const float base = c.rope_use_theta ? c.rope_theta : 10000.0f;
-    PRISM_TRY(set_scalars(e, (int32_t)pos0, 0, 0));
     PRISM_TRY(launch_embed(ctx, ctx->tensors[e->embed], toks, T, e->pf_x, nullptr));
     for (uint32_t l = 0; l < c.num_layers; l++) {
         const LutTensor &tqkv = ctx->tensors[e->wqkv[l]], &to = ctx->tensors[e->wo[l]], &tg = ctx->tensors[e->wg[l]],
                         &tu = ctx->tensors[e->wu[l]], &td = ctx->tensors[e->wd[l]];
         PRISM_TRY(launch_rms_norm(ctx, e->pf_x, e->pf_xn, H, c.norm_eps, T));
         PRISM_TRY(launch_gemm(ctx, tqkv, e->pf_xn, T, e->pf_qkv));
-        AttnArgs aa{};
-        aa.q = e->pf_qkv; aa.q_stride = wq;
-        aa.k = (char *)e->kc + (size_t)l * e->kv_layer_bytes;
-        aa.v = (char *)e->vc + (size_t)l * e->kv_layer_bytes;
-        aa.out = e->pf_att;
-        aa.pos_dev = e->scalars; aa.slot_mul = 1; aa.slot_add = 0;
-        aa.nh = e->nh_l; aa.nkv = e->nkv_l; aa.hd = e->hd; aa.batch = T;
-        aa.seq_stride = e->kv_seq_stride; aa.int8 = 0; aa.max_seq = e->kv_slots;
-        aa.prefill = 1; aa.prefill_seq = b;
-        aa.page_tbl = e->page_tbl; aa.page_shift = e->page_shift; aa.tbl_stride = e->pages_per_seq;
-        PRISM_TRY(launch_attn_fused(ctx, aa, e->pf_qkv + e->qd_l, e->pf_qkv + e->qd_l + e->kvd_l, c.rope_k, base));
+        PrefillAttn pa{};
+        pa.qkv = e->pf_qkv; pa.stride = wq;
+        pa.kc = reinterpret_cast<uint16_t *>((char *)e->kc + (size_t)l * e->kv_layer_bytes);
+        pa.vc = reinterpret_cast<uint16_t *>((char *)e->vc + (size_t)l * e->kv_layer_bytes);
+        pa.cache_rows = e->kv_layer_bytes / 2 / e->kvd_l;
+        pa.out = e->pf_att;
+        pa.nh = e->nh_l; pa.nkv = e->nkv_l; pa.hd = e->hd; pa.T = T; pa.n_seq = 1; pa.pos0 = pos0;
+        pa.seq0 = b; pa.seq_rows = e->kv_slots; pa.max_seq = e->kv_slots;
+        pa.rope_k = c.rope_k; pa.rope_base = base;
+        pa.page_tbl = e->page_tbl; pa.page_shift = e->page_shift; pa.tbl_stride = e->pages_per_seq;
+        PRISM_TRY(launch_prefill_attn(ctx, pa));
         PRISM_TRY(launch_gemm(ctx, to, e->pf_att, T, e->pf_g));
         PRISM_TRY(launch_vec_add(ctx, e->pf_x, e->pf_g, T * H));            // h = f16(o + hr)
         PRISM_TRY(launch_rms_norm(ctx, e->pf_x, e->pf_xn, H, c.norm_eps, T));
