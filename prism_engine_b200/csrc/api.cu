@@ -48,6 +48,7 @@ static int grow(prism_cuda_ctx *ctx, T **p, size_t *have, size_t want, bool *gre
     GrowBuf b{*p, *have};
     CudaScratchAlloc al{ctx};
     const int rc = grow_buf(al, b, want, sizeof(T), grew);
+    if (b.ptr != *p) ctx->option_epoch++;  // a captured step that holds the old buffer is captured again
     *p = static_cast<T *>(b.ptr);
     *have = b.count;
     if (rc) {
