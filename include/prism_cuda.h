@@ -86,9 +86,10 @@ int prism_cuda_synchronize(prism_cuda_ctx *ctx);
  * "wait_limit_polls" (default 0 = built-in, about fifteen seconds: polls after which a kernel stops
  * waiting for a tensor-parallel peer or a grid-wide arrival, records a device error code and goes on;
  * the next synchronising call then returns PRISM_E_TIMEOUT and the context stays usable),
- * "prefill_chunk" (default 512: prism_cuda_engine_generate puts up to this many prompt tokens of a sequence
+ * "prefill_chunk" (prism_cuda_engine_generate puts up to this many prompt tokens, of one sequence or of several,
  * through the layers at once -- tensor-core GEMMs, causal attention over the cache, no LM head -- instead of
- * one step per token as the reference's prefill_cpu does; 0 = one step per token.  Single GPU, fp16 KV),
+ * one step per token as the reference's prefill_cpu does; not set: the engine's choice, at most 2048; 0 = one
+ * step per token.  Single GPU, fp16 KV),
  * "layered_chunk" (default 2048: the same for models described layer by layer; read when the engine is created),
  * "tp_fused_ar" (batch-1 tensor-parallel decode, how the partial sums of a row-parallel matmul are reduced:
  * 0 = the GEMV leaves fp32 partial sums, one kernel pushes them to the peers and reduces; 1 = the GEMV's epilogue

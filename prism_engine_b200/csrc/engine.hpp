@@ -43,10 +43,9 @@ struct prism_cuda_engine {
     std::vector<int32_t> page_tbl_host, free_pages;
     std::vector<uint32_t> seq_pages;         // pages each sequence holds
     uint32_t page_shift = 0, pages_per_seq = 0, pool_pages = 0;
-    // batched prefill scratch (one chunk of prompt tokens of one sequence), grown on demand
+    // batched prefill scratch (one portion of prompt tokens), grown on demand
     uint16_t *pf_x = nullptr, *pf_xn = nullptr, *pf_qkv = nullptr, *pf_att = nullptr, *pf_g = nullptr, *pf_u = nullptr,
              *pf_act = nullptr;
-    uint32_t *pf_tok = nullptr;
     uint32_t pf_cap = 0;         // tokens the buffers hold
     cudaGraphExec_t graph = nullptr;
     uint32_t graph_batch = 0;
