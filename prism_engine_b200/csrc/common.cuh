@@ -81,7 +81,6 @@ struct prism_cuda_ctx {
     int ws_whole_blocks = 1024;  // warp-specialised GEMV: one whole block per CTA when there are almost as many blocks as SMs and rows have at most this many chunks; 0: never
     int ws_whole_fill = 50;  // ... for one activation row, when the matrix has at least this many blocks per 100 SMs
     int attn_group = 0;      // most query heads of a KV group one cluster of the fused attention serves (1/2/4/8); 0: chosen from the shape
-    int gemm_reuse_x = 0;    // set by a caller for the second of two GEMMs over the same activations: skip the re-lay
     int pdl = 1;  // programmatic dependent launch between the kernels of the decode chain
     int prefill_chunk = -1;  // most prompt tokens generate() puts through the layers at once (tensor-core GEMMs); -1: the engine's choice, 0: one step per token
     int layered_chunk = 2048;  // layered models: most prompt tokens of a sequence that go through the layers at once (read at engine creation)
@@ -305,9 +304,11 @@ bool tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t batch);
 int launch_gemv_tc5(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x,
                     void *y, const uint16_t *resid);
 
-// gemm_tc5.cu: tcgen05/TMEM prefill GEMM (4-bit, K % 32 == 0, >= 32 tokens)
+// gemm_tc5.cu: tcgen05/TMEM GEMM (K % 128 == 0, >= 8 tokens); with `resid`: Y = f16(f16(X W^T) + resid), resid may be Y.
+// launch_swiglu_tc5: act = f16(f16(silu(X Wg^T)) * (X Wu^T)), act is written twice; leaves *done false where two launches pay.
 bool gemm_tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok);
-int launch_gemm_tc5(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y);
+int launch_gemm_tc5(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y, const uint16_t *resid);
+int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, bool *done);
 
 // glue.cu
 int launch_rms_norm(prism_cuda_ctx *ctx, const uint16_t *in, uint16_t *out, uint32_t n, float eps,
@@ -382,4 +383,8 @@ int synth_shard(prism_cuda_ctx *ctx, const char *name, uint32_t rows, uint32_t c
                 uint64_t seed, float sigma, uint32_t row0, uint32_t col0, int32_t *handle);
 // gemm.cu: Y[m_tok][m] = X[m_tok][k] * W^T (fp16 in/out, fp32 accumulate)
 int launch_gemm(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y);
+// h = f16(f16(X W^T) + h); `tmp` holds m_tok * m values
+int launch_gemm_add(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *h, uint16_t *tmp);
+// act = f16(f16(silu(X Wg^T)) * (X Wu^T)); `g` and `u` hold m_tok * m values
+int launch_gemm_swiglu(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, uint16_t *g, uint16_t *u);
 }  // namespace prism

@@ -129,20 +129,13 @@ static int linear(prism_cuda_engine *e, GemvMode mode, const LutTensor &t, const
     if (!gemm_ok) return launch_gemv(ctx, mode, t, t2, x, xs, y, ys, resid, B);
     if (mode == GEMV_PLAIN) return launch_gemm(ctx, t, x, B, y);
     if (mode == GEMV_RESID) {  // y (== resid, in place) = f16( f16(W x) + resid )
+        if (y == resid) return launch_gemm_add(ctx, t, x, B, y, e->gu);
         PRISM_TRY(launch_gemm(ctx, t, x, B, e->gu));
-        if (y == resid) return launch_vec_add(ctx, y, e->gu, B * t.m);  // in place: the add commutes
         PRISM_TRY(launch_vec_add(ctx, e->gu, resid, B * t.m));
         PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(y, e->gu, (size_t)B * t.m * 2, cudaMemcpyDeviceToDevice, ctx->stream));
         return PRISM_OK;
     }
-    // SwiGLU: gate and up GEMMs, then f16(f16(silu(g)) * u)
-    uint16_t *g = e->gu, *u = e->gu + (size_t)B * t.m;
-    PRISM_TRY(launch_gemm(ctx, t, x, B, g));
-    ctx->gemm_reuse_x = 1;  // same activations, same token tile: the re-laid copy is still in scratch
-    const int rc_up = launch_gemm(ctx, *t2, x, B, u);
-    ctx->gemm_reuse_x = 0;
-    PRISM_TRY(rc_up);
-    return launch_silu_mul(ctx, y, g, u, B * t.m);
+    return launch_gemm_swiglu(ctx, t, *t2, x, B, y, e->gu, e->gu + (size_t)B * t.m);
 }
 
 // Rope(q), Rope(k), KV append and Attention of layer l (cache slot li): one fused kernel when the
@@ -450,7 +443,7 @@ static int ensure_prefill(prism_cuda_engine *e, uint32_t T) {
 static int prefill_portion(prism_cuda_engine *e, uint32_t b, uint32_t n_seq, uint32_t pos0, uint32_t T, const uint32_t *toks) {
     prism_cuda_ctx *ctx = e->ctx;
     const prism_model_config &c = e->cfg;
-    const uint32_t H = e->H, I = e->I_l, wq = e->qd_l + 2 * e->kvd_l, R = n_seq * T;
+    const uint32_t H = e->H, wq = e->qd_l + 2 * e->kvd_l, R = n_seq * T;
     const float base = c.rope_use_theta ? c.rope_theta : 10000.0f;
     PRISM_TRY(launch_embed(ctx, ctx->tensors[e->embed], toks, R, e->pf_x, nullptr));
     for (uint32_t l = 0; l < c.num_layers; l++) {
@@ -469,17 +462,10 @@ static int prefill_portion(prism_cuda_engine *e, uint32_t b, uint32_t n_seq, uin
         pa.rope_k = c.rope_k; pa.rope_base = base;
         pa.page_tbl = e->page_tbl; pa.page_shift = e->page_shift; pa.tbl_stride = e->pages_per_seq;
         PRISM_TRY(launch_prefill_attn(ctx, pa));
-        PRISM_TRY(launch_gemm(ctx, to, e->pf_att, R, e->pf_g));
-        PRISM_TRY(launch_vec_add(ctx, e->pf_x, e->pf_g, R * H));            // h = f16(o + hr)
+        PRISM_TRY(launch_gemm_add(ctx, to, e->pf_att, R, e->pf_x, e->pf_g));  // h = f16(o + hr)
         PRISM_TRY(launch_rms_norm(ctx, e->pf_x, e->pf_xn, H, c.norm_eps, R));
-        PRISM_TRY(launch_gemm(ctx, tg, e->pf_xn, R, e->pf_g));
-        ctx->gemm_reuse_x = 1;  // same activations, same token tile: the re-laid copy is still in scratch
-        const int rc_up = launch_gemm(ctx, tu, e->pf_xn, R, e->pf_u);
-        ctx->gemm_reuse_x = 0;
-        PRISM_TRY(rc_up);
-        PRISM_TRY(launch_silu_mul(ctx, e->pf_act, e->pf_g, e->pf_u, R * I));
-        PRISM_TRY(launch_gemm(ctx, td, e->pf_act, R, e->pf_g));
-        PRISM_TRY(launch_vec_add(ctx, e->pf_x, e->pf_g, R * H));            // h = f16(d + hr)
+        PRISM_TRY(launch_gemm_swiglu(ctx, tg, tu, e->pf_xn, R, e->pf_act, e->pf_g, e->pf_u));
+        PRISM_TRY(launch_gemm_add(ctx, td, e->pf_act, R, e->pf_x, e->pf_g));  // h = f16(d + hr)
     }
     return PRISM_OK;
 }

@@ -7,7 +7,7 @@ namespace prism {
 
 int launch_gemm(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y) {
     if (t.k % 8) return fail(ctx, PRISM_E_ARG, "gemm: dim_n must be a multiple of 8");
-    if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, t, m_tok)) return launch_gemm_tc5(ctx, t, X, m_tok, Y);
+    if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, t, m_tok)) return launch_gemm_tc5(ctx, t, X, m_tok, Y, nullptr);
     // activation rows as the batch dimension of the GEMV kernel, 32768 rows per launch
     for (uint32_t t0 = 0; t0 < m_tok; t0 += 32768) {
         const uint32_t nb = m_tok - t0 < 32768 ? m_tok - t0 : 32768;
@@ -15,6 +15,22 @@ int launch_gemm(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint
                               nullptr, nb));
     }
     return PRISM_OK;
+}
+
+int launch_gemm_add(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *h, uint16_t *tmp) {
+    if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, t, m_tok)) return launch_gemm_tc5(ctx, t, X, m_tok, h, h);
+    PRISM_TRY(launch_gemm(ctx, t, X, m_tok, tmp));
+    return launch_vec_add(ctx, h, tmp, m_tok * t.m);
+}
+
+int launch_gemm_swiglu(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, uint16_t *g, uint16_t *u) {
+    bool done = false;
+    if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, tg, m_tok) && gemm_tc5_eligible(ctx, tu, m_tok) && tg.bits == tu.bits)
+        PRISM_TRY(launch_swiglu_tc5(ctx, tg, tu, X, m_tok, act, &done));
+    if (done) return PRISM_OK;
+    PRISM_TRY(launch_gemm(ctx, tg, X, m_tok, g));
+    PRISM_TRY(launch_gemm(ctx, tu, X, m_tok, u));
+    return launch_silu_mul(ctx, act, g, u, m_tok * tg.m);
 }
 
 }  // namespace prism

@@ -1,21 +1,32 @@
-// Prefill palettized GEMM on tcgen05 / TMEM:  Y[t][r] = f16( sum_k f32(X[t][k]) * f32(W[r][k]) )
+// Palettized GEMM on tcgen05 / TMEM:  Y[t][r] = f16( sum_k f32(X[t][k]) * f32(W[r][k]) )
 // -- one lut_gemv_cpu per activation row (prefill_cpu, src/lut/engine_impl.rs:1046-1053; the
 // reference's never-dispatched kernel for the same job is templates/palettized_gemm.metal:16-117).
 //
-// One persistent CTA per SM computes tiles of 128 weight rows x 256 tokens over the whole K:
-//  * weights: 16 warps dequantise with the lane-private pair tables of gemv.cu / gemv_tc5.cu
-//    (one row per lane = one TMEM lane) and store 32 k at a time into a ring of TMEM stages --
-//    the A operand never touches shared memory;
-//  * activations: X is re-laid once per call into 16-byte units [k/8][token][8] so that a
-//    256-token x 32-k stage is four contiguous 4 KB runs, fetched by one thread with 1-D bulk
-//    copies that complete on an mbarrier; in shared memory the runs are exactly the K-major,
-//    no-swizzle core-matrix layout the B operand descriptor addresses;
-//  * one thread issues two tcgen05.mma (M = 128, N = 256, K = 16) per 32-k chunk; the fp32
-//    accumulators (256 TMEM columns) are read back with tcgen05.ld, rounded to fp16 and stored.
-// 2-bit tensors (4-entry palettes; BITS = 2) run the same pipeline: a 16-byte index chunk then holds
-// 64 weights of a row and expands into two 32-k chunks of the A operand through a 16-entry pair table
-// indexed by nibbles (sk_expand2, pair_table.cuh).
+// A persistent pair of CTAs (cta_group::2) computes tiles of 256 weight rows x nt tokens over a range of K:
+//  * weights: the 16 dequantising warps of a CTA expand its 128 rows with lane-private pair tables (one row per
+//    lane = one TMEM lane) and store 128 k at a time into a ring of TMEM stages -- the A operand never touches
+//    shared memory;
+//  * activations: TMA boxes of 64 k x nt/2 tokens straight from X, swizzled; each CTA fetches its half of the
+//    tokens and one tcgen05.mma reads both halves, so a token tile crosses L2 once per PAIR;
+//  * one thread of the pair issues the products (M = 256, N = nt, K = 16); the fp32 sums (nt TMEM columns) leave
+//    through registers: they are taken out of TMEM first, the accumulator goes back to the issuing thread, and the
+//    rounding, the residual or the SwiGLU product and the stores run under the next tile's products.  The first
+//    stages of that tile are expanded before the sums are waited for.
+// Where the tiles do not fill the GPU K is cut into ranges; their fp32 sums meet in scratch memory and the last
+// warp to arrive adds them in a fixed order.
+// 2-bit tensors (4-entry palettes; BITS = 2) run the same pipeline: a 16-byte index chunk then holds 64 weights of
+// a row and expands into two 32-k chunks of the A operand through a 16-entry pair table indexed by nibbles
+// (sk_expand2, pair_table.cuh).
+// Bound: with many tokens the tensor core under the power cap; with few, the table lookups (256 cycles of the
+// shared-memory pipe per 128 x 128 weights) and the latency of a short chain of stages.
+// Measured, 4 bit, against one CTA per 128 x 256 tile whose single issuing thread spent 1 700 cycles on a stage of 1 024
+// (waits one after the other, descriptors through vector registers, three commits) and which used as many CTAs as there were
+// row tiles: 18944 x 3584, 2048 tokens 266 -> 216 us (1 287 TFLOP/s, 0.78 of measured burst), 512 tokens 67 -> 54, 32 tokens
+// 26 -> 22.5; 4608 x 3584, 2048 tokens 72 -> 53, 32 tokens 23.4 -> 15.1; 3584 x 18944, 2048 tokens 320 -> 275, 32 tokens
+// 96.5 -> 26.9.  The first three without residual or SwiGLU passes and the re-laid activations that went with them.
 // Every mbarrier wait is bounded; a wait that gives up raises the context's device error word.
+#include <cuda.h>
+
 #include <algorithm>
 
 #include "common.cuh"
@@ -25,364 +36,604 @@
 namespace prism {
 
 constexpr int GM_DEQ_WARPS = 16;
-constexpr int GM_MMA_WARP = 16, GM_X_WARP = 17;
+constexpr int GM_MMA_WARP = 16;  // the warp after it loads the activations
 constexpr int GM_THREADS = 18 * 32;
-constexpr int GM_NT_MAX = 256;                // largest token tile = N of the MMA (template parameter NT <= 256)
-constexpr int GM_TBL_BYTES = 2 * 65536;
-// A pipeline stage is CPS index chunks (32 k each): the hand-over between the dequantising warps,
-// the MMA thread and the activation loader costs a few hundred cycles of single-thread control
-// whatever the stage holds, so a weight stage is four chunks (the A operand occupies 256 TMEM
-// columns, 16 per chunk); an activation stage is four chunks too, two for 256-token tiles.
-constexpr int GM_SA = 8;                      // most A stages (two chunks each)
-constexpr int GM_D_COL = 256;                 // accumulator: up to 256 columns after the A stages
-constexpr int GM_X_BYTES = 6 * GM_NT_MAX * 32 * 2;   // activation staging area: 96 KB (three 32 KB stages at 128- and 256-token tiles)
-constexpr int GM_SX_MAX = 32;                 // most X stages (small token tiles): a stage is NT tokens x 32 k fp16 = NT*64 bytes
-// X stages for a token tile of NT: as many as fit the staging area, at most GM_SX_MAX.  Small tiles
-// need the depth: a stage is refilled by a bulk copy whose latency is the same whatever its size.
-template <int NT>
-struct GmX {
-    static constexpr int CPS = 4;                             // chunks per A (weight) stage
-    static constexpr int XC = NT <= 128 ? 4 : 2;              // chunks per X (activation) stage: at most 32 KB
-    static constexpr int SA = GM_D_COL / (16 * CPS);          // A stages: 4
-    static constexpr int STAGE_BYTES = NT * 64 * XC;
-    static constexpr int SX = (GM_X_BYTES / STAGE_BYTES) < GM_SX_MAX ? (GM_X_BYTES / STAGE_BYTES) : GM_SX_MAX;
-};
-constexpr int GM_TMEM_COLS = 512;
-constexpr int GM_PF = 4;
-constexpr int GM_SBASE = 1024;
-constexpr int GM_X_OFF = GM_TBL_BYTES;
-constexpr int GM_BAR_OFF = GM_X_OFF + GM_X_BYTES;
-// barriers (8 B each): afull[SA], aempty[SA], xfull[SX], xempty[SX], dfull, dempty
-constexpr int GM_STATE_OFF = GM_BAR_OFF + 8 * (2 * GM_SA + 2 * GM_SX_MAX + 2);
-constexpr size_t GM_SMEM_BYTES = GM_STATE_OFF + 64;
+constexpr int GM_STAGE_K = 128;               // k of a weight stage: 64 TMEM columns
+constexpr int GM_SA = 4;                      // weight stages; a warp of slot j fills every fourth, ring position j
+constexpr int GM_D_COL = GM_SA * 64;          // accumulator: up to 256 columns after the A stages
+constexpr int GM_SX_MAX = 2 * GM_SA;          // most activation stages, of 64 k each
+// The two pair tables start on 64 KB boundaries of the shared-memory window, so that a lookup's address is one
+// permute of an index byte; barriers and activation stages lie before and after them.
+constexpr uint32_t GM_SBASE = 1024;           // where dynamic shared memory starts (checked)
+constexpr uint32_t GM_TBL = 65536;
+constexpr uint32_t GM_OUT_LOW = 2048, GM_OUT_LOW_WARPS = 12;      // 1 KB per dequantising warp on the way out: 16 tokens x 32 rows
+constexpr uint32_t GM_X_LOW = GM_OUT_LOW + GM_OUT_LOW_WARPS * 1024, GM_X_HIGH = GM_TBL + 2 * 65536;
+constexpr uint32_t GM_END = GM_SBASE + 227 * 1024;
+constexpr uint32_t GM_OUT_HIGH = GM_END - (GM_DEQ_WARPS - GM_OUT_LOW_WARPS) * 1024;
+// barriers (8 B each) at GM_SBASE: afull[SA], done[SA], xfull[SX], dfull, dempty; error flag, TMEM base.  One commit per
+// weight stage gives back its TMEM columns and the activation stages it used.
+constexpr uint32_t GM_STATE = GM_SBASE + 8 * (2 * GM_SA + GM_SX_MAX + 2);
+constexpr size_t GM_SMEM_BYTES = GM_END - GM_SBASE;
+static_assert(GM_STATE + 16 <= GM_OUT_LOW, "barriers overlap what follows");
+
+enum GemmOut { GM_PLAIN = 0, GM_RESID = 1, GM_SWIGLU = 2 };
 
 struct GemmArgs {
-    const uint8_t *idx;
-    const uint16_t *pal;
-    uint32_t n_chunks, n_hb, m;       // 32-k chunks per row (K/32), half-blocks, valid weight rows
+    const uint8_t *idx, *idx2;        // weights: one tensor, or gate and up
+    const uint16_t *pal, *pal2;
+    uint32_t n_hb, m;                 // half-blocks, valid weight rows
     uint32_t n_ichunks;               // 16-byte index chunks per row (K/32 at 4 bit, K/64 at 2 bit)
-    uint32_t n_rt, n_tt;              // row tiles (128 rows), token tiles (256 tokens)
-    uint32_t m_tok, m_tok_pad;
-    const uint8_t *xc;                // [token tile][K/8][NT][16 B]
+    uint32_t n_st;                    // weight stages (K/128)
+    uint32_t n_rp, n_tt, splits;      // pairs of 128-row tiles, token tiles, ranges of K
+    uint32_t subs;                    // tensors a tile goes through one after the other: 2 for SwiGLU
+    uint32_t nt;                      // tokens of a tile, a multiple of 32
+    uint32_t sx_low, sx;              // activation stages before the tables, and in all
+    uint32_t m_tok, mode;
+    uint32_t wide;                    // rows of y (and resid) can be moved 8 values at a time
     uint16_t *y;                      // [m_tok][m]
+    const uint16_t *resid;            // [m_tok][m] (GM_RESID), may be y
+    float *part;                      // [item][CTA][warp][column][lane] sums of a range
+    unsigned int *arrived;            // [tile][CTA][warp]
     unsigned int *err;
 };
 
-// X [m_tok][k] fp16 -> Xc [token tile][k/8][nt][8]: the 32 k of one chunk for the nt tokens of one
-// tile are one contiguous run of nt*64 bytes, already in the order the shared-memory B operand
-// wants (k-blocks of 8, then tokens), so a stage is filled by ONE bulk copy.  Padded token rows are
-// zero.
-__global__ void gemm_relay_x_kernel(const uint16_t *__restrict__ x, uint32_t m_tok, uint32_t m_tok_pad, uint32_t k,
-                                    uint32_t nt, uint4 *__restrict__ xc) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // index into the output
-    const size_t k8n = k / 8;
-    if (i >= k8n * m_tok_pad) return;
-    const uint32_t tin = (uint32_t)(i % nt);
-    const size_t rest = i / nt;
-    const uint32_t k8 = (uint32_t)(rest % k8n), tt = (uint32_t)(rest / k8n);
-    const uint32_t t = tt * nt + tin;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (t < m_tok) v = *reinterpret_cast<const uint4 *>(x + (size_t)t * k + (size_t)k8 * 8);
-    xc[i] = v;
+namespace {
+
+__device__ __forceinline__ void gm_tma_pair(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t mbar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(y), "r"(mbar)
+                 : "memory");
+}
+__device__ __forceinline__ void gm_mma_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// K-major operand of 128-byte rows, 128-byte swizzle, eight-row groups 1024 bytes apart.
+__device__ __forceinline__ uint64_t gm_desc(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
 }
 
-__device__ __forceinline__ uint32_t gm_lds(uint32_t off, int slot) {
+template <int SLOT>
+__device__ __forceinline__ uint32_t gm_lds(uint32_t off) {
     uint32_t v;
-    if (slot == 0) asm volatile("ld.shared.u32 %0, [%1+%2];\n" : "=r"(v) : "r"(off), "n"(GM_SBASE));
-    else asm volatile("ld.shared.u32 %0, [%1+%2];\n" : "=r"(v) : "r"(off), "n"(GM_SBASE + 128));
+    asm volatile("ld.shared.u32 %0, [%1+%2];\n" : "=r"(v) : "r"(off), "n"(SLOT * 128));
     return v;
 }
-
 // The 16 table lookups of one 32-k chunk of a row: bytes of the index words -> half2 entries.
-__device__ __forceinline__ void gm_lookup16(uint32_t (&A)[16], const uint4 &wv, uint32_t laneq, uint32_t slot) {
+template <int SLOT>
+__device__ __forceinline__ void gm_lookup(uint32_t (&A)[16], const uint4 &wv, uint32_t laneq) {
     const uint32_t aw[4] = {wv.x, wv.y, wv.z, wv.w};
-    if (slot == 0) {
 #pragma unroll
-        for (int hh = 0; hh < 4; hh++) {
-            A[4 * hh + 0] = gm_lds(__byte_perm(aw[hh], laneq, 0x7604), 0);
-            A[4 * hh + 1] = gm_lds(__byte_perm(aw[hh], laneq, 0x7614), 0);
-            A[4 * hh + 2] = gm_lds(__byte_perm(aw[hh], laneq, 0x7624), 0);
-            A[4 * hh + 3] = gm_lds(__byte_perm(aw[hh], laneq, 0x7634), 0);
-        }
-    } else {
-#pragma unroll
-        for (int hh = 0; hh < 4; hh++) {
-            A[4 * hh + 0] = gm_lds(__byte_perm(aw[hh], laneq, 0x7604), 1);
-            A[4 * hh + 1] = gm_lds(__byte_perm(aw[hh], laneq, 0x7614), 1);
-            A[4 * hh + 2] = gm_lds(__byte_perm(aw[hh], laneq, 0x7624), 1);
-            A[4 * hh + 3] = gm_lds(__byte_perm(aw[hh], laneq, 0x7634), 1);
-        }
+    for (int hh = 0; hh < 4; hh++) {
+        A[4 * hh + 0] = gm_lds<SLOT>(__byte_perm(aw[hh], laneq, 0x7604));
+        A[4 * hh + 1] = gm_lds<SLOT>(__byte_perm(aw[hh], laneq, 0x7614));
+        A[4 * hh + 2] = gm_lds<SLOT>(__byte_perm(aw[hh], laneq, 0x7624));
+        A[4 * hh + 3] = gm_lds<SLOT>(__byte_perm(aw[hh], laneq, 0x7634));
     }
 }
+__device__ __forceinline__ void gm_lookup16(uint32_t (&A)[16], const uint4 &wv, uint32_t laneq, uint32_t slot) {
+    if (slot == 0) gm_lookup<0>(A, wv, laneq);
+    else gm_lookup<1>(A, wv, laneq);
+}
 
-template <int NT, int BITS>
-__global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmArgs a) {
+struct GmItem {
+    uint32_t rp, tt, k0, k1;  // k in stages
+};
+__device__ __forceinline__ GmItem gm_item(const GemmArgs &a, uint32_t w) {
+    if (a.splits == 1) return GmItem{w % a.n_rp, w / a.n_rp, 0, a.n_st};
+    const uint32_t s = w % a.splits, t = w / a.splits;
+    return GmItem{t % a.n_rp, t / a.n_rp, a.n_st * s / a.splits, a.n_st * (s + 1) / a.splits};
+}
+
+// 16 tokens of one weight row, rounded (pairs, the first in the low half): the residual, or the product with silu of the gate
+// values this thread stored for the tile before (f16(f16(silu(g)) * u), engine_impl.rs:1355-1366).
+__device__ __forceinline__ void gm_store(const GemmArgs &a, const uint32_t (&v)[8], uint32_t t0, uint32_t row, uint32_t sub) {
+    if (row >= a.m || t0 >= a.m_tok) return;
+    const uint32_t n = min(16u, a.m_tok - t0);
+    uint16_t *y = a.y + (size_t)t0 * a.m + row;
+    const bool product = a.mode == GM_SWIGLU && sub == 1;
+    if (a.mode == GM_RESID || product) {
+        const uint16_t *src = product ? y : a.resid + (size_t)t0 * a.m + row;
+        uint16_t o[16];
+#pragma unroll
+        for (uint32_t i = 0; i < 16; i++) o[i] = i < n ? src[(size_t)i * a.m] : 0;
+#pragma unroll
+        for (uint32_t i = 0; i < 16; i++) {
+            const float h = __half2float(__ushort_as_half((uint16_t)(v[i / 2] >> (16 * (i & 1))))), x = __half2float(__ushort_as_half(o[i]));
+            const float r = product ? __half2float(__float2half_rn(x / (1.0f + expf(-x)))) * h : h + x;
+            if (i < n) y[(size_t)i * a.m] = __half_as_ushort(__float2half_rn(r));
+        }
+        return;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i++)
+        if (i < n) y[(size_t)i * a.m] = (uint16_t)(v[i / 2] >> (16 * (i & 1)));
+}
+// The same for a whole warp's 32 rows x 16 tokens, 16 bytes a lane: the values change places in the warp's 1 KB of shared
+// memory, so that a lane holds 8 rows of a token.
+__device__ __forceinline__ void gm_store_wide(const GemmArgs &a, const uint32_t (&v)[8], uint32_t t0, uint32_t row0, uint32_t sub, uint8_t *out) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint16_t *mine = reinterpret_cast<uint16_t *>(out) + lane;
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i++) mine[i * 32] = (uint16_t)(v[i / 2] >> (16 * (i & 1)));
+    __syncwarp();
+    const uint32_t r = row0 + (lane & 3) * 8;
+    const bool product = a.mode == GM_SWIGLU && sub == 1;
+#pragma unroll
+    for (uint32_t p = 0; p < 2; p++) {
+        const uint32_t t = t0 + p * 8 + (lane >> 2);
+        if (t >= a.m_tok || r >= a.m) continue;
+        uint4 w = reinterpret_cast<const uint4 *>(out)[p * 32 + lane];
+        uint16_t *y = a.y + (size_t)t * a.m + r;
+        if (a.mode == GM_RESID || product) {
+            const uint4 o = *reinterpret_cast<const uint4 *>(product ? y : a.resid + (size_t)t * a.m + r);
+            const uint32_t ov[4] = {o.x, o.y, o.z, o.w};
+            uint32_t wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&wv[i])), x = __half22float2(*reinterpret_cast<const __half2 *>(&ov[i]));
+                __half2 res;
+                if (product)
+                    res = __floats2half2_rn(__half2float(__float2half_rn(x.x / (1.0f + expf(-x.x)))) * h.x, __half2float(__float2half_rn(x.y / (1.0f + expf(-x.y)))) * h.y);
+                else
+                    res = __floats2half2_rn(h.x + x.x, h.y + x.y);
+                wv[i] = *reinterpret_cast<const uint32_t *>(&res);
+            }
+            w = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+        }
+        *reinterpret_cast<uint4 *>(y) = w;
+    }
+    __syncwarp();
+}
+__device__ __forceinline__ uint32_t gm_pack(float x, float y) {
+    const __half2 h = __floats2half2_rn(x, y);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+}  // namespace
+
+template <int BITS>
+__global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem);
-    if (smem_base != (uint32_t)GM_SBASE) {  // layout assumption broken: refuse to compute
+    if ((smem_base & 0xFFFFu) != GM_SBASE) {  // layout assumption broken: refuse to compute
         if (threadIdx.x == 0) atomicExch(a.err, 1u);
         return;
     }
-    // Tables, barriers and TMEM are set up from weights alone while the previous kernel drains; the
-    // loader thread waits for it before the first activation copy, and everything that reads or
-    // writes activations (MMAs, epilogue) follows that copy through the mbarriers.
+    uint8_t *const win = smem - GM_SBASE;               // 64 KB-aligned start of the window
+    const uint32_t base = smem_base - GM_SBASE;
+    // Tables, barriers and TMEM are set up from weights alone while the previous kernel drains.
     pdl_launch_dependents();
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t bar = smem_base + GM_BAR_OFF;
-    const uint32_t b_afull = bar, b_aempty = bar + 8 * GM_SA, b_xfull = bar + 16 * GM_SA,
-                   b_xempty = b_xfull + 8 * GM_SX_MAX, b_dfull = b_xempty + 8 * GM_SX_MAX, b_dempty = b_dfull + 8;
-    constexpr int SX = GmX<NT>::SX, XSTAGE = GmX<NT>::STAGE_BYTES, CPS = GmX<NT>::CPS, SA = GmX<NT>::SA, XC = GmX<NT>::XC;
-    constexpr int ICPS = BITS == 4 ? CPS : CPS / 2;  // 16-byte index chunks per weight stage
-    constexpr int NSI = GM_PF / ICPS;                // stages whose index chunks a warp keeps in flight
-    volatile uint32_t *err_flag = reinterpret_cast<volatile uint32_t *>(smem + GM_STATE_OFF);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + GM_STATE_OFF + 8);
-    const uint32_t nch = a.n_chunks;
-    const uint32_t n_items = a.n_rt * a.n_tt;  // item w: row tile w % n_rt, token tile w / n_rt
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), rank = t5::cluster_rank();
+    // afull, xfull and dempty: the pair's, in CTA 0 (it issues the products); done and dfull: each CTA's own
+    const uint32_t b_afull = base + GM_SBASE, b_done = b_afull + 8 * GM_SA, b_xfull = b_done + 8 * GM_SA,
+                   b_dfull = b_xfull + 8 * GM_SX_MAX, b_dempty = b_dfull + 8;
+    constexpr int ICPS = BITS == 4 ? 4 : 2;             // 16-byte index chunks per weight stage
+    volatile uint32_t *err_flag = reinterpret_cast<volatile uint32_t *>(win + GM_STATE);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(win + GM_STATE + 8);
+    const uint32_t n_items = a.n_rp * a.n_tt * a.splits, pair_id = blockIdx.x / 2, n_pairs = gridDim.x / 2;
+    const uint32_t xstage = a.nt * 64;                  // bytes of this CTA's half of the tokens
+    auto x_addr = [&](uint32_t s) { return base + (s < a.sx_low ? GM_X_LOW + s * xstage : GM_X_HIGH + (s - a.sx_low) * xstage); };
 
     if (tid == 0) {
-        for (int s = 0; s < SA; s++) { t5::mbar_init(b_afull + 8 * s, 4); t5::mbar_init(b_aempty + 8 * s, 1); }
-        for (int s = 0; s < SX; s++) { t5::mbar_init(b_xfull + 8 * s, 1); t5::mbar_init(b_xempty + 8 * s, 1); }
+        for (int s = 0; s < GM_SA; s++) { t5::mbar_init(b_afull + 8 * s, 8); t5::mbar_init(b_done + 8 * s, 1); }
+        for (int s = 0; s < GM_SX_MAX; s++) t5::mbar_init(b_xfull + 8 * s, 1);
         t5::mbar_init(b_dfull, 1);
-        t5::mbar_init(b_dempty, GM_DEQ_WARPS);
+        t5::mbar_init(b_dempty, 2 * GM_DEQ_WARPS);
         *err_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if (warp == GM_MMA_WARP) t5::tmem_alloc(smem_base + GM_STATE_OFF + 8, GM_TMEM_COLS);
+    if (warp == GM_MMA_WARP) t5::tmem_alloc_pair(base + GM_STATE + 8, 512);
     t5::fence_before();
     __syncthreads();
+    t5::cluster_sync();  // the other CTA's barriers exist before anything arrives there
     t5::fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
 
     if (warp < GM_DEQ_WARPS) {
         // =============================== dequantising warps ===============================
         const uint32_t q = warp & 3, j = warp >> 2;      // TMEM lane quarter, slot within the quarter
-        const uint32_t pair = q & 1, slot = q >> 1;      // table area, row slot inside its entries
-        const uint32_t laneq = (pair << 16) | (lane * 4);
+        const uint32_t area = q & 1, slot = q >> 1;      // table area, row slot inside its entries
+        const uint32_t laneq = base + GM_TBL + area * 65536 + lane * 4;
         const uint32_t tmem_lane = tmem_base + ((q * 32) << 16);
-        uint32_t n_base = 0, ti = 0, cur_rt = 0xFFFFFFFFu;
-        for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x, ti++) {
-            const uint32_t rt = w % a.n_rt, tt = w / a.n_rt;
-            const uint32_t hb = 4 * rt + q;
-            const bool ok = hb < a.n_hb;
-            const uint32_t h = ok ? hb : a.n_hb - 1;
-            const uint32_t nich = a.n_ichunks;
-            const uint8_t *sp = a.idx + (size_t)h * nich * 512 + lane * 16;
-            uint4 r[GM_PF];
-#pragma unroll
-            for (int i = 0; i < GM_PF; i++) {  // r[i]: index chunk (i % ICPS) of this warp's stage number i / ICPS
-                const uint32_t c = (j + 4 * (i / ICPS)) * ICPS + (i % ICPS);
-                if (c < nich) r[i] = t5::ldg128_nc(sp + (size_t)c * 512);
-            }
-            if (rt != cur_rt) {  // same decision in all warps: they walk the same item list
-                cur_rt = rt;
-                asm volatile("bar.sync %0, 256;\n" ::"r"(1 + pair) : "memory");  // lookups of the previous tile are done
-                if (BITS == 4) {
-                    const uint16_t *prow = a.pal + ((size_t)h * 32 + lane) * 16;
-                    const uint4 p0 = *reinterpret_cast<const uint4 *>(prow);
-                    const uint4 p1 = *reinterpret_cast<const uint4 *>(prow + 8);
-                    const uint32_t cbp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-                    const uint32_t hp0 = reinterpret_cast<const uint32_t *>(prow)[2 * j];
-                    const uint32_t hp1 = reinterpret_cast<const uint32_t *>(prow)[2 * j + 1];
-                    uint8_t *tb = smem + pair * 65536 + j * 16384 + lane * 4 + slot * 128;
-#pragma unroll
-                    for (int lo = 0; lo < 16; lo++) {
-#pragma unroll
-                        for (int hs = 0; hs < 4; hs++) {
-                            const uint32_t sel = (((hs & 1) ? 0x76u : 0x54u) << 8) | ((lo & 1) ? 0x32u : 0x10u);
-                            *reinterpret_cast<uint32_t *>(tb + lo * 256 + hs * 4096) =
-                                __byte_perm(cbp[lo >> 1], (hs & 2) ? hp1 : hp0, sel);
-                        }
-                    }
-                } else {
-                    // 16-entry nibble table: entry e = i0 | i1 << 2 -> half2{pal[i0], pal[i1]}; slot j writes e = 4j..4j+3
-                    const uint2 pp = *reinterpret_cast<const uint2 *>(a.pal + ((size_t)h * 32 + lane) * 4);
-                    const uint32_t v1 = ((j & 2) ? pp.y : pp.x) >> ((j & 1) * 16) & 0xFFFFu;  // pal[i1], i1 = j
-                    uint8_t *tb = smem + pair * 65536 + lane * 4 + slot * 128;
-#pragma unroll
-                    for (uint32_t i0 = 0; i0 < 4; i0++) {
-                        const uint32_t v0 = ((i0 & 2) ? pp.y : pp.x) >> ((i0 & 1) * 16) & 0xFFFFu;
-                        *reinterpret_cast<uint32_t *>(tb + (4 * j + i0) * 256) = v0 | (v1 << 16);
-                    }
-                }
-                asm volatile("bar.sync %0, 256;\n" ::"r"(1 + pair) : "memory");
-            }
-            // Everything so far read weights only.  The waits below depend on the activations, which come after the
-            // loader's dependency wait: wait for the same dependency first, so that no bounded wait runs while the
-            // kernel before this one (under tensor parallelism: a late peer) is still at work.
-            if (w == blockIdx.x) pdl_wait();
-            // ---- K loop: lookups -> TMEM stage -> signal the MMA thread ----
-            // a stage is CPS consecutive chunks; warp slot j takes the stages j, j+4, ...
-            const uint32_t nst = nch / CPS;
-            for (uint32_t s0 = j; s0 < nst; s0 += 4 * NSI) {
-#pragma unroll
-                for (int i = 0; i < NSI; i++) {
-                    const uint32_t su = s0 + 4 * i;
-                    if (su < nst) {
-                        uint32_t A[CPS][16];
-#pragma unroll
-                        for (int cc = 0; cc < ICPS; cc++) {
-                            const uint32_t c = su * ICPS + cc;
-                            const uint4 wv = r[i * ICPS + cc];
-                            const uint32_t nc = c + 4 * GM_PF;
-                            if (nc < nich) r[i * ICPS + cc] = t5::ldg128_nc(sp + (size_t)nc * 512);
-                            if (BITS == 4) {
-                                gm_lookup16(A[cc], wv, laneq, slot);
-                            } else {
-                                uint4 pa, pb;
-                                sk_expand2(pa, pb, wv);
-                                gm_lookup16(A[2 * cc], pa, laneq, slot);
-                                gm_lookup16(A[2 * cc + 1], pb, laneq, slot);
-                            }
-                        }
-                        const uint32_t n = n_base + su, stage = n % SA, ph = (n / SA) & 1;
-                        t5::mbar_wait_warp(b_aempty + 8 * stage, ph ^ 1, err_flag);
-                        t5::fence_after();
-#pragma unroll
-                        for (int cc = 0; cc < CPS; cc++) t5::st16(tmem_lane + stage * 16 * CPS + cc * 16, A[cc]);
-                        t5::wait_st();
-                        t5::fence_before();
-                        if (lane == 0) t5::mbar_arrive(b_afull + 8 * stage);
-                    }
-                }
-            }
-            n_base += nst;
-            // ---- epilogue: warp (q, j) converts token columns [64j, 64j+64) of its 32 rows ----
+        const uint32_t afull0 = t5::map_rank(b_afull + 8 * j, 0), dempty0 = t5::map_rank(b_dempty, 0);
+        uint8_t *out = win + (warp < GM_OUT_LOW_WARPS ? GM_OUT_LOW + warp * 1024 : GM_OUT_HIGH + (warp - GM_OUT_LOW_WARPS) * 1024);
+        const uint32_t groups = a.nt / 16;               // of 16 accumulator columns; this warp takes j, j + 4, ...
+        uint32_t n = 0, ti = 0, cur = 0xFFFFFFFFu;
+        uint32_t pend_w = 0xFFFFFFFFu, pend_sub = 0;     // the tile whose sums are still in TMEM
+        bool waited = false;
+
+        auto epilogue = [&](uint32_t w, uint32_t sub) {
+            const GmItem it = gm_item(a, w);
+            const uint32_t row = (2 * it.rp + rank) * 128 + q * 32 + lane, tile = w / a.splits, place = rank * GM_DEQ_WARPS + warp;
+            const uint32_t per = (groups + 3) / 4 * 512;  // floats of a warp
             t5::mbar_wait_warp(b_dfull, ti & 1, err_flag);
             t5::fence_after();
-            const uint32_t row = hb * 32 + lane;
-            const bool row_ok = ok && row < a.m;
-            constexpr int CW = NT / 4 > 16 ? NT / 4 : 16;  // accumulator columns (tokens) per warp of a quarter
-            if ((int)j * CW < NT) {
-#pragma unroll 1
-                for (int g = 0; g < CW / 16; g++) {
-                    uint32_t v[16];
-                    t5::ld16(tmem_lane + GM_D_COL + j * CW + g * 16, v);
-                    t5::wait_ld();
-                    const uint32_t t0 = tt * NT + j * CW + g * 16;
+            ti++;
+            uint32_t sums[4][8];
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const uint32_t t = t0 + i;
-                        if (row_ok && t < a.m_tok)
-                            a.y[(size_t)t * a.m + row] = __half_as_ushort(__float2half_rn(__uint_as_float(v[i])));
-                    }
+            for (uint32_t i = 0; i < 4; i++) {
+                if (j + 4 * i >= groups) break;
+                uint32_t v[16];
+                t5::ld16(tmem_lane + GM_D_COL + (j + 4 * i) * 16, v);
+                t5::wait_ld();
+                if (a.splits == 1) {
+#pragma unroll
+                    for (uint32_t c = 0; c < 8; c++) sums[i][c] = gm_pack(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
+                } else {
+                    float *mine = a.part + ((size_t)w * 2 * GM_DEQ_WARPS + place) * per + i * 512 + lane;
+#pragma unroll
+                    for (uint32_t c = 0; c < 16; c++) __stcg(mine + c * 32, __uint_as_float(v[c]));
                 }
             }
             t5::fence_before();
-            if (lane == 0) t5::mbar_arrive(b_dempty);
-        }
-    } else if (warp == GM_MMA_WARP && lane == 0) {
-        // =============================== MMA issuing thread ===============================
-        const uint32_t idesc = t5::idesc_f16(128, NT);
-        const uint32_t x_addr = smem_base + GM_X_OFF;
-        uint32_t n = 0, nx = 0, ti = 0;
-        pdl_wait();  // see the dequantising warps: no bounded wait before the dependency is met
-        for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x, ti++) {
-            t5::mbar_wait_bounded(b_dempty, (ti & 1) ^ 1, err_flag);  // epilogue of the previous tile has read D
-            t5::fence_after();
-            const uint32_t dcol = tmem_base + GM_D_COL;
-            for (uint32_t su = 0; su < nch / CPS; su++, n++) {
-                const uint32_t sa = n % SA, pa = (n / SA) & 1;
-                t5::mbar_wait_bounded(b_afull + 8 * sa, pa, err_flag);
-                const uint32_t acol = tmem_base + sa * 16 * CPS;
+            __syncwarp();
+            if (lane == 0) t5::mbar_arrive_tmem(dempty0);
+            if (a.splits > 1) {
+                __threadfence();
+                __syncwarp();
+                uint32_t before = 0;
+                if (lane == 0) before = atomicAdd(a.arrived + (size_t)tile * 2 * GM_DEQ_WARPS + place, 1u);
+                if (__shfl_sync(0xFFFFFFFFu, before, 0) != a.splits - 1) return;
+                __threadfence();
+                if (lane == 0) a.arrived[(size_t)tile * 2 * GM_DEQ_WARPS + place] = 0;
+            }
 #pragma unroll
-                for (int xi = 0; xi < CPS / XC; xi++, nx++) {
-                    const uint32_t sx = nx % SX, px = (nx / SX) & 1;
-                    t5::mbar_wait_bounded(b_xfull + 8 * sx, px, err_flag);
-                    t5::fence_after();
-                    const uint32_t xs = x_addr + sx * XSTAGE;
-                    // B: NT tokens x 16 k; core matrices of 8 tokens are 128 B apart, k-blocks of 8 are NT*16 B apart
+            for (uint32_t i = 0; i < 4; i++) {
+                if (j + 4 * i >= groups) break;
+                if (a.splits > 1) {
+                    const float *p = a.part + ((size_t)tile * a.splits * 2 * GM_DEQ_WARPS + place) * per + i * 512 + lane;
+                    float f[16];
 #pragma unroll
-                    for (int cc = 0; cc < XC; cc++) {
-                        const uint32_t ac = acol + (xi * XC + cc) * 16;
-                        t5::mma_ts(dcol, ac, t5::smem_desc(xs + cc * NT * 64, NT * 16, 128), idesc, (su | xi | cc) != 0);
-                        t5::mma_ts(dcol, ac + 8, t5::smem_desc(xs + cc * NT * 64 + 2 * NT * 16, NT * 16, 128), idesc, 1);
-                    }
-                    t5::commit(b_xempty + 8 * sx);
+                    for (uint32_t c = 0; c < 16; c++) f[c] = 0.0f;
+                    for (uint32_t s = 0; s < a.splits; s++, p += (size_t)2 * GM_DEQ_WARPS * per)
+#pragma unroll
+                        for (uint32_t c = 0; c < 16; c++) f[c] += __ldcg(p + c * 32);
+#pragma unroll
+                    for (uint32_t c = 0; c < 8; c++) sums[i][c] = gm_pack(f[2 * c], f[2 * c + 1]);
                 }
-                t5::commit(b_aempty + 8 * sa);
+                const uint32_t t0 = it.tt * a.nt + (j + 4 * i) * 16;
+                if (a.wide) gm_store_wide(a, sums[i], t0, row - lane, sub, out);
+                else gm_store(a, sums[i], t0, row, sub);
             }
-            t5::commit(b_dfull);
+            __syncwarp();
+        };
+
+        uint4 r[ICPS];
+        bool ahead = false;                              // r holds this slot's first stage of the tile already
+        bool late = false;                               // this slot's last stage was one of the last two of its tile
+        auto row_block = [&](const GmItem &i) { return min(4 * (2 * i.rp + rank) + q, a.n_hb - 1); };
+        auto chunks = [&](const GmItem &i, uint32_t sub) { return (sub ? a.idx2 : a.idx) + (size_t)row_block(i) * a.n_ichunks * 512 + lane * 16; };
+        for (uint32_t w = pair_id, sub = 0;;) {
+            const bool over = w >= n_items;              // past the last tile: its sums are still to be stored
+            GmItem it = gm_item(a, w);
+            if (over) it.k0 = it.k1 = 0;
+            {
+                uint32_t su = it.k0 + ((j - n) & 3);     // this slot's first stage: ring position j
+                const uint8_t *sp = chunks(it, sub);
+                if (su < it.k1 && !ahead)
+#pragma unroll
+                    for (int c = 0; c < ICPS; c++) r[c] = t5::ldg128_nc(sp + (size_t)(su * ICPS + c) * 512);
+                ahead = false;
+                if (!over && it.rp * 2 + sub != cur) {  // same decision in all warps: they walk the same item list
+                    cur = it.rp * 2 + sub;
+                    asm volatile("bar.sync %0, 256;\n" ::"r"(1 + area) : "memory");  // lookups of the previous tile are done
+                    uint8_t *tb = win + GM_TBL + area * 65536 + lane * 4 + slot * 128;
+                    if (BITS == 4) {
+                        const uint16_t *prow = (sub ? a.pal2 : a.pal) + ((size_t)row_block(it) * 32 + lane) * 16;
+                        const uint4 p0 = *reinterpret_cast<const uint4 *>(prow);
+                        const uint4 p1 = *reinterpret_cast<const uint4 *>(prow + 8);
+                        const uint32_t cbp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+                        const uint32_t hp0 = reinterpret_cast<const uint32_t *>(prow)[2 * j];
+                        const uint32_t hp1 = reinterpret_cast<const uint32_t *>(prow)[2 * j + 1];
+                        tb += j * 16384;
+#pragma unroll
+                        for (int lo = 0; lo < 16; lo++) {
+#pragma unroll
+                            for (int hs = 0; hs < 4; hs++) {
+                                const uint32_t sel = (((hs & 1) ? 0x76u : 0x54u) << 8) | ((lo & 1) ? 0x32u : 0x10u);
+                                *reinterpret_cast<uint32_t *>(tb + lo * 256 + hs * 4096) = __byte_perm(cbp[lo >> 1], (hs & 2) ? hp1 : hp0, sel);
+                            }
+                        }
+                    } else {
+                        // 16-entry nibble table: entry e = i0 | i1 << 2 -> half2{pal[i0], pal[i1]}; slot j writes e = 4j..4j+3
+                        const uint2 pp = *reinterpret_cast<const uint2 *>((sub ? a.pal2 : a.pal) + ((size_t)row_block(it) * 32 + lane) * 4);
+                        const uint32_t v1 = ((j & 2) ? pp.y : pp.x) >> ((j & 1) * 16) & 0xFFFFu;  // pal[i1], i1 = j
+#pragma unroll
+                        for (uint32_t i0 = 0; i0 < 4; i0++) {
+                            const uint32_t v0 = ((i0 & 2) ? pp.y : pp.x) >> ((i0 & 1) * 16) & 0xFFFFu;
+                            *reinterpret_cast<uint32_t *>(tb + (4 * j + i0) * 256) = v0 | (v1 << 16);
+                        }
+                    }
+                    asm volatile("bar.sync %0, 256;\n" ::"r"(1 + area) : "memory");
+                }
+                // Everything so far read weights only.  The waits below depend on the activations: wait for the kernel
+                // before this one first, so that no bounded wait runs while it (under tensor parallelism: a late peer) is
+                // still at work.
+                if (!waited) {
+                    pdl_wait();
+                    waited = true;
+                }
+                for (bool first = true; first || su < it.k1; first = false, su += 4) {
+                    // The tile before.  A slot that finished early expands its first stage of this one before it waits for the sums, so
+                    // that the tensor core has something to go on with; the slots of the last two stages take the sums out first.  Nobody
+                    // comes to a second stage before that: it waits for products that wait for these sums.
+                    if (pend_w != 0xFFFFFFFFu && (!first || late || su >= it.k1)) {
+                        epilogue(pend_w, pend_sub);
+                        pend_w = 0xFFFFFFFFu;
+                    }
+                    if (su < it.k1) {
+                        // what r takes next: this slot's next stage, of this tile or of the one after it
+                        const uint8_t *np = sp + (size_t)(su + 4) * ICPS * 512;
+                        bool fill = su + 4 < it.k1;
+                        if (!fill) {
+                            const uint32_t nsub = sub + 1 == a.subs ? 0 : sub + 1, nw = nsub ? w : w + n_pairs;
+                            const GmItem ni = gm_item(a, nw);
+                            const uint32_t nsu = ni.k0 + ((j - (n + it.k1 - it.k0)) & 3);
+                            ahead = fill = nw < n_items && nsu < ni.k1;
+                            np = chunks(ni, nsub) + (size_t)nsu * ICPS * 512;
+                            late = su + 2 >= it.k1;
+                        }
+#pragma unroll
+                        for (int half = 0; half < 2; half++) {  // 64 k at a time: 32 registers of weights
+                            uint32_t A[2][16];
+                            if (BITS == 4) {
+#pragma unroll
+                                for (int c = 0; c < 2; c++) {
+                                    const uint4 wv = r[2 * half + c];
+                                    if (fill) r[2 * half + c] = t5::ldg128_nc(np + (2 * half + c) * 512);
+                                    gm_lookup16(A[c], wv, laneq, slot);
+                                }
+                            } else {
+                                uint4 pa, pb;
+                                sk_expand2(pa, pb, r[half]);
+                                if (fill) r[half] = t5::ldg128_nc(np + half * 512);
+                                gm_lookup16(A[0], pa, laneq, slot);
+                                gm_lookup16(A[1], pb, laneq, slot);
+                            }
+                            if (half == 0) {
+                                t5::mbar_wait_warp(b_done + 8 * j, (((n + su - it.k0) / GM_SA) & 1) ^ 1, err_flag);
+                                t5::fence_after();
+                            }
+                            t5::st16(tmem_lane + j * 64 + half * 32, A[0]);
+                            t5::st16(tmem_lane + j * 64 + half * 32 + 16, A[1]);
+                        }
+                        t5::wait_st();
+                        t5::fence_before();
+                        if (lane == 0) t5::mbar_arrive_tmem(afull0);
+                    }
+                }
+                if (over) break;
+                if (pend_w != 0xFFFFFFFFu) epilogue(pend_w, pend_sub);
+            }
+            pend_w = w;
+            pend_sub = sub;
+            n += it.k1 - it.k0;
+            if (++sub == a.subs) {
+                sub = 0;
+                w += n_pairs;
+            }
         }
-    } else if (warp == GM_X_WARP && lane == 0) {
+    } else if (warp == GM_MMA_WARP) {
+        // =============================== MMA issuing warp ===============================
+        // The whole warp walks the stages, so that the compiler keeps descriptors and addresses in uniform registers, and one
+        // elected lane issues.  A test of a barrier takes about 250 cycles behind the lookups of the other warps: those of the
+        // next stage are under way while the products of this one are issued.
+        if (rank == 0) {
+            const uint32_t idesc = t5::idesc_f16(256, a.nt), dcol = tmem_base + GM_D_COL;
+            uint32_t n = 0, sx = 0, px = 0, ti = 0;
+            pdl_wait();  // see the dequantising warps: no bounded wait before the dependency is met
+            uint32_t ra = 0, r0 = 0, r1 = 0;               // this stage's weights and activations have been seen to be there
+            for (uint32_t w = pair_id; w < n_items; w += n_pairs) {
+                const GmItem it = gm_item(a, w);
+                for (uint32_t sub = 0; sub < a.subs; sub++, ti++) {
+                    t5::mbar_wait_bounded(b_dempty, (ti & 1) ^ 1, err_flag);  // the sums of the tile before have left D
+                    for (uint32_t su = it.k0; su < it.k1; su++, n++) {
+                        const uint32_t sa = n % GM_SA, acol = tmem_base + sa * 64;
+                        const uint32_t s1 = sx + 1 == a.sx ? 0 : sx + 1, p1 = px ^ (s1 == 0), s2 = s1 + 1 == a.sx ? 0 : s1 + 1,
+                                       p2 = p1 ^ (s2 == 0), s3 = s2 + 1 == a.sx ? 0 : s2 + 1, p3 = p2 ^ (s3 == 0);
+                        if (!ra) t5::mbar_wait_bounded(b_afull + 8 * sa, (n / GM_SA) & 1, err_flag);
+                        if (!r0) t5::mbar_wait_bounded(b_xfull + 8 * sx, px, err_flag);
+                        const uint32_t na = t5::mbar_test(b_afull + 8 * ((n + 1) % GM_SA), ((n + 1) / GM_SA) & 1),
+                                       n0 = t5::mbar_test(b_xfull + 8 * s2, p2), n1 = t5::mbar_test(b_xfull + 8 * s3, p3);
+                        __syncwarp();
+                        t5::fence_after();
+                        const uint64_t x0 = gm_desc(x_addr(sx)), x1 = gm_desc(x_addr(s1));
+                        if (t5::elect_one()) {
+#pragma unroll
+                            for (uint32_t kk = 0; kk < 4; kk++)  // 16 k are 32 bytes of the swizzled row
+                                gm_mma_pair(dcol, acol + kk * 8, x0 + kk * 2, idesc, kk ? 1u : su - it.k0);
+                        }
+                        if (!r1) t5::mbar_wait_bounded(b_xfull + 8 * s1, p1, err_flag);
+                        __syncwarp();
+                        t5::fence_after();
+                        if (t5::elect_one()) {
+#pragma unroll
+                            for (uint32_t kk = 0; kk < 4; kk++) gm_mma_pair(dcol, acol + 32 + kk * 8, x1 + kk * 2, idesc, 1u);
+                            t5::commit_pair(b_done + 8 * sa);
+                        }
+                        ra = na; r0 = n0; r1 = n1;
+                        sx = s2; px = p2;
+                    }
+                    if (t5::elect_one()) t5::commit_pair(b_dfull);
+                }
+            }
+        }
+    } else if (lane == 0) {
         // =============================== activation loader ===============================
-        const uint32_t x_addr = smem_base + GM_X_OFF;
-        uint32_t n = 0;
+        const uint32_t full0 = t5::map_rank(b_xfull, 0);
+        uint32_t sx = 0, h = 0;                            // h: activation stages so far, two per weight stage
+        auto wait_step = [&](uint32_t step) { t5::mbar_wait_bounded(b_done + 8 * (step % GM_SA), (step / GM_SA) & 1, err_flag); };
         pdl_wait();
-        for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x) {
-            const uint32_t tt = w / a.n_rt;
-            const uint8_t *src0 = a.xc + (size_t)tt * nch * NT * 64;
-            for (uint32_t su = 0; su < nch / XC; su++, n++) {
-                const uint32_t sx = n % SX, px = (n / SX) & 1;
-                t5::mbar_wait_bounded(b_xempty + 8 * sx, px ^ 1, err_flag);
-                t5::mbar_arrive_expect_tx(b_xfull + 8 * sx, XSTAGE);
-                t5::bulk_g2s(x_addr + sx * XSTAGE, src0 + (size_t)su * XSTAGE, XSTAGE, b_xfull + 8 * sx);
+        for (uint32_t w = pair_id; w < n_items; w += n_pairs) {
+            const GmItem it = gm_item(a, w);
+            const int32_t t0 = (int32_t)(it.tt * a.nt + rank * (a.nt / 2));
+            for (uint32_t sub = 0; sub < a.subs; sub++) {
+                for (uint32_t k = it.k0 * 128; k < it.k1 * 128; k += 64, h++) {
+                    if (h >= a.sx) wait_step((h - a.sx) / 2);  // at most GM_SA steps back: its barrier has not come round again
+                    if (rank == 0) t5::mbar_arrive_expect_tx(b_xfull + 8 * sx, 2 * xstage);
+                    gm_tma_pair(x_addr(sx), &xmap, (int32_t)k, t0, full0 + 8 * sx);
+                    if (++sx == a.sx) sx = 0;
+                }
             }
         }
+        // every copy in flight lands before the CTA leaves: a stage is done after its products
+        for (uint32_t step = h / 2 > (uint32_t)GM_SA ? h / 2 - GM_SA : 0; step < h / 2; step++) wait_step(step);
     }
     t5::fence_before();
     __syncthreads();
-    if (warp == GM_MMA_WARP) t5::tmem_dealloc(tmem_base, GM_TMEM_COLS);
+    t5::cluster_sync();  // nothing arrives in a CTA that has left
+    t5::fence_after();
+    if (warp == GM_MMA_WARP) t5::tmem_dealloc_pair(tmem_base, 512);
     if (tid == 0 && *err_flag) atomicExch(a.err, 5u);
 }
 
 // ---- host side ---------------------------------------------------------------------------------
+typedef CUresult (*TensorMapEncode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                    const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static int encode_x(prism_cuda_ctx *ctx, CUtensorMap *map, const uint16_t *x, uint32_t k, uint32_t m_tok, uint32_t box_rows) {
+    static TensorMapEncode enc = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult st;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess) f = nullptr;
+        return reinterpret_cast<TensorMapEncode>(f);
+    }();
+    if (!enc) return fail(ctx, PRISM_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    const cuuint64_t dims[2] = {k, m_tok}, strides[1] = {(cuuint64_t)k * 2};
+    const cuuint32_t b[2] = {64, box_rows}, estr[2] = {1, 1};
+    const CUresult rc = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(x), dims, strides, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return rc == CUDA_SUCCESS ? PRISM_OK : fail(ctx, PRISM_E_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)rc));
+}
 
 bool gemm_tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok) {
     // whole weight stages of 128 k (four 32-k chunks: four index chunks at 4 bit, two at 2 bit)
-    return ctx->smem_base == GM_SBASE && (t.bits == 4 || t.bits == 2) && t.k % 128 == 0 && m_tok >= 8;
+    return ctx->smem_base == (int)GM_SBASE && (t.bits == 4 || t.bits == 2) && t.k % GM_STAGE_K == 0 && m_tok >= 8;
 }
 
-template <int NT, int BITS>
-static int launch_gemm_nt(prism_cuda_ctx *ctx, GemmArgs &a, const LutTensor &t, const uint16_t *X) {
-    static bool configured[PRISM_MAX_DEVICES] = {false};
-    if (!configured[ctx->device]) {
-        PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(lut_gemm_tc5_kernel<NT, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)GM_SMEM_BYTES));
-        configured[ctx->device] = true;
+// Tokens of a tile and ranges of K with the least estimated cycles.  A stage takes the tensor core 4 nt cycles; expanding
+// its weights takes 256 of the shared-memory pipe and streaming them about 350 at the HBM rate.  A tile's fill and last
+// stores cost about 2500 once, 700 for each further tile of the same pair.  A split pays for its sums' way through L2 and
+// for the wait for the last of them.
+struct GmPlan {
+    uint32_t nt = 32, splits = 1;
+    double cycles = 1e30;
+};
+static GmPlan gm_plan(uint32_t pairs, uint32_t n_rp, uint32_t n_st, uint32_t m_tok, uint32_t subs, uint32_t most_splits) {
+    GmPlan best;
+    const uint32_t top = std::min(256u, round_up_u32(m_tok, 32));
+    for (uint32_t nt = top; nt >= 32 && nt + 128 > top; nt -= 32) {
+        const uint64_t tiles = (uint64_t)n_rp * ((m_tok + nt - 1) / nt);
+        for (uint32_t cut = 1; cut <= most_splits && cut <= n_st; cut++) {
+            if (cut > 1 && tiles * cut * 256 * nt * 4 > (64u << 20)) break;  // bytes of partial sums
+            const uint64_t waves = (tiles * cut + pairs - 1) / pairs;
+            double t = (double)waves * subs * ((n_st + cut - 1) / cut * std::max(4.0 * nt, 350.0) + 700.0) + 2500.0;
+            if (cut > 1) t += 2500.0 + (double)waves * nt * 20.0 + cut * nt * 8.0;
+            if (t < best.cycles * 0.999) {
+                best.cycles = t;
+                best.nt = nt;
+                best.splits = cut;
+            }
+        }
     }
-    a.m_tok_pad = round_up_u32(a.m_tok, NT);
-    a.n_tt = a.m_tok_pad / NT;
-    // X -> [token tile][k/8][NT][8] (context scratch)
-    const size_t xc_halfs = (size_t)t.k * a.m_tok_pad;
-    PRISM_TRY(ensure_tmp(ctx, xc_halfs));
-    const size_t units = xc_halfs / 8;
-    if (!ctx->gemm_reuse_x) {
-        launch_pdl(ctx, "gemm_relay_x_kernel", gemm_relay_x_kernel, dim3((unsigned)((units + 255) / 256)), dim3(256), 0, X, a.m_tok,
-                   a.m_tok_pad, t.k, (uint32_t)NT, reinterpret_cast<uint4 *>(ctx->tmp_scratch));
-        PRISM_TRY(after_launch(ctx, "gemm_relay_x_kernel"));
+    return best;
+}
+
+template <int BITS>
+static int gm_pairs(prism_cuda_ctx *ctx, uint32_t *out) {  // pairs that are resident at once
+    static int pairs[PRISM_MAX_DEVICES] = {0};
+    if (!pairs[ctx->device]) {
+        PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(lut_gemm_tc5_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GM_SMEM_BYTES));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2 * ((unsigned)ctx->sm_count / 2));
+        cfg.blockDim = dim3(GM_THREADS);
+        cfg.dynamicSmemBytes = GM_SMEM_BYTES;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        PRISM_CUDA_TRY(ctx, cudaOccupancyMaxActiveClusters(&n, lut_gemm_tc5_kernel<BITS>, &cfg));
+        pairs[ctx->device] = std::max(1, std::min(n, ctx->sm_count / 2));
     }
-    a.xc = reinterpret_cast<const uint8_t *>(ctx->tmp_scratch);
-    // one row tile per CTA when possible, so its tables are built once
-    const uint32_t G = (uint32_t)ctx->sm_count;
-    uint32_t grid;
-    if (a.n_rt <= G) grid = a.n_rt * std::max(1u, std::min(G / a.n_rt, a.n_tt));
-    else grid = G;
-    launch_pdl(ctx, "lut_gemm_tc5_kernel", lut_gemm_tc5_kernel<NT, BITS>, dim3(grid), dim3(GM_THREADS), GM_SMEM_BYTES, a);
+    *out = (uint32_t)pairs[ctx->device];
+    return PRISM_OK;
+}
+
+template <int BITS>
+static int launch_gm(prism_cuda_ctx *ctx, GemmArgs &a, const LutTensor &t, const uint16_t *X, const GmPlan &p, uint32_t pairs) {
+    a.nt = p.nt;
+    a.splits = p.splits;
+    a.n_tt = (a.m_tok + a.nt - 1) / a.nt;
+    a.wide = a.m % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.resid)) & 15) == 0;
+    const uint32_t xstage = a.nt * 64;
+    a.sx_low = std::min((uint32_t)GM_SX_MAX, (GM_TBL - GM_X_LOW) / xstage);
+    a.sx = std::min((uint32_t)GM_SX_MAX, a.sx_low + (GM_OUT_HIGH - GM_X_HIGH) / xstage);
+    const size_t tiles = (size_t)a.n_rp * a.n_tt;
+    if (a.splits > 1) {
+        const uint32_t per = (a.nt / 16 + 3) / 4 * 512;
+        PRISM_TRY(ensure_splitk(ctx, tiles * a.splits * 2 * GM_DEQ_WARPS * per, tiles * 2 * GM_DEQ_WARPS));
+        a.part = ctx->splitk_partials;
+        a.arrived = ctx->splitk_counters;
+    }
+    CUtensorMap xmap;
+    PRISM_TRY(encode_x(ctx, &xmap, X, t.k, a.m_tok, a.nt / 2));
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(pairs, (uint64_t)tiles * a.splits);
+    launch_cluster_pdl(ctx, lut_gemm_tc5_kernel<BITS>, dim3(2 * grid), dim3(GM_THREADS), GM_SMEM_BYTES, 2u, a, xmap);
     return after_launch(ctx, "lut_gemm_tc5_kernel");
 }
 
-int launch_gemm_tc5(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y) {
-    if (reinterpret_cast<uintptr_t>(X) & 15) return fail(ctx, PRISM_E_ARG, "gemm: X must be 16-byte aligned");
+static GemmArgs gm_args(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok, uint16_t *Y) {
     GemmArgs a{};
     a.idx = t.idx; a.pal = t.pal;
-    a.n_chunks = t.k / 32; a.n_ichunks = t.n_chunks; a.n_hb = t.n_hb; a.m = t.m;
-    a.n_rt = (t.n_hb + 3) / 4;
+    a.n_st = t.k / GM_STAGE_K; a.n_ichunks = t.n_chunks; a.n_hb = t.n_hb; a.m = t.m;
+    a.n_rp = (t.n_hb + 7) / 8;
+    a.subs = 1;
     a.m_tok = m_tok;
     a.y = Y; a.err = ctx->dev_err;
-    // token tile = N of the MMA: as small as the batch allows (the activation tile is the operand
-    // that has to come through L2 for every 32-k chunk)
-    if (t.bits == 2) {
-        if (m_tok <= 32) return launch_gemm_nt<32, 2>(ctx, a, t, X);
-        if (m_tok <= 64) return launch_gemm_nt<64, 2>(ctx, a, t, X);
-        if (m_tok <= 128) return launch_gemm_nt<128, 2>(ctx, a, t, X);
-        return launch_gemm_nt<256, 2>(ctx, a, t, X);
-    }
-    if (m_tok <= 32) return launch_gemm_nt<32, 4>(ctx, a, t, X);
-    if (m_tok <= 64) return launch_gemm_nt<64, 4>(ctx, a, t, X);
-    if (m_tok <= 128) return launch_gemm_nt<128, 4>(ctx, a, t, X);
-    return launch_gemm_nt<256, 4>(ctx, a, t, X);
+    return a;
+}
+constexpr uint32_t GM_MAX_SPLITS = 8;
+
+template <int BITS>
+static int gemm_bits(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y, const uint16_t *resid) {
+    uint32_t pairs = 0;
+    PRISM_TRY(gm_pairs<BITS>(ctx, &pairs));
+    GemmArgs a = gm_args(ctx, t, m_tok, Y);
+    a.mode = resid ? GM_RESID : GM_PLAIN;
+    a.resid = resid;
+    return launch_gm<BITS>(ctx, a, t, X, gm_plan(pairs, a.n_rp, a.n_st, m_tok, 1, GM_MAX_SPLITS), pairs);
+}
+int launch_gemm_tc5(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y, const uint16_t *resid) {
+    if (reinterpret_cast<uintptr_t>(X) & 15) return fail(ctx, PRISM_E_ARG, "gemm: X must be 16-byte aligned");
+    return t.bits == 2 ? gemm_bits<2>(ctx, t, X, m_tok, Y, resid) : gemm_bits<4>(ctx, t, X, m_tok, Y, resid);
+}
+
+// Gate and up of a tile one after the other by the same CTA, whose threads meet their own gate values again, unless the
+// tiles are so few that two launches with K cut into ranges and a pass over their outputs take less.
+template <int BITS>
+static int swiglu_bits(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, bool *done) {
+    uint32_t pairs = 0;
+    PRISM_TRY(gm_pairs<BITS>(ctx, &pairs));
+    GemmArgs a = gm_args(ctx, tg, m_tok, act);
+    const GmPlan both = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 2, 1), one = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 1, GM_MAX_SPLITS);
+    *done = both.cycles <= 2 * one.cycles + 4000.0 + (double)m_tok * tg.m * 8.0 / 3500.0;
+    if (!*done) return PRISM_OK;
+    a.idx2 = tu.idx; a.pal2 = tu.pal;
+    a.subs = 2;
+    a.mode = GM_SWIGLU;
+    return launch_gm<BITS>(ctx, a, tg, X, both, pairs);
+}
+int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, bool *done) {
+    if (reinterpret_cast<uintptr_t>(X) & 15) return fail(ctx, PRISM_E_ARG, "gemm: X must be 16-byte aligned");
+    return tg.bits == 2 ? swiglu_bits<2>(ctx, tg, tu, X, m_tok, act, done) : swiglu_bits<4>(ctx, tg, tu, X, m_tok, act, done);
 }
 
 }  // namespace prism

@@ -38,16 +38,26 @@ __device__ __forceinline__ void mbar_wait_bounded(uint32_t addr, uint32_t parity
     }
     *err_flag = 1;
 }
-// Whole-warp wait: lane 0 polls (with a short back-off), the other lanes park at the warp barrier.
-// Thirty-two lanes polling one barrier word multiply the traffic on it and delay the arrivals.
+__device__ __forceinline__ uint32_t mbar_try(uint32_t addr, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    return ok;
+}
+// Whole-warp wait: lane 0 waits (each try is suspended by the hardware for some microseconds at most), the other lanes
+// park at the warp barrier.  Thirty-two lanes polling one barrier word multiply the traffic on it and delay the arrivals.
 __device__ __forceinline__ void mbar_wait_warp(uint32_t addr, uint32_t parity, volatile uint32_t *err_flag,
-                                               uint32_t limit = 16u << 20) {
+                                               uint32_t limit = 4u << 20) {
     if ((threadIdx.x & 31) == 0) {
         for (uint32_t i = 0; i < limit; i++) {
-            if (mbar_test(addr, parity)) break;
-            if ((i & 63) == 63 && *err_flag) break;
+            if (mbar_try(addr, parity)) break;
+            if ((i & 15) == 15 && *err_flag) break;
             if (i + 1 == limit) *err_flag = 1;
-            __nanosleep(32);
         }
     }
     __syncwarp();
@@ -129,6 +139,16 @@ __device__ __forceinline__ void mma_ss_pair(uint32_t d_tmem, uint64_t a_desc, ui
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// One lane of a converged warp, the same one every time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok));
+    return ok != 0;
+}
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
@@ -142,6 +162,11 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
 }
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
+}
+// The same where only tensor-memory accesses are handed over (ordered by tcgen05.fence): release at CTA scope.  At cluster scope
+// the arrival would first wait for every load the thread has in flight.
+__device__ __forceinline__ void mbar_arrive_tmem(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
