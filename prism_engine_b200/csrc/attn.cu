@@ -3,19 +3,23 @@
 // kernel.  It stands for four nodes of step() (src/lut/engine_impl.rs:1076-1459): Rope(q),
 // Rope(k), KVCache::append and Attention (attention_cpu, src/lut/cpu_fallback.rs:84-127;
 // rope_inplace, cpu_fallback.rs:131-143), with the same fp16 rounding points: q and k are rounded
-// to fp16 after the rotation, the output after the weighted sum.
+// to fp16 after the rotation, the output after the weighted sum.  Scores, softmax and sums are fp32.
 //
-// A thread-block cluster of S CTAs serves one (KV head, sequence) and ALL the query heads that
-// share that KV head (grouped-query attention: up to GT = 8 heads per pass over the cache), so a
-// cached row is read once per group instead of once per query head.  CTA r scores and weighs the
-// positions [r*chunk, (r+1)*chunk): one warp per cached row, every row of a pass in flight at once,
-// the value rows requested together with the key rows so that their latency hides behind the
-// softmax.  The softmax is the reference's two-pass form (global maximum, exp, global sum, `* inv`
-// inside the weighted sum); the S CTAs exchange their maxima, sums and partial outputs through
-// distributed shared memory, so nothing goes through global scratch and the result does not
-// depend on scheduling.
+// A thread-block cluster of S CTAs serves one (KV head, sequence) and up to 8 of the query heads that
+// share that KV head, so a cached row is read once per group instead of once per query head.  A WARP owns
+// every (warps of the cluster)-th tile of 16 positions: it copies the tile's keys and values into its own part
+// of shared memory (two tiles in flight), takes scores = K q^T (m16n8k16: 16 positions x 8 heads) and keeps
+// its own running maximum, sum and O^T = V^T p^T; the weights enter that product as two fp16 parts (22 bits of
+// the fp32 weight).  So no warp waits for another until the end, where every warp stores its maximum, sum and O
+// into the shared memory of the CTA that finishes those outputs, and ONE cluster barrier later they are merged in
+// a fixed order.
+// Bound: the latency of that chain (dependency wait, rotation, two products, merge) for the contexts of a chat, the
+// cache's bytes for long ones.  A launch inside a step, against one warp per cached row, tiles staged by the whole CTA in
+// turn and three cluster barriers: 14 heads over 2 of 64 at 160 positions 6.8 -> 4.6 us; 64 over 8 of 128 at 530 13.5 -> 6.3;
+// 8 sequences, 28 over 4 of 128, at 215 23.3 -> 6.4; one at 8 200 118 -> 16.8.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -24,8 +28,21 @@ namespace cg = cooperative_groups;
 
 namespace prism {
 
-constexpr int FA_THREADS = 256;
-constexpr int FA_WARPS = FA_THREADS / 32;
+constexpr uint32_t FA_ROWS = 16;     // positions of a tile
+constexpr uint32_t FA_MAX_S = 16;    // CTAs of a cluster
+template <int HD>
+struct FaCfg {
+    static constexpr int WARPS = HD == 256 ? 4 : 8;
+    static constexpr int THREADS = WARPS * 32;
+    static constexpr int MT = HD / 16;                      // 16-element pieces of a head
+    static constexpr int PPR = HD / 8;                      // 16-byte pieces of a row
+    static constexpr int TILE = FA_ROWS * HD * 2;           // bytes of a key (or value) tile
+    static constexpr int Q_OFF = WARPS * 4 * TILE;          // [8][HD] rotated q, [HD] new k, [HD] new v
+    static constexpr int ML_OFF = Q_OFF + 10 * HD * 2;      // [entries][8] maxima, then sums, then weights
+    // per warp of the cluster: the O pieces this CTA finishes, 128 floats each
+    static __host__ __device__ constexpr uint32_t pieces(uint32_t S) { return (MT + S - 1) / S; }
+    static __host__ __device__ constexpr size_t smem(uint32_t S) { return ML_OFF + (size_t)S * WARPS * (3 * 8 * 4 + pieces(S) * 512); }
+};
 
 __device__ __forceinline__ float fa_h2f(uint16_t v) { return __half2float(__ushort_as_half(v)); }
 __device__ __forceinline__ uint16_t fa_f2h(float v) { return __half_as_ushort(__float2half_rn(v)); }
@@ -40,7 +57,7 @@ struct FusedAttnArgs {
     uint32_t nh, nkv, batch;
     uint64_t seq_stride;        // halfs between sequences in the cache
     uint32_t max_seq;           // slots per sequence
-    uint32_t chunk_cap;         // positions of score buffer per CTA
+    uint32_t gt;                // query heads of a cluster, at most 8
     uint32_t rope_k;
     const float *inv_freq;      // [hd/2] rotation frequencies base^(-2j/hd), computed once on the host
     // Paged cache: position p of cache sequence c lives in row (page_tbl[c*tbl_stride + (p >> page_shift)]
@@ -74,13 +91,6 @@ __device__ __forceinline__ void fa_rope_angles(float (&ca)[VEC], float (&sa)[VEC
     }
 }
 
-// Stores a value into the same shared-memory word of every CTA of the cluster (at most 8), its own included.
-template <typename G>
-__device__ __forceinline__ void fa_scatter(G &cluster, float *word, uint32_t S, float value) {
-#pragma unroll
-    for (uint32_t r = 0; r < 8; r++)
-        if (r < S) *cluster.map_shared_rank(word, r) = value;
-}
 // Rotates a lane's elements; the partner element j +- hd/2 lives in lane ^ 16.
 template <int VEC>
 __device__ __forceinline__ void fa_rope_apply(float (&x)[VEC], const float (&ca)[VEC], const float (&sa)[VEC], uint32_t lane) {
@@ -96,106 +106,91 @@ __device__ __forceinline__ void fa_rope_apply(float (&x)[VEC], const float (&ca)
     }
 }
 
-// Sums each of GT per-lane values over the 32 lanes of a warp.  log2(GT) exchange rounds halve the
-// number of values a lane carries (offsets 16, 8, ...), the rest are plain butterfly adds: 9
-// shuffles for GT = 8 instead of 40.  Returns the total of value number (lane >> (5 - log2 GT)).
-template <int GT>
-__device__ __forceinline__ float fa_reduce_heads(float (&s)[GT], uint32_t lane) {
-    int off = 16;
-#pragma unroll
-    for (int n = GT; n > 1; n >>= 1, off >>= 1) {
-        const bool up = (lane & off) != 0;
-#pragma unroll
-        for (int j = 0; j < n / 2; j++) {
-            const float send = up ? s[j] : s[j + n / 2];
-            const float keep = up ? s[j + n / 2] : s[j];
-            s[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, off);
-        }
-    }
-    float v = s[0];
-#pragma unroll
-    for (; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
-    return v;
+// 16-byte asynchronous copy global -> shared
+__device__ __forceinline__ void fa_cp16(uint32_t dst_smem, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst_smem), "l"(src) : "memory");
+}
+__device__ __forceinline__ void fa_ldm(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void fa_ldm_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void fa_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t fa_transpose(uint32_t v) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(r) : "r"(v));
+    return r;
+}
+// Two weights as an fp16 pair and what that rounding left over as another.
+__device__ __forceinline__ void fa_split(float a, float b, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
-// 16-byte asynchronous copy global -> shared (the cached rows of a pass are all requested before any is used)
-__device__ __forceinline__ void fa_cp16(void *dst_smem, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void fa_cp_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-
-// rows of a tile: K and V tiles together take 48 KB of shared memory
-__host__ __device__ constexpr uint32_t fa_tile_rows(uint32_t hd) { return 24576u / (hd * 2u); }
-
-// The loops over cached rows are real loops (two rows per trip): a kernel that runs once per layer and
-// token pays for every instruction it has to fetch, so the code is kept small and the memory
-// parallelism comes from the asynchronous copies, not from unrolling.
-template <int VEC, int GT>
-__global__ void __launch_bounds__(FA_THREADS) attn_fused_kernel(const FusedAttnArgs a) {
+template <int HD>
+__global__ void __launch_bounds__(FaCfg<HD>::THREADS) attn_fused_kernel(const FusedAttnArgs a) {
+    using C = FaCfg<HD>;
+    constexpr int VEC = HD / 32, W = C::WARPS, MT = C::MT, PPR = C::PPR;
     pdl_launch_dependents();
     // first half of a cluster barrier that only says "this CTA has started": its second half stands before the
     // first store into a peer's shared memory and has long completed by then
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
     cg::cluster_group cluster = cg::this_cluster();
-    const uint32_t S = cluster.dim_blocks().x, rank = cluster.block_rank();
-    constexpr uint32_t hd = 32 * VEC;
-    constexpr uint32_t PR = fa_tile_rows(hd);      // cached rows staged per pass
-    constexpr uint32_t HL = 32 / GT;               // lanes that end up with the same head's score
-    extern __shared__ __align__(16) float fa_dyn[];
-    float *sc = fa_dyn;                                            // [chunk_cap][GT] scores, then exp
-    float *qs = fa_dyn + (((size_t)a.chunk_cap * GT + 3) & ~(size_t)3);  // [GT][hd] rotated q (16-byte aligned)
-    uint16_t *newk = reinterpret_cast<uint16_t *>(qs + GT * hd);   // [hd] this token's rotated k, [hd] its v
-    uint16_t *newv = newk + hd;
-    uint16_t *kt = newv + hd;                                      // [PR][hd] key tile
-    uint16_t *vt = kt + PR * hd;                                   // [PR][hd] value tile
-    float *part = reinterpret_cast<float *>(kt);                   // after the last tile: [FA_WARPS][GT*hd] partial outputs
-    float *recv = reinterpret_cast<float *>(vt + PR * hd);         // [S][slice]: every rank's partial sums of the outputs this CTA finishes
-    __shared__ float sh[FA_WARPS][GT];
-    __shared__ float xall[2][8][GT];               // maxima and sums of every CTA of the cluster, stored here by their owners
-    __shared__ float sinv[GT];
+    const uint32_t S = cluster.dim_blocks().x, rank = cluster.block_rank(), E = S * W;
+    extern __shared__ __align__(16) uint8_t fa_smem[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = blockIdx.y;
-    const uint32_t g = a.nh / a.nkv, n_tiles = (g + GT - 1) / GT, kvd = a.nkv * hd;
-    const uint32_t cl = blockIdx.x / S, kh = cl / n_tiles, tile = cl - kh * n_tiles;
-    const uint32_t h0 = kh * g + tile * GT;        // first query head of this cluster
-    const uint32_t nhl = min((uint32_t)GT, g - tile * GT);
-
-    uint16_t *kcb = a.kc + (size_t)kh * hd;
-    uint16_t *vcb = a.vc + (size_t)kh * hd;
+    uint16_t *qs = reinterpret_cast<uint16_t *>(fa_smem + C::Q_OFF), *newk = qs + 8 * HD, *newv = newk + HD;
+    float *mx_all = reinterpret_cast<float *>(fa_smem + C::ML_OFF), *sum_all = mx_all + E * 8, *wgt = sum_all + E * 8;
+    float *recv = wgt + E * 8;                     // [entry][piece][lane][4]
+    const uint32_t tiles_at = (uint32_t)__cvta_generic_to_shared(fa_smem) + warp * 4 * C::TILE;  // stage s: keys at 2 s, values at 2 s + 1
+    const uint32_t g = a.nh / a.nkv, n_ht = (g + a.gt - 1) / a.gt, kvd = a.nkv * HD;
+    const uint32_t cl = blockIdx.x / S, kh = cl / n_ht, ht = cl - kh * n_ht;
+    const uint32_t h0 = kh * g + ht * a.gt;        // first query head of this cluster
+    const uint32_t nhl = min(a.gt, g - ht * a.gt);
+    uint16_t *kcb = a.kc + (size_t)kh * HD;
+    uint16_t *vcb = a.vc + (size_t)kh * HD;
     const uint64_t seq_rows = a.seq_stride / kvd;  // rows of a sequence's slab (contiguous cache)
     auto row_of = [&](uint32_t p) { return fa_row(a.page_tbl, a.page_shift, a.tbl_stride, seq_rows, b, p) * kvd; };
-    constexpr uint32_t PPR = hd / 8;               // 16-byte pieces per row
+    auto place_of = [](uint32_t r, uint32_t c) { return r * (HD * 2) + ((PPR >= 8 ? c ^ (r & 7) : c ^ ((r >> 1) & 3)) << 4); };
 
-    // Everything that follows from the token position: which cache rows this CTA covers, where the new row goes.
+    // Everything that follows from the token position: the positions seen, where the new row goes.
+    const uint32_t entry = warp * S + rank;        // of the cluster's warps: neighbouring tiles lie on different SMs
     int32_t pos;
     bool have_new;
-    uint32_t sl, new_slot, p_begin, p_end, n_loc, n_pass;
+    uint32_t sl, new_slot, n_tiles;
     auto place = [&](int32_t pos_now) {
         pos = pos_now;
         const int64_t slot64 = (int64_t)pos * a.slot_mul + a.slot_add;
         have_new = slot64 >= 0 && slot64 < (int64_t)a.max_seq;  // a full cache takes no new row
-        sl = (uint32_t)(slot64 + 1);
-        if (slot64 < 0) sl = 0;
-        if (sl > a.max_seq) sl = a.max_seq;
+        sl = slot64 < 0 ? 0 : (uint32_t)min(slot64 + 1, (int64_t)a.max_seq);
         new_slot = have_new ? (uint32_t)slot64 : 0xFFFFFFFFu;
-        uint32_t chunk = (sl + S - 1) / S;
-        if (chunk > a.chunk_cap) chunk = a.chunk_cap;  // cannot happen with chunk_cap = ceil(max_seq / S)
-        p_begin = min(sl, rank * chunk);
-        p_end = min(sl, p_begin + chunk);
-        n_loc = p_end - p_begin;
-        n_pass = (n_loc + PR - 1) / PR;
+        n_tiles = (sl + FA_ROWS - 1) / FA_ROWS;
     };
-    // rows [r0, r0 + n) of this CTA's range into the tiles (the new token's row comes from registers instead)
-    auto stage = [&](uint32_t r0, uint32_t n, bool with_k) {
-        for (uint32_t i = threadIdx.x; i < n * PPR; i += FA_THREADS) {
-            const uint32_t r = i / PPR, c = i - r * PPR, p = p_begin + r0 + r;
-            if (p == new_slot) continue;
-            const size_t ro = row_of(p);
-            if (with_k) fa_cp16(kt + r * hd + c * 8, kcb + ro + c * 8);
-            fa_cp16(vt + r * hd + c * 8, vcb + ro + c * 8);
+    // a tile's rows into stage s; rows past the end are zero, the new token's row comes later
+    auto fetch = [&](uint32_t t, uint32_t s) {
+        if (t < n_tiles) {
+            const uint32_t kt = tiles_at + s * 2 * C::TILE;
+#pragma unroll
+            for (uint32_t i = lane; i < FA_ROWS * PPR; i += 32) {
+                const uint32_t r = i / PPR, c = i % PPR, p = t * FA_ROWS + r, at = kt + place_of(r, c);
+                if (p >= sl) {
+                    asm volatile("st.shared.v4.u32 [%0], {%2,%2,%2,%2};\nst.shared.v4.u32 [%1], {%2,%2,%2,%2};\n" ::"r"(at), "r"(at + C::TILE), "r"(0u) : "memory");
+                } else if (p != new_slot) {
+                    const size_t ro = row_of(p) + c * 8;
+                    fa_cp16(at, kcb + ro);
+                    fa_cp16(at + C::TILE, vcb + ro);
+                }
+            }
         }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
     // A decode step's predecessor in the stream (the q/k/v projection) does not touch the cache, and the rows
     // below the new token's were written steps ago: with `early_cache` the first tiles are requested and the
@@ -207,195 +202,173 @@ __global__ void __launch_bounds__(FA_THREADS) attn_fused_kernel(const FusedAttnA
     if (!early) pdl_wait();
     const int32_t pos_seen = *pos_ptr;
     place(pos_seen);
-    stage(0, min(n_loc, PR), true);                // requested before anything else is computed
+    fetch(entry, 0);
+    fetch(entry + E, 1);
     float ca[VEC], sa[VEC];
     fa_rope_angles<VEC>(ca, sa, lane, (float)pos, a.inv_freq);
     if (early) {
         pdl_wait();
         const int32_t pos_now = *pos_ptr;
         if (pos_now != pos_seen) {                 // the same value in every thread of the cluster
-            fa_cp_wait_all();
-            __syncthreads();
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            __syncwarp();
             place(pos_now);
-            stage(0, min(n_loc, PR), true);
+            fetch(entry, 0);
+            fetch(entry + E, 1);
             fa_rope_angles<VEC>(ca, sa, lane, (float)pos, a.inv_freq);
         }
     }
 
-    // ---- rotation: warp w prepares query head w of the group, warp 0 also the new token's k and v ----
-    {
-        for (uint32_t hh = warp; hh < (uint32_t)GT; hh += FA_WARPS) {
-            float x[VEC];
-            const uint16_t *q = a.q + (size_t)b * a.src_stride + (size_t)(h0 + hh) * hd + lane * VEC;
+    // ---- rotation: warp w prepares query heads w, w + W, ...; the last warp also the new token's k and v ----
+    for (uint32_t hh = warp; hh < 8; hh += W) {
+        float x[VEC];
+        const uint16_t *q = a.q + (size_t)b * a.src_stride + (size_t)(h0 + hh) * HD + lane * VEC;
 #pragma unroll
-            for (int i = 0; i < VEC; i++) x[i] = hh < nhl ? fa_h2f(q[i]) : 0.0f;
-            fa_rope_apply<VEC>(x, ca, sa, lane);
+        for (int i = 0; i < VEC; i++) x[i] = hh < nhl ? fa_h2f(q[i]) : 0.0f;
+        fa_rope_apply<VEC>(x, ca, sa, lane);
 #pragma unroll
-            for (int i = 0; i < VEC; i++) qs[hh * hd + lane * VEC + i] = x[i];
-        }
-        if (warp == 0) {
-            float kn[VEC];
-            const uint16_t *k = a.k + (size_t)b * a.src_stride + (size_t)kh * hd + lane * VEC;
-            const uint16_t *v = a.v + (size_t)b * a.src_stride + (size_t)kh * hd + lane * VEC;
+        for (int i = 0; i < VEC; i++) qs[hh * HD + lane * VEC + i] = fa_f2h(x[i]);
+    }
+    const uint32_t new_tile = new_slot / FA_ROWS;
+    if (warp == W - 1) {
+        float kn[VEC];
+        const uint16_t *k = a.k + (size_t)b * a.src_stride + (size_t)kh * HD + lane * VEC;
+        const uint16_t *v = a.v + (size_t)b * a.src_stride + (size_t)kh * HD + lane * VEC;
 #pragma unroll
-            for (int i = 0; i < VEC; i++) kn[i] = fa_h2f(k[i]);
-            if (a.rope_k) fa_rope_apply<VEC>(kn, ca, sa, lane);
-            const bool own_new = have_new && new_slot >= p_begin && new_slot < p_end;
-            const size_t new_off = (own_new && tile == 0) ? row_of(new_slot) : 0;
+        for (int i = 0; i < VEC; i++) kn[i] = fa_h2f(k[i]);
+        if (a.rope_k) fa_rope_apply<VEC>(kn, ca, sa, lane);
+        const bool append = have_new && ht == 0 && rank == new_tile % S;
+        const size_t new_off = append ? row_of(new_slot) : 0;
 #pragma unroll
-            for (int i = 0; i < VEC; i++) {
-                const uint16_t kb = fa_f2h(kn[i]), vb = v[i];
-                newk[lane * VEC + i] = kb;
-                newv[lane * VEC + i] = vb;
-                // KVCache::append: the first head tile of a group stores the row for all later steps
-                if (own_new && tile == 0) {
-                    kcb[new_off + lane * VEC + i] = kb;
-                    vcb[new_off + lane * VEC + i] = vb;
-                }
+        for (int i = 0; i < VEC; i++) {
+            const uint16_t kb = fa_f2h(kn[i]), vb = v[i];
+            newk[lane * VEC + i] = kb;
+            newv[lane * VEC + i] = vb;
+            // KVCache::append: the first head tile of a group stores the row for all later steps
+            if (append) {
+                kcb[new_off + lane * VEC + i] = kb;
+                vcb[new_off + lane * VEC + i] = vb;
             }
         }
     }
-    fa_cp_wait_all();
     __syncthreads();
 
-    // ---- q of every head of the group in registers --------------------------------------------------
-    float qf[GT][VEC];
+    // ---- this warp's tiles ---------------------------------------------------------------------------
+    const uint32_t mat = lane >> 3, hp = (lane & 3) * 2;  // the lane's heads: hp, hp + 1
+    uint32_t qf[MT][2];                                   // q^T, 16 elements at a time
 #pragma unroll
-    for (int hh = 0; hh < GT; hh++)
-#pragma unroll
-        for (int i = 0; i < VEC; i++) qf[hh][i] = qs[hh * hd + lane * VEC + i];
-
-    // ---- scores of this CTA's positions: one warp per position, GT heads per row -------------------
-    const float div = sqrtf((float)hd);
-    for (uint32_t ps = 0; ps < n_pass; ps++) {
-        const uint32_t r0 = ps * PR, n = min(PR, n_loc - r0);
-        if (ps > 0) {
-            __syncthreads();                       // every warp is done with the previous tile
-            stage(r0, n, true);
-            fa_cp_wait_all();
-            __syncthreads();
-        }
-#pragma unroll 2
-        for (uint32_t r = warp; r < n; r += FA_WARPS) {
-            const uint32_t p = p_begin + r0 + r;
-            const uint16_t *krow = (p == new_slot ? newk : kt + r * hd) + lane * VEC;
-            float kf[VEC], s[GT];
-#pragma unroll
-            for (int i = 0; i < VEC; i++) kf[i] = fa_h2f(krow[i]);
-#pragma unroll
-            for (int hh = 0; hh < GT; hh++) {
-                s[hh] = 0.0f;
-#pragma unroll
-                for (int i = 0; i < VEC; i++) s[hh] += qf[hh][i] * kf[i];
-            }
-            const float tot = fa_reduce_heads<GT>(s, lane);
-            if ((lane & (HL - 1)) == 0) sc[(size_t)(r0 + r) * GT + lane / HL] = tot / div;
-        }
+    for (int i = 0; i < MT; i++) {
+        const uint16_t *src = qs + (lane >> 2) * HD + i * 16 + hp;
+        qf[i][0] = *reinterpret_cast<const uint32_t *>(src);
+        qf[i][1] = *reinterpret_cast<const uint32_t *>(src + 8);
     }
-    __syncthreads();
-
-    // ---- maximum over all positions, per head: local, then across the cluster --------------------
-    // entry idx of the score buffer belongs to head idx % GT; FA_THREADS is a multiple of GT, so a
-    // thread only ever sees its own head hm = threadIdx.x % GT
-    const uint32_t hm = threadIdx.x % GT;
-    float mx = -INFINITY;
-    for (uint32_t idx = threadIdx.x; idx < n_loc * GT; idx += FA_THREADS) mx = fmaxf(mx, sc[idx]);
+    const float scale2 = 1.4426950408889634f / sqrtf((float)HD);
+    float o[MT][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
 #pragma unroll
-    for (int o = 16; o >= GT; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-    if (lane < GT) sh[warp][lane] = mx;
-    __syncthreads();
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) o[i][c] = 0.0f;
+    uint32_t st = 0;
+    for (uint32_t t = entry; t < n_tiles; t += E, st ^= 1) {
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        const uint32_t kt = tiles_at + st * 2 * C::TILE, vt = kt + C::TILE;
+        if (have_new && t == new_tile)
+            for (uint32_t c = lane; c < PPR; c += 32) {
+                const uint4 kv = reinterpret_cast<const uint4 *>(newk)[c], vv = reinterpret_cast<const uint4 *>(newv)[c];
+                const uint32_t at = kt + place_of(new_slot % FA_ROWS, c);
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(at), "r"(kv.x), "r"(kv.y), "r"(kv.z), "r"(kv.w) : "memory");
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(at + C::TILE), "r"(vv.x), "r"(vv.y), "r"(vv.z), "r"(vv.w) : "memory");
+            }
+        __syncwarp();
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, s2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < MT; i++) {
+            uint32_t k4[4];
+            fa_ldm(k4, kt + place_of(lane & 15, 2 * i + (lane >> 4)));
+            fa_mma(i & 1 ? s2 : s, k4, qf[i][0], qf[i][1]);
+        }
+        const uint32_t p0 = t * FA_ROWS + (lane >> 2);
+        float w[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) w[c] = p0 + (c >> 1) * 8 < sl ? (s[c] + s2[c]) * scale2 : -INFINITY;
+        float f[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            float top = fmaxf(w[j], w[2 + j]);
+#pragma unroll
+            for (int x = 4; x < 32; x <<= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, x));
+            top = fmaxf(top, m[j]);
+            f[j] = exp2f(m[j] - top);
+            m[j] = top;
+            w[j] = exp2f(w[j] - top);
+            w[2 + j] = exp2f(w[2 + j] - top);
+            l[j] = l[j] * f[j] + (w[j] + w[2 + j]);
+        }
+        uint32_t hi[2], lo[2];
+        fa_split(w[0], w[1], hi[0], lo[0]);
+        fa_split(w[2], w[3], hi[1], lo[1]);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            hi[j] = fa_transpose(hi[j]);
+            lo[j] = fa_transpose(lo[j]);
+        }
+#pragma unroll
+        for (int i = 0; i < MT; i++) {
+            uint32_t v4[4];
+            fa_ldm_t(v4, vt + place_of((lane & 7) + (mat >> 1) * 8, 2 * i + (mat & 1)));
+#pragma unroll
+            for (int c = 0; c < 4; c++) o[i][c] *= f[c & 1];
+            fa_mma(o[i], v4, hi[0], hi[1]);
+            fa_mma(o[i], v4, lo[0], lo[1]);
+        }
+        __syncwarp();                              // the whole warp is done with the stage
+        fetch(t + 2 * E, st);
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+
+    // ---- merge: every warp that had a tile stores its part where it is finished ----------------------
+    const uint32_t used = min(E, n_tiles), per = C::pieces(S);
     asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
-    if (threadIdx.x < GT) {
-        float m = -INFINITY;
-        for (int w = 0; w < FA_WARPS; w++) m = fmaxf(m, sh[w][threadIdx.x]);
-        fa_scatter(cluster, &xall[0][rank][threadIdx.x], S, m);
-    }
-    cluster.sync();
-    mx = -INFINITY;
-    for (uint32_t r = 0; r < S; r++) mx = fmaxf(mx, xall[0][r][hm]);
-
-    // ---- exp and its sum: local in warp order, then across the cluster in rank order -------------
-    float es = 0.0f;
-    for (uint32_t idx = threadIdx.x; idx < n_loc * GT; idx += FA_THREADS) {
-        const float e = expf(sc[idx] - mx);
-        sc[idx] = e;
-        es += e;
-    }
+    if (entry < used) {
 #pragma unroll
-    for (int o = 16; o >= GT; o >>= 1) es += __shfl_xor_sync(0xFFFFFFFFu, es, o);
-    if (lane < GT) sh[warp][lane] = es;
-    __syncthreads();
-    if (threadIdx.x < GT) {
-        float t = 0.0f;
-        for (int w = 0; w < FA_WARPS; w++) t += sh[w][threadIdx.x];
-        fa_scatter(cluster, &xall[1][rank][threadIdx.x], S, t);
-    }
-    cluster.sync();
-    if (threadIdx.x < GT) {
-        float t = 0.0f;
-        for (uint32_t r = 0; r < S; r++) t += xall[1][r][threadIdx.x];  // rank order
-        sinv[threadIdx.x] = 1.0f / (t + 1e-10f);
-    }
-    __syncthreads();
-    float inv[GT];
+        for (int j = 0; j < 2; j++)
 #pragma unroll
-    for (int hh = 0; hh < GT; hh++) inv[hh] = sinv[hh];
-
-    // ---- weighted sum of the value rows -----------------------------------------------------------
-    float ac[GT][VEC];
-#pragma unroll
-    for (int hh = 0; hh < GT; hh++)
-#pragma unroll
-        for (int i = 0; i < VEC; i++) ac[hh][i] = 0.0f;
-    for (uint32_t ps = 0; ps < n_pass; ps++) {
-        const uint32_t r0 = ps * PR, n = min(PR, n_loc - r0);
-        if (n_pass > 1) {                          // with one pass the value tile is still the one staged at the start
-            __syncthreads();
-            stage(r0, n, false);
-            fa_cp_wait_all();
-            __syncthreads();
+            for (int x = 4; x < 32; x <<= 1) l[j] += __shfl_xor_sync(0xFFFFFFFFu, l[j], x);
+        for (uint32_t r = lane >> 2; r < S; r += 8) {
+            *reinterpret_cast<float2 *>(cluster.map_shared_rank(mx_all + entry * 8 + hp, r)) = make_float2(m[0], m[1]);
+            *reinterpret_cast<float2 *>(cluster.map_shared_rank(sum_all + entry * 8 + hp, r)) = make_float2(l[0], l[1]);
         }
-#pragma unroll 2
-        for (uint32_t r = warp; r < n; r += FA_WARPS) {
-            const uint32_t p = p_begin + r0 + r;
-            const uint16_t *vrow = (p == new_slot ? newv : vt + r * hd) + lane * VEC;
-            const float *ep = sc + (size_t)(r0 + r) * GT;
-            float vf[VEC];
 #pragma unroll
-            for (int i = 0; i < VEC; i++) vf[i] = fa_h2f(vrow[i]);
-#pragma unroll
-            for (int hh = 0; hh < GT; hh++) {
-                const float e = ep[hh];
-#pragma unroll
-                for (int i = 0; i < VEC; i++) ac[hh][i] += __fmul_rn(__fmul_rn(e, vf[i]), inv[hh]);
-            }
+        for (int i = 0; i < MT; i++) {
+            const uint32_t owner = i / per;
+            *reinterpret_cast<float4 *>(cluster.map_shared_rank(recv + ((size_t)(entry * per + (i - owner * per)) * 32 + lane) * 4, owner)) =
+                make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
         }
     }
-    __syncthreads();                               // the tiles are dead: their space takes the partial outputs
+    cluster.sync();                                // nobody touches a peer's memory after this barrier
+    for (uint32_t hh = warp; hh < 8; hh += W) {
+        float top = -INFINITY, sum = 0.0f;
+        for (uint32_t e = lane; e < used; e += 32) top = fmaxf(top, mx_all[e * 8 + hh]);
 #pragma unroll
-    for (int hh = 0; hh < GT; hh++)
+        for (int x = 16; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, x));
+        for (uint32_t e = lane; e < used; e += 32) {
+            const float f = exp2f(mx_all[e * 8 + hh] - top);
+            wgt[e * 8 + hh] = f;
+            sum += sum_all[e * 8 + hh] * f;
+        }
 #pragma unroll
-        for (int i = 0; i < VEC; i++) part[(size_t)warp * (GT * hd) + hh * hd + lane * VEC + i] = ac[hh][i];
+        for (int x = 16; x > 0; x >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, x);
+        const float inv = 1.0f / (sum + 1e-10f);
+        __syncwarp();
+        for (uint32_t e = lane; e < used; e += 32) wgt[e * 8 + hh] *= inv;
+    }
     __syncthreads();
-    // Output element t is finished by rank t / per: every CTA adds its warps' partial sums and stores the result
-    // into slot [its rank] of the finishing CTA's receive buffer; after one cluster barrier the finisher adds the
-    // slots in rank order from its own shared memory.  Nobody touches a peer's memory after that barrier.
-    const uint32_t n_out = nhl * hd, per = (n_out + S - 1) / S;
-    for (uint32_t t = threadIdx.x; t < n_out; t += FA_THREADS) {
+    const uint32_t own = rank * per < (uint32_t)MT ? min(per, MT - rank * per) : 0;
+    for (uint32_t t = threadIdx.x; t < own * 128; t += C::THREADS) {
+        const uint32_t i = t >> 7, ln = (t >> 2) & 31, c = t & 3, hh = (ln & 3) * 2 + (c & 1);
         float v = 0.0f;
-#pragma unroll
-        for (uint32_t w = 0; w < (uint32_t)FA_WARPS; w++) v += part[(size_t)w * (GT * hd) + t];
-        const uint32_t owner = t / per;
-        *cluster.map_shared_rank(recv + rank * per + (t - owner * per), owner) = v;
-    }
-    cluster.sync();
-    {
-        const uint32_t t_end = min(n_out, (rank + 1) * per);
-        for (uint32_t t = rank * per + threadIdx.x; t < t_end; t += FA_THREADS) {
-            float o = 0.0f;
-            for (uint32_t r = 0; r < S; r++) o += recv[r * per + (t - rank * per)];  // rank order
-            a.out[(size_t)b * a.nh * hd + (size_t)h0 * hd + t] = fa_f2h(o);
-        }
+        for (uint32_t e = 0; e < used; e++) v += recv[(size_t)(e * per + i) * 128 + (t & 127)] * wgt[e * 8 + hh];
+        if (hh < nhl) a.out[(size_t)b * a.nh * HD + (size_t)(h0 + hh) * HD + (rank * per + i) * 16 + (ln >> 2) + (c >> 1) * 8] = fa_f2h(v);
     }
 }
 
@@ -405,30 +378,30 @@ bool attn_fused_eligible(const AttnArgs &a) {
            reinterpret_cast<uintptr_t>(a.k) % 16 == 0 && reinterpret_cast<uintptr_t>(a.v) % 16 == 0;
 }
 
-// shared memory of a launch: the score buffer and the per-warp partial outputs
-static size_t fa_smem_bytes(uint32_t chunk_cap, uint32_t gt, uint32_t hd) {
-    // scores, rotated q, the new token's k and v, and the key/value tiles (48 KB; the per-warp partial
-    // outputs, at most 32 KB, reuse the tiles' space)
-    // and the receive buffer of the final reduction (one slice per rank, together at most gt*hd + 8 floats)
-    return (((size_t)chunk_cap * gt + 3) & ~(size_t)3) * 4 + (size_t)gt * hd * 4 + 2 * hd * 2 + 2 * (size_t)fa_tile_rows(hd) * hd * 2 +
-           ((size_t)gt * hd + 8) * 4;
-}
-
-template <int VEC, int GT>
-static int launch_attn_fused_v(prism_cuda_ctx *ctx, const FusedAttnArgs &fa, uint32_t S) {
-    const uint32_t g = fa.nh / fa.nkv, n_tiles = (g + GT - 1) / GT;
-    const size_t smem = fa_smem_bytes(fa.chunk_cap, GT, 32 * VEC);
-    if (smem > 215 * 1024) return fail(ctx, PRISM_E_ARG, "fused attention: max_seq too large for the score buffer");
+template <int HD>
+static int launch_attn_fused_hd(prism_cuda_ctx *ctx, FusedAttnArgs &fa) {
+    using C = FaCfg<HD>;
+    const uint32_t g = fa.nh / fa.nkv;
+    fa.gt = std::min(8u, g);
+    if (ctx->attn_group > 0) fa.gt = std::min(fa.gt, (uint32_t)ctx->attn_group);
+    const uint32_t clusters = fa.nkv * ((g + fa.gt - 1) / fa.gt) * fa.batch;
+    // CTAs per cluster: a tile of 16 positions per warp while there are SMs to give one CTA each; more than 8 (a
+    // non-portable size) only for contexts that still give every warp two tiles
+    uint32_t S = 1;
+    while (S < 8 && S * C::WARPS * FA_ROWS < fa.max_seq && 2 * S * clusters <= (uint32_t)ctx->sm_count) S *= 2;
+    if (S == 8 && 16 * clusters <= (uint32_t)ctx->sm_count && fa.max_seq >= 32 * C::WARPS * FA_ROWS) S = 16;
+    if (ctx->attn_cluster == 1 || ctx->attn_cluster == 2 || ctx->attn_cluster == 4 || ctx->attn_cluster == 8)
+        S = (uint32_t)ctx->attn_cluster;
     static bool configured[PRISM_MAX_DEVICES] = {false};
-    if (smem > 32 * 1024 && !configured[ctx->device]) {
-        PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_fused_kernel<VEC, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 215 * 1024));
+    if (!configured[ctx->device]) {
+        PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_fused_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(C::smem(1), C::smem(FA_MAX_S))));
+        PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_fused_kernel<HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         configured[ctx->device] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(fa.nkv * n_tiles * S, fa.batch);
-    cfg.blockDim = dim3(FA_THREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3(clusters / fa.batch * S, fa.batch);
+    cfg.blockDim = dim3(C::THREADS);
+    cfg.dynamicSmemBytes = C::smem(S);
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -439,24 +412,8 @@ static int launch_attn_fused_v(prism_cuda_ctx *ctx, const FusedAttnArgs &fa, uin
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->pdl ? 2 : 1;
-    (void)cudaLaunchKernelEx(&cfg, attn_fused_kernel<VEC, GT>, fa);
+    (void)cudaLaunchKernelEx(&cfg, attn_fused_kernel<HD>, fa);
     return after_launch(ctx, "attn_fused_kernel");
-}
-
-template <int VEC>
-static int launch_attn_fused_g(prism_cuda_ctx *ctx, const FusedAttnArgs &fa, uint32_t S) {
-    // query heads served per pass over the cache: the group size rounded up to a power of two, at
-    // most 8 (4 for 256-wide heads: registers)
-    const uint32_t g = fa.nh / fa.nkv;
-    uint32_t cap = VEC == 8 ? 4 : 8;
-    // A small model with few KV heads would leave most of the GPU idle (0.5B: 2 KV heads x 2 CTAs): serve fewer
-    // heads per cluster until about two dozen CTAs run; the cached rows are then read once per cluster, from L2.
-    while (cap > 1 && fa.nkv * ((g + cap - 1) / cap) * S * fa.batch < 24 && g > cap / 2) cap /= 2;
-    if (ctx->attn_group > 0) cap = min(cap, (uint32_t)ctx->attn_group);
-    if (g >= 5 && cap >= 8) return launch_attn_fused_v<VEC, (VEC == 8 ? 4 : 8)>(ctx, fa, S);
-    if (g >= 3 && cap >= 4) return launch_attn_fused_v<VEC, 4>(ctx, fa, S);
-    if (g >= 2 && cap >= 2) return launch_attn_fused_v<VEC, 2>(ctx, fa, S);
-    return launch_attn_fused_v<VEC, 1>(ctx, fa, S);
 }
 
 // The rotation frequencies base^(-2j/hd), j < hd/2, as the CPU path computes them (powf in fp32,
@@ -498,17 +455,11 @@ int launch_attn_fused(prism_cuda_ctx *ctx, const AttnArgs &a, const uint16_t *k_
     fa.page_tbl = a.page_tbl; fa.page_shift = a.page_shift; fa.tbl_stride = a.tbl_stride;
     fa.early_cache = a.early_cache;
     PRISM_TRY(rope_table(ctx, a.hd, rope_base, &fa.inv_freq));
-    // cluster size: a CTA stages up to 96 cached rows of 128-wide heads per pass; more CTAs per group
-    // spread the rows (and the latency of fetching them) over more SMs
-    uint32_t S = a.max_seq > 512 ? 8 : a.max_seq > 256 ? 4 : a.max_seq > 128 ? 2 : 1;
-    if (ctx->attn_cluster == 1 || ctx->attn_cluster == 2 || ctx->attn_cluster == 4 || ctx->attn_cluster == 8)
-        S = (uint32_t)ctx->attn_cluster;
-    fa.chunk_cap = (a.max_seq + S - 1) / S;
     switch (a.hd) {
-    case 32: return launch_attn_fused_g<1>(ctx, fa, S);
-    case 64: return launch_attn_fused_g<2>(ctx, fa, S);
-    case 128: return launch_attn_fused_g<4>(ctx, fa, S);
-    default: return launch_attn_fused_g<8>(ctx, fa, S);
+    case 32: return launch_attn_fused_hd<32>(ctx, fa);
+    case 64: return launch_attn_fused_hd<64>(ctx, fa);
+    case 128: return launch_attn_fused_hd<128>(ctx, fa);
+    default: return launch_attn_fused_hd<256>(ctx, fa);
     }
 }
 
