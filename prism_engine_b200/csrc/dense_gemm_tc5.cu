@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(DgCfg<NT>::THREADS, 1) dense_gemm_tc5_kernel(c
     uint8_t *smem = dg_smem_raw + (1024 - ((uint32_t)__cvta_generic_to_shared(dg_smem_raw) & 1023u)) % 1024;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
     pdl_launch_dependents();
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
     const uint32_t b_full = base + C::BAR_OFF, b_empty = b_full + 8 * C::S, b_dfull = b_empty + 8 * C::S, b_dempty = b_dfull + 16;
     const uint32_t state = C::BAR_OFF + 8 * (2 * C::S + 4);
     volatile uint32_t *err_flag = reinterpret_cast<volatile uint32_t *>(smem + state);
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(DgCfg<NT>::THREADS, 1) dense_gemm_tc5_kernel(c
     t5::fence_before();
     __syncthreads();
     t5::fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
     pdl_wait();  // before any bounded wait: the kernel before this one may still be at work
     if (MOE) {
         if (warp == 2) dg_expert_table<NT>(a, tile_end, row_end, lane);
@@ -279,25 +279,28 @@ __global__ void __launch_bounds__(DgCfg<NT>::THREADS, 1) dense_gemm_tc5_kernel(c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = t5::idesc_f16(128, NT) | a.types;
-            uint32_t n = 0, ti = 0;
-            for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x, ti++) {
-                const DgItem it = dg_locate<NT, 1, MOE>(a, w, tile_end, row_end);
-                const uint32_t kb = dense_seg(a.epi, it.rt * 128).k / 64, d = tmem + (ti & 1) * NT;
-                t5::mbar_wait_bounded(b_dempty + 8 * (ti & 1), ((ti >> 1) & 1) ^ 1, err_flag);
+        // The whole warp walks the stages, so that descriptors stay in uniform registers, and one elected lane issues; the
+        // test of the next stage's barrier is under way while the products of this one are issued.
+        const uint32_t idesc = t5::idesc_f16(128, NT) | a.types;
+        uint32_t n = 0, ti = 0, ready = 0;
+        for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x, ti++) {
+            const DgItem it = dg_locate<NT, 1, MOE>(a, w, tile_end, row_end);
+            const uint32_t kb = dense_seg(a.epi, it.rt * 128).k / 64, d = tmem + (ti & 1) * NT;
+            t5::mbar_wait_bounded(b_dempty + 8 * (ti & 1), ((ti >> 1) & 1) ^ 1, err_flag);
+            for (uint32_t k = 0; k < kb; k++, n++) {
+                const uint32_t s = n % C::S, sa = base + s * C::STAGE, sb = sa + C::A_BYTES;
+                if (!ready) t5::mbar_wait_bounded(b_full + 8 * s, (n / C::S) & 1, err_flag);
+                ready = t5::mbar_test(b_full + 8 * ((n + 1) % C::S), ((n + 1) / C::S) & 1);
+                __syncwarp();
                 t5::fence_after();
-                for (uint32_t k = 0; k < kb; k++, n++) {
-                    const uint32_t s = n % C::S, ph = (n / C::S) & 1, sa = base + s * C::STAGE, sb = sa + C::A_BYTES;
-                    t5::mbar_wait_bounded(b_full + 8 * s, ph, err_flag);
-                    t5::fence_after();
+                if (t5::elect_one()) {
 #pragma unroll
                     for (int j = 0; j < 4; j++)  // 16 k each: two k/8 slabs of 2 KB in A, 32 bytes inside the swizzled rows of B
-                        mma_ss(d, t5::smem_desc(sa + j * 4096, 2048, 128), desc_sw128(sb + j * 32), idesc, (k | j) != 0);
+                        mma_ss(d, t5::smem_desc(sa + j * 4096, 2048, 128), desc_sw128(sb + j * 32), idesc, j ? 1u : k);
                     t5::commit(b_empty + 8 * s);
                 }
-                t5::commit(b_dfull + 8 * (ti & 1));
             }
+            if (t5::elect_one()) t5::commit(b_dfull + 8 * (ti & 1));
         }
     } else {
         const uint32_t q = warp & 3;  // the TMEM lanes a warp may read
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(DpCfg<NT>::THREADS, 1) dense_gemm_pair_kernel(
     uint8_t *smem = dg_smem_raw + (1024 - ((uint32_t)__cvta_generic_to_shared(dg_smem_raw) & 1023u)) % 1024;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem), rank = t5::cluster_rank();
     pdl_launch_dependents();
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
     // full and dempty: the pair's, in CTA 0 (it issues the products); empty and dfull: each CTA's own
     const uint32_t b_full = base + C::BAR_OFF, b_empty = b_full + 8 * C::S, b_dfull = b_empty + 8 * C::S, b_dempty = b_dfull + 16;
     const uint32_t state = C::BAR_OFF + 8 * (2 * C::S + 4);
@@ -350,7 +353,7 @@ __global__ void __launch_bounds__(DpCfg<NT>::THREADS, 1) dense_gemm_pair_kernel(
     __syncthreads();
     t5::cluster_sync();  // the other CTA's barriers exist before anything arrives there
     t5::fence_after();
-    const uint32_t tmem = *tmem_slot, pair = blockIdx.x / 2, n_pairs = gridDim.x / 2;
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0), pair = blockIdx.x / 2, n_pairs = gridDim.x / 2;
     pdl_wait();  // before any bounded wait: the kernel before this one may still be at work
     if (MOE) {
         if (warp == 2) dg_expert_table<NT>(a, tile_end, row_end, lane);
@@ -382,25 +385,28 @@ __global__ void __launch_bounds__(DpCfg<NT>::THREADS, 1) dense_gemm_pair_kernel(
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {  // as in dense_gemm_tc5_kernel
             const uint32_t idesc = t5::idesc_f16(256, NT) | a.types;
-            uint32_t n = 0, ti = 0;
+            uint32_t n = 0, ti = 0, ready = 0;
             for (uint32_t w = pair; w < n_items; w += n_pairs, ti++) {
                 const DgItem it = dg_locate<NT, 2, MOE>(a, w / a.splits, tile_end, row_end);
                 const DenseEpiSeg &seg = dense_seg(a.epi, it.rt * 256);
                 const uint32_t kb = dg_k(a, seg, w % a.splits + 1) - dg_k(a, seg, w % a.splits), d = tmem + (ti & 1) * NT;
                 t5::mbar_wait_bounded(b_dempty + 8 * (ti & 1), ((ti >> 1) & 1) ^ 1, err_flag);
-                t5::fence_after();
                 for (uint32_t k = 0; k < kb; k++, n++) {
-                    const uint32_t s = n % C::S, ph = (n / C::S) & 1, sa = base + s * C::STAGE, sb = sa + DG_A_BYTES;
-                    t5::mbar_wait_bounded(b_full + 8 * s, ph, err_flag);
+                    const uint32_t s = n % C::S, sa = base + s * C::STAGE, sb = sa + DG_A_BYTES;
+                    if (!ready) t5::mbar_wait_bounded(b_full + 8 * s, (n / C::S) & 1, err_flag);
+                    ready = t5::mbar_test(b_full + 8 * ((n + 1) % C::S), ((n + 1) / C::S) & 1);
+                    __syncwarp();
                     t5::fence_after();
+                    if (t5::elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        t5::mma_ss_pair(d, t5::smem_desc(sa + j * 4096, 2048, 128), desc_sw128(sb + j * 32), idesc, (k | j) != 0);
-                    t5::commit_pair(b_empty + 8 * s);
+                        for (int j = 0; j < 4; j++)
+                            t5::mma_ss_pair(d, t5::smem_desc(sa + j * 4096, 2048, 128), desc_sw128(sb + j * 32), idesc, j ? 1u : k);
+                        t5::commit_pair(b_empty + 8 * s);
+                    }
                 }
-                t5::commit_pair(b_dfull + 8 * (ti & 1));
+                if (t5::elect_one()) t5::commit_pair(b_dfull + 8 * (ti & 1));
             }
         }
     } else {

@@ -19,8 +19,8 @@
 // against about 1 000 for the 16 384 exponentials.  Masked positions carry weight 0; value rows past the portion's
 // end (stale cache) are zeroed in shared memory before the product, so no stale NaN meets a zero weight.
 // Measured, 28 query / 4 KV heads of 128: the attention of an 8190-token prompt through two layers took 128 ms with one
-// cluster of the decode kernel per token, on the CUDA cores; with this kernel the whole pass takes 20.2 ms instead of
-// 142.5, a 2048-token prompt through four layers 7.7 ms instead of 23.8.
+// cluster of the decode kernel per token, on the CUDA cores; this kernel took 1.87 ms with a single issuing thread (descriptors
+// through vector registers), 1.38 with a whole warp walking the tiles.
 #include <cuda.h>
 
 #include <algorithm>
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
     uint8_t *smem = pa_raw + (1024 - ((uint32_t)__cvta_generic_to_shared(pa_raw) & 1023u)) % 1024;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
     pdl_launch_dependents();
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
     const uint32_t b_kfull = base + C::BAR_OFF, b_kempty = b_kfull + 8 * ST, b_vfull = b_kempty + 8 * ST, b_vempty = b_vfull + 8 * ST,
                    b_sfull = b_vempty + 8 * ST, b_pfull = b_sfull + 16, b_ofull = b_pfull + 16, b_qfull = b_ofull + 16;
     volatile uint32_t *err_flag = reinterpret_cast<volatile uint32_t *>(smem + C::STATE_OFF);
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
     t5::fence_before();
     __syncthreads();
     t5::fence_after();
-    const uint32_t tmem = *tmem_slot;  // S of tile q at column 128 q, O at 256 + HD q
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);  // S of tile q at column 128 q, O at 256 + HD q
     pdl_wait();                        // before any bounded wait: the kernel before this one may still be at work
 
     const uint32_t h = blockIdx.x, kh = h / a.group, sq = blockIdx.y, qb = (gridDim.z - 1 - blockIdx.z) * (QT * 128);
@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
         }
         __syncwarp();
     } else {
-        // ================= products: lane 0 issues; the whole warp clears stale value rows =================
+        // ================= products: the whole warp walks the tiles (descriptors stay in uniform registers), an elected lane
+        // issues; all lanes clear stale value rows =================
         const uint32_t id_s = t5::idesc_f16(128, PA_K), id_o = t5::idesc_f16(128, HD) | (1u << 16);  // V is read across its rows
         auto scores = [&](uint32_t q, uint32_t j) {
             const uint32_t qa = base + q * C::TILE, ka = base + C::K_OFF + (j % ST) * C::TILE;
@@ -277,18 +278,19 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
             }
             t5::commit(b_sfull + 8 * q);
         };
-        if (lane == 0) {
-            t5::mbar_wait_bounded(b_qfull, 0, err_flag);
-            t5::mbar_wait_bounded(b_kfull, 0, err_flag);
-            t5::fence_after();
+        t5::mbar_wait_bounded(b_qfull, 0, err_flag);
+        t5::mbar_wait_bounded(b_kfull, 0, err_flag);
+        __syncwarp();
+        t5::fence_after();
+        if (t5::elect_one()) {
             for (uint32_t q = 0; q < (uint32_t)QT; q++)
                 if (n_kt[q]) scores(q, 0);
             t5::commit(b_kempty);
         }
         __syncwarp();
         for (uint32_t j = 0; j < n; j++) {
-            const uint32_t st = j % ST, ph = (j / ST) & 1, va = base + C::V_OFF + st * C::TILE;
-            if (lane == 0) t5::mbar_wait_bounded(b_vfull + 8 * st, ph, err_flag);
+            const uint32_t st = j % ST, ph = (j / ST) & 1, va = base + C::V_OFF + st * C::TILE, jn = j + 1;
+            t5::mbar_wait_bounded(b_vfull + 8 * st, ph, err_flag);
             __syncwarp();
             if (kv_end - j * PA_K < (uint32_t)PA_K) {
                 const uint32_t first = kv_end - j * PA_K, per = C::ROWB / 16, cells = (PA_K - first) * per * C::PANELS;
@@ -299,22 +301,26 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 __syncwarp();
             }
-            if (lane == 0) {
-                const uint32_t jn = j + 1;
-                if (jn < n) t5::mbar_wait_bounded(b_kfull + 8 * (jn % ST), (jn / ST) & 1, err_flag);
-                for (uint32_t q = 0; q < (uint32_t)QT; q++) {
-                    if (j >= n_kt[q]) continue;
-                    t5::mbar_wait_bounded(b_pfull + 8 * q, j & 1, err_flag);
-                    t5::fence_after();
+            if (jn < n) t5::mbar_wait_bounded(b_kfull + 8 * (jn % ST), (jn / ST) & 1, err_flag);
+#pragma unroll
+            for (uint32_t q = 0; q < (uint32_t)QT; q++) {
+                if (j >= n_kt[q]) continue;
+                t5::mbar_wait_bounded(b_pfull + 8 * q, j & 1, err_flag);
+                __syncwarp();
+                t5::fence_after();
+                if (t5::elect_one()) {
 #pragma unroll
                     for (int part = 0; part < 2; part++)
 #pragma unroll
                         for (int k = 0; k < PA_K / 16; k++)
                             t5::mma_ts(tmem + 256 + q * HD, tmem + q * 128 + part * 64 + k * 8, pa_desc<C::ROWB>(va + k * 16 * C::ROWB, C::PANEL), id_o,
-                                       (j | part | k) != 0);
+                                       part | k ? 1u : j);
                     if (jn < n_kt[q]) scores(q, jn);
                     else t5::commit(b_ofull + 8 * q);
                 }
+                __syncwarp();
+            }
+            if (t5::elect_one()) {
                 t5::commit(b_vempty + 8 * st);
                 if (jn < n) t5::commit(b_kempty + 8 * (jn % ST));
             }
