@@ -22,8 +22,8 @@
 // Measured, 4 bit, against one CTA per 128 x 256 tile whose single issuing thread spent 1 700 cycles on a stage of 1 024
 // (waits one after the other, descriptors through vector registers, three commits) and which used as many CTAs as there were
 // row tiles: 18944 x 3584, 2048 tokens 266 -> 216 us (1 287 TFLOP/s, 0.78 of measured burst), 512 tokens 67 -> 54, 32 tokens
-// 26 -> 22.5; 4608 x 3584, 2048 tokens 72 -> 53, 32 tokens 23.4 -> 15.1; 3584 x 18944, 2048 tokens 320 -> 275, 32 tokens
-// 96.5 -> 26.9.  The first three without residual or SwiGLU passes and the re-laid activations that went with them.
+// 26 -> 19.9; 4608 x 3584, 2048 tokens 72 -> 53, 32 tokens 23.4 -> 15.1; 3584 x 18944, 2048 tokens 320 -> 278, 32 tokens
+// 96.5 -> 25.0.  The times before are without the residual or SwiGLU passes and the re-laid activations that went with them.
 // Every mbarrier wait is bounded; a wait that gives up raises the context's device error word.
 #include <cuda.h>
 
@@ -41,7 +41,8 @@ constexpr int GM_THREADS = 18 * 32;
 constexpr int GM_STAGE_K = 128;               // k of a weight stage: 64 TMEM columns
 constexpr int GM_SA = 4;                      // weight stages; a warp of slot j fills every fourth, ring position j
 constexpr int GM_D_COL = GM_SA * 64;          // accumulator: up to 256 columns after the A stages
-constexpr int GM_SX_MAX = 2 * GM_SA;          // most activation stages, of 64 k each
+constexpr int GM_SX_MAX = 32;                 // most activation stages, of 64 k each
+constexpr int GM_XD = GM_SX_MAX / 2;          // weight stages that many belong to
 // The two pair tables start on 64 KB boundaries of the shared-memory window, so that a lookup's address is one
 // permute of an index byte; barriers and activation stages lie before and after them.
 constexpr uint32_t GM_SBASE = 1024;           // where dynamic shared memory starts (checked)
@@ -50,9 +51,10 @@ constexpr uint32_t GM_OUT_LOW = 2048, GM_OUT_LOW_WARPS = 12;      // 1 KB per de
 constexpr uint32_t GM_X_LOW = GM_OUT_LOW + GM_OUT_LOW_WARPS * 1024, GM_X_HIGH = GM_TBL + 2 * 65536;
 constexpr uint32_t GM_END = GM_SBASE + 227 * 1024;
 constexpr uint32_t GM_OUT_HIGH = GM_END - (GM_DEQ_WARPS - GM_OUT_LOW_WARPS) * 1024;
-// barriers (8 B each) at GM_SBASE: afull[SA], done[SA], xfull[SX], dfull, dempty; error flag, TMEM base.  One commit per
-// weight stage gives back its TMEM columns and the activation stages it used.
-constexpr uint32_t GM_STATE = GM_SBASE + 8 * (2 * GM_SA + GM_SX_MAX + 2);
+// barriers (8 B each) at GM_SBASE: afull[SA], done[SA], xfull[SX], xdone[XD], dfull, dempty; error flag, TMEM base.  One commit
+// per weight stage gives back its TMEM columns and the activation stages it used; where small token tiles leave room for more
+// activation stages than SA weight stages use, another says so on a ring of their length.
+constexpr uint32_t GM_STATE = GM_SBASE + 8 * (2 * GM_SA + GM_SX_MAX + GM_XD + 2);
 constexpr size_t GM_SMEM_BYTES = GM_END - GM_SBASE;
 static_assert(GM_STATE + 16 <= GM_OUT_LOW, "barriers overlap what follows");
 
@@ -211,7 +213,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), rank = t5::cluster_rank();
     // afull, xfull and dempty: the pair's, in CTA 0 (it issues the products); done and dfull: each CTA's own
     const uint32_t b_afull = base + GM_SBASE, b_done = b_afull + 8 * GM_SA, b_xfull = b_done + 8 * GM_SA,
-                   b_dfull = b_xfull + 8 * GM_SX_MAX, b_dempty = b_dfull + 8;
+                   b_xdone = b_xfull + 8 * GM_SX_MAX, b_dfull = b_xdone + 8 * GM_XD, b_dempty = b_dfull + 8;
+    const bool deep = a.sx > 2 * GM_SA;
     constexpr int ICPS = BITS == 4 ? 4 : 2;             // 16-byte index chunks per weight stage
     volatile uint32_t *err_flag = reinterpret_cast<volatile uint32_t *>(win + GM_STATE);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(win + GM_STATE + 8);
@@ -222,6 +225,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
     if (tid == 0) {
         for (int s = 0; s < GM_SA; s++) { t5::mbar_init(b_afull + 8 * s, 8); t5::mbar_init(b_done + 8 * s, 1); }
         for (int s = 0; s < GM_SX_MAX; s++) t5::mbar_init(b_xfull + 8 * s, 1);
+        for (int s = 0; s < GM_XD; s++) t5::mbar_init(b_xdone + 8 * s, 1);
         t5::mbar_init(b_dfull, 1);
         t5::mbar_init(b_dempty, 2 * GM_DEQ_WARPS);
         *err_flag = 0;
@@ -421,13 +425,13 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
     } else if (warp == GM_MMA_WARP) {
         // =============================== MMA issuing warp ===============================
         // The whole warp walks the stages, so that the compiler keeps descriptors and addresses in uniform registers, and one
-        // elected lane issues.  A test of a barrier takes about 250 cycles behind the lookups of the other warps: those of the
-        // next stage are under way while the products of this one are issued.
+        // elected lane issues.  A test of a barrier takes some 100 to 250 cycles behind the lookups of the other warps: three
+        // lanes test the three of the next stage at once.
         if (rank == 0) {
             const uint32_t idesc = t5::idesc_f16(256, a.nt), dcol = tmem_base + GM_D_COL;
             uint32_t n = 0, sx = 0, px = 0, ti = 0;
             pdl_wait();  // see the dequantising warps: no bounded wait before the dependency is met
-            uint32_t ra = 0, r0 = 0, r1 = 0;               // this stage's weights and activations have been seen to be there
+            uint32_t ready = 0;                            // this stage's weights (1) and activations (2, 4) have been seen to be there
             for (uint32_t w = pair_id; w < n_items; w += n_pairs) {
                 const GmItem it = gm_item(a, w);
                 for (uint32_t sub = 0; sub < a.subs; sub++, ti++) {
@@ -436,11 +440,10 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                         const uint32_t sa = n % GM_SA, acol = tmem_base + sa * 64;
                         const uint32_t s1 = sx + 1 == a.sx ? 0 : sx + 1, p1 = px ^ (s1 == 0), s2 = s1 + 1 == a.sx ? 0 : s1 + 1,
                                        p2 = p1 ^ (s2 == 0), s3 = s2 + 1 == a.sx ? 0 : s2 + 1, p3 = p2 ^ (s3 == 0);
-                        if (!ra) t5::mbar_wait_bounded(b_afull + 8 * sa, (n / GM_SA) & 1, err_flag);
-                        if (!r0) t5::mbar_wait_bounded(b_xfull + 8 * sx, px, err_flag);
-                        const uint32_t na = t5::mbar_test(b_afull + 8 * ((n + 1) % GM_SA), ((n + 1) / GM_SA) & 1),
-                                       n0 = t5::mbar_test(b_xfull + 8 * s2, p2), n1 = t5::mbar_test(b_xfull + 8 * s3, p3);
-                        __syncwarp();
+                        if (!(ready & 1)) t5::mbar_wait_bounded(b_afull + 8 * sa, (n / GM_SA) & 1, err_flag);
+                        if (!(ready & 2)) t5::mbar_wait_bounded(b_xfull + 8 * sx, px, err_flag);
+                        const uint32_t next = __ballot_sync(0xFFFFFFFFu, t5::mbar_test(lane == 0 ? b_afull + 8 * ((n + 1) % GM_SA) : b_xfull + 8 * (lane == 1 ? s2 : s3),
+                                                                                       lane == 0 ? ((n + 1) / GM_SA) & 1 : lane == 1 ? p2 : p3));
                         t5::fence_after();
                         const uint64_t x0 = gm_desc(x_addr(sx)), x1 = gm_desc(x_addr(s1));
                         if (t5::elect_one()) {
@@ -448,15 +451,16 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                             for (uint32_t kk = 0; kk < 4; kk++)  // 16 k are 32 bytes of the swizzled row
                                 gm_mma_pair(dcol, acol + kk * 8, x0 + kk * 2, idesc, kk ? 1u : su - it.k0);
                         }
-                        if (!r1) t5::mbar_wait_bounded(b_xfull + 8 * s1, p1, err_flag);
+                        if (!(ready & 4)) t5::mbar_wait_bounded(b_xfull + 8 * s1, p1, err_flag);
                         __syncwarp();
                         t5::fence_after();
                         if (t5::elect_one()) {
 #pragma unroll
                             for (uint32_t kk = 0; kk < 4; kk++) gm_mma_pair(dcol, acol + 32 + kk * 8, x1 + kk * 2, idesc, 1u);
                             t5::commit_pair(b_done + 8 * sa);
+                            if (deep) t5::commit_pair(b_xdone + 8 * (n % GM_XD));
                         }
-                        ra = na; r0 = n0; r1 = n1;
+                        ready = next;
                         sx = s2; px = p2;
                     }
                     if (t5::elect_one()) t5::commit_pair(b_dfull);
@@ -467,14 +471,15 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
         // =============================== activation loader ===============================
         const uint32_t full0 = t5::map_rank(b_xfull, 0);
         uint32_t sx = 0, h = 0;                            // h: activation stages so far, two per weight stage
-        auto wait_step = [&](uint32_t step) { t5::mbar_wait_bounded(b_done + 8 * (step % GM_SA), (step / GM_SA) & 1, err_flag); };
+        const uint32_t ring = deep ? GM_XD : GM_SA, b_step = deep ? b_xdone : b_done;
+        auto wait_step = [&](uint32_t step) { t5::mbar_wait_bounded(b_step + 8 * (step % ring), (step / ring) & 1, err_flag); };
         pdl_wait();
         for (uint32_t w = pair_id; w < n_items; w += n_pairs) {
             const GmItem it = gm_item(a, w);
             const int32_t t0 = (int32_t)(it.tt * a.nt + rank * (a.nt / 2));
             for (uint32_t sub = 0; sub < a.subs; sub++) {
                 for (uint32_t k = it.k0 * 128; k < it.k1 * 128; k += 64, h++) {
-                    if (h >= a.sx) wait_step((h - a.sx) / 2);  // at most GM_SA steps back: its barrier has not come round again
+                    if (h >= a.sx) wait_step((h - a.sx) / 2);  // at most `ring` stages back: its barrier has not come round again
                     if (rank == 0) t5::mbar_arrive_expect_tx(b_xfull + 8 * sx, 2 * xstage);
                     gm_tma_pair(x_addr(sx), &xmap, (int32_t)k, t0, full0 + 8 * sx);
                     if (++sx == a.sx) sx = 0;
@@ -482,7 +487,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
             }
         }
         // every copy in flight lands before the CTA leaves: a stage is done after its products
-        for (uint32_t step = h / 2 > (uint32_t)GM_SA ? h / 2 - GM_SA : 0; step < h / 2; step++) wait_step(step);
+        for (uint32_t step = h / 2 > ring ? h / 2 - ring : 0; step < h / 2; step++) wait_step(step);
     }
     t5::fence_before();
     __syncthreads();
