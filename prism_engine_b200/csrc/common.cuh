@@ -252,8 +252,7 @@ int launch_relay(prism_cuda_ctx *ctx, const uint8_t *payload_dev, uint32_t src_m
 int launch_unrelay(prism_cuda_ctx *ctx, const LutTensor &t, uint8_t *payload_dev);
 int launch_dequant(prism_cuda_ctx *ctx, const LutTensor &t, uint16_t *out_dev);
 int launch_synth(prism_cuda_ctx *ctx, LutTensor &t, uint64_t seed, float sigma, uint32_t row0, uint32_t col0);
-int launch_embed(prism_cuda_ctx *ctx, const LutTensor &t, const uint32_t *tokens_dev, uint32_t batch,
-                 uint16_t *out_dev, uint16_t *out2_dev);
+int launch_embed(prism_cuda_ctx *ctx, const LutTensor &t, const uint32_t *tokens_dev, uint32_t batch, uint16_t *out_dev);
 
 // gemv.cu
 enum GemvMode { GEMV_PLAIN = 0, GEMV_RESID = 1, GEMV_SWIGLU = 2, GEMV_F32 = 3, GEMV_TP = 4 };

@@ -186,7 +186,7 @@ static int enqueue_step(prism_cuda_engine *e) {
     const bool tp = e->T > 1;
     const bool fused = ctx->fuse != 0;
     const LutTensor &emb = ctx->tensors[e->embed];
-    PRISM_TRY(launch_embed(ctx, emb, e->tok, B, e->h, nullptr));
+    PRISM_TRY(launch_embed(ctx, emb, e->tok, B, e->h));
     uint32_t li = 0;
     for (uint32_t l = 0; l < c.num_layers; l++) {
         const LutTensor &tq = ctx->tensors[e->wq[l]], &tk = ctx->tensors[e->wk[l]], &tv = ctx->tensors[e->wv[l]],
@@ -450,7 +450,7 @@ static int prefill_portion(prism_cuda_engine *e, uint32_t b, uint32_t n_seq, uin
     const prism_model_config &c = e->cfg;
     const uint32_t H = e->H, wq = e->qd_l + 2 * e->kvd_l, R = n_seq * T;
     const float base = c.rope_use_theta ? c.rope_theta : 10000.0f;
-    PRISM_TRY(launch_embed(ctx, ctx->tensors[e->embed], toks, R, e->pf_x, nullptr));
+    PRISM_TRY(launch_embed(ctx, ctx->tensors[e->embed], toks, R, e->pf_x));
     for (uint32_t l = 0; l < c.num_layers; l++) {
         const LutTensor &tqkv = ctx->tensors[e->wqkv[l]], &to = ctx->tensors[e->wo[l]], &tg = ctx->tensors[e->wg[l]],
                         &tu = ctx->tensors[e->wu[l]], &td = ctx->tensors[e->wd[l]];
