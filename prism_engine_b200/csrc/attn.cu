@@ -9,8 +9,9 @@
 // share that KV head, so a cached row is read once per group instead of once per query head.  A WARP owns
 // every (warps of the cluster)-th tile of 16 positions: it copies the tile's keys and values into its own part
 // of shared memory (two tiles in flight), takes scores = K q^T (m16n8k16: 16 positions x 8 heads) and keeps
-// its own running maximum, sum and O^T = V^T p^T; the weights enter that product as two fp16 parts (22 bits of
-// the fp32 weight).  So no warp waits for another until the end, where every warp stores its maximum, sum and O
+// its own running maximum, sum and O^T = V^T p^T; the weights (at most 1) enter that product 2^15-fold as two fp16 parts:
+// 22 bits of the fp32 weight down to 2^-18 of the largest, below that to 2^-40 of it, so that keys beside one that takes
+// nearly all the weight keep theirs.  So no warp waits for another until the end, where every warp stores its maximum, sum and O
 // into the shared memory of the CTA that finishes those outputs, and ONE cluster barrier later they are merged in
 // a fixed order.
 // Bound: the latency of that chain (dependency wait, rotation, two products, merge) for the contexts of a chat, the
@@ -30,6 +31,7 @@ namespace prism {
 
 constexpr uint32_t FA_ROWS = 16;     // positions of a tile
 constexpr uint32_t FA_MAX_S = 16;    // CTAs of a cluster
+constexpr float FA_PARTS = 32768.0f; // weights, at most 1, times this are what the fp16 parts hold
 template <int HD>
 struct FaCfg {
     static constexpr int WARPS = HD == 256 ? 4 : 8;
@@ -126,11 +128,11 @@ __device__ __forceinline__ uint32_t fa_transpose(uint32_t v) {
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(r) : "r"(v));
     return r;
 }
-// Two weights as an fp16 pair and what that rounding left over as another.
+// Two weights, FA_PARTS-fold, as an fp16 pair and what that rounding left over as another.
 __device__ __forceinline__ void fa_split(float a, float b, uint32_t &hi, uint32_t &lo) {
-    const __half2 h = __floats2half2_rn(a, b);
+    const __half2 h = __floats2half2_rn(a * FA_PARTS, b * FA_PARTS);
     const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    const __half2 l = __floats2half2_rn(fmaf(a, FA_PARTS, -f.x), fmaf(b, FA_PARTS, -f.y));
     hi = *reinterpret_cast<const uint32_t *>(&h);
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(FaCfg<HD>::THREADS) attn_fused_kernel(const Fu
         for (int x = 16; x > 0; x >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, x);
         const float inv = 1.0f / (sum + 1e-10f);
         __syncwarp();
-        for (uint32_t e = lane; e < used; e += 32) wgt[e * 8 + hh] *= inv;
+        for (uint32_t e = lane; e < used; e += 32) wgt[e * 8 + hh] *= inv * (1.0f / FA_PARTS);
     }
     __syncthreads();
     const uint32_t own = rank * per < (uint32_t)MT ? min(per, MT - rank * per) : 0;
