@@ -10,8 +10,8 @@
 // every (warps of the cluster)-th tile of 16 positions: it copies the tile's keys and values into its own part
 // of shared memory (two tiles in flight), takes scores = K q^T (m16n8k16: 16 positions x 8 heads) and keeps
 // its own running maximum, sum and O^T = V^T p^T; the weights (at most 1) enter that product 2^15-fold as two fp16 parts:
-// 22 bits of the fp32 weight down to 2^-18 of the largest, below that to 2^-40 of it, so that keys beside one that takes
-// nearly all the weight keep theirs.  So no warp waits for another until the end, where every warp stores its maximum, sum and O
+// 21 bits of the fp32 weight down to 2^-18 of the largest, below that to 2^-38 of it, so that keys beside one that takes
+// nearly all the weight keep theirs, both positive, so that an infinite value stays one.  So no warp waits for another until the end, where every warp stores its maximum, sum and O
 // into the shared memory of the CTA that finishes those outputs, and ONE cluster barrier later they are merged in
 // a fixed order.
 // Bound: the latency of that chain (dependency wait, rotation, two products, merge) for the contexts of a chat, the
@@ -128,12 +128,20 @@ __device__ __forceinline__ uint32_t fa_transpose(uint32_t v) {
     asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(r) : "r"(v));
     return r;
 }
-// Two weights, FA_PARTS-fold, as an fp16 pair and what that rounding left over as another.
+// Two weights, FA_PARTS-fold, as an fp16 pair rounded down and what is left over as another.  Both parts of a positive weight
+// are positive (at least the smallest fp16 value, 2^-39 of the largest weight), so that an infinite value times the one and the
+// other has one sign and is no NaN.
 __device__ __forceinline__ void fa_split(float a, float b, uint32_t &hi, uint32_t &lo) {
-    const __half2 h = __floats2half2_rn(a * FA_PARTS, b * FA_PARTS);
+    a *= FA_PARTS;
+    b *= FA_PARTS;
+    const uint32_t least = (a > 0.0f ? 1u : 0u) | (b > 0.0f ? 0x10000u : 0u);
+    const __half2 floor2 = *reinterpret_cast<const __half2 *>(&least);
+    uint32_t d;
+    asm("cvt.rz.f16x2.f32 %0, %1, %2;\n" : "=r"(d) : "f"(b), "f"(a));  // the first source goes to the upper half
+    const __half2 h = *reinterpret_cast<const __half2 *>(&d);
     const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(fmaf(a, FA_PARTS, -f.x), fmaf(b, FA_PARTS, -f.y));
-    hi = *reinterpret_cast<const uint32_t *>(&h);
+    const __half2 l = __hmax2_nan(__floats2half2_rn(a - f.x, b - f.y), floor2), h1 = __hmax2_nan(h, floor2);
+    hi = *reinterpret_cast<const uint32_t *>(&h1);
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
@@ -300,10 +308,11 @@ __global__ void __launch_bounds__(FaCfg<HD>::THREADS) attn_fused_kernel(const Fu
 #pragma unroll
             for (int x = 4; x < 32; x <<= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, x));
             top = fmaxf(top, m[j]);
-            f[j] = exp2f(m[j] - top);
+            const float sub = top == -INFINITY ? 0.0f : top;  // nothing but scores of -inf so far: weights 0
+            f[j] = exp2f(m[j] - sub);
             m[j] = top;
-            w[j] = exp2f(w[j] - top);
-            w[2 + j] = exp2f(w[2 + j] - top);
+            w[j] = exp2f(w[j] - sub);
+            w[2 + j] = exp2f(w[2 + j] - sub);
             l[j] = l[j] * f[j] + (w[j] + w[2 + j]);
         }
         uint32_t hi[2], lo[2];

@@ -2,7 +2,8 @@
 heads attend to): the output is the sum of small weights.  Against the same attention in 64 bits on the rotated query.
 
 Tolerance: the rounding of the fp16 output (at most 2^-11 of a value, 2.8e-4 in the mean) is far above scores, sums and parts
-of weights, of which the parts resolve 2^-40 of the largest weight, 2^-14 of a weight at e^-18: 4e-4 of the norm."""
+of weights, of which the parts resolve 2^-38 of the largest weight, 2^-12 of a weight at e^-18 at most and a quarter of that
+in the mean: 4e-4 of the norm."""
 import numpy as np
 import pytest
 
