@@ -17,7 +17,10 @@
 //                         maximum in use.
 // Bound: the tensor core -- per 128 x 128 tile and 128-wide head three products of 2*128^3 flops, about 1 570 cycles,
 // against about 1 000 for the 16 384 exponentials.  Masked positions carry weight 0; value rows past the portion's
-// end (stale cache) are zeroed in shared memory before the product, so no stale NaN meets a zero weight.
+// end (stale cache) are zeroed in shared memory before the product, so no stale NaN meets a zero weight.  A value row of a later
+// token that overflowed still does, and an attended one meets the second part of its weight, which may be 0 or negative; scores of
+// -inf may leave a row's first tile without a maximum.  Each of these ends in a NaN or an infinity, and a row with one is taken again
+// position by position in fp32 over what it may see (pa_plain_row), so a later token's overflow stays out of earlier ones.
 // Measured, 28 query / 4 KV heads of 128: the attention of an 8190-token prompt through two layers took 128 ms with one
 // cluster of the decode kernel per token, on the CUDA cores; this kernel took 1.87 ms with a single issuing thread (descriptors
 // through vector registers), 1.38 with a whole warp walking the tiles.
@@ -53,6 +56,8 @@ struct PrefillAttnDev {
     const int32_t *page_tbl;
     uint32_t page_shift, tbl_stride;
     float scale2;                    // log2(e) / sqrt(head size)
+    const uint16_t *q, *kc, *vc;     // rotated queries (rows q_stride apart) and the cache, for the rows taken again
+    uint32_t q_stride;
     uint16_t *out;                   // [n_seq * T][nh * HD]
     unsigned int *err;
 };
@@ -93,10 +98,64 @@ __device__ __forceinline__ void pa_split(float a, float b, uint32_t &hi, uint32_
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
+// Row of the cache that holds position p of cache sequence c.
+__device__ __forceinline__ size_t pa_row(const PrefillAttnDev &a, uint32_t c, uint32_t p) {
+    if (!a.page_tbl) return (size_t)c * a.seq_rows + p;
+    return ((size_t)__ldg(a.page_tbl + (size_t)c * a.tbl_stride + (p >> a.page_shift)) << a.page_shift) + (p & ((1u << a.page_shift) - 1u));
+}
+// One token's output for one head by one warp, position by position in fp32: a lane takes the scores of every 32nd position and
+// HD / 32 columns.  About 20 instructions a position; only rows with infinities or NaN come here.
+template <int HD>
+__device__ __noinline__ void pa_plain_row(const PrefillAttnDev &a, uint32_t token, uint32_t cseq, uint32_t pos, uint32_t h, uint32_t lane) {
+    constexpr uint32_t VEC = HD / 32;
+    const uint32_t kh = h / a.group, kvd = a.nh / a.group * HD;
+    const uint16_t *q = a.q + (size_t)token * a.q_stride + (size_t)h * HD;
+    auto score = [&](uint32_t p) {
+        if (p > pos) return -INFINITY;
+        const uint4 *k = reinterpret_cast<const uint4 *>(a.kc + pa_row(a, cseq, p) * kvd + (size_t)kh * HD);
+        float d = 0.0f;
+#pragma unroll 2
+        for (uint32_t i = 0; i < HD / 8; i++) {
+            const uint4 qv = reinterpret_cast<const uint4 *>(q)[i], kv = k[i];
+            const uint32_t qw[4] = {qv.x, qv.y, qv.z, qv.w}, kw[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float2 x = __half22float2(*reinterpret_cast<const __half2 *>(&qw[j])), y = __half22float2(*reinterpret_cast<const __half2 *>(&kw[j]));
+                d += x.x * y.x;
+                d += x.y * y.y;
+            }
+        }
+        return d / sqrtf((float)HD);
+    };
+    float top = -INFINITY, sum = 0.0f;
+    for (uint32_t p = lane; p <= pos; p += 32) top = fmaxf(top, score(p));
+#pragma unroll
+    for (int x = 16; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, x));
+    for (uint32_t p = lane; p <= pos; p += 32) sum += expf(score(p) - top);
+#pragma unroll
+    for (int x = 16; x > 0; x >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, x);
+    const float inv = 1.0f / (sum + 1e-10f);
+    float acc[VEC];
+#pragma unroll
+    for (uint32_t i = 0; i < VEC; i++) acc[i] = 0.0f;
+    for (uint32_t p0 = 0; p0 <= pos; p0 += 32) {
+        const float mine = expf(score(p0 + lane) - top);
+        for (uint32_t j = 0; j < 32 && p0 + j <= pos; j++) {
+            const float e = __shfl_sync(0xFFFFFFFFu, mine, j);
+            const uint16_t *v = a.vc + pa_row(a, cseq, p0 + j) * kvd + (size_t)kh * HD + lane;
+#pragma unroll
+            for (uint32_t i = 0; i < VEC; i++) acc[i] += e * __half2float(__ushort_as_half(v[i * 32])) * inv;
+        }
+    }
+    uint16_t *dst = a.out + (size_t)token * a.nh * HD + (size_t)h * HD + lane;
+#pragma unroll
+    for (uint32_t i = 0; i < VEC; i++) dst[i * 32] = __half_as_ushort(__float2half_rn(acc[i]));
+}
+
 }  // namespace
 
 template <int HD>
-__global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(const PrefillAttnDev a, const __grid_constant__ CUtensorMap qmap,
+__global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(const __grid_constant__ PrefillAttnDev a, const __grid_constant__ CUtensorMap qmap,
                                                                              const __grid_constant__ CUtensorMap kmap,
                                                                              const __grid_constant__ CUtensorMap vmap) {
     using C = PaCfg<HD>;
@@ -208,6 +267,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
             const float inv = 1.0f / l;
             const uint32_t t = qb + q * 128 + row;
             uint16_t *dst = a.out + ((size_t)sq * a.T + t) * a.nh * HD + (size_t)h * HD;
+            float odd = 0.0f;  // NaN once an output was not finite
 #pragma unroll 1
             for (int c = 0; c < HD / 32; c++) {
                 uint32_t o[32];
@@ -216,8 +276,10 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
                 uint32_t p[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    const __half2 v = __floats2half2_rn(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
+                    const float x = __uint_as_float(o[2 * i]) * inv, y = __uint_as_float(o[2 * i + 1]) * inv;
+                    const __half2 v = __floats2half2_rn(x, y);
                     p[i] = *reinterpret_cast<const uint32_t *>(&v);
+                    odd = fmaf(x, 0.0f, fmaf(y, 0.0f, odd));
                 }
                 if (t < a.T) {
 #pragma unroll
@@ -225,6 +287,10 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
                         reinterpret_cast<uint4 *>(dst + c * 32)[i] = make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
                 }
                 __syncwarp();  // the next TMEM read takes the whole warp
+            }
+            for (uint32_t rows = __ballot_sync(0xFFFFFFFFu, t < a.T && odd != 0.0f); rows; rows &= rows - 1) {
+                const uint32_t r = __ffs(rows) - 1, tr = t - lane + r;
+                pa_plain_row<HD>(a, sq * a.T + tr, a.seq0 + sq, a.pos0 + tr, h, lane);
             }
         }
         t5::fence_before();
@@ -430,6 +496,7 @@ int launch_prefill_attn(prism_cuda_ctx *ctx, const PrefillAttn &a) {
     d.page_tbl = a.page_tbl; d.page_shift = a.page_shift; d.tbl_stride = a.tbl_stride;
     d.box = a.page_tbl ? std::min(128u, 1u << a.page_shift) : 128u;
     d.scale2 = 1.4426950408889634f / sqrtf((float)a.hd);
+    d.q = a.qkv; d.q_stride = a.stride; d.kc = a.kc; d.vc = a.vc;
     d.out = a.out; d.err = ctx->dev_err;
     switch (a.hd) {
     case 32: return launch_pa<32>(ctx, d, a);
