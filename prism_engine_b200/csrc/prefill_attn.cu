@@ -9,12 +9,12 @@
 //                         the softmax warps of one tile work, the tensor core has the other's products).  Keys and
 //                         values come by TMA, 128 positions a stage, straight from the cache (page by page when it is
 //                         paged).  S = Q K^T goes to TMEM; a thread owns one query row, so the softmax needs no
-//                         exchange; the weights go back to TMEM over the scores they came from, as TWO fp16 parts
-//                         (hi + lo: 22 bits of each weight, so nothing of the fp32 softmax is lost to the 16-bit
-//                         operand) and meet V, read from shared memory along its rows, in two products each.
-//                         The running maximum is only moved when it grows by more than 2^8: O is rescaled a few
-//                         times per row tile instead of at every key tile, and the sums stay exact relative to the
-//                         maximum in use.
+//                         exchange; the weights go back to TMEM over the scores they came from, 2^12-fold as TWO fp16
+//                         parts (22 bits of each weight down to 2^-15 of the maximum in use, below that to 2^-37 of it,
+//                         so that keys beside one that takes nearly all the weight keep theirs) and meet V, read from
+//                         shared memory along its rows, in two products each.
+//                         The running maximum is only moved when it grows by more than 2^3: O is rescaled a few
+//                         times per row tile instead of at every key tile, and a weight is at most 2^15 in the parts.
 // Bound: the tensor core -- per 128 x 128 tile and 128-wide head three products of 2*128^3 flops, about 1 570 cycles,
 // against about 1 000 for the 16 384 exponentials.  Masked positions carry weight 0; value rows past the portion's
 // end (stale cache) are zeroed in shared memory before the product, so no stale NaN meets a zero weight.  A value row of a later
@@ -34,6 +34,9 @@
 namespace prism {
 
 constexpr int PA_K = 128;  // keys of a stage
+// A score may lie PA_GROW (in powers of two) above the maximum in use before that is moved; the fp16 parts hold the weights times
+// PA_PARTS: at most 2^PA_GROW * PA_PARTS = 2^15.
+constexpr float PA_GROW = 3.0f, PA_PARTS = 4096.0f;
 template <int HD>
 struct PaCfg {
     static constexpr int QT = HD <= 128 ? 2 : 1;           // query tiles of 128 rows
@@ -89,11 +92,11 @@ __device__ __forceinline__ float pa_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
     return y;
 }
-// Two weights as an fp16 pair (first in the low half) and what that rounding left over as another.
+// Two weights, PA_PARTS-fold, as an fp16 pair (first in the low half) and what that rounding left over as another.
 __device__ __forceinline__ void pa_split(float a, float b, uint32_t &hi, uint32_t &lo) {
-    const __half2 h = __floats2half2_rn(a, b);
+    const __half2 h = __floats2half2_rn(a * PA_PARTS, b * PA_PARTS);
     const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    const __half2 l = __floats2half2_rn(fmaf(a, PA_PARTS, -f.x), fmaf(b, PA_PARTS, -f.y));
     hi = *reinterpret_cast<const uint32_t *>(&h);
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
                 for (int i = 1; i < 32; i++) mx[c] = fmaxf(mx[c], __uint_as_float(s[c][i]));
             }
             const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.scale2;
-            const bool grow = top > m + 8.0f;  // the first tile: m is -inf (every row sees its position 0)
+            const bool grow = top > m + PA_GROW;  // the first tile: m is -inf (every row sees its position 0)
             if (j == 0) {
                 m = top;
             } else if (__any_sync(0xFFFFFFFFu, grow)) {
@@ -264,7 +267,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
         if (n_kt[q]) {
             t5::mbar_wait_warp(b_ofull + 8 * q, 0, err_flag);
             t5::fence_after();
-            const float inv = 1.0f / l;
+            const float inv = 1.0f / (l * PA_PARTS);
             const uint32_t t = qb + q * 128 + row;
             uint16_t *dst = a.out + ((size_t)sq * a.T + t) * a.nh * HD + (size_t)h * HD;
             float odd = 0.0f;  // NaN once an output was not finite

@@ -108,3 +108,37 @@ def test_not_a_number(backend, what):
         got, want = _attend(backend, qkv, nh, nkv, hd, T)
         assert want.isnan().any() and want[:150].isfinite().all()
         _compare(got, want)
+
+
+@pytest.mark.parametrize("hd,nh,nkv", HEADS)
+def test_maximum_moves(backend, hd, nh, nkv):
+    """Keys that grow along the prompt, scores of tens of nats: the maximum moves in every key tile, in some rows of a warp by
+    more than the others, so sums and outputs of the tiles before are scaled down."""
+    import torch
+
+    T = 700
+    qkv = _inputs(nh, nkv, hd, T)
+    grow = (torch.arange(T, device="cuda")[:, None] / 64.0).exp2().clamp(max=30.0)
+    qkv[:, nh * hd:(nh + nkv) * hd] = (qkv[:, nh * hd:(nh + nkv) * hd].float() * grow).half()
+    _compare(*_attend(backend, qkv, nh, nkv, hd, T))
+
+
+@pytest.mark.parametrize("lead", [4.0, 10.0, 13.0, 16.0])
+@pytest.mark.parametrize("hd,nh,nkv", HEADS)
+def test_one_key_takes_the_weight_and_carries_nothing(backend, hd, nh, nkv, lead):
+    """The first position leads all scores by `lead` nats, its value row is zero: outputs are sums of weights of e^-lead.
+    The parts of a weight resolve 2^-37 of the largest weight, a seventh of TOL of a weight of e^-16."""
+    T = 700
+    qkv = _inputs(nh, nkv, hd, T)
+    c = hd // 2 - 1  # turns slowly
+    q, k = qkv[:, :nh * hd].view(T, nh, hd), qkv[:, nh * hd:(nh + nkv) * hd].view(T, nkv, hd)
+    q *= 0.25
+    q[:, :, c], q[:, :, c + hd // 2] = 4.0, 0.0
+    k[:, :, c], k[:, :, c + hd // 2] = 0.0, 0.0
+    k[0] = 0.0
+    k[0, :, c] = lead / 4.0 * hd ** 0.5
+    v = qkv[:, (nh + nkv) * hd:]
+    v *= 4096.0
+    v[0] = 0.0
+    got, want = _attend(backend, qkv, nh, nkv, hd, T, rope_k=0)
+    _compare(got[1:], want[1:])
