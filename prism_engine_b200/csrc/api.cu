@@ -42,13 +42,13 @@ struct CudaScratchAlloc {
 
 // Grows one of the context's scratch buffers to `want` elements.  Pointer and element count are
 // written back whatever happens: after a failed allocation both are zero, never a stale size
-// beside a null pointer.
+// beside a null pointer.  `in_steps`: kernels of a decode step use the buffer.
 template <typename T>
-static int grow(prism_cuda_ctx *ctx, T **p, size_t *have, size_t want, bool *grew = nullptr) {
+static int grow(prism_cuda_ctx *ctx, T **p, size_t *have, size_t want, bool in_steps, bool *grew = nullptr) {
     GrowBuf b{*p, *have};
     CudaScratchAlloc al{ctx};
     const int rc = grow_buf(al, b, want, sizeof(T), grew);
-    if (b.ptr != *p) ctx->option_epoch++;  // a captured step that holds the old buffer is captured again
+    if (in_steps && b.ptr != *p) ctx->option_epoch++;  // a captured step that holds the old buffer is captured again
     *p = static_cast<T *>(b.ptr);
     *have = b.count;
     if (rc) {
@@ -59,23 +59,23 @@ static int grow(prism_cuda_ctx *ctx, T **p, size_t *have, size_t want, bool *gre
 }
 
 int ensure_stage(prism_cuda_ctx *ctx, size_t in_bytes, size_t out_bytes) {
-    PRISM_TRY(grow(ctx, &ctx->stage_in, &ctx->stage_in_bytes, in_bytes));
-    return grow(ctx, &ctx->stage_out, &ctx->stage_out_bytes, out_bytes);
+    PRISM_TRY(grow(ctx, &ctx->stage_in, &ctx->stage_in_bytes, in_bytes, false));
+    return grow(ctx, &ctx->stage_out, &ctx->stage_out_bytes, out_bytes, false);
 }
 
 int ensure_splitk(prism_cuda_ctx *ctx, size_t floats, size_t counters) {
-    PRISM_TRY(grow(ctx, &ctx->splitk_partials, &ctx->splitk_floats, floats));
+    PRISM_TRY(grow(ctx, &ctx->splitk_partials, &ctx->splitk_floats, floats, true));
     bool grew = false;
-    PRISM_TRY(grow(ctx, &ctx->splitk_counters, &ctx->splitk_counter_n, counters, &grew));
+    PRISM_TRY(grow(ctx, &ctx->splitk_counters, &ctx->splitk_counter_n, counters, true, &grew));
     // arrival counters start at zero; each kernel leaves them at zero again
     if (grew)
         PRISM_CUDA_TRY(ctx, cudaMemsetAsync(ctx->splitk_counters, 0, ctx->splitk_counter_n * sizeof(unsigned int), ctx->stream));
     return PRISM_OK;
 }
 
-int ensure_act(prism_cuda_ctx *ctx, size_t halfs) { return grow(ctx, &ctx->act_scratch, &ctx->act_halfs, halfs); }
+int ensure_act(prism_cuda_ctx *ctx, size_t halfs) { return grow(ctx, &ctx->act_scratch, &ctx->act_halfs, halfs, true); }
 
-int ensure_tmp(prism_cuda_ctx *ctx, size_t halfs) { return grow(ctx, &ctx->tmp_scratch, &ctx->tmp_halfs, halfs); }
+int ensure_tmp(prism_cuda_ctx *ctx, size_t halfs) { return grow(ctx, &ctx->tmp_scratch, &ctx->tmp_halfs, halfs, true); }
 
 int check_device_error(prism_cuda_ctx *ctx) {
     unsigned int v = 0;

@@ -374,9 +374,9 @@ int run_step(prism_cuda_engine *e) {
             e->graph = nullptr;
         }
         e->graph_batch = e->batch;
-        e->graph_epoch = ctx->option_epoch;
         const uint64_t l0 = ctx->launches;
         PRISM_TRY(enqueue_step(e));
+        e->graph_epoch = ctx->option_epoch;  // now: scratch that this step had to grow is what the captured one will use
         e->kernels_per_step = (uint32_t)(ctx->launches - l0);
         return PRISM_OK;
     }
