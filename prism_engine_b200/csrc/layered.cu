@@ -350,6 +350,11 @@ static int build_layer(prism_cuda_engine *e, uint32_t i, const prism_layer_confi
     return PRISM_OK;
 }
 
+// Pinned words of a step of n rows: slots, positions, tokens; greedy tokens, the device error word; then the logits of its
+// rows.  At most 16 MB stay with the model; logits that do not fit are copied to the caller's memory directly.
+constexpr size_t STEP_HOST_MAX = 4u << 20;
+static size_t step_host_words(size_t n) { return 4 * n + 4; }
+
 static int build_model(prism_cuda_engine *e, const prism_layer_config *layers) {
     LayeredModel *m = e->lm;
     const prism_layered_config &c = m->c;
@@ -434,6 +439,16 @@ static int build_model(prism_cuda_engine *e, const prism_layer_config *layers) {
         PRISM_TRY(model_alloc(e, m->rows_scratch.ml, ml * m->rows_scratch.rows_cap));
     }
     m->slot_pos.assign(c.max_batch, -1);
+    // Once, here: allocated by the first decode step it took 2 to 4 ms of that call, and up to 80 on a busy host.
+    const size_t least = step_host_words(c.max_batch);
+    size_t words = std::max(least, std::min(least + (size_t)c.max_batch * c.vocab, STEP_HOST_MAX));
+    if (cudaHostAlloc((void **)&m->host, words * 4, cudaHostAllocDefault) != cudaSuccess) {
+        (void)cudaGetLastError();
+        m->host = nullptr;
+        words = least;
+        PRISM_CUDA_TRY(e->ctx, cudaHostAlloc((void **)&m->host, words * 4, cudaHostAllocDefault));
+    }
+    m->host_n = words;
     PRISM_CUDA_TRY(e->ctx, cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking));
     PRISM_CUDA_TRY(e->ctx, cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming));
     PRISM_CUDA_TRY(e->ctx, cudaEventCreateWithFlags(&m->join, cudaEventDisableTiming));
@@ -868,22 +883,6 @@ __global__ void step_begin_kernel(const uint32_t *__restrict__ host, uint32_t n,
     }
     if (threadIdx.x < 3) scalars[threadIdx.x] = 0;
 }
-// Pinned words of a step of n rows: slots, positions, tokens; greedy tokens, the device error word; logits of the rows.
-// At most 16 MB stay with the model; the logits of larger steps are copied to the caller's memory directly.
-constexpr size_t STEP_HOST_MAX = 4u << 20;
-static int step_host(prism_cuda_engine *e, size_t n, bool with_logits, bool *logits_fit) {
-    LayeredModel *m = e->lm;
-    const size_t small = 4 * n + 4, all = small + n * m->c.vocab;
-    *logits_fit = with_logits && all <= STEP_HOST_MAX;
-    const size_t want = *logits_fit ? all : small;
-    if (want <= m->host_n) return PRISM_OK;
-    cudaFreeHost(m->host);  // no step is at work: every call waits for its own
-    m->host = nullptr;
-    m->host_n = 0;
-    PRISM_CUDA_TRY(e->ctx, cudaHostAlloc((void **)&m->host, want * 4, cudaHostAllocDefault));
-    m->host_n = want;
-    return PRISM_OK;
-}
 // One step of the rows in m->host, up to the copies back; nothing is waited for.
 static int step_rows(prism_cuda_engine *e, uint32_t n, bool logits) {
     prism_cuda_ctx *ctx = e->ctx;
@@ -894,7 +893,7 @@ static int step_rows(prism_cuda_engine *e, uint32_t n, bool logits) {
     PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(m->host + 3 * n, e->next, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(m->host + 4 * n, ctx->dev_err, 4, cudaMemcpyDeviceToHost, ctx->stream));
     if (!logits) return PRISM_OK;
-    PRISM_CUDA_TRY(ctx, cudaMemcpy2DAsync(m->host + 4 * n + 4, (size_t)m->c.vocab * 4, m->logits, (size_t)m->vocab_pad * 4, (size_t)m->c.vocab * 4, n,
+    PRISM_CUDA_TRY(ctx, cudaMemcpy2DAsync(m->host + step_host_words(n), (size_t)m->c.vocab * 4, m->logits, (size_t)m->vocab_pad * 4, (size_t)m->c.vocab * 4, n,
                                           cudaMemcpyDeviceToHost, ctx->stream));
     return PRISM_OK;
 }
@@ -1140,9 +1139,9 @@ int prism_cuda_engine_extend(prism_cuda_engine *e, uint32_t n, const uint32_t *s
         if (n_tokens[i] == 1) one.push_back(i);
     if (!one.empty()) {
         const size_t B = one.size();
-        bool wanted = false, fit = false;
+        bool wanted = false;
         for (uint32_t i : one) wanted = wanted || (n_want && n_want[i]);
-        PRISM_TRY(step_host(e, B, wanted, &fit));
+        const bool fit = wanted && step_host_words(B) + B * m->c.vocab <= m->host_n;
         for (size_t r = 0; r < B; r++) {
             const uint32_t i = one[r];
             m->host[r] = seqs[i];
@@ -1165,7 +1164,7 @@ int prism_cuda_engine_extend(prism_cuda_engine *e, uint32_t n, const uint32_t *s
             const uint32_t i = one[r];
             m->slot_pos[seqs[i]] += 1;
             for (uint32_t k = 0; fit && n_want && k < n_want[i]; k++)
-                memcpy(logits + (want0[i] + k) * m->c.vocab, m->host + 4 * B + 4 + r * m->c.vocab, (size_t)m->c.vocab * 4);
+                memcpy(logits + (want0[i] + k) * m->c.vocab, m->host + step_host_words(B) + r * m->c.vocab, (size_t)m->c.vocab * 4);
             if (next_tokens) next_tokens[i] = m->host[3 * B + r];
         }
         if (B == n) return device_error_result(ctx, m->host[4 * B]);

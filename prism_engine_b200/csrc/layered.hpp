@@ -88,7 +88,7 @@ struct LayeredModel {
     bf16 *ex_lat = nullptr, *ex_krot = nullptr, *ex_kv = nullptr;
     size_t ex_lat_n = 0, ex_krot_n = 0, ex_kv_n = 0;
     int32_t *row_slot = nullptr, *row_pos = nullptr;
-    uint32_t *host = nullptr;                      // pinned: what a step of extend() takes in and gives back (see step_host)
+    uint32_t *host = nullptr;                      // pinned: what a step of extend() takes in and gives back (step_host_words)
     size_t host_n = 0;                             // its words
     std::vector<int64_t> slot_pos;                 // tokens a slot holds; -1: free
     std::vector<void *> allocs;                    // everything above that lives as long as the model
