@@ -350,8 +350,8 @@ static int build_layer(prism_cuda_engine *e, uint32_t i, const prism_layer_confi
     return PRISM_OK;
 }
 
-// Pinned words of a step of n rows: slots, positions, tokens; greedy tokens, the device error word; then the logits of its
-// rows.  At most 16 MB stay with the model; logits that do not fit are copied to the caller's memory directly.
+// Pinned words of a step of n rows: slots, positions, tokens; greedy tokens, the device error word; then the logits of the
+// rows that want them.  At most 16 MB stay with the model; logits that do not fit are copied to the caller's memory directly.
 constexpr size_t STEP_HOST_MAX = 4u << 20;
 static size_t step_host_words(size_t n) { return 4 * n + 4; }
 
@@ -883,8 +883,8 @@ __global__ void step_begin_kernel(const uint32_t *__restrict__ host, uint32_t n,
     }
     if (threadIdx.x < 3) scalars[threadIdx.x] = 0;
 }
-// One step of the rows in m->host, up to the copies back; nothing is waited for.
-static int step_rows(prism_cuda_engine *e, uint32_t n, bool logits) {
+// One step of the rows in m->host, up to the copies back, with the logits of the rows `want` (ascending); nothing is waited for.
+static int step_rows(prism_cuda_engine *e, uint32_t n, const std::vector<uint32_t> &want) {
     prism_cuda_ctx *ctx = e->ctx;
     LayeredModel *m = e->lm;
     step_begin_kernel<<<1, 64, 0, ctx->stream>>>(m->host, n, m->row_slot, m->row_pos, e->tok, e->scalars);
@@ -892,9 +892,11 @@ static int step_rows(prism_cuda_engine *e, uint32_t n, bool logits) {
     PRISM_TRY(run_step(e));
     PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(m->host + 3 * n, e->next, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(m->host + 4 * n, ctx->dev_err, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (!logits) return PRISM_OK;
-    PRISM_CUDA_TRY(ctx, cudaMemcpy2DAsync(m->host + step_host_words(n), (size_t)m->c.vocab * 4, m->logits, (size_t)m->vocab_pad * 4, (size_t)m->c.vocab * 4, n,
-                                          cudaMemcpyDeviceToHost, ctx->stream));
+    for (size_t i = 0, run; i < want.size(); i += run) {  // neighbouring rows in one copy
+        for (run = 1; i + run < want.size() && want[i + run] == want[i] + run;) run++;
+        PRISM_CUDA_TRY(ctx, cudaMemcpy2DAsync(m->host + step_host_words(n) + i * m->c.vocab, (size_t)m->c.vocab * 4, m->logits + (size_t)want[i] * m->vocab_pad,
+                                              (size_t)m->vocab_pad * 4, (size_t)m->c.vocab * 4, run, cudaMemcpyDeviceToHost, ctx->stream));
+    }
     return PRISM_OK;
 }
 int layered_set_rows(prism_cuda_engine *e, uint32_t pos) {
@@ -1139,9 +1141,10 @@ int prism_cuda_engine_extend(prism_cuda_engine *e, uint32_t n, const uint32_t *s
         if (n_tokens[i] == 1) one.push_back(i);
     if (!one.empty()) {
         const size_t B = one.size();
-        bool wanted = false;
-        for (uint32_t i : one) wanted = wanted || (n_want && n_want[i]);
-        const bool fit = wanted && step_host_words(B) + B * m->c.vocab <= m->host_n;
+        std::vector<uint32_t> wanted;              // rows with logits to give back
+        for (size_t r = 0; r < B; r++)
+            if (n_want && n_want[one[r]]) wanted.push_back((uint32_t)r);
+        const bool fit = step_host_words(B) + wanted.size() * m->c.vocab <= m->host_n;
         for (size_t r = 0; r < B; r++) {
             const uint32_t i = one[r];
             m->host[r] = seqs[i];
@@ -1149,12 +1152,12 @@ int prism_cuda_engine_extend(prism_cuda_engine *e, uint32_t n, const uint32_t *s
             m->host[2 * B + r] = tokens[tok0[i]];
         }
         e->batch = (uint32_t)B;
-        const int rc = step_rows(e, (uint32_t)B, fit);
+        const int rc = step_rows(e, (uint32_t)B, fit ? wanted : std::vector<uint32_t>());
         cudaError_t ce = cudaSuccess;
-        if (rc == PRISM_OK && wanted && !fit)
-            for (size_t r = 0; r < B; r++)
+        if (rc == PRISM_OK && !fit)
+            for (uint32_t r : wanted)
                 for (uint32_t k = 0; k < n_want[one[r]] && ce == cudaSuccess; k++)
-                    ce = cudaMemcpyAsync(logits + (want0[one[r]] + k) * m->c.vocab, m->logits + r * m->vocab_pad, (size_t)m->c.vocab * 4,
+                    ce = cudaMemcpyAsync(logits + (want0[one[r]] + k) * m->c.vocab, m->logits + (size_t)r * m->vocab_pad, (size_t)m->c.vocab * 4,
                                          cudaMemcpyDeviceToHost, ctx->stream);
         const cudaError_t se = cudaStreamSynchronize(ctx->stream);  // also after a failure: the step may still read the pinned words
         PRISM_TRY(rc);
@@ -1163,9 +1166,12 @@ int prism_cuda_engine_extend(prism_cuda_engine *e, uint32_t n, const uint32_t *s
         for (size_t r = 0; r < B; r++) {
             const uint32_t i = one[r];
             m->slot_pos[seqs[i]] += 1;
-            for (uint32_t k = 0; fit && n_want && k < n_want[i]; k++)
-                memcpy(logits + (want0[i] + k) * m->c.vocab, m->host + step_host_words(B) + r * m->c.vocab, (size_t)m->c.vocab * 4);
             if (next_tokens) next_tokens[i] = m->host[3 * B + r];
+        }
+        for (size_t j = 0; fit && j < wanted.size(); j++) {
+            const uint32_t i = one[wanted[j]];
+            for (uint32_t k = 0; k < n_want[i]; k++)
+                memcpy(logits + (want0[i] + k) * m->c.vocab, m->host + step_host_words(B) + j * m->c.vocab, (size_t)m->c.vocab * 4);
         }
         if (B == n) return device_error_result(ctx, m->host[4 * B]);
     }

@@ -42,3 +42,29 @@ def test_second_layered_step_is_captured(batch):
         n = _launches(be, lambda i: eng.extend([(s, np.array([5 + i], np.uint32), [0]) for s in seqs]), 4)
         assert n[1] == n[2] == n[3] < n[0], n
         eng.close()
+
+
+def test_logits_of_the_rows_that_want_them(backend):
+    """Steps of several rows of which some want logits, once or twice, alone or side by side, and a step whose logits are more
+    than the model's pinned memory: what each row gets is what it gets alone with all rows wanting."""
+    for vocab in (256, 900000):
+        cfg = u.model([u.lightning(2, 64, 64, ff=128)], width=128, vocab=vocab)
+        eng = u.engine(backend, cfg, u.weights(cfg, seed=1), dtype="bfloat16", max_seq=16, max_batch=6)
+        tokens = [np.array([7 + 3 * i], np.uint32) for i in range(6)]
+
+        def step(wants):
+            seqs = [eng.open_sequence() for _ in range(6)]
+            out = eng.extend([(s, t, w) for s, t, w in zip(seqs, tokens, wants)])
+            for s in seqs:
+                eng.close_sequence(s)
+            return out
+
+        alone = [step([[0] if i == j else [] for i in range(6)])[0] for j in range(6)]
+        assert not np.array_equal(alone[0], alone[1])
+        for wants in ([1, 1, 1, 1, 1, 1], [0, 1, 2, 0, 0, 1], [0, 0, 0, 0, 2, 1], [0, 0, 0, 0, 0, 0]):
+            got = step([[0] * n for n in wants])
+            rows = [j for j, n in enumerate(wants) for _ in range(n)]
+            assert len(got) == len(rows)
+            for g, j in zip(got, rows):
+                assert np.array_equal(g, alone[j]), (vocab, wants, j)
+        eng.close()
