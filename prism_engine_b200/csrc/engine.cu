@@ -13,6 +13,7 @@
 
 #include "../../include/prism_cuda_bench.h"
 #include "engine.hpp"
+#include "scratch.hpp"
 
 namespace prism {
 
@@ -140,7 +141,7 @@ static int linear(prism_cuda_engine *e, GemvMode mode, const LutTensor &t, const
         PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(y, e->gu, (size_t)B * t.m * 2, cudaMemcpyDeviceToDevice, ctx->stream));
         return PRISM_OK;
     }
-    return launch_gemm_swiglu(ctx, t, *t2, x, B, y, e->gu, e->gu + (size_t)B * t.m);
+    return launch_gemm_swiglu(ctx, t, *t2, x, B, y, e->gu);
 }
 
 // Rope(q), Rope(k), KV append and Attention of layer l (cache slot li): one fused kernel when the
@@ -424,22 +425,30 @@ static int ensure_prefill(prism_cuda_engine *e, uint32_t T) {
     if (T <= e->pf_cap) return PRISM_OK;
     prism_cuda_ctx *ctx = e->ctx;
     PRISM_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    void **ptrs[] = {(void **)&e->pf_x, (void **)&e->pf_xn, (void **)&e->pf_qkv, (void **)&e->pf_att, (void **)&e->pf_g,
-                     (void **)&e->pf_u, (void **)&e->pf_act};
+    void **ptrs[] = {(void **)&e->pf_x, (void **)&e->pf_xn, (void **)&e->pf_qkv, (void **)&e->pf_att, (void **)&e->pf_act};
     for (void **p : ptrs) {
         cudaFree(*p);
         *p = nullptr;
     }
     e->pf_cap = 0;
     const uint32_t wq = e->qd_l + 2 * e->kvd_l;
-    const size_t wide = std::max<size_t>(e->I_l, e->H);
-    const size_t bytes[] = {(size_t)T * e->H * 2, (size_t)T * e->H * 2, (size_t)T * wq * 2, (size_t)T * e->qd_l * 2,
-                            (size_t)T * wide * 2, (size_t)T * wide * 2, (size_t)T * wide * 2};
+    const size_t bytes[] = {(size_t)T * e->H * 2, (size_t)T * e->H * 2, (size_t)T * wq * 2, (size_t)T * e->qd_l * 2, (size_t)T * e->I_l * 2};
     for (size_t i = 0; i < sizeof(ptrs) / sizeof(ptrs[0]); i++) {
         cudaError_t ce = cudaMalloc(ptrs[i], (bytes[i] + 255) / 256 * 256);
         if (ce != cudaSuccess) return cuda_fail(ctx, ce, "cudaMalloc(prefill scratch)");
     }
     e->pf_cap = T;
+    return PRISM_OK;
+}
+// Rows of up where gate and up do not go through one kernel: few rows, or shapes that take the GEMV.
+static int ensure_prefill_up(prism_cuda_engine *e, uint32_t T) {
+    if (T <= e->pf_up_cap) return PRISM_OK;
+    PRISM_CUDA_TRY(e->ctx, cudaStreamSynchronize(e->ctx->stream));
+    cudaFree(e->pf_u);
+    e->pf_u = nullptr;
+    e->pf_up_cap = 0;
+    PRISM_CUDA_TRY(e->ctx, cudaMalloc((void **)&e->pf_u, (size_t)T * e->I_l * 2));
+    e->pf_up_cap = T;
     return PRISM_OK;
 }
 
@@ -467,10 +476,14 @@ static int prefill_portion(prism_cuda_engine *e, uint32_t b, uint32_t n_seq, uin
         pa.rope_k = c.rope_k; pa.rope_base = base;
         pa.page_tbl = e->page_tbl; pa.page_shift = e->page_shift; pa.tbl_stride = e->pages_per_seq;
         PRISM_TRY(launch_prefill_attn(ctx, pa));
-        PRISM_TRY(launch_gemm_add(ctx, to, e->pf_att, R, e->pf_x, e->pf_g));  // h = f16(o + hr)
+        // pf_xn has been read when o, and again when down, may need rows for a product of their own
+        PRISM_TRY(launch_gemm_add(ctx, to, e->pf_att, R, e->pf_x, e->pf_xn));  // h = f16(o + hr)
         PRISM_TRY(launch_rms_norm(ctx, e->pf_x, e->pf_xn, H, c.norm_eps, R));
-        PRISM_TRY(launch_gemm_swiglu(ctx, tg, tu, e->pf_xn, R, e->pf_act, e->pf_g, e->pf_u));
-        PRISM_TRY(launch_gemm_add(ctx, td, e->pf_act, R, e->pf_x, e->pf_g));  // h = f16(d + hr)
+        bool fused = false;
+        PRISM_TRY(gemm_swiglu_fused(ctx, tg, tu, R, &fused));
+        if (!fused) PRISM_TRY(ensure_prefill_up(e, R));
+        PRISM_TRY(launch_gemm_swiglu(ctx, tg, tu, e->pf_xn, R, e->pf_act, e->pf_u));
+        PRISM_TRY(launch_gemm_add(ctx, td, e->pf_act, R, e->pf_x, e->pf_xn));  // h = f16(d + hr)
     }
     return PRISM_OK;
 }
@@ -483,14 +496,11 @@ static int prefill_portion(prism_cuda_engine *e, uint32_t b, uint32_t n_seq, uin
 static int prefill_batched(prism_cuda_engine *e, uint32_t batch, uint32_t n_prompt) {
     prism_cuda_ctx *ctx = e->ctx;
     uint32_t rows = ctx->prefill_chunk > 0 ? (uint32_t)ctx->prefill_chunk : 2048u;
-    const auto most = [&] { return (uint32_t)std::min<uint64_t>(rows, (uint64_t)batch * n_prompt); };
-    int rc = ensure_prefill(e, most());
-    while (rc != PRISM_OK && ctx->prefill_chunk < 0 && rows > 512) {  // too large for what memory is left: smaller portions
-        cudaGetLastError();
-        rows /= 2;
-        rc = ensure_prefill(e, most());
-    }
-    PRISM_TRY(rc);
+    // too large for what memory is left: smaller portions, down to one prompt at a time
+    PRISM_TRY(fit_rows(rows, std::min(std::min(rows, 512u), n_prompt), [&](uint32_t n) {
+        (void)cudaGetLastError();
+        return ensure_prefill(e, (uint32_t)std::min<uint64_t>(n, (uint64_t)batch * n_prompt));
+    }));
     if (n_prompt <= rows) {
         const uint32_t fit = rows / n_prompt, portions = (batch + fit - 1) / fit, per = (batch + portions - 1) / portions;
         for (uint32_t b = 0; b < batch; b += per)
@@ -621,7 +631,7 @@ int prism_cuda_engine_create(prism_cuda_ctx *ctx, const prism_model_config *cfg,
     ALLOC(e->h, (size_t)B * e->H * 2);
     ALLOC(e->xn, (size_t)B * e->H * 2);
     ALLOC(e->qkv, (size_t)B * e->qkv_stride * 2);
-    if (B >= 8) ALLOC(e->gu, 2 * (size_t)B * std::max(e->act_stride, e->H) * 2);
+    if (B >= 8) ALLOC(e->gu, (size_t)B * std::max(e->act_stride, e->H) * 2);
     ALLOC(e->att, (size_t)B * e->qd_l * 2);
     ALLOC(e->act, (size_t)B * e->act_stride * 2);
     ALLOC(e->logits, (size_t)B * round_up_u32(e->V_l, 8) * 2);
@@ -662,7 +672,7 @@ void prism_cuda_engine_destroy(prism_cuda_engine *e) {
     if (e->lm) layered_destroy(e);
     for (int32_t h : e->wqkv)
         if (h >= 0) prism_cuda_free_tensor(e->ctx, h);
-    void *ptrs[] = {e->page_tbl, e->pf_x, e->pf_xn, e->pf_qkv, e->pf_att, e->pf_g, e->pf_u, e->pf_act, e->gu, e->h, e->xn, e->qkv, e->att, e->act, e->logits, e->part, e->tok, e->next,
+    void *ptrs[] = {e->page_tbl, e->pf_x, e->pf_xn, e->pf_qkv, e->pf_att, e->pf_u, e->pf_act, e->gu, e->h, e->xn, e->qkv, e->att, e->act, e->logits, e->part, e->tok, e->next,
                     e->out_tokens, e->prompts, e->pairs_send, e->pairs_recv, e->scalars, e->kc, e->vc};
     for (void *p : ptrs) cudaFree(p);
     if (e->ev0) cudaEventDestroy(e->ev0);

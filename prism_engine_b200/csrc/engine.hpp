@@ -44,9 +44,8 @@ struct prism_cuda_engine {
     std::vector<uint32_t> seq_pages;         // pages each sequence holds
     uint32_t page_shift = 0, pages_per_seq = 0, pool_pages = 0;
     // batched prefill scratch (one portion of prompt tokens), grown on demand
-    uint16_t *pf_x = nullptr, *pf_xn = nullptr, *pf_qkv = nullptr, *pf_att = nullptr, *pf_g = nullptr, *pf_u = nullptr,
-             *pf_act = nullptr;
-    uint32_t pf_cap = 0;         // tokens the buffers hold
+    uint16_t *pf_x = nullptr, *pf_xn = nullptr, *pf_qkv = nullptr, *pf_att = nullptr, *pf_u = nullptr, *pf_act = nullptr;
+    uint32_t pf_cap = 0, pf_up_cap = 0;  // tokens the buffers hold; those of pf_u
     cudaGraphExec_t graph = nullptr;
     uint32_t graph_batch = 0;
     uint64_t graph_epoch = ~0ull;  // option epoch of the context when the graph (or its eager warm-up) was made

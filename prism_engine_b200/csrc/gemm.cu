@@ -23,14 +23,18 @@ int launch_gemm_add(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, 
     return launch_vec_add(ctx, h, tmp, m_tok * t.m);
 }
 
-int launch_gemm_swiglu(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, uint16_t *g, uint16_t *u) {
-    bool done = false;
-    if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, tg, m_tok) && gemm_tc5_eligible(ctx, tu, m_tok) && tg.bits == tu.bits)
-        PRISM_TRY(launch_swiglu_tc5(ctx, tg, tu, X, m_tok, act, &done));
-    if (done) return PRISM_OK;
-    PRISM_TRY(launch_gemm(ctx, tg, X, m_tok, g));
+int gemm_swiglu_fused(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, uint32_t m_tok, bool *fused) {
+    *fused = false;
+    if (ctx->gemm_variant != 1 || !gemm_tc5_eligible(ctx, tg, m_tok) || !gemm_tc5_eligible(ctx, tu, m_tok) || tg.bits != tu.bits) return PRISM_OK;
+    return swiglu_tc5_pays(ctx, tg, m_tok, fused);
+}
+int launch_gemm_swiglu(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, uint16_t *u) {
+    bool fused = false;
+    PRISM_TRY(gemm_swiglu_fused(ctx, tg, tu, m_tok, &fused));
+    if (fused) return launch_swiglu_tc5(ctx, tg, tu, X, m_tok, act);
+    PRISM_TRY(launch_gemm(ctx, tg, X, m_tok, act));
     PRISM_TRY(launch_gemm(ctx, tu, X, m_tok, u));
-    return launch_silu_mul(ctx, act, g, u, m_tok * tg.m);
+    return launch_silu_mul(ctx, act, act, u, m_tok * tg.m);
 }
 
 }  // namespace prism

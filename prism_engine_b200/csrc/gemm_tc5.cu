@@ -621,24 +621,29 @@ int launch_gemm_tc5(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, 
     return t.bits == 2 ? gemm_bits<2>(ctx, t, X, m_tok, Y, resid) : gemm_bits<4>(ctx, t, X, m_tok, Y, resid);
 }
 
-// Gate and up of a tile one after the other by the same CTA, whose threads meet their own gate values again, unless the
-// tiles are so few that two launches with K cut into ranges and a pass over their outputs take less.
+// Gate and up of a tile one after the other by the same CTA, whose threads meet their own gate values again.
 template <int BITS>
-static int swiglu_bits(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, bool *done) {
+static int swiglu_bits(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act) {
     uint32_t pairs = 0;
     PRISM_TRY(gm_pairs<BITS>(ctx, &pairs));
     GemmArgs a = gm_args(ctx, tg, m_tok, act);
-    const GmPlan both = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 2, 1), one = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 1, GM_MAX_SPLITS);
-    *done = both.cycles <= 2 * one.cycles + 4000.0 + (double)m_tok * tg.m * 8.0 / 3500.0;
-    if (!*done) return PRISM_OK;
     a.idx2 = tu.idx; a.pal2 = tu.pal;
     a.subs = 2;
     a.mode = GM_SWIGLU;
-    return launch_gm<BITS>(ctx, a, tg, X, both, pairs);
+    return launch_gm<BITS>(ctx, a, tg, X, gm_plan(pairs, a.n_rp, a.n_st, m_tok, 2, 1), pairs);
 }
-int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, bool *done) {
+int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act) {
     if (reinterpret_cast<uintptr_t>(X) & 15) return fail(ctx, PRISM_E_ARG, "gemm: X must be 16-byte aligned");
-    return tg.bits == 2 ? swiglu_bits<2>(ctx, tg, tu, X, m_tok, act, done) : swiglu_bits<4>(ctx, tg, tu, X, m_tok, act, done);
+    return tg.bits == 2 ? swiglu_bits<2>(ctx, tg, tu, X, m_tok, act) : swiglu_bits<4>(ctx, tg, tu, X, m_tok, act);
+}
+// Whether that pays: tiles may be so few that two launches with K cut into ranges and a pass over their outputs take less.
+int swiglu_tc5_pays(prism_cuda_ctx *ctx, const LutTensor &tg, uint32_t m_tok, bool *pays) {
+    uint32_t pairs = 0;
+    PRISM_TRY(tg.bits == 2 ? gm_pairs<2>(ctx, &pairs) : gm_pairs<4>(ctx, &pairs));
+    const GemmArgs a = gm_args(ctx, tg, m_tok, nullptr);
+    const GmPlan both = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 2, 1), one = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 1, GM_MAX_SPLITS);
+    *pays = both.cycles <= 2 * one.cycles + 4000.0 + (double)m_tok * tg.m * 8.0 / 3500.0;
+    return PRISM_OK;
 }
 
 }  // namespace prism

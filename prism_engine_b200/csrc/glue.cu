@@ -160,8 +160,8 @@ int launch_silu(prism_cuda_ctx *ctx, uint16_t *x, uint32_t n) {
 }
 
 // Activation arm of step() (engine_impl.rs:1355-1366): g = f16(silu(g)); g = f16(g*u).
-__global__ void silu_mul_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ g,
-                                const uint16_t *__restrict__ u, uint32_t n) {
+// `out` may be g.
+__global__ void silu_mul_kernel(uint16_t *out, const uint16_t *g, const uint16_t *__restrict__ u, uint32_t n) {
     pdl_launch_dependents();
     pdl_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -40,4 +40,14 @@ int grow_buf(Alloc &al, GrowBuf &b, size_t want, size_t elem_size, bool *grew = 
     return 0;
 }
 
+// The most rows, from `rows` down by halves to `least`, for which `ensure(rows)` returns 0; its last result if none does.
+template <typename F>
+int fit_rows(unsigned &rows, unsigned least, F &&ensure) {
+    for (;;) {
+        const int rc = ensure(rows);
+        if (rc == 0 || rows <= least) return rc;
+        rows = rows / 2 > least ? rows / 2 : least;
+    }
+}
+
 }  // namespace prism
