@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "attn_plan.hpp"
 #include "common.cuh"
 
 namespace cg = cooperative_groups;
@@ -396,19 +397,30 @@ static int launch_attn_fused_hd(prism_cuda_ctx *ctx, FusedAttnArgs &fa) {
     fa.gt = std::min(8u, g);
     if (ctx->attn_group > 0) fa.gt = std::min(fa.gt, (uint32_t)ctx->attn_group);
     const uint32_t clusters = fa.nkv * ((g + fa.gt - 1) / fa.gt) * fa.batch;
-    // CTAs per cluster: a tile of 16 positions per warp while there are SMs to give one CTA each; more than 8 (a
-    // non-portable size) only for contexts that still give every warp two tiles
-    uint32_t S = 1;
-    while (S < 8 && S * C::WARPS * FA_ROWS < fa.max_seq && 2 * S * clusters <= (uint32_t)ctx->sm_count) S *= 2;
-    if (S == 8 && 16 * clusters <= (uint32_t)ctx->sm_count && fa.max_seq >= 32 * C::WARPS * FA_ROWS) S = 16;
-    if (ctx->attn_cluster == 1 || ctx->attn_cluster == 2 || ctx->attn_cluster == 4 || ctx->attn_cluster == 8)
-        S = (uint32_t)ctx->attn_cluster;
-    static bool configured[PRISM_MAX_DEVICES] = {false};
-    if (!configured[ctx->device]) {
+    static int resident16[PRISM_MAX_DEVICES] = {0};  // plus one; 0: not asked yet
+    if (!resident16[ctx->device]) {
         PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_fused_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(C::smem(1), C::smem(FA_MAX_S))));
         PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_fused_kernel<HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        configured[ctx->device] = true;
+        cudaLaunchConfig_t big = {};
+        big.gridDim = dim3(FA_MAX_S);
+        big.blockDim = dim3(C::THREADS);
+        big.dynamicSmemBytes = C::smem(FA_MAX_S);
+        cudaLaunchAttribute shape;
+        shape.id = cudaLaunchAttributeClusterDimension;
+        shape.val.clusterDim.x = FA_MAX_S;
+        shape.val.clusterDim.y = shape.val.clusterDim.z = 1;
+        big.attrs = &shape;
+        big.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, attn_fused_kernel<HD>, &big) != cudaSuccess) {
+            (void)cudaGetLastError();  // no such cluster on this GPU
+            n = 0;
+        }
+        resident16[ctx->device] = 1 + n;
     }
+    uint32_t S = attn_cluster_ctas((uint32_t)ctx->sm_count, clusters, fa.max_seq, C::WARPS * FA_ROWS, (uint32_t)resident16[ctx->device] - 1);
+    if (ctx->attn_cluster == 1 || ctx->attn_cluster == 2 || ctx->attn_cluster == 4 || ctx->attn_cluster == 8)
+        S = (uint32_t)ctx->attn_cluster;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(clusters / fa.batch * S, fa.batch);
     cfg.blockDim = dim3(C::THREADS);
