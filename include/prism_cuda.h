@@ -237,7 +237,8 @@ int prism_cuda_mlp_dev(prism_cuda_ctx *ctx, int32_t gate, int32_t up, int32_t do
  *      with the CPU prefill's numerics: one lut_gemv_cpu per activation row
  *      (prefill_cpu, engine_impl.rs:1046-1053) ----------------------------- */
 
-/* Y[m_tok][dim_m] = X[m_tok][dim_n] * W^T, fp16 in, fp32 accumulate, fp16 out. */
+/* Y[m_tok][dim_m] = X[m_tok][dim_n] * W^T, fp16 in, fp32 accumulate, fp16 out.  Y_dev may lie over X_dev (X is then copied to
+ * the context's scratch first). */
 int prism_cuda_gemm(prism_cuda_ctx *ctx, int32_t handle, const uint16_t *X, uint32_t m_tok,
                     uint16_t *Y);
 int prism_cuda_gemm_dev(prism_cuda_ctx *ctx, int32_t handle, const void *X_dev, uint32_t m_tok,

@@ -5,8 +5,20 @@
 
 namespace prism {
 
+// X, or a copy of it in scratch where Y's rows lie over X's: the kernels read X while they store Y.
+static int gemm_input(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t **X, uint32_t m_tok, const uint16_t *Y) {
+    const size_t xn = (size_t)m_tok * t.k, yn = (size_t)m_tok * t.m;
+    if (*X >= Y + yn || Y >= *X + xn) return PRISM_OK;
+    if (reinterpret_cast<uintptr_t>(*X) & 15) return fail(ctx, PRISM_E_ARG, "gemm: X must be 16-byte aligned");
+    PRISM_TRY(ensure_tmp(ctx, xn));
+    PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->tmp_scratch, *X, xn * 2, cudaMemcpyDeviceToDevice, ctx->stream));
+    *X = ctx->tmp_scratch;
+    return PRISM_OK;
+}
+
 int launch_gemm(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y) {
     if (t.k % 8) return fail(ctx, PRISM_E_ARG, "gemm: dim_n must be a multiple of 8");
+    PRISM_TRY(gemm_input(ctx, t, &X, m_tok, Y));
     if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, t, m_tok)) return launch_gemm_tc5(ctx, t, X, m_tok, Y, nullptr);
     // activation rows as the batch dimension of the GEMV kernel, 32768 rows per launch
     for (uint32_t t0 = 0; t0 < m_tok; t0 += 32768) {
