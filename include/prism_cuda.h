@@ -66,7 +66,7 @@ int prism_cuda_synchronize(prism_cuda_ctx *ctx);
  * default 1: fused epilogues), "pdl" (0/1, default 1: programmatic dependent launch between
  * the kernels of a decode step, so a kernel's weight-only prologue overlaps its predecessor),
  * "batch_gemv_max" (decode batches up to this many sequences stream the weights once through the batched
- * GEMV, in groups of 8; larger batches use the tcgen05 GEMM; not set: 8, for linears of 2^25 weights and more 7),
+ * GEMV, in groups of 8; larger batches use the tcgen05 GEMM; 0, default: 8, for linears of 2^25 weights and more 7),
  * "attn_cluster" (0 = from max_seq, default; 1/2/4/8 CTAs per KV head and sequence in the fused
  * attention kernel),
  * "attn_group" (0 = from the shape, default; 1/2/4/8 = most query heads of a KV group one cluster of the
@@ -88,7 +88,7 @@ int prism_cuda_synchronize(prism_cuda_ctx *ctx);
  * the next synchronising call then returns PRISM_E_TIMEOUT and the context stays usable),
  * "prefill_chunk" (prism_cuda_engine_generate puts up to this many prompt tokens, of one sequence or of several,
  * through the layers at once -- tensor-core GEMMs, causal attention over the cache, no LM head -- instead of
- * one step per token as the reference's prefill_cpu does; not set: the engine's choice, at most 2048; 0 = one
+ * one step per token as the reference's prefill_cpu does; -1, default: the engine's choice, at most 2048; 0 = one
  * step per token.  Single GPU, fp16 KV),
  * "layered_chunk" (default 2048: the same for models described layer by layer; read when the engine is created),
  * "tp_fused_ar" (batch-1 tensor-parallel decode, how the partial sums of a row-parallel matmul are reduced:

@@ -259,7 +259,7 @@ int prism_cuda_set_option(prism_cuda_ctx *ctx, const char *key, int64_t value) {
         if (value < 0 || value > (1 << 24)) return fail(ctx, PRISM_E_ARG, "cl_max_units must be in 0..2^24");
         ctx->cl_max_units = (int)value;
     } else if (!strcmp(key, "batch_gemv_max")) {
-        if (value < 1 || value > 4096) return fail(ctx, PRISM_E_ARG, "batch_gemv_max must be in 1..4096");
+        if (value < 0 || value > 4096) return fail(ctx, PRISM_E_ARG, "batch_gemv_max must be in 0..4096");
         ctx->batch_gemv_max = (int)value;
     } else if (!strcmp(key, "attn_cluster")) {
         if (value != 0 && value != 1 && value != 2 && value != 4 && value != 8)
@@ -283,7 +283,7 @@ int prism_cuda_set_option(prism_cuda_ctx *ctx, const char *key, int64_t value) {
     } else if (!strcmp(key, "pdl")) {
         ctx->pdl = value ? 1 : 0;
     } else if (!strcmp(key, "prefill_chunk")) {
-        if (value < 0 || value > 65536) return fail(ctx, PRISM_E_ARG, "prefill_chunk must be in 0..65536");
+        if (value < -1 || value > 65536) return fail(ctx, PRISM_E_ARG, "prefill_chunk must be in -1..65536");
         ctx->prefill_chunk = (int)value;
     } else if (!strcmp(key, "layered_chunk")) {
         if (value < 1 || value > 65536) return fail(ctx, PRISM_E_ARG, "layered_chunk must be in 1..65536");
