@@ -746,6 +746,17 @@ static int feed_forward(prism_cuda_engine *e, LayeredLayer &ly, const DenseIn &i
     return launch_moe_gemm_tc5(ctx, ly.down, plan, act, yo, pairs);
 }
 
+// What of the context and the model a mixer's kernels write beside its own state and columns.  Two mixers that share any of it
+// run one after the other on one stream: SCRATCH_GEMM is the split sums and counters that the dense GEMM leaves in the context.
+enum MixerScratch { SCRATCH_GEMM = 1, SCRATCH_LATENT = 2, SCRATCH_DELTA = 4 };
+static uint32_t mixer_scratch(uint32_t mixer) {
+    switch (mixer) {
+    case PRISM_MIXER_LATENT_ATTENTION: return SCRATCH_GEMM | SCRATCH_LATENT;  // queries; expanded keys and values
+    case PRISM_MIXER_GATED_DELTA: return SCRATCH_DELTA;                       // convolved rows, chunk transforms, fp32 outputs
+    default: return 0;                                                        // lightning, grouped attention: registers and shared memory
+    }
+}
+
 // All mixers of a layer.  In a prompt portion the second of a pair runs on a stream of its own: its chunks follow one
 // another on a part of the GPU.
 static int run_mixers(prism_cuda_engine *e, LayeredLayer &ly, const RowMap &rows, uint32_t n, bool seq) {
@@ -759,7 +770,8 @@ static int run_mixers(prism_cuda_engine *e, LayeredLayer &ly, const RowMap &rows
         lightning_norm(m, ly, mx, h);
         return launch_dense_norm(ctx, h, at(m, m->cat, mx.col), m->cat_pitch, n, m->act32);
     };
-    if (!seq || ly.mix.size() != 2 || ly.mix[0].c.mixer == ly.mix[1].c.mixer || n <= DENSE_GEMV_ROWS) {  // mixers of a kind share scratch
+    if (!seq || ly.mix.size() != 2 || n <= DENSE_GEMV_ROWS || ly.mix[0].c.mixer == ly.mix[1].c.mixer ||
+        (mixer_scratch(ly.mix[0].c.mixer) & mixer_scratch(ly.mix[1].c.mixer))) {
         for (LayeredMixer &mx : ly.mix) PRISM_TRY(whole(mx));
         return PRISM_OK;
     }
