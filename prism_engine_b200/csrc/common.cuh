@@ -306,6 +306,7 @@ int launch_gemv_tc5(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, cons
 // gemm_tc5.cu: tcgen05/TMEM GEMM (K % 128 == 0, >= 8 tokens); with `resid`: Y = f16(f16(X W^T) + resid), resid may be Y.
 // launch_swiglu_tc5: act = f16(f16(silu(X Wg^T)) * (X Wu^T)), act is written twice; swiglu_tc5_pays: false where two launches take less.
 bool gemm_tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok);
+bool gemm_tc5_wide(const LutTensor &t, const uint16_t *y);  // rows of y can be moved 16 bytes at a time, as `resid` and SwiGLU need it
 int launch_gemm_tc5(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y, const uint16_t *resid);
 int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act);
 int swiglu_tc5_pays(prism_cuda_ctx *ctx, const LutTensor &tg, uint32_t m_tok, bool *pays);
@@ -386,6 +387,6 @@ int launch_gemm(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint
 // h = f16(f16(X W^T) + h); `tmp` holds m_tok * m values
 int launch_gemm_add(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *h, uint16_t *tmp);
 // act = f16(f16(silu(X Wg^T)) * (X Wu^T)); `u` holds m_tok * m values and is not used where gemm_swiglu_fused says so
-int gemm_swiglu_fused(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, uint32_t m_tok, bool *fused);
+int gemm_swiglu_fused(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, uint32_t m_tok, const uint16_t *act, bool *fused);
 int launch_gemm_swiglu(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, uint16_t *u);
 }  // namespace prism

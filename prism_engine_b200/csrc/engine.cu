@@ -131,16 +131,10 @@ static int linear(prism_cuda_engine *e, GemvMode mode, const LutTensor &t, const
     const uint64_t weights = (uint64_t)t.m * t.k * (mode == GEMV_SWIGLU ? 2 : 1);
     const uint32_t gemv_max = ctx->batch_gemv_max ? (uint32_t)ctx->batch_gemv_max : weights >= 1u << 25 ? 7 : 8;
     const bool gemm_ok = B > gemv_max && ctx->gemm_variant == 1 && e->gu && gemm_tc5_eligible(ctx, t, B) && xs == t.k &&
-                         (mode == GEMV_SWIGLU ? ys == t.m : ys == t.m);
+                         ys == t.m && (mode != GEMV_RESID || y == resid);
     if (!gemm_ok) return launch_gemv(ctx, mode, t, t2, x, xs, y, ys, resid, B);
     if (mode == GEMV_PLAIN) return launch_gemm(ctx, t, x, B, y);
-    if (mode == GEMV_RESID) {  // y (== resid, in place) = f16( f16(W x) + resid )
-        if (y == resid) return launch_gemm_add(ctx, t, x, B, y, e->gu);
-        PRISM_TRY(launch_gemm(ctx, t, x, B, e->gu));
-        PRISM_TRY(launch_vec_add(ctx, e->gu, resid, B * t.m));
-        PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(y, e->gu, (size_t)B * t.m * 2, cudaMemcpyDeviceToDevice, ctx->stream));
-        return PRISM_OK;
-    }
+    if (mode == GEMV_RESID) return launch_gemm_add(ctx, t, x, B, y, e->gu);  // y = f16( f16(W x) + y )
     return launch_gemm_swiglu(ctx, t, *t2, x, B, y, e->gu);
 }
 
@@ -480,7 +474,7 @@ static int prefill_portion(prism_cuda_engine *e, uint32_t b, uint32_t n_seq, uin
         PRISM_TRY(launch_gemm_add(ctx, to, e->pf_att, R, e->pf_x, e->pf_xn));  // h = f16(o + hr)
         PRISM_TRY(launch_rms_norm(ctx, e->pf_x, e->pf_xn, H, c.norm_eps, R));
         bool fused = false;
-        PRISM_TRY(gemm_swiglu_fused(ctx, tg, tu, R, &fused));
+        PRISM_TRY(gemm_swiglu_fused(ctx, tg, tu, R, e->pf_act, &fused));
         if (!fused) PRISM_TRY(ensure_prefill_up(e, R));
         PRISM_TRY(launch_gemm_swiglu(ctx, tg, tu, e->pf_xn, R, e->pf_act, e->pf_u));
         PRISM_TRY(launch_gemm_add(ctx, td, e->pf_act, R, e->pf_x, e->pf_xn));  // h = f16(d + hr)

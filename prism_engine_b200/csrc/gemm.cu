@@ -30,19 +30,19 @@ int launch_gemm(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint
 }
 
 int launch_gemm_add(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *h, uint16_t *tmp) {
-    if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, t, m_tok)) return launch_gemm_tc5(ctx, t, X, m_tok, h, h);
+    if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, t, m_tok) && gemm_tc5_wide(t, h)) return launch_gemm_tc5(ctx, t, X, m_tok, h, h);
     PRISM_TRY(launch_gemm(ctx, t, X, m_tok, tmp));
     return launch_vec_add(ctx, h, tmp, m_tok * t.m);
 }
 
-int gemm_swiglu_fused(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, uint32_t m_tok, bool *fused) {
+int gemm_swiglu_fused(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, uint32_t m_tok, const uint16_t *act, bool *fused) {
     *fused = false;
-    if (ctx->gemm_variant != 1 || !gemm_tc5_eligible(ctx, tg, m_tok) || !gemm_tc5_eligible(ctx, tu, m_tok) || tg.bits != tu.bits) return PRISM_OK;
+    if (ctx->gemm_variant != 1 || !gemm_tc5_eligible(ctx, tg, m_tok) || !gemm_tc5_eligible(ctx, tu, m_tok) || tg.bits != tu.bits || !gemm_tc5_wide(tg, act)) return PRISM_OK;
     return swiglu_tc5_pays(ctx, tg, m_tok, fused);
 }
 int launch_gemm_swiglu(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, uint16_t *u) {
     bool fused = false;
-    PRISM_TRY(gemm_swiglu_fused(ctx, tg, tu, m_tok, &fused));
+    PRISM_TRY(gemm_swiglu_fused(ctx, tg, tu, m_tok, act, &fused));
     if (fused) return launch_swiglu_tc5(ctx, tg, tu, X, m_tok, act);
     PRISM_TRY(launch_gemm(ctx, tg, X, m_tok, act));
     PRISM_TRY(launch_gemm(ctx, tu, X, m_tok, u));

@@ -71,7 +71,7 @@ struct GemmArgs {
     uint32_t nt;                      // tokens of a tile, a multiple of 32
     uint32_t sx_low, sx;              // activation stages before the tables, and in all
     uint32_t m_tok, mode;
-    uint32_t wide;                    // rows of y (and resid) can be moved 8 values at a time
+    uint32_t wide;                    // rows of y (and resid) can be moved 8 values at a time; GM_PLAIN only without
     uint16_t *y;                      // [m_tok][m]
     const uint16_t *resid;            // [m_tok][m] (GM_RESID), may be y
     float *part;                      // [item][CTA][warp][column][lane] sums of a range
@@ -131,32 +131,18 @@ __device__ __forceinline__ GmItem gm_item(const GemmArgs &a, uint32_t w) {
     return GmItem{t % a.n_rp, t / a.n_rp, a.n_st * s / a.splits, a.n_st * (s + 1) / a.splits};
 }
 
-// 16 tokens of one weight row, rounded (pairs, the first in the low half): the residual, or the product with silu of the gate
-// values this thread stored for the tile before (f16(f16(silu(g)) * u), engine_impl.rs:1355-1366).
-__device__ __forceinline__ void gm_store(const GemmArgs &a, const uint32_t (&v)[8], uint32_t t0, uint32_t row, uint32_t sub) {
+// 16 tokens of one weight row, rounded (pairs, the first in the low half), where rows of y cannot be moved 8 values at a time.
+__device__ __forceinline__ void gm_store(const GemmArgs &a, const uint32_t (&v)[8], uint32_t t0, uint32_t row) {
     if (row >= a.m || t0 >= a.m_tok) return;
     const uint32_t n = min(16u, a.m_tok - t0);
     uint16_t *y = a.y + (size_t)t0 * a.m + row;
-    const bool product = a.mode == GM_SWIGLU && sub == 1;
-    if (a.mode == GM_RESID || product) {
-        const uint16_t *src = product ? y : a.resid + (size_t)t0 * a.m + row;
-        uint16_t o[16];
-#pragma unroll
-        for (uint32_t i = 0; i < 16; i++) o[i] = i < n ? src[(size_t)i * a.m] : 0;
-#pragma unroll
-        for (uint32_t i = 0; i < 16; i++) {
-            const float h = __half2float(__ushort_as_half((uint16_t)(v[i / 2] >> (16 * (i & 1))))), x = __half2float(__ushort_as_half(o[i]));
-            const float r = product ? __half2float(__float2half_rn(x / (1.0f + expf(-x)))) * h : h + x;
-            if (i < n) y[(size_t)i * a.m] = __half_as_ushort(__float2half_rn(r));
-        }
-        return;
-    }
 #pragma unroll
     for (uint32_t i = 0; i < 16; i++)
         if (i < n) y[(size_t)i * a.m] = (uint16_t)(v[i / 2] >> (16 * (i & 1)));
 }
-// The same for a whole warp's 32 rows x 16 tokens, 16 bytes a lane: the values change places in the warp's 1 KB of shared
-// memory, so that a lane holds 8 rows of a token.
+// A whole warp's 32 rows x 16 tokens, 16 bytes a lane: the values change places in the warp's 1 KB of shared memory, so that a
+// lane holds 8 rows of a token; with the residual, or the product with silu of the gate values this lane stored for the tile
+// before (f16(f16(silu(g)) * u), engine_impl.rs:1355-1366).
 __device__ __forceinline__ void gm_store_wide(const GemmArgs &a, const uint32_t (&v)[8], uint32_t t0, uint32_t row0, uint32_t sub, uint8_t *out) {
     const uint32_t lane = threadIdx.x & 31;
     uint16_t *mine = reinterpret_cast<uint16_t *>(out) + lane;
@@ -302,7 +288,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                 }
                 const uint32_t t0 = it.tt * a.nt + (j + 4 * i) * 16;
                 if (a.wide) gm_store_wide(a, sums[i], t0, row - lane, sub, out);
-                else gm_store(a, sums[i], t0, row, sub);
+                else gm_store(a, sums[i], t0, row);
             }
             __syncwarp();
         };
@@ -520,6 +506,7 @@ bool gemm_tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok) 
     // whole weight stages of 128 k (four 32-k chunks: four index chunks at 4 bit, two at 2 bit)
     return ctx->smem_base == (int)GM_SBASE && (t.bits == 4 || t.bits == 2) && t.k % GM_STAGE_K == 0 && m_tok >= 8;
 }
+bool gemm_tc5_wide(const LutTensor &t, const uint16_t *y) { return t.m % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0; }
 
 // Tokens of a tile and ranges of K with the least estimated cycles.  A stage takes the tensor core 4 nt cycles; expanding
 // its weights takes 256 of the shared-memory pipe and streaming them about 350 at the HBM rate.  A tile's fill and last
@@ -577,7 +564,8 @@ static int launch_gm(prism_cuda_ctx *ctx, GemmArgs &a, const LutTensor &t, const
     a.nt = p.nt;
     a.splits = p.splits;
     a.n_tt = (a.m_tok + a.nt - 1) / a.nt;
-    a.wide = a.m % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.resid)) & 15) == 0;
+    a.wide = gemm_tc5_wide(t, a.y) && (reinterpret_cast<uintptr_t>(a.resid) & 15) == 0;
+    if (a.mode != GM_PLAIN && !a.wide) return fail(ctx, PRISM_E_ARG, "gemm: a residual or gated product needs rows of a multiple of 8 values, 16-byte aligned");
     const uint32_t xstage = a.nt * 64;
     a.sx_low = std::min((uint32_t)GM_SX_MAX, (GM_TBL - GM_X_LOW) / xstage);
     a.sx = std::min((uint32_t)GM_SX_MAX, a.sx_low + (GM_OUT_HIGH - GM_X_HIGH) / xstage);

@@ -31,3 +31,29 @@ def prompt_attention(backend, qkv, kc, vc, nh, nkv, hd, T, pos0=0, n_seq=1, rope
                     0 if page_tbl is None else page_tbl.shape[1])
     _call(backend, "_ZN5prism19launch_prefill_attnEP14prism_cuda_ctxRKNS_11PrefillAttnE", C.byref(a))
     return out
+
+
+def _tensor(backend, handle):
+    f = backend.L._ZN5prism10get_tensorEP14prism_cuda_ctxi
+    f.restype, f.argtypes = C.c_void_p, [C.c_void_p, C.c_int32]
+    return C.c_void_p(f(backend.ctx, handle))
+
+
+def gemm_add(backend, handle, x, h):
+    """h += x W^T, rounded after the product and after the sum."""
+    import torch
+
+    tmp = torch.empty_like(h)
+    _call(backend, "_ZN5prism15launch_gemm_addEP14prism_cuda_ctxRKNS_9LutTensorEPKtjPtS7_", _tensor(backend, handle), C.c_void_p(x.data_ptr()),
+          C.c_uint32(x.shape[0]), C.c_void_p(h.data_ptr()), C.c_void_p(tmp.data_ptr()))
+
+
+def gemm_swiglu(backend, gate, up, x, out, fused):
+    """out = silu(x Wg^T) * (x Wu^T), rounded after each; by one kernel, or as the engine chooses."""
+    import torch
+
+    a = [_tensor(backend, gate), _tensor(backend, up), C.c_void_p(x.data_ptr()), C.c_uint32(x.shape[0]), C.c_void_p(out.data_ptr())]
+    if fused:
+        return _call(backend, "_ZN5prism17launch_swiglu_tc5EP14prism_cuda_ctxRKNS_9LutTensorES4_PKtjPt", *a)
+    u = torch.empty_like(out)
+    _call(backend, "_ZN5prism18launch_gemm_swigluEP14prism_cuda_ctxRKNS_9LutTensorES4_PKtjPtS7_", *a, C.c_void_p(u.data_ptr()))
