@@ -25,6 +25,7 @@
 
 #include "attn_plan.hpp"
 #include "common.cuh"
+#include "tensor_map.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(FaCfg<HD>::THREADS) attn_fused_kernel(const Fu
     if (early) {
         pdl_wait();
         const int32_t pos_now = *pos_ptr;
-        if (pos_now != pos_seen) {                 // the same value in every thread of the cluster
+        if (pos_now != pos_seen) {                 // uniform in a warp only (others may have read the old position): nothing here waits for more
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             __syncwarp();
             place(pos_now);
@@ -401,21 +402,7 @@ static int launch_attn_fused_hd(prism_cuda_ctx *ctx, FusedAttnArgs &fa) {
     if (!resident16[ctx->device]) {
         PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_fused_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(C::smem(1), C::smem(FA_MAX_S))));
         PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(attn_fused_kernel<HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchConfig_t big = {};
-        big.gridDim = dim3(FA_MAX_S);
-        big.blockDim = dim3(C::THREADS);
-        big.dynamicSmemBytes = C::smem(FA_MAX_S);
-        cudaLaunchAttribute shape;
-        shape.id = cudaLaunchAttributeClusterDimension;
-        shape.val.clusterDim.x = FA_MAX_S;
-        shape.val.clusterDim.y = shape.val.clusterDim.z = 1;
-        big.attrs = &shape;
-        big.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, attn_fused_kernel<HD>, &big) != cudaSuccess) {
-            (void)cudaGetLastError();  // no such cluster on this GPU
-            n = 0;
-        }
+        const int n = resident_clusters(attn_fused_kernel<HD>, FA_MAX_S, C::THREADS, C::smem(FA_MAX_S), FA_MAX_S);
         resident16[ctx->device] = 1 + n;
     }
     uint32_t S = attn_cluster_ctas((uint32_t)ctx->sm_count, clusters, fa.max_seq, C::WARPS * FA_ROWS, (uint32_t)resident16[ctx->device] - 1);

@@ -15,12 +15,11 @@
 // (rows past the end are filled with zeros).  One thread issues the products; four warps per 128 rows read an
 // accumulator back, apply the epilogue of the tile's segment and store.
 // Every mbarrier wait is bounded; one that gives up raises the context's device error word.
-#include <cuda.h>
-
 #include <algorithm>
 
 #include "dense.cuh"
 #include "tc5_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace prism {
 
@@ -66,30 +65,6 @@ struct DgArgs {
     unsigned int *arrived;    // [tile][CTA][warp], zero between launches
 };
 constexpr uint32_t DG_MAX_EXPERTS = 1024;
-
-__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t mbar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-                 "l"(map), "r"(x), "r"(y), "r"(mbar)
-                 : "memory");
-}
-// The same where the barrier is the pair's, in CTA 0.
-__device__ __forceinline__ void tma_2d_pair(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t mbar) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-                 "l"(map), "r"(x), "r"(y), "r"(mbar)
-                 : "memory");
-}
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// K-major operand with the 128-byte swizzle: rows of 128 bytes, eight-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
 
 // Walk of the tiles: groups of rt_group row tiles over all token tiles, so that the CTAs of one wave share a
 // few weights and a few rows of x in L2.
@@ -269,7 +244,7 @@ __global__ void __launch_bounds__(DgCfg<NT>::THREADS, 1) dense_gemm_tc5_kernel(c
                     t5::mbar_wait_bounded(b_empty + 8 * s, ph ^ 1, err_flag);
                     t5::mbar_arrive_expect_tx(b_full + 8 * s, C::STAGE);
                     t5::bulk_g2s(dst, wsrc + (size_t)k * DG_A_BYTES, DG_A_BYTES, b_full + 8 * s);
-                    tma_2d(dst + C::A_BYTES, map, (int32_t)(k * 64), (int32_t)it.t0, b_full + 8 * s);
+                    t5::tma_2d(dst + C::A_BYTES, map, (int32_t)(k * 64), (int32_t)it.t0, b_full + 8 * s);
                 }
             }
             // every copy in flight lands before the CTA leaves (a stage's last use is committed to its empty barrier)
@@ -296,7 +271,7 @@ __global__ void __launch_bounds__(DgCfg<NT>::THREADS, 1) dense_gemm_tc5_kernel(c
                 if (t5::elect_one()) {
 #pragma unroll
                     for (int j = 0; j < 4; j++)  // 16 k each: two k/8 slabs of 2 KB in A, 32 bytes inside the swizzled rows of B
-                        mma_ss(d, t5::smem_desc(sa + j * 4096, 2048, 128), desc_sw128(sb + j * 32), idesc, j ? 1u : k);
+                        t5::mma_ss(d, t5::smem_desc(sa + j * 4096, 2048, 128), t5::desc_swizzled<128>(sb + j * 32), idesc, j ? 1u : k);
                     t5::commit(b_empty + 8 * s);
                 }
             }
@@ -374,8 +349,8 @@ __global__ void __launch_bounds__(DpCfg<NT>::THREADS, 1) dense_gemm_pair_kernel(
                     const uint32_t s = n % C::S, ph = (n / C::S) & 1, dst = base + s * C::STAGE;
                     t5::mbar_wait_bounded(b_empty + 8 * s, ph ^ 1, err_flag);
                     if (rank == 0) t5::mbar_arrive_expect_tx(b_full + 8 * s, 2 * C::STAGE);
-                    tma_2d_pair(dst, &wmap, 0, (int32_t)((w0 + k) * 32), full0 + 8 * s);
-                    tma_2d_pair(dst + DG_A_BYTES, map, (int32_t)(k * 64), (int32_t)(it.t0 + rank * (NT / 2)), full0 + 8 * s);
+                    t5::tma_2d_pair(dst, &wmap, 0, (int32_t)((w0 + k) * 32), full0 + 8 * s);
+                    t5::tma_2d_pair(dst + DG_A_BYTES, map, (int32_t)(k * 64), (int32_t)(it.t0 + rank * (NT / 2)), full0 + 8 * s);
                 }
             }
             // every copy in flight lands before the CTA leaves: a stage is given back after its products
@@ -402,7 +377,7 @@ __global__ void __launch_bounds__(DpCfg<NT>::THREADS, 1) dense_gemm_pair_kernel(
                     if (t5::elect_one()) {
 #pragma unroll
                         for (int j = 0; j < 4; j++)
-                            t5::mma_ss_pair(d, t5::smem_desc(sa + j * 4096, 2048, 128), desc_sw128(sb + j * 32), idesc, j ? 1u : k);
+                            t5::mma_ss_pair(d, t5::smem_desc(sa + j * 4096, 2048, 128), t5::desc_swizzled<128>(sb + j * 32), idesc, j ? 1u : k);
                         t5::commit_pair(b_empty + 8 * s);
                     }
                 }
@@ -465,30 +440,10 @@ __global__ void __launch_bounds__(DpCfg<NT>::THREADS, 1) dense_gemm_pair_kernel(
 }
 
 // ---- host side ---------------------------------------------------------------------------------
-typedef CUresult (*TensorMapEncode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                    const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static TensorMapEncode tensor_map_encode() {
-    static TensorMapEncode fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult st;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<TensorMapEncode>(p);
-    }();
-    return fn;
-}
-
 static int encode_2d(prism_cuda_ctx *ctx, CUtensorMap *map, const void *p, uint64_t cols, uint64_t rows, uint64_t pitch, uint32_t box_cols, uint32_t box_rows,
                      bool swizzle) {
-    TensorMapEncode enc = tensor_map_encode();
-    if (!enc) return fail(ctx, PRISM_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {pitch * 2};
-    const cuuint32_t box[2] = {box_cols, box_rows}, estr[2] = {1, 1};
-    const CUresult rc = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(p), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return rc == CUDA_SUCCESS ? PRISM_OK : fail(ctx, PRISM_E_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)rc));
+    return encode_tensor_map(ctx, map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, p, cols, rows, pitch, box_cols, box_rows,
+                             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 static int encode_inputs(prism_cuda_ctx *ctx, const DgArgs &a, const DenseIn &in, uint32_t box_rows, CUtensorMap *map, CUtensorMap *map2) {
     uint32_t k[2] = {0, 0};  // columns of each input that a segment reads
@@ -534,18 +489,7 @@ static int launch_dp(prism_cuda_ctx *ctx, const DenseLinear &l, DgArgs &a, const
     static int pairs[PRISM_MAX_DEVICES] = {0};  // pairs that are resident at once (a GPC with an odd number of SMs leaves one idle)
     if (!pairs[ctx->device]) {
         PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(dense_gemm_pair_kernel<NT, MOE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * ((unsigned)ctx->sm_count / 2));
-        cfg.blockDim = dim3(C::THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        PRISM_CUDA_TRY(ctx, cudaOccupancyMaxActiveClusters(&n, dense_gemm_pair_kernel<NT, MOE>, &cfg));
+        const int n = resident_clusters(dense_gemm_pair_kernel<NT, MOE>, 2, C::THREADS, smem, 2 * ((uint32_t)ctx->sm_count / 2));
         pairs[ctx->device] = std::max(1, std::min(n, ctx->sm_count / 2));
     }
     CUtensorMap wmap, map, map2;

@@ -25,13 +25,12 @@
 // 26 -> 19.9; 4608 x 3584, 2048 tokens 72 -> 53, 32 tokens 23.4 -> 15.1; 3584 x 18944, 2048 tokens 320 -> 278, 32 tokens
 // 96.5 -> 25.0.  The times before are without the residual or SwiGLU passes and the re-laid activations that went with them.
 // Every mbarrier wait is bounded; a wait that gives up raises the context's device error word.
-#include <cuda.h>
-
 #include <algorithm>
 
 #include "common.cuh"
 #include "pair_table.cuh"
 #include "tc5_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace prism {
 
@@ -81,11 +80,6 @@ struct GemmArgs {
 
 namespace {
 
-__device__ __forceinline__ void gm_tma_pair(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t mbar) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-                 "l"(map), "r"(x), "r"(y), "r"(mbar)
-                 : "memory");
-}
 __device__ __forceinline__ void gm_mma_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -94,11 +88,6 @@ __device__ __forceinline__ void gm_mma_pair(uint32_t d_tmem, uint32_t a_tmem, ui
         "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// K-major operand of 128-byte rows, 128-byte swizzle, eight-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t gm_desc(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
-
 template <int SLOT>
 __device__ __forceinline__ uint32_t gm_lds(uint32_t off) {
     uint32_t v;
@@ -431,7 +420,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                         const uint32_t next = __ballot_sync(0xFFFFFFFFu, t5::mbar_test(lane == 0 ? b_afull + 8 * ((n + 1) % GM_SA) : b_xfull + 8 * (lane == 1 ? s2 : s3),
                                                                                        lane == 0 ? ((n + 1) / GM_SA) & 1 : lane == 1 ? p2 : p3));
                         t5::fence_after();
-                        const uint64_t x0 = gm_desc(x_addr(sx)), x1 = gm_desc(x_addr(s1));
+                        const uint64_t x0 = t5::desc_swizzled<128>(x_addr(sx)), x1 = t5::desc_swizzled<128>(x_addr(s1));
                         if (t5::elect_one()) {
 #pragma unroll
                             for (uint32_t kk = 0; kk < 4; kk++)  // 16 k are 32 bytes of the swizzled row
@@ -467,7 +456,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                 for (uint32_t k = it.k0 * 128; k < it.k1 * 128; k += 64, h++) {
                     if (h >= a.sx) wait_step((h - a.sx) / 2);  // at most `ring` stages back: its barrier has not come round again
                     if (rank == 0) t5::mbar_arrive_expect_tx(b_xfull + 8 * sx, 2 * xstage);
-                    gm_tma_pair(x_addr(sx), &xmap, (int32_t)k, t0, full0 + 8 * sx);
+                    t5::tma_2d_pair(x_addr(sx), &xmap, (int32_t)k, t0, full0 + 8 * sx);
                     if (++sx == a.sx) sx = 0;
                 }
             }
@@ -484,24 +473,6 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
 }
 
 // ---- host side ---------------------------------------------------------------------------------
-typedef CUresult (*TensorMapEncode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                    const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static int encode_x(prism_cuda_ctx *ctx, CUtensorMap *map, const uint16_t *x, uint32_t k, uint32_t m_tok, uint32_t box_rows) {
-    static TensorMapEncode enc = [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult st;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess) f = nullptr;
-        return reinterpret_cast<TensorMapEncode>(f);
-    }();
-    if (!enc) return fail(ctx, PRISM_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    const cuuint64_t dims[2] = {k, m_tok}, strides[1] = {(cuuint64_t)k * 2};
-    const cuuint32_t b[2] = {64, box_rows}, estr[2] = {1, 1};
-    const CUresult rc = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(x), dims, strides, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return rc == CUDA_SUCCESS ? PRISM_OK : fail(ctx, PRISM_E_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)rc));
-}
-
 bool gemm_tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok) {
     // whole weight stages of 128 k (four 32-k chunks: four index chunks at 4 bit, two at 2 bit)
     return ctx->smem_base == (int)GM_SBASE && (t.bits == 4 || t.bits == 2) && t.k % GM_STAGE_K == 0 && m_tok >= 8;
@@ -541,18 +512,7 @@ static int gm_pairs(prism_cuda_ctx *ctx, uint32_t *out) {  // pairs that are res
     static int pairs[PRISM_MAX_DEVICES] = {0};
     if (!pairs[ctx->device]) {
         PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(lut_gemm_tc5_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GM_SMEM_BYTES));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * ((unsigned)ctx->sm_count / 2));
-        cfg.blockDim = dim3(GM_THREADS);
-        cfg.dynamicSmemBytes = GM_SMEM_BYTES;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        PRISM_CUDA_TRY(ctx, cudaOccupancyMaxActiveClusters(&n, lut_gemm_tc5_kernel<BITS>, &cfg));
+        const int n = resident_clusters(lut_gemm_tc5_kernel<BITS>, 2, GM_THREADS, GM_SMEM_BYTES, 2 * ((uint32_t)ctx->sm_count / 2));
         pairs[ctx->device] = std::max(1, std::min(n, ctx->sm_count / 2));
     }
     *out = (uint32_t)pairs[ctx->device];
@@ -577,7 +537,7 @@ static int launch_gm(prism_cuda_ctx *ctx, GemmArgs &a, const LutTensor &t, const
         a.arrived = ctx->splitk_counters;
     }
     CUtensorMap xmap;
-    PRISM_TRY(encode_x(ctx, &xmap, X, t.k, a.m_tok, a.nt / 2));
+    PRISM_TRY(encode_tensor_map(ctx, &xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, X, t.k, a.m_tok, t.k, 64, a.nt / 2, CU_TENSOR_MAP_SWIZZLE_128B));
     const uint32_t grid = (uint32_t)std::min<uint64_t>(pairs, (uint64_t)tiles * a.splits);
     launch_cluster_pdl(ctx, lut_gemm_tc5_kernel<BITS>, dim3(2 * grid), dim3(GM_THREADS), GM_SMEM_BYTES, 2u, a, xmap);
     return after_launch(ctx, "lut_gemm_tc5_kernel");

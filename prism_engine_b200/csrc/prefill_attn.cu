@@ -24,12 +24,11 @@
 // Measured, 28 query / 4 KV heads of 128: the attention of an 8190-token prompt through two layers took 128 ms with one
 // cluster of the decode kernel per token, on the CUDA cores; this kernel took 1.87 ms with a single issuing thread (descriptors
 // through vector registers), 1.38 with a whole warp walking the tiles.
-#include <cuda.h>
-
 #include <algorithm>
 
 #include "common.cuh"
 #include "tc5_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace prism {
 
@@ -67,26 +66,6 @@ struct PrefillAttnDev {
 
 namespace {
 
-__device__ __forceinline__ void pa_tma(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t mbar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-                 "l"(map), "r"(x), "r"(y), "r"(mbar)
-                 : "memory");
-}
-__device__ __forceinline__ void pa_mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Swizzled operand of ROWB-byte rows: eight-row groups 8 * ROWB apart; lbo only matters along the other dimension of
-// an operand that is read across its rows (V): the distance between panels.
-template <int ROWB>
-__device__ __forceinline__ uint64_t pa_desc(uint32_t addr, uint32_t lbo) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(8 * ROWB >> 4) << 32 | (uint64_t)1 << 46 |
-           (uint64_t)(ROWB == 128 ? 2 : 4) << 61;
-}
 __device__ __forceinline__ float pa_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
@@ -304,7 +283,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
             for (uint32_t q = 0; q < (uint32_t)QT; q++)
                 if (n_kt[q])
                     for (uint32_t p = 0; p < (uint32_t)C::PANELS; p++)
-                        pa_tma(base + q * C::TILE + p * C::PANEL, &qmap, (int32_t)(h * HD + p * (C::ROWB / 2)), (int32_t)(sq * a.T + qb + q * 128), b_qfull);
+                        t5::tma_2d(base + q * C::TILE + p * C::PANEL, &qmap, (int32_t)(h * HD + p * (C::ROWB / 2)), (int32_t)(sq * a.T + qb + q * 128), b_qfull);
             auto load = [&](const CUtensorMap *map, uint32_t dst, uint32_t k0, uint32_t mbar) {
                 const uint32_t rows = min((uint32_t)PA_K, kv_end - k0), boxes = (rows + a.box - 1) / a.box;
                 t5::mbar_arrive_expect_tx(mbar, boxes * a.box * HD * 2);
@@ -316,7 +295,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
                         r = (page << a.page_shift) + (pos & ((1u << a.page_shift) - 1u));
                     }
                     for (uint32_t p = 0; p < (uint32_t)C::PANELS; p++)
-                        pa_tma(dst + p * C::PANEL + b * a.box * C::ROWB, map, (int32_t)(kh * HD + p * (C::ROWB / 2)), (int32_t)r, mbar);
+                        t5::tma_2d(dst + p * C::PANEL + b * a.box * C::ROWB, map, (int32_t)(kh * HD + p * (C::ROWB / 2)), (int32_t)r, mbar);
                 }
             };
             for (uint32_t j = 0; j < n; j++) {
@@ -343,7 +322,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
 #pragma unroll
             for (int k = 0; k < HD / 16; k++) {
                 const uint32_t off = (k * 32 / C::ROWB) * C::PANEL + (k * 32) % C::ROWB;
-                pa_mma_ss(tmem + q * 128, pa_desc<C::ROWB>(qa + off, 16), pa_desc<C::ROWB>(ka + off, 16), id_s, k != 0);
+                t5::mma_ss(tmem + q * 128, t5::desc_swizzled<C::ROWB>(qa + off, 16), t5::desc_swizzled<C::ROWB>(ka + off, 16), id_s, k != 0);
             }
             t5::commit(b_sfull + 8 * q);
         };
@@ -382,7 +361,7 @@ __global__ void __launch_bounds__(PaCfg<HD>::THREADS, 1) prefill_attn_kernel(con
                     for (int part = 0; part < 2; part++)
 #pragma unroll
                         for (int k = 0; k < PA_K / 16; k++)
-                            t5::mma_ts(tmem + 256 + q * HD, tmem + q * 128 + part * 64 + k * 8, pa_desc<C::ROWB>(va + k * 16 * C::ROWB, C::PANEL), id_o,
+                            t5::mma_ts(tmem + 256 + q * HD, tmem + q * 128 + part * 64 + k * 8, t5::desc_swizzled<C::ROWB>(va + k * 16 * C::ROWB, C::PANEL), id_o,
                                        part | k ? 1u : j);
                     if (jn < n_kt[q]) scores(q, jn);
                     else t5::commit(b_ofull + 8 * q);
@@ -448,23 +427,9 @@ __global__ void __launch_bounds__(256) prefill_rope_kernel(uint16_t *qkv, uint32
 }
 
 // ---- host side ---------------------------------------------------------------------------------
-typedef CUresult (*TensorMapEncode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                    const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static int encode_rows(prism_cuda_ctx *ctx, CUtensorMap *map, const void *p, uint64_t cols, uint64_t rows, uint64_t pitch, uint32_t box_cols, uint32_t box_rows) {
-    static TensorMapEncode enc = [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult st;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess) f = nullptr;
-        return reinterpret_cast<TensorMapEncode>(f);
-    }();
-    if (!enc) return fail(ctx, PRISM_E_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {pitch * 2};
-    const cuuint32_t box[2] = {box_cols, box_rows}, estr[2] = {1, 1};
-    const CUresult rc = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return rc == CUDA_SUCCESS ? PRISM_OK : fail(ctx, PRISM_E_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)rc));
+    return encode_tensor_map(ctx, map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p, cols, rows, pitch, box_cols, box_rows,
+                             box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 template <int HD>

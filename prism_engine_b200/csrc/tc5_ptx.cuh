@@ -2,6 +2,8 @@
 // used by the prefill GEMM.  Every wait is bounded (see mbar_wait_bounded).
 #pragma once
 
+#include <cuda.h>
+
 #include <cstdint>
 
 namespace prism {
@@ -131,6 +133,15 @@ __device__ __forceinline__ void commit_pair(uint32_t mbar_addr) {
                  "h"((uint16_t)3)
                  : "memory");
 }
+// D[tmem] (+)= A[smem descriptor] * B[smem descriptor], and the same over the two CTAs of a pair.
+__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 __device__ __forceinline__ void mma_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -171,6 +182,18 @@ __device__ __forceinline__ void mbar_arrive_tmem(uint32_t cluster_addr) {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
+// Box of a tensor map at column x, row y -> shared memory, completion counted in bytes on an mbarrier; tma_2d_pair: one of CTA 0
+// of the pair.
+__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t mbar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(y), "r"(mbar)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_2d_pair(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t mbar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(y), "r"(mbar)
+                 : "memory");
+}
 // 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier (no tensor map).
 // Source, destination and size are multiples of 16 bytes.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void *src, uint32_t bytes, uint32_t mbar) {
@@ -188,6 +211,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t smem_addr, uint32_t lbo, 
     d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
     d |= (uint64_t)1 << 46;  // descriptor version of sm_100
     return d;                // layout type 0: no swizzle
+}
+// The same for rows of ROWB bytes in the swizzle of that width, eight-row groups 8 * ROWB apart; lbo only matters along the other
+// dimension of an operand that is read across its rows.
+template <int ROWB>
+__device__ __forceinline__ uint64_t desc_swizzled(uint32_t addr, uint32_t lbo = 16) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(8 * ROWB >> 4) << 32 | (uint64_t)1 << 46 |
+           (uint64_t)(ROWB == 128 ? 2 : 4) << 61;
 }
 // Instruction descriptor for kind::f16: D fp32, A and B fp16, both K-major, M x N tile.
 __device__ __forceinline__ uint32_t idesc_f16(uint32_t m, uint32_t n) {
