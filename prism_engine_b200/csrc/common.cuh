@@ -76,7 +76,7 @@ struct prism_cuda_ctx {
     int sk_min_chunks = 8;      // stream-K GEMV, small matrices: fewest 1 KB index chunks a CTA is given
     int sk_stream_chunks = 64;  // chunks per CTA from which the balanced contiguous partition is used
     int cl_max_units = 16384;    // cluster GEMV for matrices of at most this many (64-row block, 1 KB chunk) units; 0: never
-    int batch_gemv_max = 0;   // decode batches up to this size use the batched GEMV (groups of 8), larger ones the GEMM; 0: 8, large linears 7
+    int batch_gemv_max = 0;   // decode batches up to this size use the batched GEMV (groups of 8), larger ones the GEMM; 0: 8, or 7 (gemm_pays_at_8)
     int attn_cluster = 0;    // CTAs per (head, sequence) of the fused attention kernel; 0: chosen from max_seq
     int ws_whole_blocks = 1024;  // warp-specialised GEMV: one whole block per CTA when there are almost as many blocks as SMs and rows have at most this many chunks; 0: never
     int ws_whole_fill = 50;  // ... for one activation row, when the matrix has at least this many blocks per 100 SMs

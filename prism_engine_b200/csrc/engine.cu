@@ -13,6 +13,7 @@
 
 #include "../../include/prism_cuda_bench.h"
 #include "engine.hpp"
+#include "linear_plan.hpp"
 #include "scratch.hpp"
 
 namespace prism {
@@ -125,11 +126,8 @@ static int tp_reduce_add_resid(prism_cuda_engine *e, uint32_t n) {
 static int linear(prism_cuda_engine *e, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x,
                   uint32_t xs, uint16_t *y, uint32_t ys, const uint16_t *resid, uint32_t B) {
     prism_cuda_ctx *ctx = e->ctx;
-    // The GEMM costs about 12 us before its first weight, the batched GEMV twice the time per weight at 8 sequences: from 2^25
-    // weights on the GEMM is ahead (8 sequences, 40 steps: 7B with both ways for all linears 11.3 / 10.0 ms, 72B 28.5 / 24.9, 0.5B
-    // 4.9 / 6.2; 6 sequences 9.5 / 9.8, 22.7 / 24.5).
-    const uint64_t weights = (uint64_t)t.m * t.k * (mode == GEMV_SWIGLU ? 2 : 1);
-    const uint32_t gemv_max = ctx->batch_gemv_max ? (uint32_t)ctx->batch_gemv_max : weights >= 1u << 25 ? 7 : 8;
+    const uint32_t gemv_max = ctx->batch_gemv_max ? (uint32_t)ctx->batch_gemv_max
+                              : gemm_pays_at_8(t.m, t.k, t.bits, mode == GEMV_SWIGLU, (uint32_t)ctx->sm_count) ? 7 : 8;
     const bool gemm_ok = B > gemv_max && ctx->gemm_variant == 1 && e->gu && gemm_tc5_eligible(ctx, t, B) && xs == t.k &&
                          ys == t.m && (mode != GEMV_RESID || y == resid);
     if (!gemm_ok) return launch_gemv(ctx, mode, t, t2, x, xs, y, ys, resid, B);

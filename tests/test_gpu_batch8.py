@@ -1,6 +1,6 @@
-"""Eight sequences in a decode step: linears of 2^25 weights and more go through the GEMM, smaller ones through the batched GEMV.
-The engine's choice against all linears through the one and through the other (option batch_gemv_max), gate and up together just
-reaching the line.  Tolerance as in test_gpu_prefill_attention.py: another order of the fp32 sums, one layer of fp16 roundings."""
+"""Eight sequences in a decode step: large linears go through the GEMM, others through the batched GEMV (gemm_pays_at_8).
+The engine's choice against all linears through the one and through the other (option batch_gemv_max), gate and up on both sides
+of the lines for 4 bits (10240 rows) and for 2 (2^25 weights together).  Tolerance as in test_gpu_prefill_attention.py: another order of the fp32 sums, one layer of fp16 roundings."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bits", [4, 2])
-@pytest.mark.parametrize("inter", [8192, 8160])
+@pytest.mark.parametrize("inter", [8192, 8160, 10240, 10112])
 def test_choice_at_eight_sequences(inter, bits):
     cfg = dict(num_layers=1, hidden_size=2048, num_heads=16, num_kv_heads=2, head_dim=128, intermediate_size=inter, vocab_size=640,
                norm_eps=1e-6, rope_theta=1e6, tie_word_embeddings=False)
