@@ -21,7 +21,7 @@
 //    16 lanes add their cluster's elements one after the other.
 // Bound by those chains (4 cycles an element, 15 passes) and the instructions of the nearest-entry search.
 // One block per row, so 14 rows of 3584 are at work on an SM at a time.
-// 3584 x 3584 values from host memory and back, one thread per row before: 33.0 ms (25.9 of it the kernel); now 7.5 (1.08).  Rows whose distances do not fit shared
+// 3584 x 3584 values from host memory and back, one thread per row before: 33 ms (25.9 of it the kernel); now 7.5 to 9 by the host (1.08).  Rows whose distances do not fit shared
 // memory still take one thread each.
 #include "common.cuh"
 
