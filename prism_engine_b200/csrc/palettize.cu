@@ -22,7 +22,7 @@
 // Bound by those chains (4 cycles an element, 15 passes) and the instructions of the nearest-entry search.
 // One block per row, so 14 rows of 3584 are at work on an SM at a time.
 // 3584 x 3584 values from host memory and back, one thread per row before: 33 ms (25.9 of it the kernel); now 7.5 to 9 by the host (1.08).  Rows whose distances do not fit shared
-// memory still take one thread each.
+// memory, and many short rows, still take one thread each.
 #include "common.cuh"
 
 namespace prism {
@@ -372,7 +372,11 @@ __global__ void __launch_bounds__(PB_THREADS) palettize_block_kernel(const float
 int launch_palettize(prism_cuda_ctx *ctx, const float *w_dev, uint32_t dm, uint32_t dn, uint32_t k, uint32_t max_iter,
                      uint8_t *payload_dev) {
     const size_t smem = pb_smem_bytes(dn);
-    if (smem <= PB_MAX_SMEM) {
+    // Many short rows: a block pays some 15 ns of the GPU a row before its first element, a thread per row 14 us an element however
+    // many rows there are up to the GPU's threads.  100000 rows of 16 / 64 / 128 values: blocks 1541 / 2059 / 2384 us, threads 165 /
+    // 955 / 1836.
+    const bool threads = dn <= 128 && dm >= 720u * dn;
+    if (smem <= PB_MAX_SMEM && !threads) {
         if (smem > 48 * 1024)
             PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(palettize_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_MAX_SMEM));
         palettize_block_kernel<<<dm, PB_THREADS, smem, ctx->stream>>>(w_dev, dm, dn, k, max_iter, payload_dev);

@@ -15,6 +15,13 @@ def test_row_lengths(backend, oracle, m, k):
     assert np.array_equal(backend.palettize(w), oracle.palettize_to_payload(w, m, k, 16, 50))
 
 
+@pytest.mark.parametrize("m,k", [(720 * 2, 2), (720 * 16 - 1, 16), (720 * 16, 16), (720 * 34 + 5, 34)])
+def test_many_short_rows(backend, oracle, m, k):
+    """Both sides of the line from which short rows take a thread each."""
+    w = (np.random.default_rng(k).standard_normal((m, k)) * 0.5).astype(np.float32)
+    assert np.array_equal(backend.palettize(w), oracle.palettize_to_payload(w, m, k, 16, 50))
+
+
 @pytest.mark.parametrize("kind", ["huge", "inf", "nan", "zeros", "ties"])
 def test_values(backend, oracle, kind):
     m, k = 4, 200
