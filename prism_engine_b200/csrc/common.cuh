@@ -303,12 +303,19 @@ bool tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t batch);
 int launch_gemv_tc5(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x,
                     void *y, const uint16_t *resid);
 
+// gemm_reg.cu: 1..32 activation rows, palettes in registers; PLAIN, RESID and SWIGLU; norm_eps >= 0 (one row) folds RMSNorm of x.
+// gemm_reg_takes: false where a tensor or mode is not for it, or another kernel takes less time (reg_pays)
+int gemm_reg_takes(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, uint32_t batch, bool *takes);
+int launch_gemm_reg(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,
+                    uint32_t y_stride, const uint16_t *resid, uint32_t batch, float norm_eps);
+
 // gemm_tc5.cu: tcgen05/TMEM GEMM (K % 128 == 0, >= 8 tokens); with `resid`: Y = f16(f16(X W^T) + resid), resid may be Y.
 // launch_swiglu_tc5: act = f16(f16(silu(X Wg^T)) * (X Wu^T)), act is written twice; swiglu_tc5_pays: false where two launches take less.
 bool gemm_tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok);
 bool gemm_tc5_wide(const LutTensor &t, const uint16_t *y);  // rows of y can be moved 16 bytes at a time, as `resid` and SwiGLU need it
 int launch_gemm_tc5(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y, const uint16_t *resid);
 int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act);
+int gemm_tc5_stages(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok, uint32_t subs, uint32_t *stages);  // that a pair of CTAs goes through
 int swiglu_tc5_pays(prism_cuda_ctx *ctx, const LutTensor &tg, uint32_t m_tok, bool *pays);
 
 // glue.cu

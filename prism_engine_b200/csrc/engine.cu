@@ -119,13 +119,15 @@ static int tp_reduce_add_resid(prism_cuda_engine *e, uint32_t n) {
     return after_launch(ctx, "round_add_resid_kernel");
 }
 
-// One palettized linear of the step.  A batch of 8 or more sequences goes through the tensor-core
-// GEMM (weights streamed once for the whole batch) followed by the same elementwise kernels the
-// unfused path uses, so the fp16 rounding points stay those of the reference; smaller batches use
-// the GEMV kernels with their fused epilogues.
+// One palettized linear of the step, weights streamed once for the whole batch: up to 32 sequences through the register-palette
+// kernel where it takes less time than the others (reg_pays), else a batch of 8 or more through the tensor-core GEMM and smaller
+// ones through the GEMV kernels.  All round where the reference does.
 static int linear(prism_cuda_engine *e, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x,
                   uint32_t xs, uint16_t *y, uint32_t ys, const uint16_t *resid, uint32_t B) {
     prism_cuda_ctx *ctx = e->ctx;
+    bool few = false;
+    if (!ctx->batch_gemv_max && B >= 2 && ctx->gemm_variant == 1 && ctx->gemv_variant == 1 && e->gu && xs >= t.k) PRISM_TRY(gemm_reg_takes(ctx, mode, t, B, &few));
+    if (few) return launch_gemm_reg(ctx, mode, t, t2, x, xs, y, ys, resid, B, -1.0f);
     const uint32_t gemv_max = ctx->batch_gemv_max ? (uint32_t)ctx->batch_gemv_max
                               : gemm_pays_at_8(t.m, t.k, t.bits, mode == GEMV_SWIGLU, (uint32_t)ctx->sm_count) ? 7 : 8;
     const bool gemm_ok = B > gemv_max && ctx->gemm_variant == 1 && e->gu && gemm_tc5_eligible(ctx, t, B) && xs == t.k &&

@@ -584,6 +584,15 @@ int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor 
     if (reinterpret_cast<uintptr_t>(X) & 15) return fail(ctx, PRISM_E_ARG, "gemm: X must be 16-byte aligned");
     return tg.bits == 2 ? swiglu_bits<2>(ctx, tg, tu, X, m_tok, act) : swiglu_bits<4>(ctx, tg, tu, X, m_tok, act);
 }
+int gemm_tc5_stages(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok, uint32_t subs, uint32_t *stages) {
+    uint32_t pairs = 0;
+    PRISM_TRY(t.bits == 2 ? gm_pairs<2>(ctx, &pairs) : gm_pairs<4>(ctx, &pairs));
+    const GemmArgs a = gm_args(ctx, t, m_tok, nullptr);
+    const GmPlan p = gm_plan(pairs, a.n_rp, a.n_st, m_tok, subs, subs == 1 ? GM_MAX_SPLITS : 1);
+    const uint32_t tiles = a.n_rp * ((m_tok + p.nt - 1) / p.nt);
+    *stages = (tiles * p.splits + pairs - 1) / pairs * subs * ((a.n_st + p.splits - 1) / p.splits);
+    return PRISM_OK;
+}
 // Whether that pays: tiles may be so few that two launches with K cut into ranges and a pass over their outputs take less.
 int swiglu_tc5_pays(prism_cuda_ctx *ctx, const LutTensor &tg, uint32_t m_tok, bool *pays) {
     uint32_t pairs = 0;

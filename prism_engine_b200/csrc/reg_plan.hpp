@@ -1,0 +1,86 @@
+// How the register-palette GEMM (gemm_reg.cu) divides a linear; kept free of CUDA so that it can be checked on a host
+// (tests/cpp/test_reg_plan.cpp).
+#pragma once
+
+#include <cstddef>
+#include <cstdint>
+
+namespace prism {
+
+constexpr uint32_t REG_MAX_TOKENS = 32;
+
+// Whether that kernel takes less time than the ones beside it -- the batched GEMV up to 8 tokens, the tcgen05 GEMM above, the
+// stream-K GEMV for one -- for `tensors` (2: gate and up) of m rows of k weights.  `stages`: weight stages of 128 k that a pair of
+// CTAs of the GEMM goes through.  Measured on 20 shapes at 2 and 4 bits, cold weights, other / this in us:
+//  * one token: at 4 bits the pair tables are ahead wherever they are used (3584 x 3584 5.8 / 8.4, gate and up of 18944 x 3584
+//    20.3 / 30.0); at 2 bits this one has the two tensors of such a gate and up (21.9 / 18.4), less is even, more is behind
+//    (29568 x 8192 53.9 / 57.2), and single tensors (3584 x 18944 12.1 / 14.0, 19008 x 3584 11.2 / 15.6);
+//  * 2 bits, 2 tokens and more: ahead (18944 x 3584, two: 34.8 / 18.6 at 2 tokens, 32.9 / 19.3 at 8, 33.6 / 22.4 at 16) up to 24
+//    tokens, above that up to 2^25 weights (3584 x 18944 23.3 / 28.9);
+//  * 4 bits, up to 2^25 weights: ahead (3584 x 3584 13.0 / 8.4 at 8 tokens, 15.7 / 11.7 at 32; 896 x 4864 26.6 / 5.8 at 16;
+//    5120 x 2048, two: 12.0 / 10.6 at 2);
+//  * 4 bits, more weights: behind at 2 tokens (8192 x 8192 15.1 / 18.8), at 3 and 4 for long rows (8192 x 29568 44.9 / 55.4;
+//    18944 x 3584, two: 36.9 / 30.1), ahead from 5 on (26.5 / 22.9 for 3584 x 18944) to 16 unless the part of X that a CTA holds gets
+//    short of shared memory (8192 x 29568 65.5 / 74.5), and to 24 where the GEMM has 48 stages and more (18944 x 3584, one
+//    21 / 24, two 40.3 / 36.4; 19008 x 3584 33.1 / 25.3; 3584 x 18944 26.6 / 27.7).
+inline bool reg_pays(uint64_t m, uint64_t k, uint32_t bits, uint32_t tensors, uint32_t tokens, uint32_t stages) {
+    const uint64_t weights = m * k * tensors;
+    const bool few = weights < 1u << 25;
+    if (tokens <= 1) return bits == 2 && tensors == 2 && weights >= 1u << 25 && weights < 1u << 28;
+    if (bits == 2) return few || tokens <= 24;
+    if (few) return true;
+    if (tokens <= 2) return false;
+    if (tokens <= 4) return k < 8192;
+    if (tokens <= 8) return true;
+    if (tokens <= 16) return k < 24576 || tensors == 2;
+    return tokens <= 24 && stages >= 48;
+}
+constexpr size_t REG_MAX_SMEM = 227 * 1024 - 1024;
+
+// A cluster of `ctas` CTAs owns `rows` half-blocks of 32 output rows; CTA r of it takes the r-th part of K for all of them, and
+// cuts its part into `parts`: (half-block, tensor, part) is a job of one of its 16 warps.
+struct RegPlan {
+    uint32_t ctas = 0, rows = 0, parts = 0, clusters = 0;
+    size_t smem = 0;
+    double cost = 1e30;
+};
+constexpr uint32_t REG_WARPS = 16;
+constexpr uint32_t REG_NORM_BYTES = 256;  // shared memory before the activations
+
+// n_hb half-blocks of 32 rows, subs tensors (2: gate and up), n_chunks 16-byte index chunks a row; resident[i]: clusters of 2^i
+// CTAs that the GPU holds at once.
+// The cost orders the choices (it is about cycles, without what all have in common): a step, four chunks of 32 rows by one warp,
+// keeps an SM sub-partition's integer pipe busy for `busy` and takes a warp that is alone there `chain`; the activations of a part
+// come at 16 bytes a cycle; a job's sums cost 140 per eight tokens on their way, the cluster barrier 1000.  Fitted to 4 to 12 choices
+// for each of 80 cases (20 shapes of 2 and 4 bits, 8 to 32 tokens, measured back to back with cold weights): the choice takes
+// 1.1 % more than the best one on average, 12 % at most.
+inline RegPlan reg_plan(uint32_t n_hb, uint32_t subs, uint32_t n_chunks, uint32_t bits, uint32_t tokens, const uint32_t (&resident)[4]) {
+    RegPlan best;
+    const uint32_t n_steps = (n_chunks + 3) / 4, nt = (tokens + 7) / 8, units = bits == 4 ? 4 : 8;
+    const double more = nt - 1.0, busy = bits == 4 ? 800.0 + 66.0 * more : 1540.0 + 180.0 * more,
+                 chain = bits == 4 ? 2900.0 + 340.0 * more : 3450.0 + 500.0 * more;
+    for (uint32_t i = 0; i < 4; i++) {
+        const uint32_t ctas = 1u << i;
+        if (!resident[i] || ctas > n_steps) continue;
+        const uint32_t rows = (n_hb + resident[i] - 1) / resident[i], span = (n_steps + ctas - 1) / ctas;
+        for (uint32_t parts = 1; parts <= REG_WARPS && parts <= span; parts++) {
+            const uint32_t jobs = rows * subs * parts;
+            RegPlan p;
+            p.ctas = ctas;
+            p.rows = rows;
+            p.parts = parts;
+            p.clusters = (n_hb + rows - 1) / rows;
+            const size_t x = (size_t)span * units * nt * 512, sums = (size_t)((rows * 4 + ctas - 1) / ctas) * subs * ctas * parts * nt * 256;
+            p.smem = REG_NORM_BYTES + x + sums;
+            if (p.smem > REG_MAX_SMEM) break;
+            const double steps = (span + parts - 1) / parts, rounds = (jobs + REG_WARPS - 1) / REG_WARPS, last = jobs % REG_WARPS;
+            const double per = jobs / REG_WARPS * (REG_WARPS / 4) + (uint32_t)(last + 3) / 4;  // jobs of the first sub-partition
+            p.cost = x / 16.0 + (per * steps * busy > rounds * steps * chain ? per * steps * busy : rounds * steps * chain) + rounds * 150.0 +
+                     (ctas > 1 ? 1000.0 : 0.0) + jobs * nt * 140.0;
+            if (p.cost < best.cost) best = p;
+        }
+    }
+    return best;
+}
+
+}  // namespace prism

@@ -57,3 +57,11 @@ def gemm_swiglu(backend, gate, up, x, out, fused):
         return _call(backend, "_ZN5prism17launch_swiglu_tc5EP14prism_cuda_ctxRKNS_9LutTensorES4_PKtjPt", *a)
     u = torch.empty_like(out)
     _call(backend, "_ZN5prism18launch_gemm_swigluEP14prism_cuda_ctxRKNS_9LutTensorES4_PKtjPtS7_", *a, C.c_void_p(u.data_ptr()))
+
+
+def linear_few_tokens(backend, handle, x, y, resid=None, up=None, norm_eps=-1.0):
+    """y = x W^T of 1..32 rows by the register-palette kernel: plain, with a residual, or silu(gate) * up; rows of y may be apart."""
+    mode = 2 if up is not None else 0 if resid is None else 1
+    _call(backend, "_ZN5prism15launch_gemm_regEP14prism_cuda_ctxNS_8GemvModeERKNS_9LutTensorEPS4_PKtjPtjS8_jf", C.c_int(mode), _tensor(backend, handle),
+          _tensor(backend, up) if up is not None else None, C.c_void_p(x.data_ptr()), C.c_uint32(x.stride(0)), C.c_void_p(y.data_ptr()),
+          C.c_uint32(y.stride(0)), C.c_void_p(resid.data_ptr()) if resid is not None else None, C.c_uint32(x.shape[0]), C.c_float(norm_eps))
