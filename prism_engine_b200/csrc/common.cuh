@@ -315,7 +315,7 @@ bool gemm_tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok);
 bool gemm_tc5_wide(const LutTensor &t, const uint16_t *y);  // rows of y can be moved 16 bytes at a time, as `resid` and SwiGLU need it
 int launch_gemm_tc5(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *Y, const uint16_t *resid);
 int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act);
-int gemm_tc5_stages(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok, uint32_t subs, uint32_t *stages);  // that a pair of CTAs goes through
+int gemm_tc5_cycles(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok, uint32_t subs, double *cycles);  // estimated; subs 2: SwiGLU, as it pays
 int swiglu_tc5_pays(prism_cuda_ctx *ctx, const LutTensor &tg, uint32_t m_tok, bool *pays);
 
 // glue.cu

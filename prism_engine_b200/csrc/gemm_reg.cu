@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(REG_WARPS * 32, 1) lut_gemm_reg_kernel(const R
 
 // ---- host side ---------------------------------------------------------------------------------
 template <int BITS, int NT>
-static int launch_reg(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, bool dry, bool *fits) {
+static int launch_reg(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, bool dry, RegPlan *plan) {
     static uint32_t resident[PRISM_MAX_DEVICES][4] = {{0}};
     uint32_t (&res)[4] = resident[ctx->device];
     if (!res[0]) {
@@ -327,8 +327,7 @@ static int launch_reg(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, bool 
         }
         res[0] = (uint32_t)ctx->sm_count;
     }
-    const RegPlan p = reg_plan((t.m + 31) / 32, a.subs, t.n_chunks, BITS, a.batch, res);
-    *fits = p.ctas != 0;
+    const RegPlan p = *plan = reg_plan((t.m + 31) / 32, a.subs, t.n_chunks, BITS, a.batch, res);
     if (dry || !p.ctas) return PRISM_OK;
     a.ctas = p.ctas;
     a.rows = p.rows;
@@ -338,18 +337,18 @@ static int launch_reg(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, bool 
     return after_launch(ctx, "lut_gemm_reg_kernel");
 }
 
-static int reg_dispatch(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, bool dry, bool *fits) {
+static int reg_dispatch(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, bool dry, RegPlan *plan) {
     const uint32_t nt = (a.batch + 7) / 8;
     if (t.bits == 4) {
-        if (nt == 1) return launch_reg<4, 1>(ctx, a, t, dry, fits);
-        if (nt == 2) return launch_reg<4, 2>(ctx, a, t, dry, fits);
-        if (nt == 3) return launch_reg<4, 3>(ctx, a, t, dry, fits);
-        return launch_reg<4, 4>(ctx, a, t, dry, fits);
+        if (nt == 1) return launch_reg<4, 1>(ctx, a, t, dry, plan);
+        if (nt == 2) return launch_reg<4, 2>(ctx, a, t, dry, plan);
+        if (nt == 3) return launch_reg<4, 3>(ctx, a, t, dry, plan);
+        return launch_reg<4, 4>(ctx, a, t, dry, plan);
     }
-    if (nt == 1) return launch_reg<2, 1>(ctx, a, t, dry, fits);
-    if (nt == 2) return launch_reg<2, 2>(ctx, a, t, dry, fits);
-    if (nt == 3) return launch_reg<2, 3>(ctx, a, t, dry, fits);
-    return launch_reg<2, 4>(ctx, a, t, dry, fits);
+    if (nt == 1) return launch_reg<2, 1>(ctx, a, t, dry, plan);
+    if (nt == 2) return launch_reg<2, 2>(ctx, a, t, dry, plan);
+    if (nt == 3) return launch_reg<2, 3>(ctx, a, t, dry, plan);
+    return launch_reg<2, 4>(ctx, a, t, dry, plan);
 }
 
 static RegArgs reg_args(GemvMode mode, const LutTensor &t, const LutTensor *t2, uint32_t batch) {
@@ -367,12 +366,14 @@ int gemm_reg_takes(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, uint3
     *takes = false;
     if (mode != GEMV_PLAIN && mode != GEMV_RESID && mode != GEMV_SWIGLU) return PRISM_OK;
     if (batch == 0 || batch > REG_MAX_TOKENS || t.m == 0 || !((t.bits == 4 && t.k % 32 == 0 && t.k >= 32) || (t.bits == 2 && t.k % 64 == 0 && t.k >= 64))) return PRISM_OK;
-    const uint32_t tensors = mode == GEMV_SWIGLU ? 2 : 1;
-    uint32_t stages = 0xFFFFFFFFu;
-    if (batch > 16 && gemm_tc5_eligible(ctx, t, batch)) PRISM_TRY(gemm_tc5_stages(ctx, t, batch, tensors, &stages));
-    if (!reg_pays(t.m, t.k, t.bits, tensors, batch, stages) && (batch < 8 || gemm_tc5_eligible(ctx, t, batch))) return PRISM_OK;
     RegArgs a = reg_args(mode, t, nullptr, batch);
-    return reg_dispatch(ctx, a, t, true, takes);
+    RegPlan plan;
+    PRISM_TRY(reg_dispatch(ctx, a, t, true, &plan));
+    if (!plan.ctas) return PRISM_OK;
+    double gemm = 1e30;
+    if (gemm_tc5_eligible(ctx, t, batch)) PRISM_TRY(gemm_tc5_cycles(ctx, t, batch, a.subs, &gemm));
+    *takes = reg_pays(t.m, t.k, t.bits, a.subs, batch, plan.cycles, gemm);
+    return PRISM_OK;
 }
 
 int launch_gemm_reg(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,
@@ -383,9 +384,9 @@ int launch_gemm_reg(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, cons
     a.y = y; a.y_stride = y_stride; a.resid = resid;
     a.norm_eps = norm_eps;
     a.wide = y_stride % 8 == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(resid)) & 15) == 0;
-    bool fits;
-    PRISM_TRY(reg_dispatch(ctx, a, t, false, &fits));
-    return fits ? PRISM_OK : fail(ctx, PRISM_E_ARG, "gemm: this shape does not fit the register-palette kernel");
+    RegPlan plan;
+    PRISM_TRY(reg_dispatch(ctx, a, t, false, &plan));
+    return plan.ctas ? PRISM_OK : fail(ctx, PRISM_E_ARG, "gemm: this shape does not fit the register-palette kernel");
 }
 
 }  // namespace prism

@@ -19,11 +19,14 @@
 // (sk_expand2, pair_table.cuh).
 // Bound: with many tokens the tensor core under the power cap; with few, the table lookups (256 cycles of the
 // shared-memory pipe per 128 x 128 weights) and the latency of a short chain of stages.
-// Measured, 4 bit, against one CTA per 128 x 256 tile whose single issuing thread spent 1 700 cycles on a stage of 1 024
+// Measured, 4 bit, when it replaced one CTA per 128 x 256 tile whose single issuing thread spent 1 700 cycles on a stage of 1 024
 // (waits one after the other, descriptors through vector registers, three commits) and which used as many CTAs as there were
 // row tiles: 18944 x 3584, 2048 tokens 266 -> 216 us (1 287 TFLOP/s, 0.78 of measured burst), 512 tokens 67 -> 54, 32 tokens
 // 26 -> 19.9; 4608 x 3584, 2048 tokens 72 -> 53, 32 tokens 23.4 -> 15.1; 3584 x 18944, 2048 tokens 320 -> 278, 32 tokens
 // 96.5 -> 25.0.  The times before are without the residual or SwiGLU passes and the re-laid activations that went with them.
+// A kernel of its own for split K (neither form holds the other's registers: 200 bytes of spills -> none and 48), the first table
+// beside the TMEM allocation, the sums of four ranges requested together, and tiles by the fitted estimate of gm_plan: 3584 x 3584
+// 15.7 -> 11.5 at 32 tokens, 3584 x 18944 26.5 -> 20.5 at 32, 81 -> 58 at 400, 269 -> 220 at 2048, gate and up of 18944 x 3584 40.1 -> 35.1.
 // Every mbarrier wait is bounded; a wait that gives up raises the context's device error word.
 #include <algorithm>
 
@@ -114,8 +117,9 @@ __device__ __forceinline__ void gm_lookup16(uint32_t (&A)[16], const uint4 &wv, 
 struct GmItem {
     uint32_t rp, tt, k0, k1;  // k in stages
 };
+template <bool SPLIT>
 __device__ __forceinline__ GmItem gm_item(const GemmArgs &a, uint32_t w) {
-    if (a.splits == 1) return GmItem{w % a.n_rp, w / a.n_rp, 0, a.n_st};
+    if (!SPLIT) return GmItem{w % a.n_rp, w / a.n_rp, 0, a.n_st};
     const uint32_t s = w % a.splits, t = w / a.splits;
     return GmItem{t % a.n_rp, t / a.n_rp, a.n_st * s / a.splits, a.n_st * (s + 1) / a.splits};
 }
@@ -173,7 +177,7 @@ __device__ __forceinline__ uint32_t gm_pack(float x, float y) {
 
 }  // namespace
 
-template <int BITS>
+template <int BITS, bool SPLIT>
 __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem);
@@ -197,7 +201,42 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
     const uint32_t xstage = a.nt * 64;                  // bytes of this CTA's half of the tokens
     auto x_addr = [&](uint32_t s) { return base + (s < a.sx_low ? GM_X_LOW + s * xstage : GM_X_HIGH + (s - a.sx_low) * xstage); };
 
-    if (tid == 0) {
+    // Dequantising warps: TMEM lane quarter, slot within the quarter; table area, row slot inside its entries.
+    const uint32_t q = warp & 3, j = warp >> 2, area = q & 1, slot = q >> 1;
+    uint4 r[ICPS];
+    auto row_block = [&](const GmItem &i) { return min(4 * (2 * i.rp + rank) + q, a.n_hb - 1); };
+    auto chunks = [&](const GmItem &i, uint32_t sub) { return (sub ? a.idx2 : a.idx) + (size_t)row_block(i) * a.n_ichunks * 512 + lane * 16; };
+    auto build_table = [&](const GmItem &it, uint32_t sub) {
+        uint8_t *tb = win + GM_TBL + area * 65536 + lane * 4 + slot * 128;
+        if (BITS == 4) {
+            const uint16_t *prow = (sub ? a.pal2 : a.pal) + ((size_t)row_block(it) * 32 + lane) * 16;
+            const uint4 p0 = *reinterpret_cast<const uint4 *>(prow);
+            const uint4 p1 = *reinterpret_cast<const uint4 *>(prow + 8);
+            const uint32_t cbp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+            const uint32_t hp0 = reinterpret_cast<const uint32_t *>(prow)[2 * j];
+            const uint32_t hp1 = reinterpret_cast<const uint32_t *>(prow)[2 * j + 1];
+            tb += j * 16384;
+#pragma unroll
+            for (int lo = 0; lo < 16; lo++) {
+#pragma unroll
+                for (int hs = 0; hs < 4; hs++) {
+                    const uint32_t sel = (((hs & 1) ? 0x76u : 0x54u) << 8) | ((lo & 1) ? 0x32u : 0x10u);
+                    *reinterpret_cast<uint32_t *>(tb + lo * 256 + hs * 4096) = __byte_perm(cbp[lo >> 1], (hs & 2) ? hp1 : hp0, sel);
+                }
+            }
+        } else {
+            // 16-entry nibble table: entry e = i0 | i1 << 2 -> half2{pal[i0], pal[i1]}; slot j writes e = 4j..4j+3
+            const uint2 pp = *reinterpret_cast<const uint2 *>((sub ? a.pal2 : a.pal) + ((size_t)row_block(it) * 32 + lane) * 4);
+            const uint32_t v1 = ((j & 2) ? pp.y : pp.x) >> ((j & 1) * 16) & 0xFFFFu;  // pal[i1], i1 = j
+#pragma unroll
+            for (uint32_t i0 = 0; i0 < 4; i0++) {
+                const uint32_t v0 = ((i0 & 2) ? pp.y : pp.x) >> ((i0 & 1) * 16) & 0xFFFFu;
+                *reinterpret_cast<uint32_t *>(tb + (4 * j + i0) * 256) = v0 | (v1 << 16);
+            }
+        }
+    };
+
+    if (tid == GM_THREADS - 32) {
         for (int s = 0; s < GM_SA; s++) { t5::mbar_init(b_afull + 8 * s, 8); t5::mbar_init(b_done + 8 * s, 1); }
         for (int s = 0; s < GM_SX_MAX; s++) t5::mbar_init(b_xfull + 8 * s, 1);
         for (int s = 0; s < GM_XD; s++) t5::mbar_init(b_xdone + 8 * s, 1);
@@ -207,6 +246,17 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == GM_MMA_WARP) t5::tmem_alloc_pair(base + GM_STATE + 8, 512);
+    // The first tile's indices and table, beside the allocation: every pair has a tile (the grid is no larger than they are).
+    if (warp < GM_DEQ_WARPS) {
+        const GmItem it = gm_item<SPLIT>(a, pair_id);
+        const uint32_t su = it.k0 + j;
+        if (su < it.k1) {
+            const uint8_t *sp = chunks(it, 0) + (size_t)su * ICPS * 512;
+#pragma unroll
+            for (int c = 0; c < ICPS; c++) r[c] = t5::ldg128_nc(sp + c * 512);
+        }
+        build_table(it, 0);
+    }
     t5::fence_before();
     __syncthreads();
     t5::cluster_sync();  // the other CTA's barriers exist before anything arrives there
@@ -215,81 +265,97 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
 
     if (warp < GM_DEQ_WARPS) {
         // =============================== dequantising warps ===============================
-        const uint32_t q = warp & 3, j = warp >> 2;      // TMEM lane quarter, slot within the quarter
-        const uint32_t area = q & 1, slot = q >> 1;      // table area, row slot inside its entries
         const uint32_t laneq = base + GM_TBL + area * 65536 + lane * 4;
         const uint32_t tmem_lane = tmem_base + ((q * 32) << 16);
         const uint32_t afull0 = t5::map_rank(b_afull + 8 * j, 0), dempty0 = t5::map_rank(b_dempty, 0);
         uint8_t *out = win + (warp < GM_OUT_LOW_WARPS ? GM_OUT_LOW + warp * 1024 : GM_OUT_HIGH + (warp - GM_OUT_LOW_WARPS) * 1024);
         const uint32_t groups = a.nt / 16;               // of 16 accumulator columns; this warp takes j, j + 4, ...
-        uint32_t n = 0, ti = 0, cur = 0xFFFFFFFFu;
+        uint32_t n = 0, ti = 0, cur = gm_item<SPLIT>(a, pair_id).rp * 2;  // the tables are those of tensor `sub` (lowest bit), row pair
         uint32_t pend_w = 0xFFFFFFFFu, pend_sub = 0;     // the tile whose sums are still in TMEM
-        bool waited = false;
+        bool waited = false, ahead = true;                // ahead: r holds this slot's first stage of the tile already
 
         auto epilogue = [&](uint32_t w, uint32_t sub) {
-            const GmItem it = gm_item(a, w);
-            const uint32_t row = (2 * it.rp + rank) * 128 + q * 32 + lane, tile = w / a.splits, place = rank * GM_DEQ_WARPS + warp;
+            const GmItem it = gm_item<SPLIT>(a, w);
+            const uint32_t row = (2 * it.rp + rank) * 128 + q * 32 + lane, tile = SPLIT ? w / a.splits : w, place = rank * GM_DEQ_WARPS + warp;
             const uint32_t per = (groups + 3) / 4 * 512;  // floats of a warp
             t5::mbar_wait_warp(b_dfull, ti & 1, err_flag);
             t5::fence_after();
             ti++;
-            uint32_t sums[4][8];
+            auto store = [&](const uint32_t (&v)[8], uint32_t i) {
+                const uint32_t t0 = it.tt * a.nt + (j + 4 * i) * 16;
+                if (a.wide) gm_store_wide(a, v, t0, row - lane, sub, out);
+                else gm_store(a, v, t0, row);
+            };
+            if (!SPLIT) {
+                uint32_t sums[4][8];
 #pragma unroll
-            for (uint32_t i = 0; i < 4; i++) {
-                if (j + 4 * i >= groups) break;
-                uint32_t v[16];
-                t5::ld16(tmem_lane + GM_D_COL + (j + 4 * i) * 16, v);
-                t5::wait_ld();
-                if (a.splits == 1) {
+                for (uint32_t i = 0; i < 4; i++) {
+                    if (j + 4 * i >= groups) break;
+                    uint32_t v[16];
+                    t5::ld16(tmem_lane + GM_D_COL + (j + 4 * i) * 16, v);
+                    t5::wait_ld();
 #pragma unroll
                     for (uint32_t c = 0; c < 8; c++) sums[i][c] = gm_pack(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
-                } else {
+                }
+                t5::fence_before();
+                __syncwarp();
+                if (lane == 0) t5::mbar_arrive_tmem(dempty0);
+#pragma unroll
+                for (uint32_t i = 0; i < 4; i++) {
+                    if (j + 4 * i >= groups) break;
+                    store(sums[i], i);
+                }
+            } else {
+                for (uint32_t i = 0; j + 4 * i < groups; i++) {
+                    uint32_t v[16];
+                    t5::ld16(tmem_lane + GM_D_COL + (j + 4 * i) * 16, v);
+                    t5::wait_ld();
                     float *mine = a.part + ((size_t)w * 2 * GM_DEQ_WARPS + place) * per + i * 512 + lane;
 #pragma unroll
                     for (uint32_t c = 0; c < 16; c++) __stcg(mine + c * 32, __uint_as_float(v[c]));
                 }
-            }
-            t5::fence_before();
-            __syncwarp();
-            if (lane == 0) t5::mbar_arrive_tmem(dempty0);
-            if (a.splits > 1) {
-                __threadfence();
+                t5::fence_before();
                 __syncwarp();
                 uint32_t before = 0;
-                if (lane == 0) before = atomicAdd(a.arrived + (size_t)tile * 2 * GM_DEQ_WARPS + place, 1u);
+                if (lane == 0) {
+                    t5::mbar_arrive_tmem(dempty0);
+                    __threadfence();
+                    before = atomicAdd(a.arrived + (size_t)tile * 2 * GM_DEQ_WARPS + place, 1u);
+                    __threadfence();
+                }
                 if (__shfl_sync(0xFFFFFFFFu, before, 0) != a.splits - 1) return;
-                __threadfence();
+                __syncwarp();
                 if (lane == 0) a.arrived[(size_t)tile * 2 * GM_DEQ_WARPS + place] = 0;
-            }
-#pragma unroll
-            for (uint32_t i = 0; i < 4; i++) {
-                if (j + 4 * i >= groups) break;
-                if (a.splits > 1) {
+                const size_t step = (size_t)2 * GM_DEQ_WARPS * per;
+                for (uint32_t i = 0; j + 4 * i < groups; i++) {
                     const float *p = a.part + ((size_t)tile * a.splits * 2 * GM_DEQ_WARPS + place) * per + i * 512 + lane;
                     float f[16];
 #pragma unroll
                     for (uint32_t c = 0; c < 16; c++) f[c] = 0.0f;
-                    for (uint32_t s = 0; s < a.splits; s++, p += (size_t)2 * GM_DEQ_WARPS * per)
+                    for (uint32_t s = 0; s < a.splits; s += 4, p += 4 * step) {  // four ranges requested together, added in order
+                        float g[4][16];
 #pragma unroll
-                        for (uint32_t c = 0; c < 16; c++) f[c] += __ldcg(p + c * 32);
+                        for (uint32_t u = 0; u < 4; u++)
 #pragma unroll
-                    for (uint32_t c = 0; c < 8; c++) sums[i][c] = gm_pack(f[2 * c], f[2 * c + 1]);
+                            for (uint32_t c = 0; c < 16; c++) g[u][c] = s + u < a.splits ? __ldcg(p + u * step + c * 32) : 0.0f;
+#pragma unroll
+                        for (uint32_t u = 0; u < 4; u++)
+#pragma unroll
+                            for (uint32_t c = 0; c < 16; c++) f[c] += g[u][c];
+                    }
+                    uint32_t v[8];
+#pragma unroll
+                    for (uint32_t c = 0; c < 8; c++) v[c] = gm_pack(f[2 * c], f[2 * c + 1]);
+                    store(v, i);
                 }
-                const uint32_t t0 = it.tt * a.nt + (j + 4 * i) * 16;
-                if (a.wide) gm_store_wide(a, sums[i], t0, row - lane, sub, out);
-                else gm_store(a, sums[i], t0, row);
             }
             __syncwarp();
         };
 
-        uint4 r[ICPS];
-        bool ahead = false;                              // r holds this slot's first stage of the tile already
         bool late = false;                               // this slot's last stage was one of the last two of its tile
-        auto row_block = [&](const GmItem &i) { return min(4 * (2 * i.rp + rank) + q, a.n_hb - 1); };
-        auto chunks = [&](const GmItem &i, uint32_t sub) { return (sub ? a.idx2 : a.idx) + (size_t)row_block(i) * a.n_ichunks * 512 + lane * 16; };
         for (uint32_t w = pair_id, sub = 0;;) {
             const bool over = w >= n_items;              // past the last tile: its sums are still to be stored
-            GmItem it = gm_item(a, w);
+            GmItem it = gm_item<SPLIT>(a, w);
             if (over) it.k0 = it.k1 = 0;
             {
                 uint32_t su = it.k0 + ((j - n) & 3);     // this slot's first stage: ring position j
@@ -301,33 +367,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                 if (!over && it.rp * 2 + sub != cur) {  // same decision in all warps: they walk the same item list
                     cur = it.rp * 2 + sub;
                     asm volatile("bar.sync %0, 256;\n" ::"r"(1 + area) : "memory");  // lookups of the previous tile are done
-                    uint8_t *tb = win + GM_TBL + area * 65536 + lane * 4 + slot * 128;
-                    if (BITS == 4) {
-                        const uint16_t *prow = (sub ? a.pal2 : a.pal) + ((size_t)row_block(it) * 32 + lane) * 16;
-                        const uint4 p0 = *reinterpret_cast<const uint4 *>(prow);
-                        const uint4 p1 = *reinterpret_cast<const uint4 *>(prow + 8);
-                        const uint32_t cbp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-                        const uint32_t hp0 = reinterpret_cast<const uint32_t *>(prow)[2 * j];
-                        const uint32_t hp1 = reinterpret_cast<const uint32_t *>(prow)[2 * j + 1];
-                        tb += j * 16384;
-#pragma unroll
-                        for (int lo = 0; lo < 16; lo++) {
-#pragma unroll
-                            for (int hs = 0; hs < 4; hs++) {
-                                const uint32_t sel = (((hs & 1) ? 0x76u : 0x54u) << 8) | ((lo & 1) ? 0x32u : 0x10u);
-                                *reinterpret_cast<uint32_t *>(tb + lo * 256 + hs * 4096) = __byte_perm(cbp[lo >> 1], (hs & 2) ? hp1 : hp0, sel);
-                            }
-                        }
-                    } else {
-                        // 16-entry nibble table: entry e = i0 | i1 << 2 -> half2{pal[i0], pal[i1]}; slot j writes e = 4j..4j+3
-                        const uint2 pp = *reinterpret_cast<const uint2 *>((sub ? a.pal2 : a.pal) + ((size_t)row_block(it) * 32 + lane) * 4);
-                        const uint32_t v1 = ((j & 2) ? pp.y : pp.x) >> ((j & 1) * 16) & 0xFFFFu;  // pal[i1], i1 = j
-#pragma unroll
-                        for (uint32_t i0 = 0; i0 < 4; i0++) {
-                            const uint32_t v0 = ((i0 & 2) ? pp.y : pp.x) >> ((i0 & 1) * 16) & 0xFFFFu;
-                            *reinterpret_cast<uint32_t *>(tb + (4 * j + i0) * 256) = v0 | (v1 << 16);
-                        }
-                    }
+                    build_table(it, sub);
                     asm volatile("bar.sync %0, 256;\n" ::"r"(1 + area) : "memory");
                 }
                 // Everything so far read weights only.  The waits below depend on the activations: wait for the kernel
@@ -337,7 +377,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                     pdl_wait();
                     waited = true;
                 }
-                for (bool first = true; first || su < it.k1; first = false, su += 4) {
+                for (bool first = true; first || su < it.k1 || pend_w != 0xFFFFFFFFu; first = false, su += 4) {
                     // The tile before.  A slot that finished early expands its first stage of this one before it waits for the sums, so
                     // that the tensor core has something to go on with; the slots of the last two stages take the sums out first.  Nobody
                     // comes to a second stage before that: it waits for products that wait for these sums.
@@ -351,7 +391,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                         bool fill = su + 4 < it.k1;
                         if (!fill) {
                             const uint32_t nsub = sub + 1 == a.subs ? 0 : sub + 1, nw = nsub ? w : w + n_pairs;
-                            const GmItem ni = gm_item(a, nw);
+                            const GmItem ni = gm_item<SPLIT>(a, nw);
                             const uint32_t nsu = ni.k0 + ((j - (n + it.k1 - it.k0)) & 3);
                             ahead = fill = nw < n_items && nsu < ni.k1;
                             np = chunks(ni, nsub) + (size_t)nsu * ICPS * 512;
@@ -387,7 +427,6 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
                     }
                 }
                 if (over) break;
-                if (pend_w != 0xFFFFFFFFu) epilogue(pend_w, pend_sub);
             }
             pend_w = w;
             pend_sub = sub;
@@ -408,7 +447,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
             pdl_wait();  // see the dequantising warps: no bounded wait before the dependency is met
             uint32_t ready = 0;                            // this stage's weights (1) and activations (2, 4) have been seen to be there
             for (uint32_t w = pair_id; w < n_items; w += n_pairs) {
-                const GmItem it = gm_item(a, w);
+                const GmItem it = gm_item<SPLIT>(a, w);
                 for (uint32_t sub = 0; sub < a.subs; sub++, ti++) {
                     t5::mbar_wait_bounded(b_dempty, (ti & 1) ^ 1, err_flag);  // the sums of the tile before have left D
                     for (uint32_t su = it.k0; su < it.k1; su++, n++) {
@@ -450,7 +489,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) lut_gemm_tc5_kernel(const GemmA
         auto wait_step = [&](uint32_t step) { t5::mbar_wait_bounded(b_step + 8 * (step % ring), (step / ring) & 1, err_flag); };
         pdl_wait();
         for (uint32_t w = pair_id; w < n_items; w += n_pairs) {
-            const GmItem it = gm_item(a, w);
+            const GmItem it = gm_item<SPLIT>(a, w);
             const int32_t t0 = (int32_t)(it.tt * a.nt + rank * (a.nt / 2));
             for (uint32_t sub = 0; sub < a.subs; sub++) {
                 for (uint32_t k = it.k0 * 128; k < it.k1 * 128; k += 64, h++) {
@@ -479,10 +518,12 @@ bool gemm_tc5_eligible(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok) 
 }
 bool gemm_tc5_wide(const LutTensor &t, const uint16_t *y) { return t.m % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0; }
 
-// Tokens of a tile and ranges of K with the least estimated cycles.  A stage takes the tensor core 4 nt cycles; expanding
-// its weights takes 256 of the shared-memory pipe and streaming them about 350 at the HBM rate.  A tile's fill and last
-// stores cost about 2500 once, 700 for each further tile of the same pair.  A split pays for its sums' way through L2 and
-// for the wait for the last of them.
+// Tokens of a tile and ranges of K with the least estimated cycles: a stage's products or its look-ups and hand-overs, a tile's way
+// into and out of the pipeline, a launch, the tables of another pair of row tiles; a split pays for its sums' way through L2 and the
+// wait for the last of them.  Fitted to every choice (tiles of 32 to 256 tokens, 1 to 8 ranges) for 17 shapes of 2 and 4 bits and
+// 24 to 2048 tokens, cold weights: within 12 % of the times, and what it chooses takes 0.7 % more than the best choice on average,
+// 10 % at most.  The estimate before took 5 % more on average and up to 1.5 times as long: it only weighed tiles near 256 tokens
+// (3584 x 18944, 2048 tokens: 256 tokens and 112 tiles for 74 pairs 261 us, 224 and 140 220; 8192 x 8192, 100 tokens 39 and 28).
 struct GmPlan {
     uint32_t nt = 32, splits = 1;
     double cycles = 1e30;
@@ -490,13 +531,13 @@ struct GmPlan {
 static GmPlan gm_plan(uint32_t pairs, uint32_t n_rp, uint32_t n_st, uint32_t m_tok, uint32_t subs, uint32_t most_splits) {
     GmPlan best;
     const uint32_t top = std::min(256u, round_up_u32(m_tok, 32));
-    for (uint32_t nt = top; nt >= 32 && nt + 128 > top; nt -= 32) {
+    for (uint32_t nt = top; nt >= 32; nt -= 32) {
         const uint64_t tiles = (uint64_t)n_rp * ((m_tok + nt - 1) / nt);
         for (uint32_t cut = 1; cut <= most_splits && cut <= n_st; cut++) {
             if (cut > 1 && tiles * cut * 256 * nt * 4 > (64u << 20)) break;  // bytes of partial sums
-            const uint64_t waves = (tiles * cut + pairs - 1) / pairs;
-            double t = (double)waves * subs * ((n_st + cut - 1) / cut * std::max(4.0 * nt, 350.0) + 700.0) + 2500.0;
-            if (cut > 1) t += 2500.0 + (double)waves * nt * 20.0 + cut * nt * 8.0;
+            const uint64_t waves = (tiles * cut + pairs - 1) / pairs, tables = subs == 2 ? 2 * waves : cut > 1 || pairs % n_rp ? waves : 1;
+            double t = 4200.0 + (double)waves * subs * ((n_st + cut - 1) / cut * std::max(5.6 * nt, 915.0) + 6800.0) + (double)(tables - 1) * 3800.0;
+            if (cut > 1) t += 4000.0 + (double)waves * nt * 17.0 + cut * nt * 7.0;
             if (t < best.cycles * 0.999) {
                 best.cycles = t;
                 best.nt = nt;
@@ -511,8 +552,9 @@ template <int BITS>
 static int gm_pairs(prism_cuda_ctx *ctx, uint32_t *out) {  // pairs that are resident at once
     static int pairs[PRISM_MAX_DEVICES] = {0};
     if (!pairs[ctx->device]) {
-        PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(lut_gemm_tc5_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GM_SMEM_BYTES));
-        const int n = resident_clusters(lut_gemm_tc5_kernel<BITS>, 2, GM_THREADS, GM_SMEM_BYTES, 2 * ((uint32_t)ctx->sm_count / 2));
+        PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(lut_gemm_tc5_kernel<BITS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GM_SMEM_BYTES));
+        PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(lut_gemm_tc5_kernel<BITS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GM_SMEM_BYTES));
+        const int n = resident_clusters(lut_gemm_tc5_kernel<BITS, true>, 2, GM_THREADS, GM_SMEM_BYTES, 2 * ((uint32_t)ctx->sm_count / 2));
         pairs[ctx->device] = std::max(1, std::min(n, ctx->sm_count / 2));
     }
     *out = (uint32_t)pairs[ctx->device];
@@ -539,7 +581,7 @@ static int launch_gm(prism_cuda_ctx *ctx, GemmArgs &a, const LutTensor &t, const
     CUtensorMap xmap;
     PRISM_TRY(encode_tensor_map(ctx, &xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, X, t.k, a.m_tok, t.k, 64, a.nt / 2, CU_TENSOR_MAP_SWIZZLE_128B));
     const uint32_t grid = (uint32_t)std::min<uint64_t>(pairs, (uint64_t)tiles * a.splits);
-    launch_cluster_pdl(ctx, lut_gemm_tc5_kernel<BITS>, dim3(2 * grid), dim3(GM_THREADS), GM_SMEM_BYTES, 2u, a, xmap);
+    launch_cluster_pdl(ctx, a.splits > 1 ? lut_gemm_tc5_kernel<BITS, true> : lut_gemm_tc5_kernel<BITS, false>, dim3(2 * grid), dim3(GM_THREADS), GM_SMEM_BYTES, 2u, a, xmap);
     return after_launch(ctx, "lut_gemm_tc5_kernel");
 }
 
@@ -584,22 +626,34 @@ int launch_swiglu_tc5(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor 
     if (reinterpret_cast<uintptr_t>(X) & 15) return fail(ctx, PRISM_E_ARG, "gemm: X must be 16-byte aligned");
     return tg.bits == 2 ? swiglu_bits<2>(ctx, tg, tu, X, m_tok, act) : swiglu_bits<4>(ctx, tg, tu, X, m_tok, act);
 }
-int gemm_tc5_stages(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok, uint32_t subs, uint32_t *stages) {
+// Gate and up in one launch, or two launches with K cut into ranges and a pass over their outputs (5120 x 2048, 24 tokens 25.0 / 24.3 us,
+// 8192 x 4096 38.1 / 34.0; at 256 tokens 32.4 / 38.7 and 51.0 / 60.2).
+template <int BITS>
+static int gm_swiglu_cycles(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok, double *fused, double *apart) {
+    uint32_t pairs = 0;
+    PRISM_TRY(gm_pairs<BITS>(ctx, &pairs));
+    const GemmArgs a = gm_args(ctx, t, m_tok, nullptr);
+    *fused = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 2, 1).cycles;
+    *apart = 2 * gm_plan(pairs, a.n_rp, a.n_st, m_tok, 1, GM_MAX_SPLITS).cycles + 6000.0 + (double)m_tok * t.m * 8.0 / 3500.0;
+    return PRISM_OK;
+}
+int gemm_tc5_cycles(prism_cuda_ctx *ctx, const LutTensor &t, uint32_t m_tok, uint32_t subs, double *cycles) {
+    if (subs == 2) {
+        double fused = 0, apart = 0;
+        PRISM_TRY(t.bits == 2 ? gm_swiglu_cycles<2>(ctx, t, m_tok, &fused, &apart) : gm_swiglu_cycles<4>(ctx, t, m_tok, &fused, &apart));
+        *cycles = std::min(fused, apart);
+        return PRISM_OK;
+    }
     uint32_t pairs = 0;
     PRISM_TRY(t.bits == 2 ? gm_pairs<2>(ctx, &pairs) : gm_pairs<4>(ctx, &pairs));
     const GemmArgs a = gm_args(ctx, t, m_tok, nullptr);
-    const GmPlan p = gm_plan(pairs, a.n_rp, a.n_st, m_tok, subs, subs == 1 ? GM_MAX_SPLITS : 1);
-    const uint32_t tiles = a.n_rp * ((m_tok + p.nt - 1) / p.nt);
-    *stages = (tiles * p.splits + pairs - 1) / pairs * subs * ((a.n_st + p.splits - 1) / p.splits);
+    *cycles = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 1, GM_MAX_SPLITS).cycles;
     return PRISM_OK;
 }
-// Whether that pays: tiles may be so few that two launches with K cut into ranges and a pass over their outputs take less.
 int swiglu_tc5_pays(prism_cuda_ctx *ctx, const LutTensor &tg, uint32_t m_tok, bool *pays) {
-    uint32_t pairs = 0;
-    PRISM_TRY(tg.bits == 2 ? gm_pairs<2>(ctx, &pairs) : gm_pairs<4>(ctx, &pairs));
-    const GemmArgs a = gm_args(ctx, tg, m_tok, nullptr);
-    const GmPlan both = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 2, 1), one = gm_plan(pairs, a.n_rp, a.n_st, m_tok, 1, GM_MAX_SPLITS);
-    *pays = both.cycles <= 2 * one.cycles + 4000.0 + (double)m_tok * tg.m * 8.0 / 3500.0;
+    double fused = 0, apart = 0;
+    PRISM_TRY(tg.bits == 2 ? gm_swiglu_cycles<2>(ctx, tg, m_tok, &fused, &apart) : gm_swiglu_cycles<4>(ctx, tg, m_tok, &fused, &apart));
+    *pays = fused <= apart;
     return PRISM_OK;
 }
 

@@ -8,52 +8,43 @@
 namespace prism {
 
 constexpr uint32_t REG_MAX_TOKENS = 32;
+constexpr size_t REG_MAX_SMEM = 227 * 1024 - 1024;
 
-// Whether that kernel takes less time than the ones beside it -- the batched GEMV up to 8 tokens, the tcgen05 GEMM above, the
-// stream-K GEMV for one -- for `tensors` (2: gate and up) of m rows of k weights.  `stages`: weight stages of 128 k that a pair of
-// CTAs of the GEMM goes through.  Measured on 20 shapes at 2 and 4 bits, cold weights, other / this in us:
+// Whether that kernel takes less time than the ones beside it for `tensors` (2: gate and up) of m rows of k weights.  From 8 tokens
+// on the other one is the tcgen05 GEMM and the two estimates are compared (`cycles` of reg_plan, `gemm_cycles` of gm_plan, each
+// within some 12 % of the times; 1e30 where the GEMM does not take the shape).  On 40 cases of 2 and 4 bits and 8 to 32 tokens that
+// picks the slower one where they are within 10 % of each other.  Below that the others are the batched GEMV, and for one token the
+// pair-table and stream-K GEMV; measured, cold weights, other / this in us:
 //  * one token: at 4 bits the pair tables are ahead wherever they are used (3584 x 3584 5.8 / 8.4, gate and up of 18944 x 3584
 //    20.3 / 30.0); at 2 bits this one has the two tensors of such a gate and up (21.9 / 18.4), less is even, more is behind
 //    (29568 x 8192 53.9 / 57.2), and single tensors (3584 x 18944 12.1 / 14.0, 19008 x 3584 11.2 / 15.6);
-//  * 2 bits, 2 tokens and more: ahead (18944 x 3584, two: 34.8 / 18.6 at 2 tokens, 32.9 / 19.3 at 8, 33.6 / 22.4 at 16) up to 24
-//    tokens, above that up to 2^25 weights (3584 x 18944 23.3 / 28.9);
-//  * 4 bits, up to 2^25 weights: ahead (3584 x 3584 13.0 / 8.4 at 8 tokens, 15.7 / 11.7 at 32; 896 x 4864 26.6 / 5.8 at 16;
-//    5120 x 2048, two: 12.0 / 10.6 at 2);
-//  * 4 bits, more weights: behind at 2 tokens (8192 x 8192 15.1 / 18.8), at 3 and 4 for long rows (8192 x 29568 44.9 / 55.4;
-//    18944 x 3584, two: 36.9 / 30.1), ahead from 5 on (26.5 / 22.9 for 3584 x 18944) to 16 unless the part of X that a CTA holds gets
-//    short of shared memory (8192 x 29568 65.5 / 74.5), and to 24 where the GEMM has 48 stages and more (18944 x 3584, one
-//    21 / 24, two 40.3 / 36.4; 19008 x 3584 33.1 / 25.3; 3584 x 18944 26.6 / 27.7).
-inline bool reg_pays(uint64_t m, uint64_t k, uint32_t bits, uint32_t tensors, uint32_t tokens, uint32_t stages) {
+//  * 2 bits, 2 to 7 tokens: ahead (18944 x 3584, two: 34.8 / 18.6 at 2, 84.2 / 19.1 at 6);
+//  * 4 bits, up to 2^25 weights: ahead (3584 x 3584 9.6 / 8.3 at 4, 5120 x 2048, two: 12.0 / 10.6 at 2);
+//  * 4 bits, more weights: behind at 2 tokens (8192 x 8192 15.1 / 18.8), at 3 and 4 for long rows (8192 x 29568 44.9 / 55.4, but
+//    18944 x 3584, two: 36.9 / 30.1), ahead from 5 on (3584 x 18944 26.7 / 22.7 at 6).
+inline bool reg_pays(uint64_t m, uint64_t k, uint32_t bits, uint32_t tensors, uint32_t tokens, double cycles, double gemm_cycles) {
     const uint64_t weights = m * k * tensors;
-    const bool few = weights < 1u << 25;
+    if (tokens >= 8) return cycles < 0.95 * gemm_cycles;
     if (tokens <= 1) return bits == 2 && tensors == 2 && weights >= 1u << 25 && weights < 1u << 28;
-    if (bits == 2) return few || tokens <= 24;
-    if (few) return true;
-    if (tokens <= 2) return false;
-    if (tokens <= 4) return k < 8192;
-    if (tokens <= 8) return true;
-    if (tokens <= 16) return k < 24576 || tensors == 2;
-    return tokens <= 24 && stages >= 48;
+    return bits == 2 || weights < 1u << 25 || tokens > 4 || (tokens > 2 && k < 8192);
 }
-constexpr size_t REG_MAX_SMEM = 227 * 1024 - 1024;
 
 // A cluster of `ctas` CTAs owns `rows` half-blocks of 32 output rows; CTA r of it takes the r-th part of K for all of them, and
 // cuts its part into `parts`: (half-block, tensor, part) is a job of one of its 16 warps.
 struct RegPlan {
     uint32_t ctas = 0, rows = 0, parts = 0, clusters = 0;
     size_t smem = 0;
-    double cost = 1e30;
+    double cycles = 1e30;
 };
 constexpr uint32_t REG_WARPS = 16;
 constexpr uint32_t REG_NORM_BYTES = 256;  // shared memory before the activations
 
 // n_hb half-blocks of 32 rows, subs tensors (2: gate and up), n_chunks 16-byte index chunks a row; resident[i]: clusters of 2^i
 // CTAs that the GPU holds at once.
-// The cost orders the choices (it is about cycles, without what all have in common): a step, four chunks of 32 rows by one warp,
-// keeps an SM sub-partition's integer pipe busy for `busy` and takes a warp that is alone there `chain`; the activations of a part
-// come at 16 bytes a cycle; a job's sums cost 140 per eight tokens on their way, the cluster barrier 1000.  Fitted to 4 to 12 choices
-// for each of 80 cases (20 shapes of 2 and 4 bits, 8 to 32 tokens, measured back to back with cold weights): the choice takes
-// 1.1 % more than the best one on average, 12 % at most.
+// Estimated cycles: a step, four chunks of 32 rows by one warp, keeps an SM sub-partition's integer pipe busy for `busy` and takes
+// a warp that is alone there `chain`; the activations of a part come at 16 bytes a cycle; a job's sums cost 140 per eight tokens on
+// their way, the cluster barrier 1000.  Fitted to all choices for 80 cases (20 shapes of 2 and 4 bits, 8 to 32 tokens, cold weights):
+// the choice takes 1.1 % more than the best one on average, 12 % at most; scaled, the estimate is within 7 % (rms) of the times.
 inline RegPlan reg_plan(uint32_t n_hb, uint32_t subs, uint32_t n_chunks, uint32_t bits, uint32_t tokens, const uint32_t (&resident)[4]) {
     RegPlan best;
     const uint32_t n_steps = (n_chunks + 3) / 4, nt = (tokens + 7) / 8, units = bits == 4 ? 4 : 8;
@@ -75,9 +66,10 @@ inline RegPlan reg_plan(uint32_t n_hb, uint32_t subs, uint32_t n_chunks, uint32_
             if (p.smem > REG_MAX_SMEM) break;
             const double steps = (span + parts - 1) / parts, rounds = (jobs + REG_WARPS - 1) / REG_WARPS, last = jobs % REG_WARPS;
             const double per = jobs / REG_WARPS * (REG_WARPS / 4) + (uint32_t)(last + 3) / 4;  // jobs of the first sub-partition
-            p.cost = x / 16.0 + (per * steps * busy > rounds * steps * chain ? per * steps * busy : rounds * steps * chain) + rounds * 150.0 +
+            const double cost = x / 16.0 + (per * steps * busy > rounds * steps * chain ? per * steps * busy : rounds * steps * chain) + rounds * 150.0 +
                      (ctas > 1 ? 1000.0 : 0.0) + jobs * nt * 140.0;
-            if (p.cost < best.cost) best = p;
+            p.cycles = bits == 4 ? 0.93 * cost + 5500.0 - 800.0 * nt : 0.69 * cost + 4300.0 + 400.0 * nt;
+            if (p.cycles < best.cycles) best = p;
         }
     }
     return best;

@@ -37,11 +37,12 @@ int main() {
                         }
     CHECK(fits > 3000);
     using prism::reg_pays;
-    CHECK(reg_pays(18944, 3584, 2, 2, 1, 0) && !reg_pays(29568, 8192, 2, 2, 1, 0) && !reg_pays(3584, 18944, 2, 1, 1, 0) && !reg_pays(18944, 3584, 4, 2, 1, 0));
-    CHECK(reg_pays(3584, 18944, 2, 1, 24, 0) && !reg_pays(3584, 18944, 2, 1, 25, 99) && reg_pays(3584, 3584, 2, 1, 32, 0));
-    CHECK(reg_pays(3584, 3584, 4, 1, 2, 0) && reg_pays(3584, 3584, 4, 1, 32, 0) && !reg_pays(8192, 8192, 4, 1, 2, 0));
-    CHECK(reg_pays(18944, 3584, 4, 2, 3, 0) && !reg_pays(8192, 29568, 4, 1, 4, 0) && reg_pays(8192, 29568, 4, 1, 5, 0) && !reg_pays(8192, 29568, 4, 1, 9, 0));
-    CHECK(reg_pays(18944, 3584, 4, 2, 16, 0) && reg_pays(18944, 3584, 4, 2, 24, 56) && !reg_pays(18944, 3584, 4, 1, 24, 28) && !reg_pays(18944, 3584, 4, 2, 25, 56));
+    auto pays = [](uint64_t m, uint64_t k, uint32_t bits, uint32_t tensors, uint32_t tokens) { return reg_pays(m, k, bits, tensors, tokens, 2, 1); };
+    CHECK(pays(18944, 3584, 2, 2, 1) && !pays(29568, 8192, 2, 2, 1) && !pays(3584, 18944, 2, 1, 1) && !pays(18944, 3584, 4, 2, 1));
+    CHECK(pays(3584, 18944, 2, 1, 2) && pays(8192, 29568, 2, 1, 7) && !pays(3584, 18944, 2, 1, 8) && !pays(3584, 3584, 4, 1, 8));
+    CHECK(pays(3584, 3584, 4, 1, 2) && pays(3584, 3584, 4, 1, 7) && !pays(8192, 8192, 4, 1, 2));
+    CHECK(pays(18944, 3584, 4, 2, 3) && !pays(8192, 29568, 4, 1, 4) && pays(8192, 29568, 4, 1, 5));
+    CHECK(reg_pays(3584, 3584, 4, 1, 8, 94, 100) && !reg_pays(3584, 3584, 4, 1, 8, 96, 100) && reg_pays(3584, 3584, 4, 1, 32, 1e29, 1e30));
     printf("ok\n");
     return 0;
 }
