@@ -218,6 +218,7 @@ void prism_cuda_destroy(prism_cuda_ctx *ctx) {
     cudaFree(ctx->act_scratch);
     cudaFree(ctx->tmp_scratch);
     cudaFree(ctx->dev_err);
+    palettize_pool_free(ctx->palettize);
     cudaFree(ctx->kv_k);
     cudaFree(ctx->kv_v);
     for (auto *t : ctx->rope_tabs) {

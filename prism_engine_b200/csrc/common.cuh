@@ -59,6 +59,10 @@ __host__ __device__ inline size_t lut_idx_offset(uint32_t n_chunks, uint32_t hb,
 }  // namespace prism
 
 struct prism_nccl_api;
+namespace prism {
+struct PalettizePool;
+void palettize_pool_free(PalettizePool *pool);
+}  // namespace prism
 
 // The opaque context of the C ABI.
 struct prism_cuda_ctx {
@@ -135,6 +139,7 @@ struct prism_cuda_ctx {
     // backend-held KV cache of the MetalBackend-style entry points (prism_cuda_kv_init / kv_append / attention_kv)
     uint16_t *kv_k = nullptr, *kv_v = nullptr;
     uint32_t kv_layers = 0, kv_dim = 0, kv_max_seq = 0;
+    prism::PalettizePool *palettize = nullptr;  // of the quantiser's host entry point (palettize.cu)
     // execution plan of the last .cimage that was loaded (src/lut/graph.rs:552-589); version 0: none / unparseable
     struct PlanInfo {
         uint32_t version = 0, num_layers = 0, n_nodes = 0, n_gemm_nodes = 0;

@@ -21,8 +21,17 @@
 //    16 lanes add their cluster's elements one after the other.
 // Bound by those chains (4 cycles an element, 15 passes) and the instructions of the nearest-entry search.
 // One block per row, so 14 rows of 3584 are at work on an SM at a time.
-// 3584 x 3584 values from host memory and back, one thread per row before: 33 ms (25.9 of it the kernel); now 7.5 to 9 by the host (1.08).  Rows whose distances do not fit shared
-// memory, and many short rows, still take one thread each.
+// 3584 x 3584 values: 1.08 ms, 25.9 with one thread per row.  Rows whose distances do not fit shared memory, and many short rows,
+// still take one thread each.
+#include <sys/mman.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstdlib>
+#include <cstring>
+#include <new>
+#include <thread>
+
 #include "common.cuh"
 
 namespace prism {
@@ -42,10 +51,10 @@ __device__ __forceinline__ float pq_threshold(float total, uint32_t seed) {
 }
 
 __global__ void __launch_bounds__(PQ_THREADS) palettize_rows_kernel(const float *__restrict__ w, uint32_t dm,
-                                                                    uint32_t dn, uint32_t k_req, uint32_t max_iter,
-                                                                    uint8_t *__restrict__ payload) {
-    const uint32_t r = blockIdx.x * PQ_THREADS + threadIdx.x;
-    if (r >= dm) return;
+                                                                    uint32_t dn, uint32_t row0, uint32_t row1, uint32_t k_req,
+                                                                    uint32_t max_iter, uint8_t *__restrict__ payload) {
+    const uint32_t r = row0 + blockIdx.x * PQ_THREADS + threadIdx.x;
+    if (r >= row1) return;
     const float *ch = w + (size_t)r * dn;
     const uint32_t n = dn;
     float cb[16];
@@ -191,7 +200,7 @@ __device__ __forceinline__ uint32_t pb_nearest(float x, const float (&cb)[16]) {
 }
 
 __global__ void __launch_bounds__(PB_THREADS) palettize_block_kernel(const float *__restrict__ w, uint32_t dm, uint32_t n,
-                                                                     uint32_t k_req, uint32_t max_iter, uint8_t *__restrict__ payload) {
+                                                                     uint32_t row0, uint32_t k_req, uint32_t max_iter, uint8_t *__restrict__ payload) {
     extern __shared__ __align__(16) float md[];
     __shared__ float cbs[16];
     __shared__ uint32_t cnt[PB_WARPS][16], off[PB_WARPS][16], first[17];
@@ -200,8 +209,9 @@ __global__ void __launch_bounds__(PB_THREADS) palettize_block_kernel(const float
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t tiles = (n + 31) / 32;
     float *running = md + (size_t)tiles * 32;
-    const float *ch = w + (size_t)blockIdx.x * n;
-    uint8_t *idx = payload + (size_t)dm * 32 + (size_t)blockIdx.x * (n / 2);
+    const size_t row = row0 + blockIdx.x;
+    const float *ch = w + row * n;
+    uint8_t *idx = payload + (size_t)dm * 32 + row * (n / 2);
     uint32_t k = k_req > 16 ? 16 : k_req;
     if (k > n) k = n;
 
@@ -366,25 +376,141 @@ __global__ void __launch_bounds__(PB_THREADS) palettize_block_kernel(const float
     for (uint32_t i = tid; i < n / 2; i += PB_THREADS)
         idx[i] = (uint8_t)(pb_nearest(ch[2 * i], cb) | (pb_nearest(ch[2 * i + 1], cb) << 4));
     if (tid < 16)
-        reinterpret_cast<uint16_t *>(payload + (size_t)blockIdx.x * 32)[tid] = __half_as_ushort(__float2half_rn(cbs[tid]));
+        reinterpret_cast<uint16_t *>(payload + row * 32)[tid] = __half_as_ushort(__float2half_rn(cbs[tid]));
 }
 
-int launch_palettize(prism_cuda_ctx *ctx, const float *w_dev, uint32_t dm, uint32_t dn, uint32_t k, uint32_t max_iter,
-                     uint8_t *payload_dev) {
+// Rows row0 .. row1 - 1 of a matrix of dm rows.
+static cudaError_t palettize_rows(const float *w_dev, uint32_t dm, uint32_t dn, uint32_t row0, uint32_t row1, uint32_t k, uint32_t max_iter,
+                                  uint8_t *payload_dev, cudaStream_t stream) {
     const size_t smem = pb_smem_bytes(dn);
     // Many short rows: a block pays some 15 ns of the GPU a row before its first element, a thread per row 14 us an element however
     // many rows there are up to the GPU's threads.  100000 rows of 16 / 64 / 128 values: blocks 1541 / 2059 / 2384 us, threads 165 /
     // 955 / 1836.
     const bool threads = dn <= 128 && dm >= 720u * dn;
     if (smem <= PB_MAX_SMEM && !threads) {
-        if (smem > 48 * 1024)
-            PRISM_CUDA_TRY(ctx, cudaFuncSetAttribute(palettize_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_MAX_SMEM));
-        palettize_block_kernel<<<dm, PB_THREADS, smem, ctx->stream>>>(w_dev, dm, dn, k, max_iter, payload_dev);
-        return after_launch(ctx, "palettize_block_kernel");
+        if (smem > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(palettize_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_MAX_SMEM);
+            if (e != cudaSuccess) return e;
+        }
+        palettize_block_kernel<<<row1 - row0, PB_THREADS, smem, stream>>>(w_dev, dm, dn, row0, k, max_iter, payload_dev);
+    } else {
+        palettize_rows_kernel<<<(row1 - row0 + PQ_THREADS - 1) / PQ_THREADS, PQ_THREADS, 0, stream>>>(w_dev, dm, dn, row0, row1, k, max_iter, payload_dev);
     }
-    palettize_rows_kernel<<<(dm + PQ_THREADS - 1) / PQ_THREADS, PQ_THREADS, 0, ctx->stream>>>(w_dev, dm, dn, k, max_iter,
-                                                                                               payload_dev);
-    return after_launch(ctx, "palettize_rows_kernel");
+    return cudaGetLastError();
+}
+
+// ---- a matrix in host memory -----------------------------------------------------------------------
+// A copy from pageable memory goes through the driver at 12 GB/s, one thread, also when several ask, and a copy into memory that was
+// never touched at 2.  Here up to 4 threads carry a part of the rows each onto the GPU and their payload back, through two pinned
+// slots of their own.  The slots (4 MB; in huge pages their first use takes 1.5 ms, through cudaHostAlloc 3 to 15) and the device
+// buffers stay with the context and go with it; device buffers above PZ_KEEP are given back at once.
+// 3584 x 3584 values: 8.0 -> 3.4 ms (matrix 1.8, kernel 1.08, payload 0.5), a context's first call 9.9 -> 6.4; 896 x 896, one thread and
+// kept device buffers: 1.13 -> 0.5 ms.
+constexpr uint32_t PZ_WORKERS = 4;
+constexpr size_t PZ_SLOT = 512 * 1024;                  // two of them a worker
+constexpr size_t PZ_PAGE = 2 << 20;
+constexpr size_t PZ_LEAST = 8 << 20;                    // bytes of a matrix from which it is shared: below, the slots' first use takes longer than they save
+constexpr size_t PZ_KEEP = 256 << 20;
+
+struct PalettizePool {
+    uint8_t *pinned = nullptr;
+    cudaEvent_t event[PZ_WORKERS][2] = {};
+    void *dev[2] = {};                                   // matrix, payload
+    size_t bytes[2] = {};
+};
+void palettize_pool_free(PalettizePool *p) {
+    if (!p) return;
+    for (auto &w : p->event)
+        for (cudaEvent_t e : w)
+            if (e) cudaEventDestroy(e);
+    if (p->pinned) cudaHostUnregister(p->pinned);
+    free(p->pinned);
+    for (void *d : p->dev) cudaFree(d);
+    delete p;
+}
+
+struct PalettizeJob {
+    const float *w;
+    uint32_t dm, dn, k, max_iter, workers;
+    uint8_t *payload;
+    PalettizePool *pool;
+    int device;
+    cudaStream_t stream;
+    std::atomic<uint32_t> carried{0}, failed{0}, launched{0};  // shares on their way to the GPU; one of them failed; the kernel is in the stream
+};
+// Worker t's share; its copies take its two slots in turn, a slot is free again when its event has come.  Whoever has carried the
+// last share launches the kernel.
+static cudaError_t palettize_share(PalettizeJob &j, uint32_t t) {
+    PalettizePool &p = *j.pool;
+    uint8_t *slot[2] = {p.pinned + (size_t)t * 2 * PZ_SLOT, p.pinned + ((size_t)t * 2 + 1) * PZ_SLOT};
+    uint8_t *w_dev = static_cast<uint8_t *>(p.dev[0]), *p_dev = static_cast<uint8_t *>(p.dev[1]);
+    const size_t r0 = (size_t)j.dm * t / j.workers, r1 = (size_t)j.dm * (t + 1) / j.workers, row = (size_t)j.dn * 4;
+    uint32_t turn = 0;
+    cudaError_t e = cudaSetDevice(j.device);
+    for (size_t at = r0 * row; at < r1 * row && e == cudaSuccess; at += PZ_SLOT, turn ^= 1) {
+        const size_t n = std::min(r1 * row - at, PZ_SLOT);
+        if ((e = cudaEventSynchronize(p.event[t][turn])) != cudaSuccess) break;
+        memcpy(slot[turn], reinterpret_cast<const uint8_t *>(j.w) + at, n);
+        e = cudaMemcpyAsync(w_dev + at, slot[turn], n, cudaMemcpyHostToDevice, j.stream);
+        if (e == cudaSuccess) e = cudaEventRecord(p.event[t][turn], j.stream);
+    }
+    if (e != cudaSuccess) j.failed = 1;
+    if (j.carried.fetch_add(1) + 1 == j.workers) {
+        if (!j.failed && (e = palettize_rows(static_cast<const float *>(p.dev[0]), j.dm, j.dn, 0, j.dm, j.k, j.max_iter, p_dev, j.stream)) != cudaSuccess) j.failed = 1;
+        j.launched = 1;
+    }
+    while (!j.launched) std::this_thread::yield();
+    if (j.failed) return e;
+    for (int s = 0; s < 2 && e == cudaSuccess; s++) e = cudaEventSynchronize(p.event[t][s]);
+    const size_t part[2][2] = {{r0 * 32, r1 * 32}, {(size_t)j.dm * 32 + r0 * (j.dn / 2), (size_t)j.dm * 32 + r1 * (j.dn / 2)}};
+    for (const auto &range : part) {
+        size_t behind = range[0], behind_n = 0;          // what the other slot is receiving
+        for (size_t at = range[0]; e == cudaSuccess && (at < range[1] || behind_n); turn ^= 1) {
+            const size_t n = std::min(range[1] - at, PZ_SLOT);
+            if (n) {
+                e = cudaMemcpyAsync(slot[turn], p_dev + at, n, cudaMemcpyDeviceToHost, j.stream);
+                if (e == cudaSuccess) e = cudaEventRecord(p.event[t][turn], j.stream);
+            }
+            if (behind_n && e == cudaSuccess && (e = cudaEventSynchronize(p.event[t][turn ^ 1])) == cudaSuccess) memcpy(j.payload + behind, slot[turn ^ 1], behind_n);
+            behind = at;
+            behind_n = n;
+            at += n;
+        }
+    }
+    return e;
+}
+
+static cudaError_t palettize_pool(prism_cuda_ctx *ctx, bool slots) {
+    if (!ctx->palettize && !(ctx->palettize = new (std::nothrow) PalettizePool())) return cudaErrorMemoryAllocation;
+    PalettizePool &p = *ctx->palettize;
+    cudaError_t e = cudaSuccess;
+    if (!slots) return e;
+    if (!p.pinned) {
+        const size_t bytes = 2 * PZ_WORKERS * PZ_SLOT;
+        void *m = aligned_alloc(PZ_PAGE, bytes);
+        if (!m) return cudaErrorMemoryAllocation;
+        madvise(m, bytes, MADV_HUGEPAGE);                // a wish: without it registering takes longer
+        memset(m, 0, bytes);
+        if ((e = cudaHostRegister(m, bytes, cudaHostRegisterDefault)) != cudaSuccess) {
+            free(m);
+            return e;
+        }
+        p.pinned = static_cast<uint8_t *>(m);
+    }
+    for (auto &w : p.event)
+        for (cudaEvent_t &v : w)
+            if (!v && (e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) != cudaSuccess) return e;
+    return e;
+}
+static cudaError_t palettize_device(PalettizePool &p, int i, size_t bytes) {
+    if (p.bytes[i] >= bytes) return cudaSuccess;
+    cudaFree(p.dev[i]);
+    p.dev[i] = nullptr;
+    p.bytes[i] = 0;
+    const cudaError_t e = cudaMalloc(&p.dev[i], bytes);
+    if (e == cudaSuccess) p.bytes[i] = bytes;
+    else p.dev[i] = nullptr;
+    return e;
 }
 
 }  // namespace prism
@@ -396,7 +522,9 @@ extern "C" int prism_cuda_palettize_dev(prism_cuda_ctx *ctx, const float *weight
     if (!ctx || !weights_dev || !payload_dev) return fail(ctx, PRISM_E_NULL, "null argument");
     if (dim_m == 0 || dim_n == 0 || dim_n % 2 != 0 || k == 0)
         return fail(ctx, PRISM_E_ARG, "palettize: dim_m, dim_n > 0, dim_n even, k >= 1");
-    return launch_palettize(ctx, weights_dev, dim_m, dim_n, k, max_iter, payload_dev);
+    PRISM_CUDA_TRY(ctx, palettize_rows(weights_dev, dim_m, dim_n, 0, dim_m, k, max_iter, payload_dev, ctx->stream));
+    ctx->launches++;
+    return PRISM_OK;
 }
 
 extern "C" int prism_cuda_palettize(prism_cuda_ctx *ctx, const float *weights, uint32_t dim_m, uint32_t dim_n, uint32_t k,
@@ -407,23 +535,57 @@ extern "C" int prism_cuda_palettize(prism_cuda_ctx *ctx, const float *weights, u
     const size_t need = (size_t)dim_m * 32 + (size_t)dim_m * (dim_n / 2);
     if (len != need) return fail(ctx, PRISM_E_ARG, "palettize: payload must hold dim_m*32 + dim_m*dim_n/2 bytes");
     PRISM_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    float *w_dev = nullptr;
-    uint8_t *p_dev = nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PRISM_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return cuda_fail(ctx, cudaErrorStreamCaptureUnsupported, "palettize");
     const size_t w_bytes = (size_t)dim_m * dim_n * sizeof(float);
-    PRISM_CUDA_TRY(ctx, cudaMalloc((void **)&w_dev, w_bytes));
-    cudaError_t e = cudaMalloc((void **)&p_dev, need);
-    if (e != cudaSuccess) {
-        cudaFree(w_dev);
-        return cuda_fail(ctx, e, "cudaMalloc(payload)");
+    const uint32_t most = std::min(PZ_WORKERS, std::max(1u, std::thread::hardware_concurrency()));
+    const uint32_t workers = w_bytes < PZ_LEAST ? 1 : std::min(most, dim_m);
+    PRISM_CUDA_TRY(ctx, palettize_pool(ctx, workers > 1));
+    PalettizePool &pool = *ctx->palettize;
+    cudaError_t e = palettize_device(pool, 0, w_bytes);
+    if (e == cudaSuccess) e = palettize_device(pool, 1, need);
+    if (e == cudaSuccess && workers == 1) {              // not worth the slots
+        e = cudaMemcpyAsync(pool.dev[0], weights, w_bytes, cudaMemcpyHostToDevice, ctx->stream);
+        if (e == cudaSuccess) e = palettize_rows(static_cast<const float *>(pool.dev[0]), dim_m, dim_n, 0, dim_m, k, max_iter, static_cast<uint8_t *>(pool.dev[1]), ctx->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(payload, pool.dev[1], need, cudaMemcpyDeviceToHost, ctx->stream);
+        const cudaError_t done = cudaStreamSynchronize(ctx->stream);
+        if (e == cudaSuccess) e = done;
+        if (e == cudaSuccess) ctx->launches++;
+    } else if (e == cudaSuccess) {
+        // as many shares as there are threads to be had for them: the shares wait for one another
+        PalettizeJob job;
+        job.w = weights; job.dm = dim_m; job.dn = dim_n; job.k = k; job.max_iter = max_iter;
+        job.payload = payload; job.pool = &pool; job.device = ctx->device; job.stream = ctx->stream;
+        cudaError_t results[PZ_WORKERS] = {};
+        std::thread threads[PZ_WORKERS];
+        std::atomic<uint32_t> go{0};                     // workers there are, once that is known
+        uint32_t have = 1;
+        try {
+            for (; have < workers; have++)
+                threads[have] = std::thread([&job, &results, &go](uint32_t t) {
+                    while (!go) std::this_thread::yield();
+                    results[t] = palettize_share(job, t);
+                }, have);
+        } catch (...) {
+        }
+        job.workers = have;
+        go = have;
+        results[0] = palettize_share(job, 0);
+        for (std::thread &t : threads)
+            if (t.joinable()) t.join();
+        for (cudaError_t r : results)
+            if (e == cudaSuccess) e = r;
+        const cudaError_t done = cudaStreamSynchronize(ctx->stream);  // nothing of this call is left on the GPU, failed or not
+        if (e == cudaSuccess) e = done;
+        if (e == cudaSuccess) ctx->launches++;
     }
-    int rc = PRISM_OK;
-    e = cudaMemcpyAsync(w_dev, weights, w_bytes, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) rc = launch_palettize(ctx, w_dev, dim_m, dim_n, k, max_iter, p_dev);
-    if (e == cudaSuccess && rc == PRISM_OK) e = cudaMemcpyAsync(payload, p_dev, need, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess && rc == PRISM_OK) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(w_dev);
-    cudaFree(p_dev);
-    if (rc != PRISM_OK) return rc;
+    for (int i = 0; i < 2; i++)
+        if (pool.bytes[i] > PZ_KEEP || e != cudaSuccess) {
+            cudaFree(pool.dev[i]);
+            pool.dev[i] = nullptr;
+            pool.bytes[i] = 0;
+        }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "palettize");
     return PRISM_OK;
 }
