@@ -265,6 +265,16 @@ DenseEpi dense_epi(const DenseLinear &l, const DenseOut *outs);
 constexpr uint32_t DENSE_GEMV_ROWS = 8;
 bool dense_gemv_ok(const DenseIn &in, uint32_t rows);
 int launch_dense_gemv(prism_cuda_ctx *ctx, const DenseLinear &l, const DenseIn &in, const DenseOut *outs, uint32_t rows);
+// dense_stream.cu: plain inputs and large weights; writes the context's split sums.  launch_dense_gemv goes there where dense_stream_ok.
+// From these many weights on (dense_gemv / dense_stream, 4 rows, cold weights, us): 4736 x 896 5.0 / 7.5, 896 x 5760 8.8 / 8.9, 3584 x 1536
+// 7.8 / 7.3, 12288 x 896 9.7 / 8.0, 4736 x 3584 11.2 / 9.9, 8192 x 3584 17.1 / 13.0.  The line lies above where they meet: a model of
+// smaller linears has much of them in L2, and is slower through this one (0.5B shapes, 3 sequences, 2 550 / 2 730 us a call).
+constexpr uint64_t DENSE_STREAM_LEAST = 1ull << 24;
+// and, where that takes the norm out of the linear into a launch of its own (3.3 us), for one row: 8192 x 3584 16.4 / 13.0,
+// 12544 x 3584 26.9 / 17.7, 33280 x 3584 48.8 / 37.9.
+constexpr uint64_t DENSE_STREAM_LEAST_NORM = 1ull << 25;
+bool dense_stream_ok(prism_cuda_ctx *ctx, const DenseLinear &l, const DenseIn &in, uint32_t rows);
+int launch_dense_stream(prism_cuda_ctx *ctx, const DenseLinear &l, const DenseIn &in, const DenseOut *outs, uint32_t rows);
 // 32-bit activations and fp32 products (the weights are exact in fp32): any number of rows, plain inputs
 int launch_dense_f32(prism_cuda_ctx *ctx, const DenseLinear &l, const DenseIn &in, const DenseOut *outs, uint32_t rows);
 // dense_gemm_tc5.cu: tcgen05/TMEM GEMM, bf16 activations, plain inputs, pitches a multiple of 8

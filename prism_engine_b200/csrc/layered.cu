@@ -511,7 +511,8 @@ static int linear(prism_cuda_engine *e, const DenseLinear &l, const DenseIn &in,
                   uint32_t normed_pitch) {
     prism_cuda_ctx *ctx = e->ctx;
     LayeredModel *m = e->lm;
-    if (!m->act32 && ctx->fuse && dense_gemv_ok(in, rows)) return launch_dense_gemv(ctx, l, in, outs, rows);
+    const bool apart = in.norm_w && l.valid_rows() * l.k_pad >= DENSE_STREAM_LEAST_NORM;  // worth a norm of its own for the streaming kernel
+    if (!m->act32 && ctx->fuse && !apart && dense_gemv_ok(in, rows)) return launch_dense_gemv(ctx, l, in, outs, rows);
     const void *x = in.x;
     uint32_t pitch = in.pitch;
     if (in.norm_w) {

@@ -65,3 +65,40 @@ def linear_few_tokens(backend, handle, x, y, resid=None, up=None, norm_eps=-1.0)
     _call(backend, "_ZN5prism15launch_gemm_regEP14prism_cuda_ctxNS_8GemvModeERKNS_9LutTensorEPS4_PKtjPtjS8_jf", C.c_int(mode), _tensor(backend, handle),
           _tensor(backend, up) if up is not None else None, C.c_void_p(x.data_ptr()), C.c_uint32(x.stride(0)), C.c_void_p(y.data_ptr()),
           C.c_uint32(y.stride(0)), C.c_void_p(resid.data_ptr()) if resid is not None else None, C.c_uint32(x.shape[0]), C.c_float(norm_eps))
+
+
+class DenseSeg(C.Structure):  # prism::DenseSeg, dense.cuh
+    _fields_ = [("row0", C.c_uint32), ("rows", C.c_uint32), ("inp", C.c_uint32), ("k", C.c_uint32), ("act", C.c_uint32), ("mul", C.c_float), ("bias", C.c_void_p)]
+
+
+class DenseLinear(C.Structure):
+    _fields_ = [("w", C.c_void_p), ("k_pad", C.c_uint32), ("n_tiles", C.c_uint32), ("n_segs", C.c_uint32), ("experts", C.c_uint32), ("seg", DenseSeg * 12)]
+
+
+class DenseOut(C.Structure):
+    _fields_ = [("p", C.c_void_p), ("pitch", C.c_uint32), ("store", C.c_uint32)]
+
+
+class DenseIn(C.Structure):
+    _fields_ = [("x", C.c_void_p), ("pitch", C.c_uint32), ("f32", C.c_uint32), ("norm_w", C.c_void_p), ("n_norm", C.c_uint32), ("eps", C.c_float),
+                ("gate", C.c_void_p), ("gate_pitch", C.c_uint32), ("x2", C.c_void_p), ("pitch2", C.c_uint32)]
+
+
+def dense_layout(w):
+    """[rows of whole tiles of 128, k of whole 64s] bf16 in the device layout of a dense weight."""
+    rows, k = w.shape
+    return w.reshape(rows // 128, 128, k // 8, 8).permute(0, 2, 1, 3).contiguous()
+
+
+def dense_stream(backend, packed, k_pad, segs, x, outs, x2=None, wait=True):
+    """The streaming linear of few rows.  segs: dicts of DenseSeg fields; outs: (tensor, store) per segment."""
+    l = DenseLinear(packed.data_ptr(), k_pad, packed.shape[0], len(segs), 1)
+    for i, s in enumerate(segs):
+        l.seg[i] = DenseSeg(s["row0"], s["rows"], s.get("inp", 0), s.get("k", 0), s.get("act", 0), s.get("mul", 1.0), s["bias"].data_ptr() if s.get("bias") is not None else None)
+    o = (DenseOut * len(outs))(*[DenseOut(t.data_ptr(), t.stride(0), store) for t, store in outs])
+    i = DenseIn(x=x.data_ptr(), pitch=x.stride(0), x2=x2.data_ptr() if x2 is not None else None, pitch2=x2.stride(0) if x2 is not None else 0)
+    if not wait:
+        f = backend.L._ZN5prism19launch_dense_streamEP14prism_cuda_ctxRKNS_11DenseLinearERKNS_7DenseInEPKNS_8DenseOutEj
+        f.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32]
+        return f(backend.ctx, C.addressof(l), C.addressof(i), C.addressof(o), x.shape[0])
+    _call(backend, "_ZN5prism19launch_dense_streamEP14prism_cuda_ctxRKNS_11DenseLinearERKNS_7DenseInEPKNS_8DenseOutEj", C.byref(l), C.byref(i), o, C.c_uint32(x.shape[0]))
