@@ -361,7 +361,7 @@ static int build_model(prism_cuda_engine *e, const prism_layer_config *layers) {
     const size_t es = m->act32 ? 4 : 2;
     m->width_pad = round_up_u32(c.width, 64);
     m->vocab_pad = round_up_u32(c.vocab, 4);
-    m->cap = std::max(m->chunk, c.max_batch);
+    m->cap = std::max(m->portion, c.max_batch);
     m->layers.resize(c.num_layers);  // never resized again: names point into it
     PRISM_TRY(model_alloc(e, m->embed, (size_t)c.vocab * c.width));
     LayeredDst &em = add_name(m, "embed", c.vocab, c.width);
@@ -542,16 +542,35 @@ static int grow_bf16(prism_cuda_engine *e, bf16 *&p, size_t &have, size_t want) 
     return PRISM_OK;
 }
 
-// The mixers leave their heads in the rows of `cat`, from column mx.col on.
-static int mix_lightning(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t n, bool seq) {
+// The rows of a prompt portion: consecutive tokens of one or more sequences, one after the other.  Linears and row-wise kernels take
+// them all at once, what follows a sequence takes them span by span (`row0`: its first row).
+struct Span {
+    uint32_t slot, pos0, row0, n;
+};
+using Spans = std::vector<Span>;
+template <typename F>
+static int each_span(const Spans *seq, const RowMap &rows, uint32_t n, F &&f) {  // f(rows, first row, rows); a decode step is one
+    if (!seq) return f(rows, 0u, n);
+    for (const Span &sp : *seq) {
+        RowMap r;
+        r.slot0 = (int32_t)sp.slot;
+        r.pos0 = (int32_t)sp.pos0;
+        PRISM_TRY(f(r, sp.row0, sp.n));
+    }
+    return PRISM_OK;
+}
+
+// The mixers leave their heads in the rows of `cat`, from column mx.col on.  r0: the first of the n rows.
+static int mix_lightning(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t r0, uint32_t n, bool seq) {
     LayeredModel *m = e->lm;
     const DenseSeg *seg = ly.in.seg + mx.seg0;
+    const size_t p0 = (size_t)r0 * m->proj_pitch;
     LightningArgs a{};
-    a.q = at(m, m->proj, seg[0].row0);
-    a.k = at(m, m->proj, seg[1].row0);
-    a.v = at(m, m->proj, seg[2].row0);
+    a.q = at(m, m->proj, p0 + seg[0].row0);
+    a.k = at(m, m->proj, p0 + seg[1].row0);
+    a.v = at(m, m->proj, p0 + seg[2].row0);
     a.pitch = m->proj_pitch;
-    a.o = at(m, m->cat, mx.col);
+    a.o = at(m, m->cat, (size_t)r0 * m->cat_pitch + mx.col);
     a.o_pitch = m->cat_pitch;
     a.state = mx.state;
     a.decay = mx.decay;
@@ -559,12 +578,13 @@ static int mix_lightning(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &m
     return seq ? launch_lightning_seq(e->ctx, a, rows, m->act32) : launch_lightning_step(e->ctx, a, rows, m->act32);
 }
 
-static int mix_attention(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t n, bool seq, bool late) {
+static int mix_attention(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t r0, uint32_t n, bool seq, bool late) {
     prism_cuda_ctx *ctx = e->ctx;
     LayeredModel *m = e->lm;
     const DenseSeg *seg = ly.in.seg + mx.seg0;
-    const void *q = at(m, m->proj, seg[0].row0), *k = at(m, m->proj, seg[1].row0), *v = at(m, m->proj, seg[2].row0);
-    void *out = at(m, m->cat, mx.col);
+    const size_t p0 = (size_t)r0 * m->proj_pitch;
+    const void *q = at(m, m->proj, p0 + seg[0].row0), *k = at(m, m->proj, p0 + seg[1].row0), *v = at(m, m->proj, p0 + seg[2].row0);
+    void *out = at(m, m->cat, (size_t)r0 * m->cat_pitch + mx.col);
     if (!seq) return launch_grouped_rows(ctx, mx.ga, q, k, v, m->proj_pitch, out, m->cat_pitch, rows, n, m->act32, late);
     PRISM_TRY(launch_grouped_append(ctx, mx.ga, k, v, m->proj_pitch, rows, n, m->act32));
     if (!m->act32 && n > DENSE_GEMV_ROWS && tiled_attn_ok(mx.ga.dp, mx.ga.vp))
@@ -572,40 +592,45 @@ static int mix_attention(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &m
     return launch_grouped_rows(ctx, mx.ga, q, nullptr, nullptr, m->proj_pitch, out, m->cat_pitch, rows, n, m->act32);
 }
 
-static int mix_delta(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t n, bool seq, bool beside) {
+static int mix_delta(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t r0, uint32_t n, bool seq, bool beside) {
     prism_cuda_ctx *ctx = e->ctx;
     LayeredModel *m = e->lm;
     const DenseSeg *seg = ly.in.seg + mx.seg0;
     DeltaArgs a = mx.da;
     a.rows = n;
-    a.q = at(m, m->proj, seg[0].row0); a.k = at(m, m->proj, seg[1].row0); a.v = at(m, m->proj, seg[2].row0); a.pitch = m->proj_pitch;
-    a.ba = m->aux; a.ba_pitch = m->aux_pitch;
-    a.gate = at(m, m->proj, seg[4].row0); a.gate_pitch = m->proj_pitch;
-    a.o = at(m, m->cat, mx.col); a.o_pitch = m->cat_pitch;
+    const size_t p0 = (size_t)r0 * m->proj_pitch, v0 = (size_t)r0 * m->conv_pitch;
+    a.q = at(m, m->proj, p0 + seg[0].row0); a.k = at(m, m->proj, p0 + seg[1].row0); a.v = at(m, m->proj, p0 + seg[2].row0); a.pitch = m->proj_pitch;
+    a.ba = m->aux + (size_t)r0 * m->aux_pitch; a.ba_pitch = m->aux_pitch;
+    a.gate = at(m, m->proj, p0 + seg[4].row0); a.gate_pitch = m->proj_pitch;
+    a.o = at(m, m->cat, (size_t)r0 * m->cat_pitch + mx.col); a.o_pitch = m->cat_pitch;
     a.beside = beside;
     if (!seq) return launch_delta_step(ctx, a, rows, m->act32);
     const uint32_t hk = a.kv_heads * a.dim;
     ConvArgs c{};
     c.pieces = 3; c.x_pitch = m->proj_pitch; c.y_pitch = m->conv_pitch; c.taps = a.taps; c.channels = a.channels; c.w = a.conv_w; c.ring = a.ring; c.silu = 1;
-    c.piece[0] = ConvPiece{a.q, at(m, m->conv, mx.conv_col[0]), hk, 0};
-    c.piece[1] = ConvPiece{a.k, at(m, m->conv, mx.conv_col[1]), hk, hk};
-    c.piece[2] = ConvPiece{a.v, at(m, m->conv, mx.conv_col[2]), a.heads * a.vdim, 2 * hk};
+    c.piece[0] = ConvPiece{a.q, at(m, m->conv, v0 + mx.conv_col[0]), hk, 0};
+    c.piece[1] = ConvPiece{a.k, at(m, m->conv, v0 + mx.conv_col[1]), hk, hk};
+    c.piece[2] = ConvPiece{a.v, at(m, m->conv, v0 + mx.conv_col[2]), a.heads * a.vdim, 2 * hk};
     PRISM_TRY(launch_conv_seq(ctx, c, rows, n, m->act32));
     a.q = c.piece[0].y; a.k = c.piece[1].y; a.v = c.piece[2].y; a.pitch = m->conv_pitch;
     a.o32 = m->o32; a.chunk_scratch = m->delta;
     return launch_delta_seq(ctx, a, rows, m->act32);
 }
 
-static int mix_latent(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t n, bool seq) {
+static int latent_queries(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, uint32_t n) {
+    LayeredModel *m = e->lm;
+    DenseIn qi{};
+    qi.x = at(m, m->proj, ly.in.seg[mx.seg0].row0); qi.pitch = m->proj_pitch; qi.norm_w = mx.dq_norm; qi.n_norm = mx.c.q_rank; qi.eps = m->c.norm_eps;
+    const DenseOut qo{m->q, m->q_pitch, ST_ACT};
+    return linear(e, mx.uq, qi, &qo, n, m->cq, m->cq_pitch);
+}
+static int mix_latent(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t r0, uint32_t n, bool seq) {
     prism_cuda_ctx *ctx = e->ctx;
     LayeredModel *m = e->lm;
     const LatentArgs &la = mx.la;
     const DenseSeg *seg = ly.in.seg + mx.seg0;
-    void *dq = at(m, m->proj, seg[0].row0), *dkv = at(m, m->proj, seg[1].row0), *gate = at(m, m->proj, seg[2].row0), *out = at(m, m->cat, mx.col);
-    DenseIn qi{};
-    qi.x = dq; qi.pitch = m->proj_pitch; qi.norm_w = mx.dq_norm; qi.n_norm = mx.c.q_rank; qi.eps = m->c.norm_eps;
-    const DenseOut qo{m->q, m->q_pitch, ST_ACT};
-    PRISM_TRY(linear(e, mx.uq, qi, &qo, n, m->cq, m->cq_pitch));
+    const size_t p0 = (size_t)r0 * m->proj_pitch, q0 = (size_t)r0 * m->q_pitch;
+    void *dkv = at(m, m->proj, p0 + seg[1].row0), *gate = at(m, m->proj, p0 + seg[2].row0), *out = at(m, m->cat, (size_t)r0 * m->cat_pitch + mx.col);
     if (seq && n > DENSE_GEMV_ROWS && mx.ukv.w) {
         const uint32_t pos0 = (uint32_t)rows.pos0, lo = la.window && pos0 + 1 > la.window ? pos0 + 1 - la.window : 0, nk = pos0 + n - lo;
         const uint32_t kv_pitch = mx.ukv.n_tiles * 128, v0 = mx.ukv.seg[1].row0;
@@ -618,7 +643,7 @@ static int mix_latent(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, 
         DenseIn ki{};
         ki.x = m->ex_lat; ki.pitch = mx.ukv.k_pad;
         PRISM_TRY(launch_dense_gemm_tc5(ctx, mx.ukv, ki, ko, nk));
-        return launch_latent_prefill(ctx, la, (const bf16 *)m->q, m->q_pitch, m->ex_kv, kv_pitch, m->ex_kv + v0, kv_pitch, m->ex_krot, lo,
+        return launch_latent_prefill(ctx, la, (const bf16 *)at(m, m->q, q0), m->q_pitch, m->ex_kv, kv_pitch, m->ex_kv + v0, kv_pitch, m->ex_krot, lo,
                                      (const bf16 *)gate, m->proj_pitch, (bf16 *)out, m->cat_pitch, pos0, n);
     }
     LatentRowsScratch s = m->rows_scratch;
@@ -632,7 +657,7 @@ static int mix_latent(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, 
         } else {
             sub.pos0 += (int32_t)r;
         }
-        PRISM_TRY(launch_latent_rows(ctx, la, s, at(m, m->q, (size_t)r * m->q_pitch), m->q_pitch, at(m, dkv, (size_t)r * m->proj_pitch),
+        PRISM_TRY(launch_latent_rows(ctx, la, s, at(m, m->q, q0 + (size_t)r * m->q_pitch), m->q_pitch, at(m, dkv, (size_t)r * m->proj_pitch),
                                      m->proj_pitch, at(m, gate, (size_t)r * m->proj_pitch), m->proj_pitch,
                                      at(m, out, (size_t)r * m->cat_pitch), m->cat_pitch, sub, k, m->act32));
     }
@@ -640,14 +665,17 @@ static int mix_latent(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, 
 }
 
 // In a decode step the two kernels of an attention and a gated delta rule run side by side: neither needs the other.
-static int run_mixer(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t n, bool seq) {
+static int run_mixer(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, const RowMap &rows, uint32_t n, const Spans *seq) {
+    if (mx.c.mixer == PRISM_MIXER_LATENT_ATTENTION) PRISM_TRY(latent_queries(e, ly, mx, n));
     const bool side = !seq && ly.mix.size() == 2 && ly.mix[0].c.mixer == PRISM_MIXER_ATTENTION && ly.mix[1].c.mixer == PRISM_MIXER_GATED_DELTA;
-    switch (mx.c.mixer) {
-    case PRISM_MIXER_LIGHTNING: return mix_lightning(e, ly, mx, rows, n, seq);
-    case PRISM_MIXER_LATENT_ATTENTION: return mix_latent(e, ly, mx, rows, n, seq);
-    case PRISM_MIXER_ATTENTION: return mix_attention(e, ly, mx, rows, n, seq, side);
-    default: return mix_delta(e, ly, mx, rows, n, seq, side);
-    }
+    return each_span(seq, rows, n, [&](const RowMap &r, uint32_t r0, uint32_t k) -> int {
+        switch (mx.c.mixer) {
+        case PRISM_MIXER_LIGHTNING: return mix_lightning(e, ly, mx, r, r0, k, seq);
+        case PRISM_MIXER_LATENT_ATTENTION: return mix_latent(e, ly, mx, r, r0, k, seq);
+        case PRISM_MIXER_ATTENTION: return mix_attention(e, ly, mx, r, r0, k, seq, side);
+        default: return mix_delta(e, ly, mx, r, r0, k, seq, side);
+        }
+    });
 }
 // Lightning: all heads normed together, then gated, as the input of the output linear takes it.
 static void lightning_norm(LayeredModel *m, const LayeredLayer &ly, const LayeredMixer &mx, DenseIn &in) {
@@ -661,7 +689,7 @@ static void in_outs(const LayeredModel *m, const LayeredLayer &ly, DenseOut *out
         if (mx.c.mixer == PRISM_MIXER_GATED_DELTA) outs[mx.seg0 + 3] = DenseOut{m->aux, m->aux_pitch, ST_F32};
 }
 
-static int forward_parallel(prism_cuda_engine *e, const RowMap &rows, uint32_t n, bool seq) {
+static int forward_parallel(prism_cuda_engine *e, const RowMap &rows, uint32_t n, const Spans *seq) {
     LayeredModel *m = e->lm;
     const uint32_t D = m->c.width;
     for (LayeredLayer &ly : m->layers) {
@@ -682,7 +710,7 @@ static int forward_parallel(prism_cuda_engine *e, const RowMap &rows, uint32_t n
 }
 
 // The row-wise kernel between two sublayers, ending with the norm (and convolution) of sublayer `which` of `next`.
-static int row_step(prism_cuda_engine *e, RowUpdate &u, const LayeredLayer *next, int which, const RowMap &rows, uint32_t n, bool seq) {
+static int row_step(prism_cuda_engine *e, RowUpdate &u, const LayeredLayer *next, int which, const RowMap &rows, uint32_t n, const Spans *seq) {
     LayeredModel *m = e->lm;
     const uint32_t D = m->c.width, taps = m->c.canon_taps;
     u.x = m->x; u.width = D; u.eps = m->c.norm_eps; u.mul = m->c.residual_mult;
@@ -701,8 +729,10 @@ static int row_step(prism_cuda_engine *e, RowUpdate &u, const LayeredLayer *next
     c.pieces = 1; c.x_pitch = c.y_pitch = m->width_pad; c.taps = taps; c.channels = D;
     c.w = which == 1 ? next->canon1 : next->canon2;
     c.ring = which == 1 ? next->ring1 : next->ring2;
-    c.piece[0] = ConvPiece{m->xn, m->xc, D, 0};
-    return launch_conv_seq(e->ctx, c, rows, n, m->act32);
+    return each_span(seq, rows, n, [&](const RowMap &r, uint32_t r0, uint32_t k) -> int {
+        c.piece[0] = ConvPiece{at(m, m->xn, (size_t)r0 * m->width_pad), at(m, m->xc, (size_t)r0 * m->width_pad), D, 0};
+        return launch_conv_seq(e->ctx, c, r, k, m->act32);
+    });
 }
 
 // Feed-forward of the rows in m->xc / m->xn, up to its result: a row each, or rows of the experts with the plan.
@@ -760,7 +790,7 @@ static uint32_t mixer_scratch(uint32_t mixer) {
 
 // All mixers of a layer.  In a prompt portion the second of a pair runs on a stream of its own: its chunks follow one
 // another on a part of the GPU.
-static int run_mixers(prism_cuda_engine *e, LayeredLayer &ly, const RowMap &rows, uint32_t n, bool seq) {
+static int run_mixers(prism_cuda_engine *e, LayeredLayer &ly, const RowMap &rows, uint32_t n, const Spans *seq) {
     prism_cuda_ctx *ctx = e->ctx;
     LayeredModel *m = e->lm;
     auto whole = [&](LayeredMixer &mx) -> int {
@@ -789,7 +819,7 @@ static int run_mixers(prism_cuda_engine *e, LayeredLayer &ly, const RowMap &rows
     return PRISM_OK;
 }
 
-static int forward_sequential(prism_cuda_engine *e, const RowMap &rows, uint32_t n, bool seq) {
+static int forward_sequential(prism_cuda_engine *e, const RowMap &rows, uint32_t n, const Spans *seq) {
     LayeredModel *m = e->lm;
     const uint32_t D = m->c.width, L = m->c.num_layers;
     DenseIn in{};  // what the sublayers read: the convolved norm, and the norm itself
@@ -845,10 +875,13 @@ static int forward_sequential(prism_cuda_engine *e, const RowMap &rows, uint32_t
     return PRISM_OK;
 }
 
-// `n` tokens (device ids) through every layer, their residual rows in m->x.
-static int forward_tokens(prism_cuda_engine *e, const uint32_t *tokens, const RowMap &rows, uint32_t n, bool seq) {
+// `n` tokens (device ids) through every layer, their residual rows in m->x: a decode step's `rows`, or the spans of a portion.
+static int forward_tokens(prism_cuda_engine *e, const uint32_t *tokens, const RowMap &rows, uint32_t n, const Spans *seq) {
     LayeredModel *m = e->lm;
-    PRISM_TRY(launch_dense_embed(e->ctx, m->embed, m->c.width, m->c.vocab, tokens, n, m->x, m->pos, m->c.max_positions, rows, m->history));
+    PRISM_TRY(each_span(seq, rows, n, [&](const RowMap &r, uint32_t r0, uint32_t k) -> int {
+        const size_t x0 = (size_t)r0 * m->c.width;
+        return launch_dense_embed(e->ctx, m->embed, m->c.width, m->c.vocab, tokens + r0, k, m->x + x0, m->pos, m->c.max_positions, r, m->history ? m->history + x0 : nullptr);
+    }));
     return m->c.arrangement == PRISM_ARRANGE_SEQUENTIAL ? forward_sequential(e, rows, n, seq) : forward_parallel(e, rows, n, seq);
 }
 
@@ -868,7 +901,7 @@ int layered_enqueue_step(prism_cuda_engine *e) {
     RowMap rows;
     rows.slot = m->row_slot;
     rows.pos = m->row_pos;
-    PRISM_TRY(forward_tokens(e, e->tok, rows, B, false));
+    PRISM_TRY(forward_tokens(e, e->tok, rows, B, nullptr));
     PRISM_TRY(head_rows(e, m->x, B));
     PRISM_TRY(launch_argmax(ctx, m->logits, m->c.vocab, m->vocab_pad, B, e->next));
     return enqueue_advance(e, m->row_pos);
@@ -943,27 +976,51 @@ int layered_reset(prism_cuda_engine *e, uint32_t batch) {
     return PRISM_OK;
 }
 
-// Prompt tokens of one slot, in chunks; after_chunk(first token, count) runs once a chunk's residual rows are in m->x.
+// Prompt tokens of one or more slots, in portions of at most m->portion tokens that take the slots one after the other.  After a
+// portion, done(part) runs for each of its parts, whose residual rows are in m->x from part.row0 on.
+// Four prompts of about 500 tokens, 7B shapes, weights read once and tiles full: a call of prompts and 12 steps 10.55 -> 9.80 ms (lightning and
+// latent layers) and 11.70 -> 10.38 (attention beside the delta rule, experts: their products 468 -> 243 us each way and layer).
+struct Part {
+    uint32_t entry, first, row0, n;  // tokens first .. first + n - 1 of the entry
+};
+struct PromptEntry {
+    uint32_t slot, n;
+    const uint32_t *tokens;
+};
 template <typename F>
-static int run_portion(prism_cuda_engine *e, uint32_t slot, const uint32_t *tokens, uint32_t n, F &&after_chunk) {
+static int run_portions(prism_cuda_engine *e, const std::vector<PromptEntry> &entries, F &&done) {
     prism_cuda_ctx *ctx = e->ctx;
     LayeredModel *m = e->lm;
-    for (uint32_t t0 = 0; t0 < n; t0 += m->chunk) {
-        const uint32_t k = std::min(m->chunk, n - t0);
-        PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(m->pf_tok, tokens + t0, (size_t)k * 4, cudaMemcpyHostToDevice, ctx->stream));
-        RowMap rows;
-        rows.slot0 = (int32_t)slot;
-        rows.pos0 = (int32_t)m->slot_pos[slot];
-        PRISM_TRY(forward_tokens(e, m->pf_tok, rows, k, true));
-        m->slot_pos[slot] += k;
-        PRISM_TRY(after_chunk(t0, k));
+    uint32_t entry = 0, first = 0;
+    while (entry < entries.size()) {
+        Spans spans;
+        std::vector<Part> parts;
+        uint32_t n = 0;
+        while (entry < entries.size() && n < m->portion) {
+            const PromptEntry &p = entries[entry];
+            const uint32_t k = std::min({m->chunk, m->portion - n, p.n - first});
+            // a part of a few tokens takes other kernels than the rest of its prompt would: it waits for the next portion
+            if (n && k < p.n - first && k <= DENSE_GEMV_ROWS) break;
+            PRISM_CUDA_TRY(ctx, cudaMemcpyAsync(m->pf_tok + n, p.tokens + first, (size_t)k * 4, cudaMemcpyHostToDevice, ctx->stream));
+            spans.push_back(Span{p.slot, (uint32_t)m->slot_pos[p.slot] , n, k});
+            parts.push_back(Part{entry, first, n, k});
+            n += k;
+            first += k;
+            if (first == p.n) {
+                entry++;
+                first = 0;
+            }
+        }
+        PRISM_TRY(forward_tokens(e, m->pf_tok, RowMap(), n, &spans));
+        for (const Span &sp : spans) m->slot_pos[sp.slot] += sp.n;
+        PRISM_TRY(done(parts));
     }
     return PRISM_OK;
 }
 int layered_prefill(prism_cuda_engine *e, uint32_t slot, const uint32_t *tokens, uint32_t n) {
     for (uint32_t i = 0; i < n; i++)
         if (tokens[i] >= e->lm->c.vocab) return fail(e->ctx, PRISM_E_ARG, "token id outside the vocabulary");
-    return run_portion(e, slot, tokens, n, [](uint32_t, uint32_t) { return PRISM_OK; });
+    return run_portions(e, {PromptEntry{slot, n, tokens}}, [](const std::vector<Part> &) { return PRISM_OK; });
 }
 
 int layered_logits_f16(prism_cuda_engine *e, uint16_t *host) {
@@ -1051,6 +1108,7 @@ int prism_cuda_engine_create_layered(prism_cuda_ctx *ctx, const prism_layered_co
     e->lm->c = c;
     e->lm->act32 = c.dtype == PRISM_DTYPE_F32;
     e->lm->chunk = std::min(c.max_seq, (uint32_t)std::max(1, ctx->layered_chunk));
+    e->lm->portion = (uint32_t)std::min<uint64_t>((uint64_t)c.max_seq * c.max_batch, (uint64_t)std::max(1, ctx->layered_chunk));
     // what the shared loop reads of the palettized configuration
     e->cfg.num_layers = c.num_layers; e->cfg.hidden_size = c.width; e->cfg.vocab_size = c.vocab; e->cfg.norm_eps = c.norm_eps;
     e->cfg.max_seq = c.max_seq; e->cfg.max_batch = c.max_batch;
@@ -1188,25 +1246,32 @@ int prism_cuda_engine_extend(prism_cuda_engine *e, uint32_t n, const uint32_t *s
         }
         if (B == n) return device_error_result(ctx, m->host[4 * B]);
     }
+    std::vector<PromptEntry> prompts;
+    std::vector<uint32_t> of;                            // which entry of the call
     for (uint32_t i = 0; i < n; i++) {
         if (n_tokens[i] == 1) continue;
-        const uint32_t nwi = n_want ? n_want[i] : 0;
-        const uint32_t *w = want + want0[i];
-        PRISM_TRY(run_portion(e, seqs[i], tokens + tok0[i], n_tokens[i], [&](uint32_t t0, uint32_t k) -> int {
-            std::vector<uint32_t> idx, dst;
-            for (uint32_t j = 0; j < nwi; j++)
-                if (w[j] >= t0 && w[j] < t0 + k) {
-                    idx.push_back(w[j] - t0);
+        prompts.push_back(PromptEntry{seqs[i], n_tokens[i], tokens + tok0[i]});
+        of.push_back(i);
+    }
+    PRISM_TRY(run_portions(e, prompts, [&](const std::vector<Part> &parts) -> int {
+        std::vector<uint32_t> idx, dst;
+        for (const Part &p : parts) {
+            const uint32_t i = of[p.entry], nwi = n_want ? n_want[i] : 0;
+            for (uint32_t j = 0; j < nwi; j++) {
+                const uint32_t w = want[want0[i] + j];
+                if (w >= p.first && w < p.first + p.n) {
+                    idx.push_back(p.row0 + w - p.first);
                     dst.push_back((uint32_t)want0[i] + j);
                 }
-            if (!idx.empty()) PRISM_TRY(logits_of(e, idx.data(), dst.data(), (uint32_t)idx.size(), logits, nullptr));
-            if (next_tokens && t0 + k == n_tokens[i]) {
-                const uint32_t last = k - 1;
-                PRISM_TRY(logits_of(e, &last, nullptr, 1, nullptr, next_tokens + i));
             }
-            return PRISM_OK;
-        }));
-    }
+        }
+        if (!idx.empty()) PRISM_TRY(logits_of(e, idx.data(), dst.data(), (uint32_t)idx.size(), logits, nullptr));
+        for (const Part &p : parts) {
+            const uint32_t i = of[p.entry], last = p.row0 + p.n - 1;
+            if (next_tokens && p.first + p.n == n_tokens[i]) PRISM_TRY(logits_of(e, &last, nullptr, 1, nullptr, next_tokens + i));
+        }
+        return PRISM_OK;
+    }));
     return check_device_error(ctx);
 }
 

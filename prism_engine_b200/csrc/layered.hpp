@@ -70,7 +70,8 @@ struct LayeredModel {
     std::unordered_map<std::string, LayeredDst> names;
     std::vector<std::string> order;                // names in layer order
     // scratch for `cap` rows
-    uint32_t cap = 0, chunk = 0, lg_cap = 0;
+    uint32_t cap = 0, lg_cap = 0;
+    uint32_t chunk = 0, portion = 0;  // most prompt tokens of one sequence, and of all together, that go through the layers at once
     float *x = nullptr, *xw = nullptr, *logits = nullptr;
     void *xn = nullptr, *proj = nullptr, *cat = nullptr, *q = nullptr, *cq = nullptr;
     uint32_t proj_pitch = 0, cat_pitch = 0, q_pitch = 0, cq_pitch = 0;
