@@ -16,7 +16,7 @@ constexpr size_t REG_MAX_SMEM = 227 * 1024 - 1024;
 // picks the slower one where they are within 10 % of each other.  Below that the others are the batched GEMV, and for one token the
 // pair-table and stream-K GEMV; measured, cold weights, other / this in us:
 //  * one token: at 4 bits the pair tables are ahead wherever they are used (3584 x 3584 5.8 / 8.4, gate and up of 18944 x 3584
-//    20.3 / 30.0); at 2 bits this one has the two tensors of such a gate and up (21.9 / 18.4), less is even, more is behind
+//    20.3 / 30.0); at 2 bits this one has the two tensors of such a gate and up (21.9 / 18.6), less is even, more is behind
 //    (29568 x 8192 53.9 / 57.2), and single tensors (3584 x 18944 12.1 / 14.0, 19008 x 3584 11.2 / 15.6);
 //  * 2 bits, 2 to 7 tokens: ahead (18944 x 3584, two: 34.8 / 18.6 at 2, 84.2 / 19.1 at 6);
 //  * 4 bits, up to 2^25 weights: ahead (3584 x 3584 9.6 / 8.3 at 4, 5120 x 2048, two: 12.0 / 10.6 at 2);
