@@ -309,8 +309,10 @@ int launch_gemv_tc5(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, cons
                     void *y, const uint16_t *resid);
 
 // gemm_reg.cu: 1..32 activation rows, palettes in registers; PLAIN, RESID and SWIGLU; norm_eps >= 0 (one row) folds RMSNorm of x.
-// gemm_reg_takes: false where a tensor or mode is not for it, or another kernel takes less time (reg_pays)
-int gemm_reg_takes(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, uint32_t batch, bool *takes);
+// gemm_few_tokens: nothing launched and `takes` false where tensor, mode or alignment are not for it, or another kernel takes less time
+// (reg_pays); launch_gemm_reg: wherever the shape fits
+int gemm_few_tokens(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,
+                    uint32_t y_stride, const uint16_t *resid, uint32_t batch, float norm_eps, bool *takes);
 int launch_gemm_reg(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,
                     uint32_t y_stride, const uint16_t *resid, uint32_t batch, float norm_eps);
 

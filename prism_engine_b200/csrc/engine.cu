@@ -126,8 +126,9 @@ static int linear(prism_cuda_engine *e, GemvMode mode, const LutTensor &t, const
                   uint32_t xs, uint16_t *y, uint32_t ys, const uint16_t *resid, uint32_t B) {
     prism_cuda_ctx *ctx = e->ctx;
     bool few = false;
-    if (!ctx->batch_gemv_max && B >= 2 && ctx->gemm_variant == 1 && ctx->gemv_variant == 1 && e->gu && xs >= t.k) PRISM_TRY(gemm_reg_takes(ctx, mode, t, B, &few));
-    if (few) return launch_gemm_reg(ctx, mode, t, t2, x, xs, y, ys, resid, B, -1.0f);
+    if (!ctx->batch_gemv_max && B >= 2 && ctx->gemm_variant == 1 && ctx->gemv_variant == 1 && e->gu && xs >= t.k)
+        PRISM_TRY(gemm_few_tokens(ctx, mode, t, t2, x, xs, y, ys, resid, B, -1.0f, &few));
+    if (few) return PRISM_OK;
     const uint32_t gemv_max = ctx->batch_gemv_max ? (uint32_t)ctx->batch_gemv_max
                               : gemm_pays_at_8(t.m, t.k, t.bits, mode == GEMV_SWIGLU, (uint32_t)ctx->sm_count) ? 7 : 8;
     const bool gemm_ok = B > gemv_max && ctx->gemm_variant == 1 && e->gu && gemm_tc5_eligible(ctx, t, B) && xs == t.k &&

@@ -331,8 +331,11 @@ static int launch_reg(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, bool 
         }
         res[0] = (uint32_t)ctx->sm_count;
     }
-    const RegPlan p = *plan = reg_plan((t.m + 31) / 32, a.subs, t.n_chunks, BITS, a.batch, res);
-    if (dry || !p.ctas) return PRISM_OK;
+    if (dry) {
+        *plan = reg_plan((t.m + 31) / 32, a.subs, t.n_chunks, BITS, a.batch, res);
+        return PRISM_OK;
+    }
+    const RegPlan &p = *plan;
     a.ctas = p.ctas;
     a.rows = p.rows;
     a.parts = p.parts;
@@ -366,31 +369,40 @@ static RegArgs reg_args(GemvMode mode, const LutTensor &t, const LutTensor *t2, 
     return a;
 }
 
-int gemm_reg_takes(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, uint32_t batch, bool *takes) {
+static int reg_launch(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, RegPlan *plan, const uint16_t *x, uint32_t x_stride, uint16_t *y, uint32_t y_stride,
+                      const uint16_t *resid, float norm_eps) {
+    if ((reinterpret_cast<uintptr_t>(x) & 15) || x_stride % 8) return fail(ctx, PRISM_E_ARG, "gemm: activations must be 16-byte aligned");
+    a.x = x; a.x_stride = x_stride;
+    a.y = y; a.y_stride = y_stride; a.resid = resid;
+    a.norm_eps = norm_eps;
+    a.wide = y_stride % 8 == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(resid)) & 15) == 0;
+    return reg_dispatch(ctx, a, t, false, plan);
+}
+
+int gemm_few_tokens(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,
+                    uint32_t y_stride, const uint16_t *resid, uint32_t batch, float norm_eps, bool *takes) {
     *takes = false;
+    if ((reinterpret_cast<uintptr_t>(x) & 15) || x_stride % 8) return PRISM_OK;
     if (mode != GEMV_PLAIN && mode != GEMV_RESID && mode != GEMV_SWIGLU) return PRISM_OK;
     if (batch == 0 || batch > REG_MAX_TOKENS || t.m == 0 || !((t.bits == 4 && t.k % 32 == 0 && t.k >= 32) || (t.bits == 2 && t.k % 64 == 0 && t.k >= 64))) return PRISM_OK;
-    RegArgs a = reg_args(mode, t, nullptr, batch);
+    RegArgs a = reg_args(mode, t, t2, batch);
+    if (batch < 8 && !reg_pays(t.m, t.k, t.bits, a.subs, batch, 0.0, 1e30)) return PRISM_OK;  // whatever the plan
     RegPlan plan;
     PRISM_TRY(reg_dispatch(ctx, a, t, true, &plan));
     if (!plan.ctas) return PRISM_OK;
     double gemm = 1e30;
     if (gemm_tc5_eligible(ctx, t, batch)) PRISM_TRY(gemm_tc5_cycles(ctx, t, batch, a.subs, &gemm));
     *takes = reg_pays(t.m, t.k, t.bits, a.subs, batch, plan.cycles, gemm);
-    return PRISM_OK;
+    return *takes ? reg_launch(ctx, a, t, &plan, x, x_stride, y, y_stride, resid, norm_eps) : PRISM_OK;
 }
 
 int launch_gemm_reg(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,
                     uint32_t y_stride, const uint16_t *resid, uint32_t batch, float norm_eps) {
-    if ((reinterpret_cast<uintptr_t>(x) & 15) || x_stride % 8) return fail(ctx, PRISM_E_ARG, "gemm: activations must be 16-byte aligned");
     RegArgs a = reg_args(mode, t, t2, batch);
-    a.x = x; a.x_stride = x_stride;
-    a.y = y; a.y_stride = y_stride; a.resid = resid;
-    a.norm_eps = norm_eps;
-    a.wide = y_stride % 8 == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(resid)) & 15) == 0;
     RegPlan plan;
-    PRISM_TRY(reg_dispatch(ctx, a, t, false, &plan));
-    return plan.ctas ? PRISM_OK : fail(ctx, PRISM_E_ARG, "gemm: this shape does not fit the register-palette kernel");
+    PRISM_TRY(reg_dispatch(ctx, a, t, true, &plan));
+    if (!plan.ctas) return fail(ctx, PRISM_E_ARG, "gemm: this shape does not fit the register-palette kernel");
+    return reg_launch(ctx, a, t, &plan, x, x_stride, y, y_stride, resid, norm_eps);
 }
 
 }  // namespace prism

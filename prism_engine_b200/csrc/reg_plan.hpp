@@ -16,16 +16,27 @@ constexpr size_t REG_MAX_SMEM = 227 * 1024 - 1024;
 // picks the slower one where they are within 10 % of each other.  Below that the others are the batched GEMV, and for one token the
 // pair-table and stream-K GEMV; measured, cold weights, other / this in us:
 //  * one token: at 4 bits the pair tables are ahead wherever they are used (3584 x 3584 5.8 / 8.4, gate and up of 18944 x 3584
-//    20.3 / 30.0); at 2 bits this one has the two tensors of such a gate and up (21.9 / 18.6), less is even, more is behind
-//    (29568 x 8192 53.9 / 57.2), and single tensors (3584 x 18944 12.1 / 14.0, 19008 x 3584 11.2 / 15.6);
+//    20.3 / 30.0), at 2 bits for single tensors (3584 x 18944 12.1 / 14.0, 19008 x 3584 11.2 / 15.6) and small gates and ups (two of
+//    9472 x 3584 8.7 / 11.8).  For larger ones it depends on how evenly this kernel's CTAs share the rows, so its estimate meets one of the
+//    stream-K GEMV (6.1 us and 0.104 us a million weights, within 7 % on 14 shapes of 117 to 283 million): two of 18944 x 3584 21.5 / 18.3,
+//    13824 x 5120 21.2 / 19.8, 23680 x 3584 24.7 / 24.1, but 19264 x 3584 21.8 / 23.7, 10240 x 8192 24.1 / 26.6, 28672 x 4096 30.6 / 33.4;
 //  * 2 bits, 2 to 7 tokens: ahead (18944 x 3584, two: 34.8 / 18.6 at 2, 84.2 / 19.1 at 6);
+//  * short rows, little work: behind, since its clusters and the staging of X cost 2.6 us at least (2 bits, k < 1024 and fewer than nine
+//    million weights x tokens: 320 x 192 1.9 / 2.9 at 12, 896 x 896 2.8 / 3.1 at 6, 960 x 320 3.1 / 3.8 at 24, but 1600 x 192 5.7 / 4.0 at
+//    32; up to 8 tokens, since from 9 on the tcgen05 GEMM is beside it where it can be: 640 x 256 5.0 / 3.0 at 12; 4 bits, k < 512 and three million:
+//    320 x 192 2.2 / 2.6 at 4, 3520 x 192 2.5 / 2.8 at 4, but 192 x 832 5.2 / 2.8 at 4);
+//  * 4 bits, single tensors of 2^22 weights with more rows than k: behind at 2 tokens (5120 x 2048 5.5 / 6.4, 4864 x 896 3.9 / 4.5,
+//    but 2048 x 5120 6.8 / 6.5), at 3 where they are four times as many (4864 x 896 4.3 / 4.5, but 5120 x 2048 6.7 / 6.4);
 //  * 4 bits, up to 2^25 weights: ahead (3584 x 3584 9.6 / 8.3 at 4, 5120 x 2048, two: 12.0 / 10.6 at 2);
 //  * 4 bits, more weights: behind at 2 tokens (8192 x 8192 15.1 / 18.8), at 3 and 4 for long rows (8192 x 29568 44.9 / 55.4, but
 //    18944 x 3584, two: 36.9 / 30.1), ahead from 5 on (3584 x 18944 26.7 / 22.7 at 6).
 inline bool reg_pays(uint64_t m, uint64_t k, uint32_t bits, uint32_t tensors, uint32_t tokens, double cycles, double gemm_cycles) {
     const uint64_t weights = m * k * tensors;
+    if (bits == 2 && k < 1024 && tokens > 1 && tokens * weights < 9000000u && (tokens <= 8 || gemm_cycles >= 1e30)) return false;
+    if (bits == 4 && k < 512 && tokens > 1 && tokens < 8 && tokens * weights < 3000000u) return false;
     if (tokens >= 8) return cycles < 0.95 * gemm_cycles;
-    if (tokens <= 1) return bits == 2 && tensors == 2 && weights >= 1u << 25 && weights < 1u << 28;
+    if (tokens <= 1) return bits == 2 && tensors == 2 && weights >= 100000000u && weights < 1u << 28 && cycles < 12000.0 + 204e-6 * (double)weights;
+    if (bits == 4 && tokens <= 3 && tensors == 1 && weights >= 1u << 22 && m > (tokens == 2 ? k : 4 * k)) return false;
     return bits == 2 || weights < 1u << 25 || tokens > 4 || (tokens > 2 && k < 8192);
 }
 

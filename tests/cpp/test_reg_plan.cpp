@@ -43,6 +43,10 @@ int main() {
     CHECK(pays(3584, 3584, 4, 1, 2) && pays(3584, 3584, 4, 1, 7) && !pays(8192, 8192, 4, 1, 2));
     CHECK(pays(18944, 3584, 4, 2, 3) && !pays(8192, 29568, 4, 1, 4) && pays(8192, 29568, 4, 1, 5));
     CHECK(reg_pays(3584, 3584, 4, 1, 8, 94, 100) && !reg_pays(3584, 3584, 4, 1, 8, 96, 100) && reg_pays(3584, 3584, 4, 1, 32, 1e29, 1e30));
+    CHECK(reg_pays(18944, 3584, 2, 2, 1, 38000, 1e30) && !reg_pays(19264, 3584, 2, 2, 1, 45800, 1e30) && !reg_pays(9472, 3584, 2, 2, 1, 24200, 1e30));
+    CHECK(!reg_pays(896, 896, 2, 1, 6, 2, 1e30) && !reg_pays(192, 832, 2, 1, 32, 2, 1e30) && reg_pays(640, 256, 2, 1, 12, 94, 100) && !reg_pays(640, 256, 2, 1, 8, 94, 100));
+    CHECK(reg_pays(1600, 192, 2, 1, 32, 2, 1e30) && !reg_pays(320, 192, 4, 1, 4, 2, 1e30) && reg_pays(192, 832, 4, 1, 4, 2, 1e30) && reg_pays(320, 192, 4, 1, 8, 2, 1e30));
+    CHECK(!reg_pays(5120, 2048, 4, 1, 2, 2, 1e30) && reg_pays(2048, 5120, 4, 1, 2, 2, 1e30) && !reg_pays(4864, 896, 4, 1, 3, 2, 1e30) && reg_pays(5120, 2048, 4, 1, 3, 2, 1e30));
     printf("ok\n");
     return 0;
 }
