@@ -66,7 +66,9 @@ int prism_cuda_synchronize(prism_cuda_ctx *ctx);
  * default 1: fused epilogues), "pdl" (0/1, default 1: programmatic dependent launch between
  * the kernels of a decode step, so a kernel's weight-only prologue overlaps its predecessor),
  * "batch_gemv_max" (decode batches up to this many sequences stream the weights once through the batched
- * GEMV, in groups of 8; larger batches use the tcgen05 GEMM; 0, default: per linear the kernel that takes least time),
+ * GEMV, in groups of 8; larger batches use the tcgen05 GEMM; 0, default: per linear the kernel that takes least time.
+ * The register-palette kernel for up to 32 rows is among those only while this option, "gemv_variant" and
+ * "gemm_variant" are all at their defaults),
  * "attn_cluster" (0 = from max_seq, default; 1/2/4/8 CTAs per KV head and sequence in the fused
  * attention kernel),
  * "attn_group" (0 = from the shape, default; 1/2/4/8 = most query heads of a KV group one cluster of the

@@ -80,7 +80,7 @@ struct prism_cuda_ctx {
     int sk_min_chunks = 8;      // stream-K GEMV, small matrices: fewest 1 KB index chunks a CTA is given
     int sk_stream_chunks = 64;  // chunks per CTA from which the balanced contiguous partition is used
     int cl_max_units = 16384;    // cluster GEMV for matrices of at most this many (64-row block, 1 KB chunk) units; 0: never
-    int batch_gemv_max = 0;   // decode batches up to this size use the batched GEMV (groups of 8), larger ones the GEMM; 0: 8, or 7 (gemm_pays_at_8)
+    int batch_gemv_max = 0;   // decode batches up to this size use the batched GEMV (groups of 8), larger ones the GEMM; 0: per linear whichever takes least time
     int attn_cluster = 0;    // CTAs per (head, sequence) of the fused attention kernel; 0: chosen from max_seq
     int ws_whole_blocks = 1024;  // warp-specialised GEMV: one whole block per CTA when there are almost as many blocks as SMs and rows have at most this many chunks; 0: never
     int ws_whole_fill = 50;  // ... for one activation row, when the matrix has at least this many blocks per 100 SMs
@@ -310,7 +310,7 @@ int launch_gemv_tc5(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, cons
 
 // gemm_reg.cu: 1..32 activation rows, palettes in registers; PLAIN, RESID and SWIGLU; norm_eps >= 0 (one row) folds RMSNorm of x.
 // gemm_few_tokens: nothing launched and `takes` false where tensor, mode or alignment are not for it, or another kernel takes less time
-// (reg_pays); launch_gemm_reg: wherever the shape fits
+// (reg_pays), or the options gemv_variant, gemm_variant and batch_gemv_max are not at their defaults; launch_gemm_reg: wherever the shape fits
 int gemm_few_tokens(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,
                     uint32_t y_stride, const uint16_t *resid, uint32_t batch, float norm_eps, bool *takes);
 int launch_gemm_reg(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,

@@ -126,7 +126,7 @@ static int linear(prism_cuda_engine *e, GemvMode mode, const LutTensor &t, const
                   uint32_t xs, uint16_t *y, uint32_t ys, const uint16_t *resid, uint32_t B) {
     prism_cuda_ctx *ctx = e->ctx;
     bool few = false;
-    if (!ctx->batch_gemv_max && B >= 2 && ctx->gemm_variant == 1 && ctx->gemv_variant == 1 && e->gu && xs >= t.k)
+    if (B >= 2 && e->gu && xs >= t.k)
         PRISM_TRY(gemm_few_tokens(ctx, mode, t, t2, x, xs, y, ys, resid, B, -1.0f, &few));
     if (few) return PRISM_OK;
     const uint32_t gemv_max = ctx->batch_gemv_max ? (uint32_t)ctx->batch_gemv_max

@@ -20,7 +20,7 @@ int launch_gemm(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint
     if (t.k % 8) return fail(ctx, PRISM_E_ARG, "gemm: dim_n must be a multiple of 8");
     PRISM_TRY(gemm_input(ctx, t, &X, m_tok, Y));
     bool few = false;
-    if (ctx->gemm_variant == 1 && m_tok >= 2) PRISM_TRY(gemm_few_tokens(ctx, GEMV_PLAIN, t, nullptr, X, t.k, Y, t.m, nullptr, m_tok, -1.0f, &few));
+    if (m_tok >= 2) PRISM_TRY(gemm_few_tokens(ctx, GEMV_PLAIN, t, nullptr, X, t.k, Y, t.m, nullptr, m_tok, -1.0f, &few));
     if (few) return PRISM_OK;
     if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, t, m_tok)) return launch_gemm_tc5(ctx, t, X, m_tok, Y, nullptr);
     // activation rows as the batch dimension of the GEMV kernel, 32768 rows per launch
@@ -34,7 +34,7 @@ int launch_gemm(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint
 
 int launch_gemm_add(prism_cuda_ctx *ctx, const LutTensor &t, const uint16_t *X, uint32_t m_tok, uint16_t *h, uint16_t *tmp) {
     bool few = false;
-    if (ctx->gemm_variant == 1 && m_tok >= 2) PRISM_TRY(gemm_few_tokens(ctx, GEMV_RESID, t, nullptr, X, t.k, h, t.m, h, m_tok, -1.0f, &few));
+    if (m_tok >= 2) PRISM_TRY(gemm_few_tokens(ctx, GEMV_RESID, t, nullptr, X, t.k, h, t.m, h, m_tok, -1.0f, &few));
     if (few) return PRISM_OK;
     if (ctx->gemm_variant == 1 && gemm_tc5_eligible(ctx, t, m_tok) && gemm_tc5_wide(t, h)) return launch_gemm_tc5(ctx, t, X, m_tok, h, h);
     PRISM_TRY(launch_gemm(ctx, t, X, m_tok, tmp));
@@ -48,7 +48,7 @@ int gemm_swiglu_fused(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor 
 }
 int launch_gemm_swiglu(prism_cuda_ctx *ctx, const LutTensor &tg, const LutTensor &tu, const uint16_t *X, uint32_t m_tok, uint16_t *act, uint16_t *u) {
     bool few = false, fused = false;
-    if (ctx->gemm_variant == 1 && m_tok >= 2 && tg.bits == tu.bits && tg.k == tu.k && tg.m == tu.m)
+    if (m_tok >= 2 && tg.bits == tu.bits && tg.k == tu.k && tg.m == tu.m)
         PRISM_TRY(gemm_few_tokens(ctx, GEMV_SWIGLU, tg, &tu, X, tg.k, act, tg.m, nullptr, m_tok, -1.0f, &few));
     if (few) return PRISM_OK;
     PRISM_TRY(gemm_swiglu_fused(ctx, tg, tu, m_tok, act, &fused));

@@ -382,6 +382,7 @@ static int reg_launch(prism_cuda_ctx *ctx, RegArgs &a, const LutTensor &t, RegPl
 int gemm_few_tokens(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const LutTensor *t2, const uint16_t *x, uint32_t x_stride, uint16_t *y,
                     uint32_t y_stride, const uint16_t *resid, uint32_t batch, float norm_eps, bool *takes) {
     *takes = false;
+    if (ctx->gemv_variant != 1 || ctx->gemm_variant != 1 || ctx->batch_gemv_max) return PRISM_OK;  // the caller names the kernels
     if ((reinterpret_cast<uintptr_t>(x) & 15) || x_stride % 8) return PRISM_OK;
     if (mode != GEMV_PLAIN && mode != GEMV_RESID && mode != GEMV_SWIGLU) return PRISM_OK;
     if (batch == 0 || batch > REG_MAX_TOKENS || t.m == 0 || !((t.bits == 4 && t.k % 32 == 0 && t.k >= 32) || (t.bits == 2 && t.k % 64 == 0 && t.k >= 64))) return PRISM_OK;

@@ -444,7 +444,7 @@ int launch_gemv(prism_cuda_ctx *ctx, GemvMode mode, const LutTensor &t, const Lu
     // 2..8 activation rows: one pass over the weights for all of them (larger batches in groups of 8)
     if (mode == GEMV_TP && batch != 1) return fail(ctx, PRISM_E_ARG, "the in-kernel all-reduce takes one activation row");
     bool use_reg = false;
-    if (v == 1 && t.bits == 2 && x_stride >= t.k && (norm_eps < 0.0f || batch == 1))
+    if (t.bits == 2 && x_stride >= t.k && (norm_eps < 0.0f || batch == 1))
         PRISM_TRY(gemm_few_tokens(ctx, mode, t, t2, x, x_stride, y, y_stride, resid, batch, norm_eps, &use_reg));
     if (use_reg) return PRISM_OK;
     const bool use_wsb = (v == 1 || v == 2) && batch >= 2 && wsb_eligible(t, batch < 8 ? batch : 8);

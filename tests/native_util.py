@@ -102,3 +102,11 @@ def dense_stream(backend, packed, k_pad, segs, x, outs, x2=None, wait=True):
         f.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32]
         return f(backend.ctx, C.addressof(l), C.addressof(i), C.addressof(o), x.shape[0])
     _call(backend, "_ZN5prism19launch_dense_streamEP14prism_cuda_ctxRKNS_11DenseLinearERKNS_7DenseInEPKNS_8DenseOutEj", C.byref(l), C.byref(i), o, C.c_uint32(x.shape[0]))
+
+
+def few_tokens_taken(backend, handle, x, y):
+    """y = x W^T where the register-palette kernel is the engine's choice for it; whether it is."""
+    takes = C.c_bool(False)
+    _call(backend, "_ZN5prism15gemm_few_tokensEP14prism_cuda_ctxNS_8GemvModeERKNS_9LutTensorEPS4_PKtjPtjS8_jfPb", C.c_int(0), _tensor(backend, handle), None,
+          C.c_void_p(x.data_ptr()), C.c_uint32(x.stride(0)), C.c_void_p(y.data_ptr()), C.c_uint32(y.stride(0)), None, C.c_uint32(x.shape[0]), C.c_float(-1.0), C.byref(takes))
+    return takes.value

@@ -1,6 +1,6 @@
-"""Eight sequences in a decode step: large linears go through the GEMM, others through the batched GEMV (gemm_pays_at_8).
-The engine's choice against all linears through the one and through the other (option batch_gemv_max), gate and up on both sides
-of the lines for 4 bits (10240 rows) and for 2 (2^25 weights together).  Tolerance as in test_gpu_prefill_attention.py: another order of the fp32 sums, one layer of fp16 roundings."""
+"""Eight sequences in a decode step: the engine's choice against all linears through the tcgen05 GEMM (option batch_gemv_max 1) and through
+the batched GEMV (8), three sets of kernels that add in other orders; gate and up on both sides of the lines of gemm_pays_at_8, for 4 bits
+(10240 rows) and for 2 (2^25 weights together).  Tolerance as in test_gpu_prefill_attention.py: another order of the fp32 sums, one layer of fp16 roundings."""
 import numpy as np
 import pytest
 
@@ -27,8 +27,9 @@ def test_choice_at_eight_sequences(inter, bits):
             return eng.generate(prompts, 3, return_logits=True)
 
     tokens, got = logits(0)
-    for most in (1, 8):
-        other, want = logits(most)
+    arms = {most: logits(most) for most in (1, 8)}
+    assert not np.array_equal(arms[1][1], arms[8][1]) and not np.array_equal(got, arms[8][1])  # other kernels
+    for most, (other, want) in arms.items():
         for b in range(8):
             if np.array_equal(tokens[b], other[b]):
                 assert rel_l2(got[b], want[b]) <= 3.2e-3, (most, b)
