@@ -92,7 +92,8 @@ int prism_cuda_synchronize(prism_cuda_ctx *ctx);
  * through the layers at once -- tensor-core GEMMs, causal attention over the cache, no LM head -- instead of
  * one step per token as the reference's prefill_cpu does; -1, default: the engine's choice, at most 2048; 0 = one
  * step per token.  Single GPU, fp16 KV),
- * "layered_chunk" (default 2048: the same for models described layer by layer; read when the engine is created),
+ * "layered_chunk" (default 2048: the same for models described layer by layer, of one sequence; of several together
+ * at most 2048, and fewer where memory is short; read when the engine is created),
  * "tp_fused_ar" (batch-1 tensor-parallel decode, how the partial sums of a row-parallel matmul are reduced:
  * 0 = the GEMV leaves fp32 partial sums, one kernel pushes them to the peers and reduces; 1 = the GEMV's epilogue
  * stores its sums into every rank's receive area, a small kernel publishes flags, waits and reduces; 2 = flags,

@@ -87,7 +87,7 @@ struct prism_cuda_ctx {
     int attn_group = 0;      // most query heads of a KV group one cluster of the fused attention serves (1/2/4/8); 0: chosen from the shape
     int pdl = 1;  // programmatic dependent launch between the kernels of the decode chain
     int prefill_chunk = -1;  // most prompt tokens generate() puts through the layers at once (tensor-core GEMMs); -1: the engine's choice, 0: one step per token
-    int layered_chunk = 2048;  // layered models: most prompt tokens of a sequence that go through the layers at once (read at engine creation)
+    int layered_chunk = 2048;  // layered models: most prompt tokens of a sequence that go through the layers at once, of several at most 2048 (read at engine creation)
     int cimage_cache = 0;  // engine_load_cimage keeps / uses the cache of the re-laid image beside the file
     // Upper bound, in polls, of the device-side waits on something outside the waiting CTA (a peer
     // GPU's flag, a grid-wide arrival); a wait that runs out sets the device error word and the

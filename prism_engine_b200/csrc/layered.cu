@@ -20,6 +20,7 @@
 #include <cstring>
 
 #include "layered.hpp"
+#include "scratch.hpp"
 
 namespace prism {
 
@@ -299,7 +300,6 @@ static int build_sequential_layer(prism_cuda_engine *e, LayeredLayer &ly, uint32
                 name_packed(m, q + ".down", D, c.ff, ly.down, 0, 0, x * ly.down.n_tiles * 128);
             }
             m->aux_pitch = std::max(m->aux_pitch, round_up_u32(c.experts, 4));
-            m->pairs_cap = std::max(m->pairs_cap, (size_t)m->cap * c.top);
             m->plan.experts = std::max(m->plan.experts, c.experts);
             m->plan.top = std::max(m->plan.top, c.top);
         } else {
@@ -355,13 +355,77 @@ static int build_layer(prism_cuda_engine *e, uint32_t i, const prism_layer_confi
 constexpr size_t STEP_HOST_MAX = 4u << 20;
 static size_t step_host_words(size_t n) { return 4 * n + 4; }
 
+// Buffers that hold a row for every token of a portion, or of a decode step: f(pointer, bytes) for each.  What follows a sequence is done
+// with one span of it before the next, so the chunked delta rule's buffers hold the longest span.
+template <typename F>
+static int row_buffers(LayeredModel *m, uint32_t cap, F &&f) {
+    const prism_layered_config &c = m->c;
+    const size_t es = m->act32 ? 4 : 2, rows = cap, pairs = rows * m->plan.top;
+    auto words = [&](auto *&p, size_t n) { return f(reinterpret_cast<void **>(&p), n * 4); };
+    auto acts = [&](void *&p, size_t n) { return f(&p, n * es); };
+    PRISM_TRY(words(m->x, rows * c.width));
+    PRISM_TRY(acts(m->xn, rows * m->width_pad));
+    PRISM_TRY(acts(m->proj, rows * m->proj_pitch));
+    PRISM_TRY(acts(m->cat, rows * m->cat_pitch));
+    if (m->q_pitch) {
+        PRISM_TRY(acts(m->q, rows * m->q_pitch));
+        PRISM_TRY(acts(m->cq, rows * m->cq_pitch));
+    }
+    PRISM_TRY(words(m->want_idx, rows));
+    PRISM_TRY(words(m->pf_tok, rows));
+    size_t delta = 0;
+    for (const LayeredLayer &ly : m->layers)
+        for (const LayeredMixer &mx : ly.mix)
+            if (mx.c.mixer == PRISM_MIXER_GATED_DELTA) delta = std::max(delta, delta_scratch_bytes(mx.da, m->chunk));
+    if (delta) {
+        PRISM_TRY(acts(m->conv, (size_t)m->chunk * m->conv_pitch));
+        PRISM_TRY(words(m->o32, (size_t)m->chunk * m->o32_width));
+        if (!m->act32) PRISM_TRY(f(&m->delta, delta));
+    }
+    if (m->aux_pitch) PRISM_TRY(words(m->aux, rows * m->aux_pitch));
+    if (c.arrangement == PRISM_ARRANGE_SEQUENTIAL) {
+        if (c.canon_taps) PRISM_TRY(acts(m->xc, rows * m->width_pad));
+        PRISM_TRY(acts(m->y, std::max(2 * rows, pairs) * m->y_pitch));
+        if (m->act_pitch) PRISM_TRY(acts(m->act, std::max(rows, pairs) * m->act_pitch));
+        if (c.depth_average) PRISM_TRY(words(m->history, (c.num_layers + 1) * rows * c.width));
+    }
+    if (pairs) {
+        MoePlan &pl = m->plan;
+        PRISM_TRY(acts(m->moe_x, pairs * m->width_pad));
+        PRISM_TRY(words(pl.idx, pairs));
+        PRISM_TRY(words(pl.wgt, pairs));
+        PRISM_TRY(words(pl.order, pairs));
+        PRISM_TRY(words(pl.inv, pairs));
+    }
+    return PRISM_OK;
+}
+// For portions of m->portion tokens, or of fewer: a portion of several sequences is worth an eighth of the memory that is left and no
+// failure, so it shrinks by halves down to m->chunk, what one sequence needs.
+static int alloc_rows(prism_cuda_engine *e) {
+    LayeredModel *m = e->lm;
+    size_t left = 0, total = 0;
+    PRISM_CUDA_TRY(e->ctx, cudaMemGetInfo(&left, &total));
+    const size_t before = m->allocs.size();
+    return fit_rows(m->portion, m->chunk, [&](uint32_t n) -> int {
+        for (; m->allocs.size() > before; m->allocs.pop_back()) cudaFree(m->allocs.back());
+        (void)cudaGetLastError();
+        m->cap = std::max(n, m->c.max_batch);
+        size_t want = 0;
+        PRISM_TRY(row_buffers(m, m->cap, [&](void **, size_t bytes) {
+            want += bytes;
+            return PRISM_OK;
+        }));
+        if (n > m->chunk && want > left / 8) return PRISM_E_CUDA;
+        return row_buffers(m, m->cap, [&](void **p, size_t bytes) { return model_alloc(e, p, bytes); });
+    });
+}
+
 static int build_model(prism_cuda_engine *e, const prism_layer_config *layers) {
     LayeredModel *m = e->lm;
     const prism_layered_config &c = m->c;
-    const size_t es = m->act32 ? 4 : 2;
     m->width_pad = round_up_u32(c.width, 64);
     m->vocab_pad = round_up_u32(c.vocab, 4);
-    m->cap = std::max(m->portion, c.max_batch);
+    m->y_pitch = round_up_u32(c.width, 8);
     m->layers.resize(c.num_layers);  // never resized again: names point into it
     PRISM_TRY(model_alloc(e, m->embed, (size_t)c.vocab * c.width));
     LayeredDst &em = add_name(m, "embed", c.vocab, c.width);
@@ -380,22 +444,11 @@ static int build_model(prism_cuda_engine *e, const prism_layer_config *layers) {
     PRISM_TRY(finish_linear(e, m->head, m->width_pad));
     name_packed(m, "head", c.vocab, c.width, m->head, 0);
     m->lg_cap = std::max(64u, c.max_batch);
-    PRISM_TRY(model_alloc(e, m->x, (size_t)m->cap * c.width));
     PRISM_TRY(model_alloc(e, m->xw, (size_t)m->lg_cap * c.width));
     PRISM_TRY(model_alloc(e, m->logits, (size_t)m->lg_cap * m->vocab_pad));
-    PRISM_TRY(model_alloc(e, &m->xn, (size_t)m->cap * m->width_pad * es));
-    PRISM_TRY(model_alloc(e, &m->proj, (size_t)m->cap * m->proj_pitch * es));
-    PRISM_TRY(model_alloc(e, &m->cat, (size_t)m->cap * m->cat_pitch * es));
-    if (m->q_pitch) {
-        PRISM_TRY(model_alloc(e, &m->q, (size_t)m->cap * m->q_pitch * es));
-        PRISM_TRY(model_alloc(e, &m->cq, (size_t)m->cap * m->cq_pitch * es));
-    }
-    PRISM_TRY(model_alloc(e, m->want_idx, m->cap));
-    PRISM_TRY(model_alloc(e, m->pf_tok, m->cap));
     PRISM_TRY(model_alloc(e, m->row_slot, c.max_batch));
     PRISM_TRY(model_alloc(e, m->row_pos, c.max_batch));
     size_t qa = 0, part = 0, ml = 0;
-    size_t delta = 0;
     for (const LayeredLayer &ly : m->layers)
         for (const LayeredMixer &mx : ly.mix)
             if (mx.c.mixer == PRISM_MIXER_LATENT_ATTENTION) {
@@ -404,29 +457,9 @@ static int build_model(prism_cuda_engine *e, const prism_layer_config *layers) {
                 qa = std::max(qa, q1);
                 part = std::max(part, p1);
                 ml = std::max(ml, m1);
-            } else if (mx.c.mixer == PRISM_MIXER_GATED_DELTA) {
-                delta = std::max(delta, delta_scratch_bytes(mx.da, m->cap));
             }
-    if (delta) {
-        PRISM_TRY(model_alloc(e, &m->conv, (size_t)m->cap * m->conv_pitch * es));
-        PRISM_TRY(model_alloc(e, m->o32, (size_t)m->cap * m->o32_width));
-        if (!m->act32) PRISM_TRY(model_alloc(e, &m->delta, delta));
-    }
-    if (m->aux_pitch) PRISM_TRY(model_alloc(e, m->aux, (size_t)m->cap * m->aux_pitch));
-    if (c.arrangement == PRISM_ARRANGE_SEQUENTIAL) {
-        m->y_pitch = round_up_u32(c.width, 8);
-        if (c.canon_taps) PRISM_TRY(model_alloc(e, &m->xc, (size_t)m->cap * m->width_pad * es));
-        PRISM_TRY(model_alloc(e, &m->y, std::max((size_t)2 * m->cap, m->pairs_cap) * m->y_pitch * es));
-        if (m->act_pitch) PRISM_TRY(model_alloc(e, &m->act, std::max((size_t)m->cap, m->pairs_cap) * m->act_pitch * es));
-        if (c.depth_average) PRISM_TRY(model_alloc(e, m->history, (size_t)(c.num_layers + 1) * m->cap * c.width));
-    }
-    if (m->pairs_cap) {
+    if (m->plan.top) {
         MoePlan &pl = m->plan;
-        PRISM_TRY(model_alloc(e, &m->moe_x, m->pairs_cap * m->width_pad * es));
-        PRISM_TRY(model_alloc(e, pl.idx, m->pairs_cap));
-        PRISM_TRY(model_alloc(e, pl.wgt, m->pairs_cap));
-        PRISM_TRY(model_alloc(e, pl.order, m->pairs_cap));
-        PRISM_TRY(model_alloc(e, pl.inv, m->pairs_cap));
         PRISM_TRY(model_alloc(e, pl.count, pl.experts));
         PRISM_TRY(model_alloc(e, pl.n_active, 1));
         PRISM_TRY(model_alloc(e, pl.active, DENSE_GEMV_ROWS * pl.top));
@@ -438,6 +471,7 @@ static int build_model(prism_cuda_engine *e, const prism_layer_config *layers) {
         PRISM_TRY(model_alloc(e, m->rows_scratch.part, part * m->rows_scratch.rows_cap));
         PRISM_TRY(model_alloc(e, m->rows_scratch.ml, ml * m->rows_scratch.rows_cap));
     }
+    PRISM_TRY(alloc_rows(e));  // last: what is left
     m->slot_pos.assign(c.max_batch, -1);
     // Once, here: allocated by the first decode step it took 2 to 4 ms of that call, and up to 80 on a busy host.
     const size_t least = step_host_words(c.max_batch);
@@ -598,7 +632,7 @@ static int mix_delta(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, c
     const DenseSeg *seg = ly.in.seg + mx.seg0;
     DeltaArgs a = mx.da;
     a.rows = n;
-    const size_t p0 = (size_t)r0 * m->proj_pitch, v0 = (size_t)r0 * m->conv_pitch;
+    const size_t p0 = (size_t)r0 * m->proj_pitch;
     a.q = at(m, m->proj, p0 + seg[0].row0); a.k = at(m, m->proj, p0 + seg[1].row0); a.v = at(m, m->proj, p0 + seg[2].row0); a.pitch = m->proj_pitch;
     a.ba = m->aux + (size_t)r0 * m->aux_pitch; a.ba_pitch = m->aux_pitch;
     a.gate = at(m, m->proj, p0 + seg[4].row0); a.gate_pitch = m->proj_pitch;
@@ -608,9 +642,9 @@ static int mix_delta(prism_cuda_engine *e, LayeredLayer &ly, LayeredMixer &mx, c
     const uint32_t hk = a.kv_heads * a.dim;
     ConvArgs c{};
     c.pieces = 3; c.x_pitch = m->proj_pitch; c.y_pitch = m->conv_pitch; c.taps = a.taps; c.channels = a.channels; c.w = a.conv_w; c.ring = a.ring; c.silu = 1;
-    c.piece[0] = ConvPiece{a.q, at(m, m->conv, v0 + mx.conv_col[0]), hk, 0};
-    c.piece[1] = ConvPiece{a.k, at(m, m->conv, v0 + mx.conv_col[1]), hk, hk};
-    c.piece[2] = ConvPiece{a.v, at(m, m->conv, v0 + mx.conv_col[2]), a.heads * a.vdim, 2 * hk};
+    c.piece[0] = ConvPiece{a.q, at(m, m->conv, mx.conv_col[0]), hk, 0};
+    c.piece[1] = ConvPiece{a.k, at(m, m->conv, mx.conv_col[1]), hk, hk};
+    c.piece[2] = ConvPiece{a.v, at(m, m->conv, mx.conv_col[2]), a.heads * a.vdim, 2 * hk};
     PRISM_TRY(launch_conv_seq(ctx, c, rows, n, m->act32));
     a.q = c.piece[0].y; a.k = c.piece[1].y; a.v = c.piece[2].y; a.pitch = m->conv_pitch;
     a.o32 = m->o32; a.chunk_scratch = m->delta;
@@ -1107,8 +1141,10 @@ int prism_cuda_engine_create_layered(prism_cuda_ctx *ctx, const prism_layered_co
     e->lm = new LayeredModel();
     e->lm->c = c;
     e->lm->act32 = c.dtype == PRISM_DTYPE_F32;
-    e->lm->chunk = std::min(c.max_seq, (uint32_t)std::max(1, ctx->layered_chunk));
-    e->lm->portion = (uint32_t)std::min<uint64_t>((uint64_t)c.max_seq * c.max_batch, (uint64_t)std::max(1, ctx->layered_chunk));
+    // the row-wise kernels have a row per block of their grid's second dimension
+    const uint32_t chunk = std::min(65535u, (uint32_t)std::max(1, ctx->layered_chunk));
+    e->lm->chunk = std::min(c.max_seq, chunk);
+    e->lm->portion = std::max(e->lm->chunk, (uint32_t)std::min<uint64_t>((uint64_t)c.max_seq * c.max_batch, std::min(chunk, LAYERED_SHARED_MOST)));
     // what the shared loop reads of the palettized configuration
     e->cfg.num_layers = c.num_layers; e->cfg.hidden_size = c.width; e->cfg.vocab_size = c.vocab; e->cfg.norm_eps = c.norm_eps;
     e->cfg.max_seq = c.max_seq; e->cfg.max_batch = c.max_batch;

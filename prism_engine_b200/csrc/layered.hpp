@@ -59,6 +59,9 @@ struct LayeredDst {
     bool bound = false;
 };
 
+// Most tokens of several sequences together, whatever one sequence may have: linears of 2048 rows fill the GPU, and row buffers grow with it.
+constexpr uint32_t LAYERED_SHARED_MOST = 2048;
+
 struct LayeredModel {
     prism_layered_config c{};
     std::vector<LayeredLayer> layers;
@@ -71,7 +74,7 @@ struct LayeredModel {
     std::vector<std::string> order;                // names in layer order
     // scratch for `cap` rows
     uint32_t cap = 0, lg_cap = 0;
-    uint32_t chunk = 0, portion = 0;  // most prompt tokens of one sequence, and of all together, that go through the layers at once
+    uint32_t chunk = 0, portion = 0;  // most prompt tokens of one sequence, and of all together, that go through the layers at once; never less than chunk
     float *x = nullptr, *xw = nullptr, *logits = nullptr;
     void *xn = nullptr, *proj = nullptr, *cat = nullptr, *q = nullptr, *cq = nullptr;
     uint32_t proj_pitch = 0, cat_pitch = 0, q_pitch = 0, cq_pitch = 0;
@@ -81,7 +84,6 @@ struct LayeredModel {
     void *xc = nullptr, *y = nullptr, *moe_x = nullptr, *act = nullptr, *conv = nullptr, *delta = nullptr;  // convolved norm, results, experts' rows
     float *aux = nullptr, *history = nullptr, *o32 = nullptr;  // fp32 projections, residual stream after every layer, outputs before their norm
     uint32_t aux_pitch = 0, y_pitch = 0, act_pitch = 0, conv_pitch = 0, o32_width = 0;
-    size_t pairs_cap = 0;                          // rows of the experts' buffers
     MoePlan plan{};                                // buffers; experts and top are the layer's
     cudaStream_t side = nullptr;                   // the second mixer of a pair, in prompt portions
     cudaEvent_t fork = nullptr, join = nullptr;

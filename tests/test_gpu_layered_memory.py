@@ -1,5 +1,5 @@
 """Row buffers of a layered model: a portion of several short sequences takes at most an eighth of the memory that is left, else it
-shrinks; what the chunked delta rule needs follows the longest sequence, not the portion; and no portion has more rows than a launch has.
+shrinks; more sequences add caches, and rows only up to 2048 however many tokens one sequence may have at once.
 
 The logits of a smaller portion differ as in test_gpu_layered_portions.py: other row counts, bf16 roundings, 2e-2 of the norm."""
 import numpy as np
@@ -17,7 +17,7 @@ def _model(chunk=2048, max_seq=MAX_SEQ, max_batch=SEQS, layers=LAYERS, hog_to=No
 
     import prism_engine_b200 as p
 
-    cfg = p.LayeredConfig.from_dict(lu.tozarax([lu.pair(lu.attention(8, 2, 128, 128), lu.delta(8, 8, 128, 128), lu.moe(4, 4, 64))] * layers, width=WIDTH))
+    cfg = p.LayeredConfig.from_dict(lu.tozarax([lu.pair(lu.attention(8, 2, 128, 128), lu.delta(8, 8, 128, 128), lu.moe(4, 4, 64))] * layers, width=WIDTH, max_positions=4096))
     hog = None
     with p.CudaBackend(device=0) as be:
         be.set_option("layered_chunk", chunk)
