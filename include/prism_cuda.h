@@ -161,7 +161,8 @@ int prism_cuda_download_payload(prism_cuda_ctx *ctx, int32_t handle, uint8_t *pa
  * the row (encode_channel, :189-217) and writes the reference payload (dim_m x 16 fp16 palettes,
  * then dim_m rows of dim_n/2 index bytes), bit-identical to the CPU quantiser.  dim_n must be even;
  * len must be dim_m*32 + dim_m*dim_n/2.  Host pointers; _dev takes device pointers and runs on the
- * context stream. */
+ * context stream.  Between host calls the context keeps 4 MB of pinned memory and device buffers of up to 64 MB,
+ * which any other allocation of the context that finds no memory takes back. */
 int prism_cuda_palettize(prism_cuda_ctx *ctx, const float *weights, uint32_t dim_m, uint32_t dim_n, uint32_t k,
                          uint32_t max_iter, uint8_t *payload, size_t len);
 int prism_cuda_palettize_dev(prism_cuda_ctx *ctx, const float *weights_dev, uint32_t dim_m, uint32_t dim_n,

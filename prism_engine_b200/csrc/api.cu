@@ -30,6 +30,16 @@ int after_launch(prism_cuda_ctx *ctx, const char *kernel) {
     return PRISM_OK;
 }
 
+cudaError_t device_malloc(prism_cuda_ctx *ctx, void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && palettize_pool_trim(ctx->palettize)) {
+        (void)cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+}
+
 // cudaMalloc / cudaFree behind the allocator interface of grow_buf (scratch.hpp).
 struct CudaScratchAlloc {
     prism_cuda_ctx *ctx;
@@ -37,7 +47,7 @@ struct CudaScratchAlloc {
     const char *what = "";
     int sync() { what = "cudaStreamSynchronize"; last = cudaStreamSynchronize(ctx->stream); return last == cudaSuccess ? 0 : 1; }
     int release(void *p) { what = "cudaFree"; last = cudaFree(p); return last == cudaSuccess ? 0 : 1; }
-    int acquire(void **p, size_t bytes) { what = "cudaMalloc"; last = cudaMalloc(p, bytes); return last == cudaSuccess ? 0 : 1; }
+    int acquire(void **p, size_t bytes) { what = "cudaMalloc"; last = device_malloc(ctx, p, bytes); return last == cudaSuccess ? 0 : 1; }
 };
 
 // Grows one of the context's scratch buffers to `want` elements.  Pointer and element count are
@@ -130,8 +140,8 @@ int alloc_tensor(prism_cuda_ctx *ctx, const char *name, uint32_t m, uint32_t k, 
     t.n_chunks = (t.row_bytes + 15) / 16;
     t.idx_bytes = (size_t)t.n_hb * t.n_chunks * 512;
     t.pal_bytes = (size_t)t.m_pad * t.n_ent() * 2;
-    PRISM_CUDA_TRY(ctx, cudaMalloc((void **)&t.idx, t.idx_bytes));
-    cudaError_t e = cudaMalloc((void **)&t.pal, t.pal_bytes);
+    PRISM_CUDA_TRY(ctx, device_malloc(ctx, (void **)&t.idx, t.idx_bytes));
+    cudaError_t e = device_malloc(ctx, (void **)&t.pal, t.pal_bytes);
     if (e != cudaSuccess) {
         cudaFree(t.idx);
         return cuda_fail(ctx, e, "cudaMalloc(palettes)");
@@ -735,8 +745,8 @@ int prism_cuda_kv_init(prism_cuda_ctx *ctx, uint32_t num_layers, uint32_t kv_dim
     ctx->kv_k = ctx->kv_v = nullptr;
     ctx->kv_layers = ctx->kv_dim = ctx->kv_max_seq = 0;
     const size_t bytes = (size_t)num_layers * max_seq * kv_dim * 2;
-    PRISM_CUDA_TRY(ctx, cudaMalloc((void **)&ctx->kv_k, bytes));
-    cudaError_t e = cudaMalloc((void **)&ctx->kv_v, bytes);
+    PRISM_CUDA_TRY(ctx, device_malloc(ctx, (void **)&ctx->kv_k, bytes));
+    cudaError_t e = device_malloc(ctx, (void **)&ctx->kv_v, bytes);
     if (e != cudaSuccess) {
         cudaFree(ctx->kv_k);
         ctx->kv_k = nullptr;

@@ -62,6 +62,7 @@ struct prism_nccl_api;
 namespace prism {
 struct PalettizePool;
 void palettize_pool_free(PalettizePool *pool);
+bool palettize_pool_trim(PalettizePool *pool);  // gives the device buffers back; whether there were any
 }  // namespace prism
 
 // The opaque context of the C ABI.
@@ -217,6 +218,8 @@ inline void launch_pdl(prism_cuda_ctx *ctx, const char *name, void (*kernel)(KAr
 }
 #endif
 
+// cudaMalloc; where memory is short it takes back what the quantiser keeps.  A failure leaves nothing in the last-error slot.
+cudaError_t device_malloc(prism_cuda_ctx *ctx, void **p, size_t bytes);
 int ensure_stage(prism_cuda_ctx *ctx, size_t in_bytes, size_t out_bytes);
 int ensure_splitk(prism_cuda_ctx *ctx, size_t floats, size_t counters);
 int ensure_act(prism_cuda_ctx *ctx, size_t halfs);

@@ -15,7 +15,7 @@ namespace prism {
 int dense_alloc(prism_cuda_ctx *ctx, DenseLinear &l, uint32_t k_pad, uint32_t n_tiles) {
     l.k_pad = k_pad;
     l.n_tiles = n_tiles;
-    PRISM_CUDA_TRY(ctx, cudaMalloc((void **)&l.w, l.bytes()));
+    PRISM_CUDA_TRY(ctx, device_malloc(ctx, (void **)&l.w, l.bytes()));
     PRISM_CUDA_TRY(ctx, cudaMemsetAsync(l.w, 0, l.bytes(), ctx->stream));
     return PRISM_OK;
 }

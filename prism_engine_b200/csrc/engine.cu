@@ -429,7 +429,7 @@ static int ensure_prefill(prism_cuda_engine *e, uint32_t T) {
     const uint32_t wq = e->qd_l + 2 * e->kvd_l;
     const size_t bytes[] = {(size_t)T * e->H * 2, (size_t)T * e->H * 2, (size_t)T * wq * 2, (size_t)T * e->qd_l * 2, (size_t)T * e->I_l * 2};
     for (size_t i = 0; i < sizeof(ptrs) / sizeof(ptrs[0]); i++) {
-        cudaError_t ce = cudaMalloc(ptrs[i], (bytes[i] + 255) / 256 * 256);
+        cudaError_t ce = device_malloc(ctx, ptrs[i], (bytes[i] + 255) / 256 * 256);
         if (ce != cudaSuccess) return cuda_fail(ctx, ce, "cudaMalloc(prefill scratch)");
     }
     e->pf_cap = T;
@@ -442,7 +442,7 @@ static int ensure_prefill_up(prism_cuda_engine *e, uint32_t T) {
     cudaFree(e->pf_u);
     e->pf_u = nullptr;
     e->pf_up_cap = 0;
-    PRISM_CUDA_TRY(e->ctx, cudaMalloc((void **)&e->pf_u, (size_t)T * e->I_l * 2));
+    PRISM_CUDA_TRY(e->ctx, device_malloc(e->ctx, (void **)&e->pf_u, (size_t)T * e->I_l * 2));
     e->pf_up_cap = T;
     return PRISM_OK;
 }
@@ -522,7 +522,7 @@ int set_scalars(prism_cuda_engine *e, int32_t pos, int32_t step, int32_t record)
 // What every engine has whatever its model: tokens in and out, the step's scalars, events.
 int engine_alloc_common(prism_cuda_engine *e, uint32_t B) {
     prism_cuda_ctx *ctx = e->ctx;
-    auto A = [&](void **p, size_t bytes) { return cudaMalloc(p, (bytes + 255) / 256 * 256); };
+    auto A = [&](void **p, size_t bytes) { return device_malloc(ctx, p, (bytes + 255) / 256 * 256); };
     cudaError_t ce = A((void **)&e->tok, (size_t)B * 4);
     if (ce == cudaSuccess) ce = A((void **)&e->next, (size_t)B * 4);
     if (ce == cudaSuccess) ce = A((void **)&e->out_tokens, (size_t)B * e->out_cap * 4);
@@ -620,7 +620,7 @@ int prism_cuda_engine_create(prism_cuda_ctx *ctx, const prism_model_config *cfg,
         e->kv_seq_stride = (uint64_t)e->kv_slots * e->kvd_l;
         e->kv_layer_bytes = (size_t)B * e->kv_seq_stride * 2;
     }
-    auto A = [&](void **p, size_t bytes) { return cudaMalloc(p, (bytes + 255) / 256 * 256); };
+    auto A = [&](void **p, size_t bytes) { return device_malloc(ctx, p, (bytes + 255) / 256 * 256); };
     cudaError_t ce = cudaSuccess;
 #define ALLOC(ptr, bytes) if (ce == cudaSuccess) ce = A((void **)&(ptr), (bytes))
     ALLOC(e->h, (size_t)B * e->H * 2);
@@ -867,7 +867,7 @@ int prism_cuda_engine_generate(prism_cuda_engine *e, const uint32_t *prompts, ui
         cudaFree(e->prompts);
         e->prompts = nullptr;
         e->prompts_cap = 0;
-        PRISM_CUDA_TRY(ctx, cudaMalloc((void **)&e->prompts, need * 4));
+        PRISM_CUDA_TRY(ctx, device_malloc(ctx, (void **)&e->prompts, need * 4));
         e->prompts_cap = need;
     }
     std::vector<uint32_t> tr;

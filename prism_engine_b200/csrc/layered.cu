@@ -28,7 +28,7 @@ namespace prism {
 
 static int model_alloc(prism_cuda_engine *e, void **p, size_t bytes) {
     *p = nullptr;
-    cudaError_t ce = cudaMalloc(p, (bytes + 255) / 256 * 256);
+    cudaError_t ce = device_malloc(e->ctx, p, (bytes + 255) / 256 * 256);
     if (ce != cudaSuccess) return cuda_fail(e->ctx, ce, "cudaMalloc(model)");
     e->lm->allocs.push_back(*p);
     // padding that a kernel reads must be finite
@@ -569,7 +569,7 @@ static int grow_bf16(prism_cuda_engine *e, bf16 *&p, size_t &have, size_t want) 
     cudaFree(p);
     p = nullptr;
     have = 0;
-    cudaError_t ce = cudaMalloc((void **)&p, want * 2);
+    cudaError_t ce = device_malloc(e->ctx, (void **)&p, want * 2);
     if (ce != cudaSuccess) return cuda_fail(e->ctx, ce, "cudaMalloc(expanded keys and values)");
     PRISM_CUDA_TRY(e->ctx, cudaMemsetAsync(p, 0, want * 2, e->ctx->stream));
     have = want;

@@ -402,15 +402,15 @@ static cudaError_t palettize_rows(const float *w_dev, uint32_t dm, uint32_t dn, 
 // ---- a matrix in host memory -----------------------------------------------------------------------
 // A copy from pageable memory goes through the driver at 12 GB/s, one thread, also when several ask, and a copy into memory that was
 // never touched at 2.  Here up to 4 threads carry a part of the rows each onto the GPU and their payload back, through two pinned
-// slots of their own.  The slots (4 MB; in huge pages their first use takes 1.5 ms, through cudaHostAlloc 3 to 15) and the device
-// buffers stay with the context and go with it; device buffers above PZ_KEEP are given back at once.
+// slots of their own.  The slots (4 MB; in huge pages their first use takes 1.5 ms, through cudaHostAlloc 3 to 15) and device buffers of
+// at most PZ_KEEP together stay with the context; another allocation that finds no memory takes the device buffers back (device_malloc).
 // 3584 x 3584 values: 8.0 -> 3.4 ms (matrix 1.8, kernel 1.08, payload 0.5), a context's first call 9.9 -> 6.4; 896 x 896, one thread and
 // kept device buffers: 1.13 -> 0.5 ms.
 constexpr uint32_t PZ_WORKERS = 4;
 constexpr size_t PZ_SLOT = 512 * 1024;                  // two of them a worker
 constexpr size_t PZ_PAGE = 2 << 20;
 constexpr size_t PZ_LEAST = 8 << 20;                    // bytes of a matrix from which it is shared: below, the slots' first use takes longer than they save
-constexpr size_t PZ_KEEP = 256 << 20;
+constexpr size_t PZ_KEEP = 64 << 20;                    // matrix and payload of 3584 x 3584 are 58
 
 struct PalettizePool {
     uint8_t *pinned = nullptr;
@@ -427,6 +427,17 @@ void palettize_pool_free(PalettizePool *p) {
     free(p->pinned);
     for (void *d : p->dev) cudaFree(d);
     delete p;
+}
+
+bool palettize_pool_trim(PalettizePool *p) {
+    bool any = false;
+    for (int i = 0; p && i < 2; i++) {
+        any = any || p->dev[i];
+        cudaFree(p->dev[i]);
+        p->dev[i] = nullptr;
+        p->bytes[i] = 0;
+    }
+    return any;
 }
 
 struct PalettizeJob {
@@ -580,12 +591,8 @@ extern "C" int prism_cuda_palettize(prism_cuda_ctx *ctx, const float *weights, u
         if (e == cudaSuccess) e = done;
         if (e == cudaSuccess) ctx->launches++;
     }
-    for (int i = 0; i < 2; i++)
-        if (pool.bytes[i] > PZ_KEEP || e != cudaSuccess) {
-            cudaFree(pool.dev[i]);
-            pool.dev[i] = nullptr;
-            pool.bytes[i] = 0;
-        }
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "palettize");
-    return PRISM_OK;
+    if (pool.bytes[0] + pool.bytes[1] > PZ_KEEP || e != cudaSuccess) palettize_pool_trim(&pool);
+    if (e == cudaSuccess) return PRISM_OK;
+    (void)cudaGetLastError();
+    return cuda_fail(ctx, e, "palettize");
 }
