@@ -51,10 +51,10 @@ __device__ __forceinline__ float pq_threshold(float total, uint32_t seed) {
 }
 
 __global__ void __launch_bounds__(PQ_THREADS) palettize_rows_kernel(const float *__restrict__ w, uint32_t dm,
-                                                                    uint32_t dn, uint32_t row0, uint32_t row1, uint32_t k_req,
-                                                                    uint32_t max_iter, uint8_t *__restrict__ payload) {
-    const uint32_t r = row0 + blockIdx.x * PQ_THREADS + threadIdx.x;
-    if (r >= row1) return;
+                                                                    uint32_t dn, uint32_t k_req, uint32_t max_iter,
+                                                                    uint8_t *__restrict__ payload) {
+    const uint32_t r = blockIdx.x * PQ_THREADS + threadIdx.x;
+    if (r >= dm) return;
     const float *ch = w + (size_t)r * dn;
     const uint32_t n = dn;
     float cb[16];
@@ -200,7 +200,7 @@ __device__ __forceinline__ uint32_t pb_nearest(float x, const float (&cb)[16]) {
 }
 
 __global__ void __launch_bounds__(PB_THREADS) palettize_block_kernel(const float *__restrict__ w, uint32_t dm, uint32_t n,
-                                                                     uint32_t row0, uint32_t k_req, uint32_t max_iter, uint8_t *__restrict__ payload) {
+                                                                     uint32_t k_req, uint32_t max_iter, uint8_t *__restrict__ payload) {
     extern __shared__ __align__(16) float md[];
     __shared__ float cbs[16];
     __shared__ uint32_t cnt[PB_WARPS][16], off[PB_WARPS][16], first[17];
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(PB_THREADS) palettize_block_kernel(const float
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t tiles = (n + 31) / 32;
     float *running = md + (size_t)tiles * 32;
-    const size_t row = row0 + blockIdx.x;
+    const size_t row = blockIdx.x;
     const float *ch = w + row * n;
     uint8_t *idx = payload + (size_t)dm * 32 + row * (n / 2);
     uint32_t k = k_req > 16 ? 16 : k_req;
@@ -379,9 +379,7 @@ __global__ void __launch_bounds__(PB_THREADS) palettize_block_kernel(const float
         reinterpret_cast<uint16_t *>(payload + row * 32)[tid] = __half_as_ushort(__float2half_rn(cbs[tid]));
 }
 
-// Rows row0 .. row1 - 1 of a matrix of dm rows.
-static cudaError_t palettize_rows(const float *w_dev, uint32_t dm, uint32_t dn, uint32_t row0, uint32_t row1, uint32_t k, uint32_t max_iter,
-                                  uint8_t *payload_dev, cudaStream_t stream) {
+static cudaError_t palettize_rows(const float *w_dev, uint32_t dm, uint32_t dn, uint32_t k, uint32_t max_iter, uint8_t *payload_dev, cudaStream_t stream) {
     const size_t smem = pb_smem_bytes(dn);
     // Many short rows: a block pays some 15 ns of the GPU a row before its first element, a thread per row 14 us an element however
     // many rows there are up to the GPU's threads.  100000 rows of 16 / 64 / 128 values: blocks 1541 / 2059 / 2384 us, threads 165 /
@@ -392,9 +390,9 @@ static cudaError_t palettize_rows(const float *w_dev, uint32_t dm, uint32_t dn, 
             const cudaError_t e = cudaFuncSetAttribute(palettize_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_MAX_SMEM);
             if (e != cudaSuccess) return e;
         }
-        palettize_block_kernel<<<row1 - row0, PB_THREADS, smem, stream>>>(w_dev, dm, dn, row0, k, max_iter, payload_dev);
+        palettize_block_kernel<<<dm, PB_THREADS, smem, stream>>>(w_dev, dm, dn, k, max_iter, payload_dev);
     } else {
-        palettize_rows_kernel<<<(row1 - row0 + PQ_THREADS - 1) / PQ_THREADS, PQ_THREADS, 0, stream>>>(w_dev, dm, dn, row0, row1, k, max_iter, payload_dev);
+        palettize_rows_kernel<<<(dm + PQ_THREADS - 1) / PQ_THREADS, PQ_THREADS, 0, stream>>>(w_dev, dm, dn, k, max_iter, payload_dev);
     }
     return cudaGetLastError();
 }
@@ -467,7 +465,7 @@ static cudaError_t palettize_share(PalettizeJob &j, uint32_t t) {
     }
     if (e != cudaSuccess) j.failed = 1;
     if (j.carried.fetch_add(1) + 1 == j.workers) {
-        if (!j.failed && (e = palettize_rows(static_cast<const float *>(p.dev[0]), j.dm, j.dn, 0, j.dm, j.k, j.max_iter, p_dev, j.stream)) != cudaSuccess) j.failed = 1;
+        if (!j.failed && (e = palettize_rows(static_cast<const float *>(p.dev[0]), j.dm, j.dn, j.k, j.max_iter, p_dev, j.stream)) != cudaSuccess) j.failed = 1;
         j.launched = 1;
     }
     while (!j.launched) std::this_thread::yield();
@@ -533,7 +531,7 @@ extern "C" int prism_cuda_palettize_dev(prism_cuda_ctx *ctx, const float *weight
     if (!ctx || !weights_dev || !payload_dev) return fail(ctx, PRISM_E_NULL, "null argument");
     if (dim_m == 0 || dim_n == 0 || dim_n % 2 != 0 || k == 0)
         return fail(ctx, PRISM_E_ARG, "palettize: dim_m, dim_n > 0, dim_n even, k >= 1");
-    PRISM_CUDA_TRY(ctx, palettize_rows(weights_dev, dim_m, dim_n, 0, dim_m, k, max_iter, payload_dev, ctx->stream));
+    PRISM_CUDA_TRY(ctx, palettize_rows(weights_dev, dim_m, dim_n, k, max_iter, payload_dev, ctx->stream));
     ctx->launches++;
     return PRISM_OK;
 }
@@ -558,7 +556,7 @@ extern "C" int prism_cuda_palettize(prism_cuda_ctx *ctx, const float *weights, u
     if (e == cudaSuccess) e = palettize_device(pool, 1, need);
     if (e == cudaSuccess && workers == 1) {              // not worth the slots
         e = cudaMemcpyAsync(pool.dev[0], weights, w_bytes, cudaMemcpyHostToDevice, ctx->stream);
-        if (e == cudaSuccess) e = palettize_rows(static_cast<const float *>(pool.dev[0]), dim_m, dim_n, 0, dim_m, k, max_iter, static_cast<uint8_t *>(pool.dev[1]), ctx->stream);
+        if (e == cudaSuccess) e = palettize_rows(static_cast<const float *>(pool.dev[0]), dim_m, dim_n, k, max_iter, static_cast<uint8_t *>(pool.dev[1]), ctx->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(payload, pool.dev[1], need, cudaMemcpyDeviceToHost, ctx->stream);
         const cudaError_t done = cudaStreamSynchronize(ctx->stream);
         if (e == cudaSuccess) e = done;
