@@ -112,6 +112,8 @@ int device_error_result(prism_cuda_ctx *ctx, unsigned int v) {
         return fail(ctx, PRISM_E_STATE, "the cluster GEMV was not launched with the cluster shape it was given" + code);
     case 5:
         return fail(ctx, PRISM_E_TIMEOUT, "a tcgen05 kernel gave up waiting on an mbarrier; its output is incomplete" + code);
+    case 7:
+        return fail(ctx, PRISM_E_TIMEOUT, "the streaming dense linear gave up waiting for one of its copies; its output is incomplete" + code);
     default:
         return fail(ctx, PRISM_E_STATE, "a kernel reported an unknown error" + code);
     }

@@ -243,6 +243,8 @@ int tp_all_reduce_ll_resid(prism_cuda_ctx *ctx, uint16_t *h, size_t n);
 //   3  the peer-memory all-reduce gave up waiting for a peer's slice                   -> PRISM_E_TIMEOUT
 //   4  a grid-wide arrival inside a persistent kernel gave up                          -> PRISM_E_TIMEOUT
 //   5  an mbarrier wait inside a tcgen05 kernel gave up                                -> PRISM_E_TIMEOUT
+//   6  the cluster GEMV found another cluster shape than it was given                  -> PRISM_E_STATE
+//   7  a wait for a copy inside the streaming dense linear gave up                     -> PRISM_E_TIMEOUT
 // The word is cleared, so the context stays usable.
 int check_device_error(prism_cuda_ctx *ctx);
 // The same translation for a caller that has already copied the word to the host (clears it if set).

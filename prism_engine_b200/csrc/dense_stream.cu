@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(DS_THREADS, DS_CTAS) dense_stream_kernel(const
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && gave_up) atomicExch(a.err, 5u);
+    if (threadIdx.x == 0 && gave_up) atomicExch(a.err, 7u);
 }
 
 // ---- host side ---------------------------------------------------------------------------------

@@ -69,3 +69,14 @@ def test_segments(backend):
         native_util.dense_stream(backend, packed, k_pad, segs, x, outs, x2=x2)
         for (o, _), z in zip(outs, want):
             _close(o, z, 1e-5)
+
+
+def test_a_wait_that_gave_up_is_named(backend):
+    """The code that the kernel leaves in the device error word, as the next host call reports it."""
+    import ctypes as C
+
+    f = backend.L._ZN5prism19device_error_resultEP14prism_cuda_ctxj
+    f.restype, f.argtypes = C.c_int, [C.c_void_p, C.c_uint32]
+    assert f(backend.ctx, 7) == -8  # PRISM_E_TIMEOUT
+    assert b"streaming dense linear" in backend.L.prism_cuda_last_error(backend.ctx)
+    backend.synchronize()
