@@ -39,6 +39,12 @@ def _tensor(backend, handle):
     return C.c_void_p(f(backend.ctx, handle))
 
 
+def gemm_tc5(backend, handle, x, y, resid=None):
+    """y = x W^T by the tcgen05 GEMM whatever the engine would choose; resid (y itself, say) is added after the rounding of the product."""
+    _call(backend, "_ZN5prism15launch_gemm_tc5EP14prism_cuda_ctxRKNS_9LutTensorEPKtjPtS6_", _tensor(backend, handle), C.c_void_p(x.data_ptr()),
+          C.c_uint32(x.shape[0]), C.c_void_p(y.data_ptr()), C.c_void_p(resid.data_ptr()) if resid is not None else None)
+
+
 def gemm_add(backend, handle, x, h):
     """h += x W^T, rounded after the product and after the sum."""
     import torch
@@ -90,17 +96,13 @@ def dense_layout(w):
     return w.reshape(rows // 128, 128, k // 8, 8).permute(0, 2, 1, 3).contiguous()
 
 
-def dense_stream(backend, packed, k_pad, segs, x, outs, x2=None, wait=True):
+def dense_stream(backend, packed, k_pad, segs, x, outs, x2=None):
     """The streaming linear of few rows.  segs: dicts of DenseSeg fields; outs: (tensor, store) per segment."""
     l = DenseLinear(packed.data_ptr(), k_pad, packed.shape[0], len(segs), 1)
     for i, s in enumerate(segs):
         l.seg[i] = DenseSeg(s["row0"], s["rows"], s.get("inp", 0), s.get("k", 0), s.get("act", 0), s.get("mul", 1.0), s["bias"].data_ptr() if s.get("bias") is not None else None)
     o = (DenseOut * len(outs))(*[DenseOut(t.data_ptr(), t.stride(0), store) for t, store in outs])
     i = DenseIn(x=x.data_ptr(), pitch=x.stride(0), x2=x2.data_ptr() if x2 is not None else None, pitch2=x2.stride(0) if x2 is not None else 0)
-    if not wait:
-        f = backend.L._ZN5prism19launch_dense_streamEP14prism_cuda_ctxRKNS_11DenseLinearERKNS_7DenseInEPKNS_8DenseOutEj
-        f.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32]
-        return f(backend.ctx, C.addressof(l), C.addressof(i), C.addressof(o), x.shape[0])
     _call(backend, "_ZN5prism19launch_dense_streamEP14prism_cuda_ctxRKNS_11DenseLinearERKNS_7DenseInEPKNS_8DenseOutEj", C.byref(l), C.byref(i), o, C.c_uint32(x.shape[0]))
 
 
