@@ -70,6 +70,9 @@ struct DenseIn {
     uint32_t pitch2 = 0;
 };
 
+// tests/native_util.py describes these field by field
+static_assert(sizeof(DenseSeg) == 32 && sizeof(DenseLinear) == 24 + 32 * DENSE_MAX_SEGS && sizeof(DenseOut) == 16 && sizeof(DenseIn) == 64, "dense structs");
+
 // Which (token, choice) pairs of a mixture-of-experts layer go through which expert; pair p = token * top + choice.
 // Written on the device by launch_moe_route, so a captured step serves any routing.
 struct MoePlan {

@@ -34,13 +34,14 @@ def test_one_segment(backend, rows, k):
     for t in (1, 2, 5, 8):
         x = _bf16(t, k + 64, t)[:, :k]
         want = x.double() @ w[:rows].double().T
-        y = torch.full((t, rows + 3), 7.0, dtype=torch.bfloat16, device="cuda")
+        y, calls = torch.empty(t, rows + 3, dtype=torch.bfloat16, device="cuda"), []
         for _ in range(3):
-            before = y.clone()
+            y.fill_(7.0)
             native_util.dense_stream(backend, packed, k, [dict(row0=0, rows=rows)], x, [(y, 0)])
             _close(y[:, :rows], want, 4e-3)
             assert bool((y[:, rows:] == 7).all())
-        assert torch.equal(before, y)
+            calls.append(y.clone())
+        assert torch.equal(calls[0], calls[1]) and torch.equal(calls[0], calls[2])
         f = torch.ones(t, rows, device="cuda")
         native_util.dense_stream(backend, packed, k, [dict(row0=0, rows=rows, mul=0.5)], x, [(f, 2)])
         _close(f, 1 + 0.5 * want, 1e-5)
@@ -66,6 +67,8 @@ def test_segments(backend):
         outs.append((torch.empty(6, r, dtype=torch.float32, device="cuda"), 1))
     packed = native_util.dense_layout(torch.cat(blocks))
     for _ in range(2):
+        for o, _ in outs:
+            o.fill_(1e6)
         native_util.dense_stream(backend, packed, k_pad, segs, x, outs, x2=x2)
         for (o, _), z in zip(outs, want):
             _close(o, z, 1e-5)
