@@ -247,7 +247,7 @@ def test_paged_kv_cache(oracle):
 
 
 def test_more_than_32_sequences(oracle):
-    """40 concurrent sequences (the reference decodes one): every linear is one tensor-core GEMM over the batch."""
+    """40 concurrent sequences (the reference decodes one): every linear is one launch over the batch."""
     cfg = dict(TINY, hidden_size=128, intermediate_size=256, head_dim=32, vocab_size=1024)
     be = p.CudaBackend(device=0)
     mc = p.model_config(**cfg, max_seq=64, max_batch=40, profile="baseline")
