@@ -489,11 +489,8 @@ static cudaError_t palettize_share(PalettizeJob &j, uint32_t t) {
     return e;
 }
 
-static cudaError_t palettize_pool(prism_cuda_ctx *ctx, bool slots) {
-    if (!ctx->palettize && !(ctx->palettize = new (std::nothrow) PalettizePool())) return cudaErrorMemoryAllocation;
-    PalettizePool &p = *ctx->palettize;
+static cudaError_t palettize_slots(PalettizePool &p) {
     cudaError_t e = cudaSuccess;
-    if (!slots) return e;
     if (!p.pinned) {
         const size_t bytes = 2 * PZ_WORKERS * PZ_SLOT;
         void *m = aligned_alloc(PZ_PAGE, bytes);
@@ -549,12 +546,16 @@ extern "C" int prism_cuda_palettize(prism_cuda_ctx *ctx, const float *weights, u
     if (capture != cudaStreamCaptureStatusNone) return cuda_fail(ctx, cudaErrorStreamCaptureUnsupported, "palettize");
     const size_t w_bytes = (size_t)dim_m * dim_n * sizeof(float);
     const uint32_t most = std::min(PZ_WORKERS, std::max(1u, std::thread::hardware_concurrency()));
-    const uint32_t workers = w_bytes < PZ_LEAST ? 1 : std::min(most, dim_m);
-    PRISM_CUDA_TRY(ctx, palettize_pool(ctx, workers > 1));
+    uint32_t workers = w_bytes < PZ_LEAST ? 1 : std::min(most, dim_m);
+    if (!ctx->palettize && !(ctx->palettize = new (std::nothrow) PalettizePool())) return fail(ctx, PRISM_E_CUDA, "palettize: out of host memory");
     PalettizePool &pool = *ctx->palettize;
+    if (workers > 1 && palettize_slots(pool) != cudaSuccess) {  // no pinned memory to be had: one thread needs none
+        (void)cudaGetLastError();
+        workers = 1;
+    }
     cudaError_t e = palettize_device(pool, 0, w_bytes);
     if (e == cudaSuccess) e = palettize_device(pool, 1, need);
-    if (e == cudaSuccess && workers == 1) {              // not worth the slots
+    if (e == cudaSuccess && workers == 1) {
         e = cudaMemcpyAsync(pool.dev[0], weights, w_bytes, cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess) e = palettize_rows(static_cast<const float *>(pool.dev[0]), dim_m, dim_n, k, max_iter, static_cast<uint8_t *>(pool.dev[1]), ctx->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(payload, pool.dev[1], need, cudaMemcpyDeviceToHost, ctx->stream);
