@@ -13,8 +13,9 @@
 // A cluster of CTAs owns some rows and divides K; each CTA stages its part of X once.  Sums travel as stores into the CTA that
 // owns eight rows, one cluster barrier later that adds them in the order of k: no scratch in global memory, no counters.
 //
-// Bound: the integer pipe (about 400 instructions per 4096 weights of a warp at 4 bits; 16 warps, since one alone issues every
-// sixth cycle), from 24 tokens on mma.sync besides.  Small linears are launch, the way of X into shared memory and the barrier.
+// Bound at 4 bits: the integer pipe (about 400 instructions per 4096 weights of a warp; 16 warps, since one alone issues every
+// sixth cycle; 65 % active at 8 tokens of 18944 x 3584), from 24 tokens on mma.sync besides.  At 2 bits that pipe is 53 % active and the
+// waits for X and at the cluster's end count as much.  Small linears are launch, the way of X into shared memory and the barrier.
 // Measured at 4 bits with cold weights, the tcgen05 GEMM or batched GEMV before / this, 8 | 16 | 32 tokens, us: 3584 x 3584 13.0 /
 // 8.4 | 15.7 / 9.2 | 15.7 / 11.7; 896 x 4864 11.2 / 5.5 | 26.6 / 5.8 | 26.5 / 7.8; gate and up of 18944 x 3584 39.3 / 30.4
 // (2.2 TB/s) | 40.2 / 33.0; 3584 x 18944 26.5 / 22.9 | 26.6 / 25.1.  Where other kernels stay ahead: reg_plan.hpp.

@@ -24,7 +24,8 @@
 // row tiles: 18944 x 3584, 2048 tokens 266 -> 216 us (1 287 TFLOP/s, 0.78 of measured burst), 512 tokens 67 -> 54, 32 tokens
 // 26 -> 19.9; 4608 x 3584, 2048 tokens 72 -> 53, 32 tokens 23.4 -> 15.1; 3584 x 18944, 2048 tokens 320 -> 278, 32 tokens
 // 96.5 -> 25.0.  The times before are without the residual or SwiGLU passes and the re-laid activations that went with them.
-// A kernel of its own for split K (neither form holds the other's registers: 200 bytes of spills -> none and 48), the first table
+// A kernel of its own for split K (neither form holds the other's registers: stores of spills at 4 | 2 bits 370 | 322 bytes
+// -> none for split K, 70 | 26 for whole K), the first table
 // beside the TMEM allocation, the sums of four ranges requested together, and tiles by the fitted estimate of gm_plan: 3584 x 3584
 // 15.7 -> 11.5 at 32 tokens, 3584 x 18944 26.5 -> 20.5 at 32, 81 -> 58 at 400, 269 -> 220 at 2048, gate and up of 18944 x 3584 40.1 -> 35.1.
 // Every mbarrier wait is bounded; a wait that gives up raises the context's device error word.

@@ -14,7 +14,7 @@
 //
 // A decode step takes one token of every row of the batch (each with its own slot and position, read from
 // device arrays, so the captured graph serves any set of sequences); a prompt portion takes consecutive
-// tokens of one slot.  Both run the same layer code.
+// tokens of one slot, or of several one after the other.  Both run the same layer code.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -10,6 +10,7 @@ namespace prism {
 constexpr uint32_t REG_MAX_TOKENS = 32;
 constexpr size_t REG_MAX_SMEM = 227 * 1024 - 1024;
 
+// Asked only while the options that name other kernels are at their defaults.
 // Whether that kernel takes less time than the ones beside it for `tensors` (2: gate and up) of m rows of k weights.  From 8 tokens
 // on the other one is the tcgen05 GEMM and the two estimates are compared (`cycles` of reg_plan, `gemm_cycles` of gm_plan, each
 // within some 12 % of the times; 1e30 where the GEMM does not take the shape).  On 40 cases of 2 and 4 bits and 8 to 32 tokens that
@@ -17,9 +18,11 @@ constexpr size_t REG_MAX_SMEM = 227 * 1024 - 1024;
 // pair-table and stream-K GEMV; measured, cold weights, other / this in us:
 //  * one token: at 4 bits the pair tables are ahead wherever they are used (3584 x 3584 5.8 / 8.4, gate and up of 18944 x 3584
 //    20.3 / 30.0), at 2 bits for single tensors (3584 x 18944 12.1 / 14.0, 19008 x 3584 11.2 / 15.6) and small gates and ups (two of
-//    9472 x 3584 8.7 / 11.8).  For larger ones it depends on how evenly this kernel's CTAs share the rows, so its estimate meets one of the
-//    stream-K GEMV (6.1 us and 0.104 us a million weights, within 7 % on 14 shapes of 117 to 283 million): two of 18944 x 3584 21.5 / 18.3,
-//    13824 x 5120 21.2 / 19.8, 23680 x 3584 24.7 / 24.1, but 19264 x 3584 21.8 / 23.7, 10240 x 8192 24.1 / 26.6, 28672 x 4096 30.6 / 33.4;
+//    9472 x 3584 8.7 / 11.8, 68 million weights).  For larger ones it depends on how evenly this kernel's CTAs share the rows, so its estimate
+//    meets one of the stream-K GEMV (6.1 us and 0.104 us a million weights, within 7 % on 14 shapes of 117 to 283 million; the bounds of 100
+//    and 268 keep to where that was fitted): two of 18944 x 3584 21.5 / 18.3, 13824 x 5120 21.2 / 19.8, 23680 x 3584 24.7 / 24.1, but
+//    19264 x 3584 21.8 / 23.7, 10240 x 8192 24.1 / 26.6, 28672 x 4096 30.6 / 33.4 (a share of nine half-blocks is 18 jobs: a second round of
+//    the 16 warps for two);
 //  * 2 bits, 2 to 7 tokens: ahead (18944 x 3584, two: 34.8 / 18.6 at 2, 84.2 / 19.1 at 6);
 //  * short rows, little work: behind, since its clusters and the staging of X cost 2.6 us at least (2 bits, k < 1024 and fewer than nine
 //    million weights x tokens: 320 x 192 1.9 / 2.9 at 12, 896 x 896 2.8 / 3.1 at 6, 960 x 320 3.1 / 3.8 at 24, but 1600 x 192 5.7 / 4.0 at
